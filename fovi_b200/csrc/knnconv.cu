@@ -117,7 +117,192 @@ __global__ void pack_points_kernel(const TX* __restrict__ x, __nv_bfloat16* __re
   }
 }
 
-// Exact float32 forward.  One CTA: one output point, BT batch rows, all output channels.
+// Exact float32 forward of a layer with at most 4 input channels (fed by the sensor).
+//
+// The contraction is short (K * c_in = 27..147 products) and every output point has its own taps, so what bounds a plain
+// kernel is not arithmetic (8 us of FMAs at 8 images, 3 -> 64 channels, 49 neighbours, 3976 points) but two loads per FMA and
+// 4-byte stores a point apart.  Here one warp owns an output point: a lane holds NO output channels x BT images in registers, the
+// neighbours' inputs are gathered once per point into shared memory (a lane per neighbour, read back as broadcasts), and the
+// filter is held in shared memory tap-major / channel-minor, so that a tap costs NO conflict-free loads for BT * NO FMAs.
+// A CTA's eight points leave through shared memory as runs of eight points (one 32-byte sector) per channel.
+// Persistent CTAs, so that the filter is staged once.  One accumulator per output, neighbours in list order, channels inside: the
+// sums are those of the general kernel below, bit for bit.
+constexpr int F32_POINTS = 8;     // output points (warps) per CTA
+constexpr int F32_NB = 32;        // neighbours staged per pass: one per lane
+
+template <typename TX, int BT, int NO, int CT, bool WS>
+__global__ void __launch_bounds__(F32_POINTS * 32) knnconv_f32_few_kernel(const TX* __restrict__ X, const float* __restrict__ Wt,
+                                                                          const float* __restrict__ bias, float* __restrict__ Y,
+                                                                          const int* __restrict__ nbr_idx, const uint16_t* __restrict__ nbr_tap,
+                                                                          const int* __restrict__ nbr_cnt, int kp, int B, int n_in, int n_out,
+                                                                          int c_in, int c_out, int cp, int V, int relu, int x_bnc, int y_bnc,
+                                                                          int n_ot, int n_bt, int total) {
+  extern __shared__ __align__(16) float f32_smem[];
+  constexpr int OT = NO * 32;
+  const int C = CT ? CT : c_in;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* xs = f32_smem + warp * (F32_NB * 4 * BT);                        // [neighbour][channel][BT images]
+  float* ys = f32_smem + F32_POINTS * F32_NB * 4 * BT;                    // [BT][OT][F32_POINTS], rows of F32_POINTS + 1
+  float* ws = ys + BT * OT * (F32_POINTS + 1);                            // [V][C][OT] (WS)
+  int staged = -1;
+  for (int item = blockIdx.x; item < total; item += gridDim.x) {
+    const int ot = item % n_ot, t = item / n_ot;                          // grid is a multiple of n_ot: a CTA keeps its channel tile
+    const int bt = t % n_bt, n0 = (t / n_bt) * F32_POINTS;
+    const int o0 = ot * OT, b0 = bt * BT, nb = min(BT, B - b0), n = n0 + warp;
+    if (WS && staged != ot) {
+      __syncthreads();
+      for (int i = threadIdx.x; i < V * C * OT; i += blockDim.x) {
+        const int o = i % OT, c = (i / OT) % C, v = i / (OT * C);
+        ws[i] = o0 + o < c_out ? __ldg(Wt + ((long long)v * c_out + o0 + o) * cp + c) : 0.f;
+      }
+      staged = ot;
+      __syncthreads();
+    }
+    float acc[NO][BT];
+#pragma unroll
+    for (int i = 0; i < NO; ++i)
+#pragma unroll
+      for (int b = 0; b < BT; ++b) acc[i][b] = 0.f;
+    const int cnt = n < n_out ? __ldg(nbr_cnt + n) : 0;
+    for (int k0 = 0; k0 < cnt; k0 += F32_NB) {
+      const int m = min(F32_NB, cnt - k0);
+      int tap = 0;
+      __syncwarp();      // the previous pass has been read
+      if (lane < m) {
+        const int j = __ldg(nbr_idx + (long long)n * kp + k0 + lane);
+        tap = __ldg(nbr_tap + (long long)n * kp + k0 + lane);
+        for (int c = 0; c < C; ++c) {
+          float v[BT];
+#pragma unroll
+          for (int b = 0; b < BT; ++b) {
+            const long long bb = b0 + b;
+            v[b] = b < nb ? ld_as_float(x_bnc ? X + (bb * n_in + j) * c_in + c : X + (bb * c_in + c) * n_in + j) : 0.f;
+          }
+          float* d = xs + (lane * C + c) * BT;
+          if constexpr (BT % 4 == 0) {
+#pragma unroll
+            for (int b = 0; b < BT; b += 4) *reinterpret_cast<float4*>(d + b) = make_float4(v[b], v[b + 1], v[b + 2], v[b + 3]);
+          } else {
+            *reinterpret_cast<float2*>(d) = make_float2(v[0], v[1]);
+          }
+        }
+      }
+      __syncwarp();
+#pragma unroll 2
+      for (int k = 0; k < m; ++k) {
+        const int tp = __shfl_sync(0xffffffffu, tap, k);
+#pragma unroll
+        for (int c = 0; c < (CT ? CT : 4); ++c) {
+          if (CT == 0 && c >= C) break;
+          float w[NO], x[BT];
+#pragma unroll
+          for (int i = 0; i < NO; ++i) {
+            const int o = lane + 32 * i;
+            if (WS) w[i] = ws[(tp * C + c) * OT + o];
+            else w[i] = o0 + o < c_out ? __ldg(Wt + ((long long)tp * c_out + o0 + o) * cp + c) : 0.f;
+          }
+          const float* xr = xs + (k * C + c) * BT;
+          if constexpr (BT % 4 == 0) {
+#pragma unroll
+            for (int b = 0; b < BT; b += 4) {
+              const float4 q = *reinterpret_cast<const float4*>(xr + b);
+              x[b] = q.x; x[b + 1] = q.y; x[b + 2] = q.z; x[b + 3] = q.w;
+            }
+          } else {
+            const float2 q = *reinterpret_cast<const float2*>(xr);
+            x[0] = q.x; x[1] = q.y;
+          }
+#pragma unroll
+          for (int i = 0; i < NO; ++i)
+#pragma unroll
+            for (int b = 0; b < BT; ++b) acc[i][b] = fmaf(x[b], w[i], acc[i][b]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NO; ++i) {
+      const int o = o0 + lane + 32 * i;
+      const float bo = bias && o < c_out ? __ldg(bias + o) : 0.f;
+#pragma unroll
+      for (int b = 0; b < BT; ++b) {
+        if (bias) acc[i][b] += bo;
+        if (relu) acc[i][b] = fmaxf(acc[i][b], 0.f);
+      }
+    }
+    if (y_bnc) {
+      if (n < n_out) {
+#pragma unroll
+        for (int i = 0; i < NO; ++i) {
+          const int o = o0 + lane + 32 * i;
+#pragma unroll
+          for (int b = 0; b < BT; ++b)
+            if (o < c_out && b < nb) Y[((long long)(b0 + b) * n_out + n) * c_out + o] = acc[i][b];
+        }
+      }
+      continue;
+    }
+    __syncthreads();     // the previous item's tile has left
+#pragma unroll
+    for (int i = 0; i < NO; ++i)
+#pragma unroll
+      for (int b = 0; b < BT; ++b) ys[(b * OT + lane + 32 * i) * (F32_POINTS + 1) + warp] = acc[i][b];
+    __syncthreads();
+    for (int i = threadIdx.x; i < nb * OT * F32_POINTS; i += blockDim.x) {
+      const int p = i % F32_POINTS, o = (i / F32_POINTS) % OT, b = i / (F32_POINTS * OT);
+      if (n0 + p < n_out && o0 + o < c_out)
+        Y[((long long)(b0 + b) * c_out + o0 + o) * n_out + n0 + p] = ys[(b * OT + o) * (F32_POINTS + 1) + p];
+    }
+  }
+}
+
+// Launch of the kernel above.  Images per warp: the tiles of at most eight images are made equal and rounded up to 2, 4 or
+// 8; channels per CTA: 32, 64 or 96, whichever wastes the fewest lanes (the wider one on a tie).  The filter goes to shared memory
+// when a channel tile of it fits next to a second CTA on the SM (up to 64 KB), else it is read through L1.
+template <typename TX, int BT, int NO, int CT, bool WS>
+int launch_f32_few_t(const fovi_knnconv_plan* p, const void* X, int x_bnc, const float* Wt, const float* bias, float* Y, int y_bnc, int B,
+                     int relu, size_t smem, cudaStream_t st) {
+  auto k = knnconv_f32_few_kernel<TX, BT, NO, CT, WS>;
+  const int n_ot = (p->c_out + NO * 32 - 1) / (NO * 32), n_bt = (B + BT - 1) / BT;
+  const long long total = (long long)((p->n_out + F32_POINTS - 1) / F32_POINTS) * n_bt * n_ot;
+  if (total >= (1ll << 31)) return FOVI_ERR_UNSUPPORTED;
+  if (smem > 48 * 1024) FOVI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 0;
+  FOVI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, F32_POINTS * 32, smem));
+  const long long slots = std::max<long long>(n_ot, (long long)std::max(per_sm, 1) * fovi::sm_count() / n_ot * n_ot);
+  const int grid = (int)std::min<long long>(total, slots);       // both are multiples of n_ot
+  k<<<grid, F32_POINTS * 32, smem, st>>>((const TX*)X, Wt, bias, Y, p->nbr_idx, p->nbr_tap, p->nbr_cnt, p->kp, B, p->n_in, p->n_out, p->c_in,
+                                         p->c_out, p->cin_packed, p->V, relu, x_bnc, y_bnc, n_ot, n_bt, (int)total);
+  return fovi::after_launch("knnconv_f32_few_kernel");
+}
+
+template <typename TX>
+int launch_f32_few(const fovi_knnconv_plan* p, const void* X, int x_bnc, const float* Wt, const float* bias, float* Y, int y_bnc, int B, int relu,
+                   cudaStream_t st) {
+  const int tiles = (B + 7) / 8, per = (B + tiles - 1) / tiles, bt = per <= 2 ? 2 : per <= 4 ? 4 : 8;
+  int no = 1, best = 1 << 30;
+  for (int i = 1; i <= 3; ++i) {
+    const int lanes = (p->c_out + 32 * i - 1) / (32 * i) * 32 * i;
+    if (lanes <= best) { best = lanes; no = i; }
+  }
+  const size_t base = sizeof(float) * ((size_t)F32_POINTS * F32_NB * 4 * bt + (size_t)bt * no * 32 * (F32_POINTS + 1));
+  const size_t wbytes = sizeof(float) * (size_t)p->V * p->c_in * no * 32;
+  const bool ws = wbytes <= 64 * 1024;
+  const size_t smem = base + (ws ? wbytes : 0);
+#define GO(BT_, NO_, CT_, WS_) return launch_f32_few_t<TX, BT_, NO_, CT_, WS_>(p, X, x_bnc, Wt, bias, Y, y_bnc, B, relu, smem, st)
+#define GO_WS(BT_, NO_, CT_) do { if (ws) GO(BT_, NO_, CT_, true); else GO(BT_, NO_, CT_, false); } while (0)
+#define GO_CT(BT_, NO_) do { if (p->c_in == 3) GO_WS(BT_, NO_, 3); else GO_WS(BT_, NO_, 0); } while (0)
+#define GO_NO(BT_) do { if (no == 1) GO_CT(BT_, 1); else if (no == 2) GO_CT(BT_, 2); else GO_CT(BT_, 3); } while (0)
+  if (bt == 2) GO_NO(2);
+  else if (bt == 4) GO_NO(4);
+  else GO_NO(8);
+#undef GO_NO
+#undef GO_CT
+#undef GO_WS
+#undef GO
+}
+
+// Exact float32 forward of any layer.  One CTA: one output point, BT batch rows, all output channels.  Serves the layers of more
+// than 4 input channels (parity runs and their gradients); the others take the kernel above.
 template <typename TX, bool X_BNC, bool Y_BNC>
 __global__ void __launch_bounds__(128) knnconv_f32_kernel(const TX* __restrict__ X, const float* __restrict__ Wt,
                                                           const float* __restrict__ bias, float* __restrict__ Y,
@@ -365,6 +550,11 @@ extern "C" int fovi_knnconv_forward_f32(const fovi_knnconv_plan* p, const void* 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int BT = 4;
   if ((B + BT - 1) / BT > 65535) return FOVI_ERR_UNSUPPORTED;
+  if (p->c_in <= 4) {
+    const int xb_ = x_layout == FOVI_ACT_BNC, yb_ = y_layout == FOVI_ACT_BNC;
+    return x_dtype == FOVI_F32 ? launch_f32_few<float>(p, X, xb_, Wt, bias, Y, yb_, B, relu, st)
+                               : launch_f32_few<__nv_bfloat16>(p, X, xb_, Wt, bias, Y, yb_, B, relu, st);
+  }
   dim3 grid(p->n_out, (B + BT - 1) / BT);
 #define RUN(TX, XL, YL)                                                                                                   \
   knnconv_f32_kernel<TX, XL, YL><<<grid, 128, 0, st>>>((const TX*)X, Wt, bias, Y, p->nbr_idx, p->nbr_tap, p->nbr_cnt, p->kp, B, \
