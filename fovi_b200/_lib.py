@@ -25,6 +25,7 @@ SIGNATURES = {
     "fovi_sample_backward": (C.c_int, [_P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P, _P, C.c_int, C.c_int, C.c_int, _P, _P]),
     "fovi_knnconv_plan_create": (C.c_int, [_P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(_P)]),
     "fovi_knnconv_plan_destroy": (None, [_P]),
+    "fovi_knnconv_plan_set_bias_period": (C.c_int, [_P, C.c_int]),
     "fovi_knnconv_cin_packed": (C.c_int, [_P]),
     "fovi_knnconv_nnz": (C.c_int64, [_P]),
     "fovi_knnconv_x_layout": (C.c_int, [_P]),

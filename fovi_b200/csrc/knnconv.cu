@@ -359,7 +359,7 @@ extern "C" int fovi_knnconv_plan_create(const int32_t* knn_idx_pad, const uint16
     nnz += m;
   }
   auto* p = new fovi_knnconv_plan();
-  p->n_in = n_in; p->n_out = n_out; p->K = K; p->V = V; p->c_in = c_in; p->c_out = c_out; p->kp = kp; p->nnz = nnz;
+  p->n_in = n_in; p->n_out = n_out; p->K = K; p->V = V; p->c_in = c_in; p->c_out = c_out; p->kp = kp; p->nnz = nnz; p->bias_period = c_out;
   p->cin_packed = (c_in % 64 == 0) ? c_in : (c_in + 7) / 8 * 8;
   p->ct = (c_out % 16 == 0) ? fovi::pick_cout_tile(c_out) : 0;
   // Pair mode for tiny channel counts: group each point's neighbours into aligned input pairs
@@ -460,6 +460,13 @@ extern "C" void fovi_knnconv_plan_destroy(fovi_knnconv_plan* p) {
   if (p->zero_block) cudaFree(p->zero_block);
   if (p->pair_run) cudaFree(p->pair_run);
   delete p;
+}
+
+extern "C" int fovi_knnconv_plan_set_bias_period(fovi_knnconv_plan* p, int period) {
+  if (!p || period <= 0 || p->c_out % period) return FOVI_ERR_INVALID_ARGUMENT;
+  if (p->x_layout != FOVI_X_PAIRS) return FOVI_ERR_UNSUPPORTED;   // only the pair-layout kernel reads the period
+  p->bias_period = period;
+  return FOVI_OK;
 }
 
 extern "C" int fovi_knnconv_cin_packed(const fovi_knnconv_plan* p) { return p ? p->cin_packed : -1; }

@@ -94,7 +94,7 @@ fovi_knnconv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   // no-ops when the kernel was launched without the attribute.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  for (int i = threadIdx.x; i < a.c_out; i += blockDim.x) bias_s[i] = a.bias ? __ldg(a.bias + i) : 0.f;
+  for (int i = threadIdx.x; i < a.c_out; i += blockDim.x) bias_s[i] = a.bias ? __ldg(a.bias + i % a.bias_period) : 0.f;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -464,6 +464,7 @@ static int knnconv_forward_impl(fovi_knnconv_plan* p, const void* X, const void*
   a.relu = relu; a.y_f32 = y_dtype == FOVI_F32;
   a.wait_limit = wait_limit; a.skip_loads = skip_loads;
   a.out_map = om.out_map; a.n_out_y = om.out_map ? om.n_out_y : p->n_out; a.accumulate = om.accumulate;
+  a.bias_period = p->bias_period;
   a.mt_fastest = pairs ? 1 : 0;
   const long long items = (long long)a.n_mt * p->n_out * a.n_ct;
   if (items >= (1ll << 31)) return FOVI_ERR_UNSUPPORTED;

@@ -39,6 +39,7 @@ struct TcArgs {
   const unsigned char* X; const unsigned char* Wt; const unsigned char* zero_block; int n_pairs;  // PAIRS mode
   uint32_t stage_bytes, table_bytes;
   const int* out_map; int n_out_y; int accumulate;   // see OutMode
+  int bias_period;       // channel o reads bias[o % bias_period]
 };
 
 // ---------------------------------------------------------------- PTX wrappers

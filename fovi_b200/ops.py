@@ -24,18 +24,48 @@ def _dt(t):
         raise TypeError(f"unsupported dtype {t}: the kernels take float32 or bfloat16") from None
 
 
+# A launch costs a Python caller more than the smallest kernels run (a 5 us sensor call took 32 us through
+# torch.cuda.current_stream, torch.cuda.device and ctypes wrapper objects), so the launch path asks torch's own bindings for the
+# raw stream and device and hands plain integers to ctypes.
+_raw_stream = torch._C._cuda_getCurrentRawStream
+_current_device = torch._C._cuda_getDevice
+_I64x4 = C.c_int64 * 4
+
+
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """Raw handle of the current device's current stream."""
+    return _raw_stream(_current_device())
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+class _Here:
+    def __enter__(self):
+        pass
+
+    def __exit__(self, *exc):
+        return False
+
+
+_HERE = _Here()
+
+
+def _on(device):
+    """Context in which `device` is the current one; no switch when it already is."""
+    return _HERE if device.index is None or device.index == _current_device() else torch.cuda.device(device)
 
 
 def _need_cuda(*ts):
     for t in ts:
         if t is not None and not t.is_cuda:
             raise ValueError("fovi_b200 kernels need CUDA tensors; there is no CPU path")
+
+
+def _bias_f32(bias):
+    """The bias as the kernels read it: float32 and contiguous."""
+    return bias if bias.dtype == torch.float32 and bias.is_contiguous() else bias.detach().to(torch.float32).contiguous()
 
 
 class SamplerPlan:
@@ -46,7 +76,7 @@ class SamplerPlan:
         self.n_points = g.shape[0]
         self.device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
         h = C.c_void_p()
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(lib.fovi_sampler_plan_create(g.ctypes.data_as(C.c_void_p), self.n_points, C.byref(h)), "fovi_sampler_plan_create")
         self._h = h
 
@@ -57,7 +87,7 @@ class SamplerPlan:
 
     def check(self):
         """Synchronise the current stream and raise if a sampler launch gave up waiting for its image copies."""
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(lib.fovi_sampler_check(self._h, _stream()), "fovi_sampler_check")
 
 
@@ -69,8 +99,10 @@ def sample(plan, img, fix_rc, fix_hw, mode=BILINEAR, pad=PAD_ZEROS, out_dtype=No
     consumes; rows past the last one are left unwritten."""
     _need_cuda(img, fix_rc, fix_hw)
     B, Cc, H, W = img.shape
-    fix_rc = fix_rc.to(torch.float32).contiguous()
-    fix_hw = fix_hw.to(torch.float32).contiguous()
+    if fix_rc.dtype != torch.float32 or not fix_rc.is_contiguous():
+        fix_rc = fix_rc.to(torch.float32).contiguous()
+    if fix_hw.dtype != torch.float32 or not fix_hw.is_contiguous():
+        fix_hw = fix_hw.to(torch.float32).contiguous()
     F = fix_rc.shape[1]
     assert fix_rc.shape == (B, F, 2) and fix_hw.shape == (B, F, 2)
     if out_dtype is None:
@@ -88,8 +120,8 @@ def sample(plan, img, fix_rc, fix_hw, mode=BILINEAR, pad=PAD_ZEROS, out_dtype=No
         out = torch.empty(shape, dtype=out_dtype, device=img.device)
     else:
         assert out.shape == shape and out.dtype == out_dtype and out.is_contiguous()
-    strides = (C.c_int64 * 4)(*img.stride())
-    with torch.cuda.device(img.device):
+    strides = _I64x4(*img.stride())
+    with _on(img.device):
         check(lib.fovi_sample_forward(plan._h, _ptr(img), U8 if img.dtype == torch.uint8 else _dt(img.dtype), B, Cc, H, W, strides, _ptr(fix_rc), _ptr(fix_hw), F,
                                       mode, pad, _ptr(out), _dt(out_dtype), layout, cp, _stream()), "fovi_sample_forward")
     return out
@@ -141,7 +173,7 @@ def sample_backward(plan, grad_out, img_shape, fix_rc, fix_hw, mode=BILINEAR, pa
     if grad_img is None:
         grad_img = torch.zeros((B, Cc, H, W), dtype=torch.float32, device=grad_out.device)
     assert grad_img.dtype == torch.float32 and grad_img.is_contiguous() and tuple(grad_img.shape) == (B, Cc, H, W)
-    with torch.cuda.device(grad_out.device):
+    with _on(grad_out.device):
         check(lib.fovi_sample_backward(plan._h, _ptr(grad_out), _dt(grad_out.dtype), layout, B, Cc, H, W, _ptr(fix_rc.to(torch.float32).contiguous()),
                                        _ptr(fix_hw.to(torch.float32).contiguous()), F, mode, pad, _ptr(grad_img), _stream()), "fovi_sample_backward")
     return grad_img
@@ -160,7 +192,7 @@ class KnnConvPlan:
         self.n_in, self.n_out, self.K, self.V, self.c_in, self.c_out = int(n_in), n_out, K, int(V), int(c_in), int(c_out)
         self.device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
         h = C.c_void_p()
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(lib.fovi_knnconv_plan_create(idx.ctypes.data_as(C.c_void_p), tp.ctypes.data_as(C.c_void_p), self.n_in, n_out, K,
                                                self.V, self.c_in, self.c_out, C.byref(h)), "fovi_knnconv_plan_create")
         self._h = h
@@ -186,12 +218,14 @@ class KnnConvPlan:
             uidx, utap, mtap = tables
             kq, ng = uidx.shape
             hg = C.c_void_p()
-            with torch.cuda.device(self.device):
+            with _on(self.device):
                 check(lib.fovi_knnconv_plan_create(uidx.ctypes.data_as(C.c_void_p), utap.ctypes.data_as(C.c_void_p), self.n_in, ng, kq, kq,
                                                    self.c_in, G * self.c_out, C.byref(hg)), "fovi_knnconv_plan_create")
             if not lib.fovi_knnconv_tc_supported(hg):
                 lib.fovi_knnconv_plan_destroy(hg)
                 continue
+            # the members' channels side by side take the layer's bias once per member
+            check(lib.fovi_knnconv_plan_set_bias_period(hg, self.c_out), "fovi_knnconv_plan_set_bias_period")
             self.group, self._hg, self._kq = G, hg, kq
             self._member_tap = torch.from_numpy(mtap.view(np.int16)).to(self.device)
             return
@@ -200,15 +234,6 @@ class KnnConvPlan:
     def _h_tc(self):
         """Handle the tensor-core entry points take: the grouped plan when there is one."""
         return self._hg if self._hg else self._h
-
-    def _tc_bias(self, bias):
-        """Bias as the tensor-core entry point wants it: a grouped plan's "channels" are the members' channels side by
-        side, so the layer's bias is repeated once per member.  Recomputed on every call (a few hundred bytes): any
-        cache keyed on the tensor's address or version would go stale when a caller passes a freshly folded temporary
-        that happens to reuse a freed address."""
-        if bias is None or self.group == 1:
-            return bias
-        return bias.detach().float().repeat(self.group)
 
     def __del__(self):
         for name in ("_h", "_hg"):
@@ -231,7 +256,7 @@ class KnnConvPlan:
             nbytes = lib.fovi_knnconv_packed_weight_bytes(self._hg, _dt(dtype))
             ng, cg = self.n_out // self.group, self.group * self.c_out
             dst = torch.empty((ng, nbytes // (ng * cg * 16), cg, 8), dtype=dtype, device=weight.device)
-            with torch.cuda.device(weight.device):
+            with _on(weight.device):
                 check(lib.fovi_knnconv_pack_weights_grouped(self._hg, _ptr(weight), _dt(weight.dtype), _ptr(self._member_tap), self.group, self.V,
                                                             _ptr(dst), _stream()), "fovi_knnconv_pack_weights_grouped")
             return dst
@@ -241,7 +266,7 @@ class KnnConvPlan:
         else:
             dst = torch.empty((self.V, self.c_out, self.cin_packed), dtype=dtype, device=weight.device)
         assert dst.numel() * dst.element_size() == nbytes
-        with torch.cuda.device(weight.device):
+        with _on(weight.device):
             check(lib.fovi_knnconv_pack_weights(self._h, _ptr(weight), _dt(weight.dtype), _ptr(dst), _dt(dtype), _stream()), "fovi_knnconv_pack_weights")
         return dst
 
@@ -259,10 +284,10 @@ class KnnConvPlan:
             assert x_bnc.shape[1:] == (self.n_in, self.cin_packed), x_bnc.shape
             assert wt.shape == (self.V, self.c_out, self.cin_packed)
         if bias is not None:
-            bias = self._tc_bias(bias).detach().to(torch.float32).contiguous()
+            bias = _bias_f32(bias)
         if out is None:
             out = torch.empty((B, self.n_out, self.c_out), dtype=out_dtype, device=x_bnc.device)
-        with torch.cuda.device(x_bnc.device):   # a grouped plan writes [B, n_out/G, G*c_out]: the same memory
+        with _on(x_bnc.device):   # a grouped plan writes [B, n_out/G, G*c_out]: the same memory
             check(lib.fovi_knnconv_forward(self._h_tc, _ptr(x_bnc), _ptr(wt), _ptr(bias) if bias is not None else None, _ptr(out),
                                            _dt(out.dtype), B, int(relu), _stream()), "fovi_knnconv_forward")
         return out
@@ -276,7 +301,7 @@ class KnnConvPlan:
         assert x_bnc.shape[1:] == (self.n_in, self.cin_packed) and wt.shape == (self.V, self.c_out, self.cin_packed)
         assert out_map.dtype == torch.int32 and out_map.is_contiguous() and out_map.numel() == self.n_out
         assert out.dtype == torch.float32 and out.is_contiguous() and out.dim() == 3 and out.shape[0] == B and out.shape[2] == self.c_out
-        with torch.cuda.device(x_bnc.device):
+        with _on(x_bnc.device):
             check(lib.fovi_knnconv_forward_scatter_add(self._h_tc, _ptr(x_bnc), _ptr(wt), _ptr(out), B, _ptr(out_map), int(out.shape[1]),
                                                        _stream()), "fovi_knnconv_forward_scatter_add")
         return out
@@ -289,10 +314,10 @@ class KnnConvPlan:
         assert x.shape[1:] == ((self.c_in, self.n_in) if x_layout == ACT_BCN else (self.n_in, self.c_in)), x.shape
         assert wt_f32.dtype == torch.float32 and wt_f32.shape == (self.V, self.c_out, self.cin_packed)
         if bias is not None:
-            bias = bias.detach().to(torch.float32).contiguous()
+            bias = _bias_f32(bias)
         shape = (B, self.c_out, self.n_out) if y_layout == ACT_BCN else (B, self.n_out, self.c_out)
         out = torch.empty(shape, dtype=torch.float32, device=x.device)
-        with torch.cuda.device(x.device):
+        with _on(x.device):
             check(lib.fovi_knnconv_forward_f32(self._h, _ptr(x), _dt(x.dtype), x_layout, _ptr(wt_f32), _ptr(bias) if bias is not None else None,
                                                _ptr(out), y_layout, B, int(relu), _stream()), "fovi_knnconv_forward_f32")
         return out
@@ -303,7 +328,7 @@ class KnnConvPlan:
         _need_cuda(x_bnc, wt)
         B = (x_bnc.shape[0] * 128 if batch is None else int(batch)) if self.x_layout == X_PAIRS else x_bnc.shape[0]
         out = torch.zeros((B, self.n_out, self.c_out), dtype=out_dtype, device=x_bnc.device)
-        with torch.cuda.device(x_bnc.device):
+        with _on(x_bnc.device):
             check(lib.fovi_knnconv_selftest_wait_timeout(self._h_tc, _ptr(x_bnc), _ptr(wt), _ptr(out), _dt(out.dtype), B, _stream()),
                   "fovi_knnconv_selftest_wait_timeout")
 
@@ -316,11 +341,11 @@ class KnnConvPlan:
         assert x.shape[1:] == ((self.c_in, self.n_in) if x_layout == ACT_BCN else (self.n_in, self.c_in)), x.shape
         assert wp.dtype == torch.float32 and wp.shape == (self.V, self.c_out) and wp.is_contiguous()
         if bias is not None:
-            bias = bias.detach().to(torch.float32).contiguous()
+            bias = _bias_f32(bias)
         out_dtype = x.dtype if out_dtype is None else out_dtype
         shape = (B, self.c_out, self.n_out) if y_layout == ACT_BCN else (B, self.n_out, self.c_out)
         out = torch.empty(shape, dtype=out_dtype, device=x.device)
-        with torch.cuda.device(x.device):
+        with _on(x.device):
             check(lib.fovi_knn_depthwise_forward(self._h, _ptr(x), _dt(x.dtype), x_layout, _ptr(wp), _ptr(bias) if bias is not None else None,
                                                  _ptr(out), _dt(out.dtype), y_layout, B, int(relu), _stream()), "fovi_knn_depthwise_forward")
         return out
@@ -332,14 +357,14 @@ class KnnConvPlan:
         B = x.shape[0]
         gx = torch.zeros(x.shape, dtype=torch.float32, device=x.device) if need_gx else None
         gw = torch.zeros((self.V, self.c_out), dtype=torch.float32, device=x.device) if need_gw else None
-        with torch.cuda.device(x.device):
+        with _on(x.device):
             check(lib.fovi_knn_depthwise_backward(self._h, _ptr(x), _dt(x.dtype), x_layout, _ptr(wp), _ptr(gy), _dt(gy.dtype), y_layout, B,
                                                   _ptr(gx) if need_gx else None, _ptr(gw) if need_gw else None, _stream()), "fovi_knn_depthwise_backward")
         return gx, gw
 
     def check(self):
         """Synchronise the current stream and raise if a tensor-core launch gave up on a wait."""
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(lib.fovi_knnconv_check(self._h, _stream()), "fovi_knnconv_check")
             if self._hg:
                 check(lib.fovi_knnconv_check(self._hg, _stream()), "fovi_knnconv_check")
@@ -359,9 +384,9 @@ def sample_knnconv_fused(splan, cplan, img, fix_rc, fix_hw, wt, bias=None, relu=
     if out is None:
         out = torch.empty((B * F, cplan.n_out, cplan.c_out), dtype=out_dtype, device=img.device)
     if bias is not None:
-        bias = cplan._tc_bias(bias).detach().to(torch.float32).contiguous()
-    strides = (C.c_int64 * 4)(*img.stride())
-    with torch.cuda.device(img.device):
+        bias = _bias_f32(bias)
+    strides = _I64x4(*img.stride())
+    with _on(img.device):
         check(lib.fovi_sample_knnconv_fused(splan._h, cplan._h_tc, _ptr(img), U8 if img.dtype == torch.uint8 else _dt(img.dtype), B, Cc, H, W, strides, _ptr(fix_rc.contiguous()),
                                             _ptr(fix_hw.contiguous()), F, mode, pad, _ptr(intermediate), _ptr(wt),
                                             _ptr(bias) if bias is not None else None, _ptr(out), _dt(out.dtype), int(relu),
@@ -383,7 +408,7 @@ class KnnPoolPlan:
         self.n_in = int(n_in)
         self.device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
         h = C.c_void_p()
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(lib.fovi_knnpool_plan_create(idx.ctypes.data_as(C.c_void_p), self.n_in, self.n_out, self.K, C.byref(h)), "fovi_knnpool_plan_create")
         self._h = h
 
@@ -396,7 +421,7 @@ class KnnPoolPlan:
         """Neighbour weights [K, n_out] float32 of the 'gaussian' mode (KNNPoolingLayer.gaussian_weights)."""
         w = np.ascontiguousarray(np.asarray(w_kn, np.float32))
         assert w.shape == (self.K, self.n_out), w.shape
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(lib.fovi_knnpool_set_weights(self._h, w.ctypes.data_as(C.c_void_p)), "fovi_knnpool_set_weights")
 
     def forward(self, x, mode="max", layout=ACT_BCN):
@@ -407,7 +432,7 @@ class KnnPoolPlan:
         Cc = x.shape[1] if layout == ACT_BCN else x.shape[2]
         assert (x.shape[2] if layout == ACT_BCN else x.shape[1]) == self.n_in, x.shape
         y = torch.empty((B, Cc, self.n_out) if layout == ACT_BCN else (B, self.n_out, Cc), dtype=x.dtype, device=x.device)
-        with torch.cuda.device(x.device):
+        with _on(x.device):
             check(lib.fovi_knnpool_forward(self._h, _ptr(x), _dt(x.dtype), layout, B, Cc, POOL_MODES[mode], _ptr(y), _stream()), "fovi_knnpool_forward")
         return y
 
@@ -420,7 +445,7 @@ class KnnPoolPlan:
         Cc = x.shape[1] if layout == ACT_BCN else x.shape[2]
         assert (x.shape[2] if layout == ACT_BCN else x.shape[1]) == self.n_in and gy.shape == ((B, Cc, self.n_out) if layout == ACT_BCN else (B, self.n_out, Cc))
         dx = torch.empty(x.shape, dtype=torch.float32, device=x.device)
-        with torch.cuda.device(x.device):
+        with _on(x.device):
             check(lib.fovi_knnpool_backward(self._h, _ptr(x), _dt(x.dtype), _ptr(gy), _dt(gy.dtype), layout, B, Cc, POOL_MODES[mode], _ptr(dx), _stream()),
                   "fovi_knnpool_backward")
         return dx
@@ -447,7 +472,7 @@ def knn_norm(x, mode, weight=None, bias=None, eps=1e-5, groups=1, layout=ACT_BCN
         prm.append(t)
     stats = torch.empty((max(ng, 1), 2), dtype=torch.float32, device=x.device)
     y = torch.empty_like(x, dtype=x.dtype if out_dtype is None else out_dtype)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib.fovi_knn_norm_forward(_ptr(x), _dt(x.dtype), layout, B, Cc, N, m, int(groups), _ptr(prm[0]) if prm[0] is not None else None,
                                         _ptr(prm[1]) if prm[1] is not None else None, float(eps), int(relu), _ptr(stats), _ptr(y), _dt(y.dtype),
                                         _stream()), "fovi_knn_norm_forward")
@@ -465,7 +490,7 @@ def pack_points(x, cp=8, x_layout=X_BNC):
     shape = ((B + 127) // 128, (N + 1) // 2, 128, 8) if x_layout == X_PAIRS else (B, N, cp)
     # the pad rows of the last 128-row tile are zeroed so that the buffer holds no stray bit patterns
     dst = (torch.zeros if x_layout == X_PAIRS else torch.empty)(shape, dtype=torch.bfloat16, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib.fovi_pack_points(_ptr(x), _dt(x.dtype), B, Cc, N, _ptr(dst), cp, x_layout, _stream()), "fovi_pack_points")
     return dst
 
@@ -483,7 +508,7 @@ def batch_to_inner(src, jp=None, bp=None, out=None):
     if out is None:
         out = torch.empty((I, jp, bp), dtype=torch.bfloat16, device=src.device)
     assert out.shape == (I, jp, bp) and out.dtype == torch.bfloat16 and out.is_contiguous()
-    with torch.cuda.device(src.device):
+    with _on(src.device):
         check(lib.fovi_batch_to_inner(_ptr(src), _dt(src.dtype), B, I, J, sb, si, sj, _ptr(out), jp, bp, _stream()), "fovi_batch_to_inner")
     return out
 
@@ -503,7 +528,7 @@ def relu_backward_to_inner(grad, act, jp=None, bp=None, want_masked=True, want_c
     masked = torch.empty_strided(grad.shape, grad.stride(), dtype=grad.dtype, device=grad.device) if want_masked else None
     out = torch.empty((I, jp, bp), dtype=torch.bfloat16, device=grad.device)
     colsum = torch.empty(F, dtype=torch.float32, device=grad.device) if want_colsum else None
-    with torch.cuda.device(grad.device):
+    with _on(grad.device):
         rc = lib.fovi_relu_backward_to_inner(_ptr(grad), _ptr(act), _dt(grad.dtype), B, I, J, sb, si, sj, _ptr(masked) if masked is not None else None,
                                              _ptr(out), jp, bp, _ptr(colsum) if colsum is not None else None, _stream())
     if rc == 2:   # FOVI_ERR_UNSUPPORTED: shapes the fused kernel does not take
@@ -518,7 +543,7 @@ def column_sum(x):
     x = x.contiguous()
     Cc = x.shape[-1]
     out = torch.empty(Cc, dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib.fovi_column_sum(_ptr(x), _dt(x.dtype), x.numel() // Cc, Cc, _ptr(out), _stream()), "fovi_column_sum")
     return out
 
@@ -530,7 +555,7 @@ def tap_segment_sum(prod, seg_start, seg_slot, dst):
     assert prod.dtype == torch.float32 and prod.is_contiguous() and prod.dim() == 3 and prod.shape[2] == 4
     assert seg_start.dtype == torch.int32 and seg_slot.dtype == torch.int32 and dst.dtype == torch.float32 and dst.is_contiguous()
     V = seg_start.numel() - 1
-    with torch.cuda.device(prod.device):
+    with _on(prod.device):
         check(lib.fovi_tap_segment_sum(_ptr(prod), prod.shape[0], prod.shape[1], _ptr(seg_start), _ptr(seg_slot), V, _ptr(dst), dst.shape[1],
                                        _stream()), "fovi_tap_segment_sum")
     return dst

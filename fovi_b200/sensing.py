@@ -23,25 +23,33 @@ _PADS = {"zeros": ops.PAD_ZEROS, "border": ops.PAD_BORDER}
 _CONST_CACHE = {}
 
 
-def _as_bf2(v, B, device, what):
+def _as_bf2(v, B, device, what, F=1):
     """Fixation argument -> float32 tensor [B,F,2] on `device` plus whether a fixation axis was given.
     A tensor that already is float32 [B,F,2] on the device is passed through untouched; Python numbers and
-    tuples (the usual default arguments) are uploaded once and cached, so steady-state calls issue no
-    host->device copy and no extra kernel."""
+    tuples (the usual default arguments) are uploaded once per (value, B, F) and cached, so steady-state calls issue no
+    host->device copy and no extra kernel (`F`: how many fixations such a constant is repeated for)."""
     if isinstance(v, torch.Tensor):
-        if v.dim() == 3 and v.dtype == torch.float32 and v.device == torch.device(device) and v.is_contiguous() and v.shape[0] == B and v.shape[2] == 2:
-            return v.detach(), True
+        if v.dim() == 3 and v.dtype == torch.float32 and v.device == device and v.is_contiguous() and v.shape[0] == B and v.shape[2] == 2:
+            return (v.detach() if v.requires_grad else v), True
         t = v.detach().to(device=device, dtype=torch.float32)
     else:
+        key = None
+        if type(v) is tuple and len(v) == 2 and type(v[0]) in (int, float) and type(v[1]) in (int, float):
+            key = (v, B, F, device)
+            hit = _CONST_CACHE.get(key)
+            if hit is not None:
+                return hit, False
         arr = np.asarray(v, dtype=np.float32)
         if arr.size <= 2:
-            key = (arr.tobytes(), arr.shape, B, str(device))
-            if key not in _CONST_CACHE:
+            key = (arr.tobytes(), arr.shape, B, F, device) if key is None else key
+            hit = _CONST_CACHE.get(key)
+            if hit is None:
                 if len(_CONST_CACHE) > 64:
                     _CONST_CACHE.clear()
                 pair = np.broadcast_to(arr.reshape(-1), (2,)) if arr.size == 2 else np.full(2, arr.reshape(-1)[0], np.float32)
-                _CONST_CACHE[key] = torch.as_tensor(np.ascontiguousarray(np.broadcast_to(pair, (B, 1, 2))), device=device)
-            return _CONST_CACHE[key], False
+                hit = torch.as_tensor(np.broadcast_to(pair, (B, F, 2)).copy(), device=device)
+                _CONST_CACHE[key] = hit
+            return hit, False
         t = torch.as_tensor(arr, device=device)
     multi = False
     if t.dim() == 0:
@@ -117,7 +125,7 @@ class GridSampler(nn.Module):
         Returns [B,C,N] (or [B,F,C,N]) — samplers.py:91-112."""
         B, _, H, W = img.shape
         fix_rc, multi = _as_bf2((0.5, 0.5) if fix_loc is None else fix_loc, B, img.device, "fix_loc")
-        fix_hw, _ = _as_bf2((H, W) if fixation_size is None else fixation_size, B, img.device, "fixation_size")
+        fix_hw, _ = _as_bf2((H, W) if fixation_size is None else fixation_size, B, img.device, "fixation_size", fix_rc.shape[1])
         if fix_hw.shape[1] != fix_rc.shape[1]:
             fix_hw = fix_hw.expand(B, fix_rc.shape[1], 2).contiguous()
         if torch.is_grad_enabled() and img.requires_grad:
@@ -167,7 +175,6 @@ class RetinalTransform(nn.Module):
         self.sampler = GridSampler(fov, cmf_a, resolution, device=device, mode="nearest" if sampler == "grid_nn" else "bilinear",
                                    style=style, padding_mode=padding_mode)
         self.scatter_sizes = self.sampler.coords.get_scatter_sizes().cpu().numpy()
-        self._hw_cache = {}
 
     def _defaults(self, fix_loc, fixation_size):
         if fix_loc is None:
@@ -211,21 +218,10 @@ class RetinalTransform(nn.Module):
         B = x.shape[0]
         fix_loc, fixation_size = self._defaults(fix_loc, fixation_size)
         fix_rc, _ = _as_bf2(fix_loc, B, x.device, "fix_loc")
-        fix_hw, _ = _as_bf2(fixation_size, B, x.device, "fixation_size")
+        fix_hw, _ = _as_bf2(fixation_size, B, x.device, "fixation_size", fix_rc.shape[1])
         if fix_hw.shape[1] != fix_rc.shape[1]:
-            fix_hw = self._expanded(fix_hw, B, fix_rc.shape[1])
+            fix_hw = fix_hw.expand(B, fix_rc.shape[1], 2).contiguous()
         return fix_rc, fix_hw
-
-    def _expanded(self, fix_hw, B, F):
-        """[B,1,2] -> contiguous [B,F,2]; the result for a cached constant is cached too."""
-        key = (fix_hw.data_ptr(), B, F)
-        hit = self._hw_cache.get(key)
-        if hit is None or hit[0] is not fix_hw:
-            if len(self._hw_cache) > 16:
-                self._hw_cache.clear()
-            hit = (fix_hw, fix_hw.expand(B, F, 2).contiguous())
-            self._hw_cache[key] = hit
-        return hit[1]
 
     def get_warp_params(self):
         return self.fov, self.cmf_a, self.resolution, self.fixation_size

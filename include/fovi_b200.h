@@ -145,6 +145,10 @@ typedef struct fovi_knnconv_plan fovi_knnconv_plan;
 int fovi_knnconv_plan_create(const int32_t* knn_idx_pad, const uint16_t* tap, int n_in, int n_out, int K, int V,
                              int c_in, int c_out, fovi_knnconv_plan** out);
 void fovi_knnconv_plan_destroy(fovi_knnconv_plan* plan);
+/* A plan whose output channels are several members' channels side by side (see fovi_knnconv_pack_weights_grouped) reads its
+   bias modulo `period`: channel o gets bias[o % period].  period divides c_out; a new plan's period is c_out.
+   Pair-layout plans only (others: FOVI_ERR_UNSUPPORTED). */
+int fovi_knnconv_plan_set_bias_period(fovi_knnconv_plan* plan, int period);
 
 /* Channel count of the packed bf16 operands: c_in rounded up to a multiple of 8 (kept when it
  * is a multiple of 64).  With FOVI_X_BNC, activations handed to the tensor-core path are
