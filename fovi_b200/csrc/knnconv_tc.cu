@@ -10,13 +10,13 @@
 // gather is needed, pad neighbours are skipped (the plan compacted them away) and the V/K-fold
 // zero work of a one-hot scatter formulation never exists.
 //
-// CTA = 6 warps, persistent over work items (batch tile, output point, c_out tile):
-//   warp 0      producer: stages the item's (idx, tap) list in shared memory, then one lane
-//               issues the TMA loads into a ring of shared-memory stages;
-//   warp 1      one lane issues tcgen05.mma (M=128, N=c_out tile, K=16) and commits to
+// Persistent CTAs over work items (batch tile, output point, c_out tile):
+//   warps 0-3   epilogue: tcgen05.ld the finished accumulator (double-buffered in tensor
+//               memory so the next item's MMAs overlap), add bias, ReLU, convert, store;
+//   warp 4      issues tcgen05.mma (M=128, N=c_out tile, K=16) and commits to
 //               mbarriers; the warp owns the tensor-memory allocation;
-//   warps 2-5   epilogue: tcgen05.ld the finished accumulator (double-buffered in tensor
-//               memory so the next item's MMAs overlap), add bias, ReLU, convert, store.
+//   warp 5 on   producers (C64: four warps that take turns, one turn per stage; else one warp that stages
+//               the item's list in shared memory): TMA loads into a ring of shared-memory stages.
 //
 // Three operand modes:
 //   C64    channels packed to a multiple of 64: a stage is one 64-channel chunk of one neighbour,
@@ -57,7 +57,7 @@
 namespace {
 
 template <int MODE>
-__global__ void __launch_bounds__(192, MODE == MODE_PAIRS ? 3 : 1)
+__global__ void __launch_bounds__(MODE == MODE_C64 ? TC_THREADS : 192, MODE == MODE_PAIRS ? 3 : 1)
 fovi_knnconv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcArgs a) {
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -71,7 +71,7 @@ fovi_knnconv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   const uint32_t stages0 = base + 1024u + a.table_bytes;  // 1024-aligned
   volatile int* abort_flag = &hdr->abort_flag;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const uint32_t b_stage_off = A_STAGE_BYTES;
   constexpr bool C64 = MODE == MODE_C64;
   // operand boxes per list entry; a last 64-channel box that reaches past cp is zero-filled by the tensor copy
@@ -84,7 +84,7 @@ fovi_knnconv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     hdr->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {  // tensor memory for two accumulators (all 512 columns when the c_out tile is wider than 128)
+  if (warp == 4) {  // tensor memory for two accumulators (all 512 columns when the c_out tile is wider than 128)
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hdr->tmem_base)), "r"(a.tmem_cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -100,7 +100,58 @@ fovi_knnconv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   tc_fence_after();
   const uint32_t tmem = hdr->tmem_base;
 
-  if (warp == 0) {
+  if (warp >= 5 && C64) {
+    // ------------------------------------------------------------ producers: warp w fills every W-th stage (see knnconv_tc2.cu); lane 0
+    // copies the activations, lane 1 the weights
+    constexpr int W = PRODUCER_WARPS;
+    int item = a.skip_loads ? a.total_items : (int)blockIdx.x, k = 0, cc = warp - 5, sel = 0;   // this warp's stage: chunk cc of neighbour k
+    uint32_t s = (uint32_t)(warp - 5), ph = 0;
+    while (s >= (uint32_t)a.nstage) { s -= (uint32_t)a.nstage; ph ^= 1u; }
+    ItemWalk it(blockIdx.x, gridDim.x, a.n_ct, a.n_out), ahead = it;        // d0 c_out tile, d1 output point, d2 batch tile
+    int cnt = item < a.total_items ? __ldg(a.nbr_cnt + it.d1) : 0, cnt_ahead = 0;
+    auto look_ahead = [&]() {
+      ahead.next();
+      if (item + (int)gridDim.x < a.total_items) cnt_ahead = __ldg(a.nbr_cnt + ahead.d1);
+    };
+    look_ahead();
+    auto settle = [&]() {   // moves on to an existing stage and requests its neighbour (lane 0) and tap (lane 1)
+      while (cc >= chunks) { cc -= chunks; ++k; }
+      while (k >= cnt) {
+        k -= cnt;
+        item += gridDim.x;
+        if (item >= a.total_items) return;
+        it = ahead; cnt = cnt_ahead;
+        look_ahead();
+      }
+      const size_t at = (size_t)it.d1 * a.kp + k;
+      if (lane == 0) sel = __ldg(a.nbr_idx + at);
+      if (lane == 1) sel = __ldg(a.nbr_tap + at);
+    };
+    if (item < a.total_items) settle();
+    uint32_t last_s = a.nstage, last_ph = 0;    // this warp's last armed stage
+    while (item < a.total_items) {
+      const uint32_t full = smem_u32(&hdr->full[s]), sa = stages0 + s * a.stage_bytes;
+      bool mine = true;
+      if (lane == 0) {
+        mine = mbar_wait(smem_u32(&hdr->empty[s]), ph ^ 1u, abort_flag, a.status, 1, a.wait_limit);
+        if (mine) mbar_expect_tx(full, a.stage_bytes);
+      }
+      if (!__all_sync(0xffffffffu, mine)) break;
+      if (lane == 0) tma_load_3d(sa, &tmA, full, cc * 64, sel, it.d2 * BM);
+      if (lane == 1) tma_load_3d(sa + b_stage_off, &tmB, full, cc * 64, it.d0 * a.ct, sel);
+      last_s = s; last_ph = ph;
+      cc += W;
+      settle();
+      for (s += W; s >= (uint32_t)a.nstage; s -= (uint32_t)a.nstage) ph ^= 1u;
+    }
+    if (lane == 0 && *abort_flag) {
+      // Drain: wait (bounded, errors ignored) for this warp's last copies, then give the others time to land.
+      if (last_s < (uint32_t)a.nstage)
+        for (uint32_t i = 0; i < (1u << 16); ++i)
+          if (mbar_try_wait(smem_u32(&hdr->full[last_s]), last_ph)) break;
+      for (int i = 0; i < 64; ++i) __nanosleep(1000);
+    }
+  } else if (warp == 5) {
     // ------------------------------------------------------------ producer
     uint32_t s = 0, ph = 0;
     uint32_t issued = 0;
@@ -216,20 +267,6 @@ fovi_knnconv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           ++issued;
           if (++s == (uint32_t)a.nstage) { s = 0; ph ^= 1u; }
         }
-      } else if (lane == 0) {
-        const int steps = cnt * chunks;
-        int k = 0, cc = 0;
-        for (int st = 0; st < steps; ++st) {
-          const uint32_t full = smem_u32(&hdr->full[s]);
-          if (!mbar_wait(smem_u32(&hdr->empty[s]), ph ^ 1u, abort_flag, a.status, 1, a.wait_limit)) { ok = false; break; }
-          mbar_expect_tx(full, a.stage_bytes);
-          const uint32_t sa = stages0 + s * a.stage_bytes;
-          tma_load_3d(sa, &tmA, full, cc * 64, tb_idx[k], m0);
-          tma_load_3d(sa + b_stage_off, &tmB, full, cc * 64, o0, tb_tap[k]);
-          ++issued;
-          if (++cc == chunks) { cc = 0; ++k; }
-          if (++s == (uint32_t)a.nstage) { s = 0; ph ^= 1u; }
-        }
       }
       if (MODE != MODE_PAIRS) {  // lane 0 carried the ring position and the outcome
         s = __shfl_sync(0xffffffffu, s, 0); ph = __shfl_sync(0xffffffffu, ph, 0); issued = __shfl_sync(0xffffffffu, issued, 0);
@@ -258,52 +295,56 @@ fovi_knnconv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           if (mbar_try_wait(smem_u32(&hdr->full[ds]), dph)) break;
       }
     }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.ct >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-      uint32_t s = 0, ph = 0, acc = 0, aph = 0;
-      bool ok = true;
-      int cnt = blockIdx.x < a.total_items ? __ldg(a.nbr_cnt + item_point(a, blockIdx.x)) : 0;
-      for (int item = blockIdx.x; item < a.total_items && ok; item += gridDim.x) {
-        const int next = item + gridDim.x;
-        const int cnt_next = next < a.total_items ? __ldg(a.nbr_cnt + item_point(a, next)) : 0;  // consumed next round
-        const int steps = C64 ? cnt * chunks : (cnt * chunks + 7) / 8;
-        if (!mbar_wait(smem_u32(&hdr->acc_empty[acc]), aph ^ 1u, abort_flag, a.status, 2, a.wait_limit)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t d_tmem = tmem + acc * a.acc_cols;
-        for (int st = 0; st < steps; ++st) {
-          if (!mbar_wait(smem_u32(&hdr->full[s]), ph, abort_flag, a.status, 3, a.wait_limit)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sa = stages0 + s * a.stage_bytes, sb = sa + b_stage_off;
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            uint64_t da, db;
-            if (C64) {
-              da = smem_desc(sa + kk * 32u, 16u, 1024u, 2u);
-              db = smem_desc(sb + kk * 32u, 16u, 1024u, 2u);
-            } else {
-              da = smem_desc(sa + kk * 4096u, 2048u, 128u, 0u);
-              db = smem_desc(sb + kk * 2u * (uint32_t)a.ct * 16u, (uint32_t)a.ct * 16u, 128u, 0u);
-            }
-            tc_mma_bf16(d_tmem, da, db, idesc, (st | kk) ? 1u : 0u);
-          }
-          tc_commit(smem_u32(&hdr->empty[s]));  // frees the stage once these MMAs have read it
-          if (++s == (uint32_t)a.nstage) { s = 0; ph ^= 1u; }
-        }
+  } else if (warp == 4) {
+    // ------------------------------------------------------------ MMA issuer (see elect_one)
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.ct >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    const uint32_t lbo_b = (uint32_t)a.ct * 16u;
+    const uint64_t desc_a = C64 ? smem_desc(0, 16u, 1024u, 2u) : smem_desc(0, 2048u, 128u, 0u);
+    const uint64_t desc_b = C64 ? desc_a : smem_desc(0, lbo_b, 128u, 0u);
+    const uint32_t step_a = C64 ? 2u : 256u, step_b = C64 ? 2u : lbo_b >> 3;     // from one K = 16 slice to the next, in 16-byte units
+    const uint32_t u_stages0 = warp_uniform(stages0), u_tmem = warp_uniform(tmem);
+    uint32_t s = 0, ph = 0, acc = 0, aph = 0;
+    bool ok = true;
+    int cnt = blockIdx.x < a.total_items ? __ldg(a.nbr_cnt + item_point(a, blockIdx.x)) : 0;
+    for (int item = blockIdx.x; item < a.total_items && ok; item += gridDim.x) {
+      const int next = item + gridDim.x;
+      const int cnt_next = next < a.total_items ? __ldg(a.nbr_cnt + item_point(a, next)) : 0;  // consumed next round
+      const int boxes = warp_uniform(cnt) * chunks;
+      const int steps = C64 ? boxes : (boxes + 7) / 8;
+      ok = mbar_wait_warp(smem_u32(&hdr->acc_empty[acc]), aph ^ 1u, abort_flag, a.status, 2, a.wait_limit);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d_tmem = u_tmem + acc * a.acc_cols;
+      for (int st = 0; st < steps; ++st) {
+        ok = mbar_wait_warp(smem_u32(&hdr->full[s]), ph, abort_flag, a.status, 3, a.wait_limit);
         if (!ok) break;
-        tc_commit(smem_u32(&hdr->acc_full[acc]));  // accumulator complete
-        if (++acc == 2) { acc = 0; aph ^= 1u; }
-        cnt = cnt_next;
+        tc_fence_after();
+        const uint32_t sa = u_stages0 + s * a.stage_bytes;
+        const uint64_t da = desc_a + (sa >> 4), db = desc_b + ((sa + b_stage_off) >> 4);
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) tc_mma_bf16(d_tmem, da + kk * step_a, db + kk * step_b, idesc, (st | kk) ? 1u : 0u);
+          tc_commit(smem_u32(&hdr->empty[s]));  // frees the stage once these MMAs have read it
+          if (st == steps - 1) tc_commit(smem_u32(&hdr->acc_full[acc]));  // accumulator complete
+        }
+        __syncwarp();
+        if (++s == (uint32_t)a.nstage) { s = 0; ph ^= 1u; }
       }
-      if (*abort_flag) {  // make sure no MMA is still reading shared memory / writing tensor memory
-        tc_commit(smem_u32(&hdr->drain));
-        for (uint32_t it = 0; it < (1u << 20); ++it)
-          if (mbar_try_wait(smem_u32(&hdr->drain), 0)) break;
+      if (!ok) break;
+      if (steps == 0) {                         // a point without neighbours: nothing to wait for
+        if (elect_one()) tc_commit(smem_u32(&hdr->acc_full[acc]));
+        __syncwarp();
       }
+      if (++acc == 2) { acc = 0; aph ^= 1u; }
+      cnt = cnt_next;
+    }
+    if (*abort_flag && elect_one()) {  // make sure no MMA is still reading shared memory / writing tensor memory
+      tc_commit(smem_u32(&hdr->drain));
+      for (uint32_t it = 0; it < (1u << 20); ++it)
+        if (mbar_try_wait(smem_u32(&hdr->drain), 0)) break;
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------ epilogue (warps 0..3)
     const int q = warp & 3;  // tensor-memory lane quarter this warp may read
     uint32_t acc = 0, aph = 0;
     bool ok = true;
@@ -390,7 +431,7 @@ fovi_knnconv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 4) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
   }
@@ -434,6 +475,20 @@ int fovi::encode_3d(CUtensorMap* m, const void* ptr, uint64_t d0, uint64_t d1, u
   return FOVI_OK;
 }
 
+int fovi::encode_4d(CUtensorMap* m, const void* ptr, const uint64_t (&dims)[4], const uint64_t (&strides)[3], const uint32_t (&box)[4]) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) { fovi::g_last_cuda_error = "cuTensorMapEncodeTiled entry point not available"; return FOVI_ERR_CUDA; }
+  const cuuint64_t d[4] = {dims[0], dims[1], dims[2], dims[3]}, st[3] = {strides[0], strides[1], strides[2]};
+  const cuuint32_t b[4] = {box[0], box[1], box[2], box[3]}, estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), d, st, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    fovi::g_last_cuda_error = "cuTensorMapEncodeTiled failed with CUresult " + std::to_string((int)r);
+    return FOVI_ERR_CUDA;
+  }
+  return FOVI_OK;
+}
+
 static int knnconv_forward_impl(fovi_knnconv_plan* p, const void* X, const void* Wt, const float* bias, void* Y, int y_dtype, int B,
                                 int relu, void* stream, int skip_loads, uint32_t wait_limit, const OutMode& om = OutMode()) {
   if (!p || B < 0 || !fovi::valid_dtype(y_dtype)) return FOVI_ERR_INVALID_ARGUMENT;
@@ -455,8 +510,8 @@ static int knnconv_forward_impl(fovi_knnconv_plan* p, const void* X, const void*
     if (rc2 != FOVI_ERR_UNSUPPORTED) return rc2;
   }
 
-  TcArgs a;
   const bool pairs = p->x_layout == FOVI_X_PAIRS;
+  TcArgs a;
   a.nbr_idx = pairs ? p->pair_idx : p->nbr_idx; a.nbr_tap = pairs ? p->pair_run : p->nbr_tap; a.nbr_cnt = pairs ? p->pair_cnt : p->nbr_cnt;
   a.bias = bias; a.Y = Y; a.status = p->status;
   a.kp = pairs ? p->sp : p->kp; a.B = B; a.n_in = p->n_in; a.n_out = p->n_out; a.c_out = p->c_out; a.cp = cp;
@@ -509,7 +564,7 @@ static int knnconv_forward_impl(fovi_knnconv_plan* p, const void* X, const void*
     FOVI_CUDA(fovi::launch_pdl(fovi_knnconv_tc_kernel<MODE_PAIRS>, grid, 192, smem, st, tmA, tmB, a));
   } else if (c64) {
     FOVI_CUDA(cudaFuncSetAttribute(fovi_knnconv_tc_kernel<MODE_C64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    FOVI_CUDA(fovi::launch_pdl(fovi_knnconv_tc_kernel<MODE_C64>, grid, 192, smem, st, tmA, tmB, a));
+    FOVI_CUDA(fovi::launch_pdl(fovi_knnconv_tc_kernel<MODE_C64>, grid, TC_THREADS, smem, st, tmA, tmB, a));
   } else {
     FOVI_CUDA(cudaFuncSetAttribute(fovi_knnconv_tc_kernel<MODE_C8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     FOVI_CUDA(fovi::launch_pdl(fovi_knnconv_tc_kernel<MODE_C8>, grid, 192, smem, st, tmA, tmB, a));

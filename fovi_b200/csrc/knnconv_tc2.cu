@@ -3,13 +3,17 @@
 // Same table-driven gather-GEMM as knnconv_tc.cu, but one work item is 256 batch rows x one c_out tile,
 // computed by a cluster of two CTAs on neighbouring SMs with a single M=256 MMA: each CTA stages its own
 // 128 batch rows of the activations (A) and only HALF of the weight slab (B: c_out tile / 2 rows), and the
-// tensor cores of both SMs read both halves.  The single-CTA kernel is bound by the L2 -> shared-memory
-// stream (16 KB of A + 24-32 KB of B per 64-channel chunk, at the 64 B/clk/SM limit); halving B per SM
-// cuts that stream by 30-33 % for the same MMA work.
+// tensor cores of both SMs read both halves.  Halving B per SM cuts the L2 -> shared-memory
+// stream (16 KB of A + 24-32 KB of B per 64-channel chunk in the single-CTA kernel) by 30-33 % for the same MMA work.
 //
-// Roles per CTA (6 warps as before): warp 0 producer (both CTAs; loads land in the CTA's own shared memory
-// but complete on the LEADER's "full" barrier), warp 1 MMA issuer (leader CTA only; both CTAs allocate and
-// free tensor memory), warps 2-5 epilogue (both CTAs, each for its own 128 rows).
+// Roles per CTA: warps 0-3 epilogue (both CTAs, each for its own 128 rows), warp 4 MMA issuer (leader CTA only; both
+// CTAs allocate and free tensor memory), four producer warps (both CTAs; loads land in the CTA's own shared memory
+// but complete on the LEADER's "full" barrier), each filling every fourth stage.  One producer thread takes 518 clocks to wait for a
+// free slot and issue a stage's two copies (a stage's MMAs: 384 at N = 192) and 2500 to change to the next item's list, and the copies land
+// 430 clocks later: the ring never held more than a stage.  Four warps with their entries requested a turn ahead keep it full.
+// 1024 rows, 225 points, one producer -> four: layer 64->192 (25 neighbours) 120 -> 106 us, 192->384 240 -> 211, 384->256 273 -> 266,
+// 256->256 188 -> 181 (with the MMA loop of a single thread before it: 126, 252, 282, 194).  A stage now takes 520 clocks at N = 256,
+// where the MMAs need 512, at the 1.41 GHz that the power limit leaves; what is left is the last round of items (12.2 per pair: 13).
 // Barriers: full[s] and acc_empty[a] are used in the leader's shared memory only (the peer's copies and
 // epilogue threads signal them through cluster addresses); empty[s] and acc_full[a] exist in both CTAs and
 // are signalled by the leader's tcgen05.commit, multicast to both.  No TMA load here is multicast.
@@ -23,7 +27,7 @@ struct Tc2Args {
   const float* bias; void* Y; int* status;
   int kp, B, n_in, n_out, c_out, cp;
   int ct, n_ct, n_mt2, nstage, relu, y_f32, total_items;
-  uint32_t stage_bytes, table_bytes;
+  uint32_t stage_bytes, bias_bytes;
   uint32_t wait_limit; int skip_loads;   // as in TcArgs
   const int* out_map; int n_out_y; int accumulate;   // see OutMode
 };
@@ -70,20 +74,18 @@ __device__ __forceinline__ void decode_item2(const Tc2Args& a, int item, int& n,
   mt2 = t / a.n_out;
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Tc2Args a) {
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* basep = smem_raw + (base - raw);
   SmemHeader* hdr = reinterpret_cast<SmemHeader*>(basep);
-  const uint32_t tbl_pitch = ((uint32_t)a.kp * 6u + 15u) & ~15u;
-  unsigned char* tbl0 = basep + 1024;
-  float* bias_s = reinterpret_cast<float*>(basep + 1024 + 2 * tbl_pitch);
-  const uint32_t stages0 = base + 1024u + a.table_bytes;
+  float* bias_s = reinterpret_cast<float*>(basep + 1024);
+  const uint32_t stages0 = base + 1024u + a.bias_bytes;
   volatile int* abort_flag = &hdr->abort_flag;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();      // 0 = leader (issues the MMAs), 1 = peer
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int chunks = (a.cp + 63) / 64;   // a last box reaching past cp is zero-filled by the tensor copy
@@ -96,7 +98,7 @@ fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
     hdr->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {  // both CTAs of the pair allocate together: 512 columns = two accumulators of up to 256
+  if (warp == 4) {  // both CTAs of the pair allocate together: 512 columns = two accumulators of up to 256
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&hdr->tmem_base)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
@@ -112,108 +114,94 @@ fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
   tc_fence_after();
   const uint32_t tmem = hdr->tmem_base;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------ producer (both CTAs)
-    uint32_t s = 0, ph = 0;
-    bool ok = true;
-    int item = a.skip_loads ? a.total_items : pair, buf = 0, cnt = 0;
-    if (item < a.total_items) {
-      int n, mt2, ctile;
-      decode_item2(a, item, n, mt2, ctile);
-      int* ti = reinterpret_cast<int*>(tbl0);
-      uint16_t* tt = reinterpret_cast<uint16_t*>(tbl0 + (size_t)a.kp * 4);
-      for (int k = lane; k < a.kp; k += 32) {
-        ti[k] = __ldg(a.nbr_idx + (size_t)n * a.kp + k);
-        tt[k] = __ldg(a.nbr_tap + (size_t)n * a.kp + k);
+  if (warp >= 5) {
+    // ------------------------------------------------------------ producers (both CTAs): warp w fills every W-th stage; lane 0
+    // copies the activations, lane 1 the weights
+    constexpr int W = PRODUCER_WARPS;
+    int item = a.skip_loads ? a.total_items : pair, k = 0, cc = warp - 5, sel = 0;   // this warp's stage: chunk cc of neighbour k
+    uint32_t s = (uint32_t)(warp - 5), ph = 0;
+    while (s >= (uint32_t)a.nstage) { s -= (uint32_t)a.nstage; ph ^= 1u; }
+    ItemWalk it(pair, n_pairs, a.n_ct, a.n_out), ahead = it;                        // d0 c_out tile, d1 output point, d2 row tile
+    int cnt = item < a.total_items ? __ldg(a.nbr_cnt + it.d1) : 0, cnt_ahead = 0;
+    auto look_ahead = [&]() {
+      ahead.next();
+      if (item + n_pairs < a.total_items) cnt_ahead = __ldg(a.nbr_cnt + ahead.d1);
+    };
+    look_ahead();
+    auto settle = [&]() {   // moves on to an existing stage and requests its neighbour (lane 0) and tap (lane 1)
+      while (cc >= chunks) { cc -= chunks; ++k; }
+      while (k >= cnt) {
+        k -= cnt;
+        item += n_pairs;
+        if (item >= a.total_items) return;
+        it = ahead; cnt = cnt_ahead;
+        look_ahead();
       }
-      cnt = __ldg(a.nbr_cnt + n);
-    }
-    __syncwarp();
-    while (item < a.total_items && ok) {
-      const int next = item + n_pairs;
-      int n, mt2, ctile;
-      decode_item2(a, item, n, mt2, ctile);
-      int r_idx[TBQ], cnt_next = 0;
-      uint16_t r_tap[TBQ];
-      if (next < a.total_items) {
-        int n2, m2, c2;
-        decode_item2(a, next, n2, m2, c2);
-#pragma unroll
-        for (int q = 0; q < TBQ; ++q) {
-          const int k = lane + 32 * q;
-          r_idx[q] = k < a.kp ? __ldg(a.nbr_idx + (size_t)n2 * a.kp + k) : 0;
-          r_tap[q] = k < a.kp ? __ldg(a.nbr_tap + (size_t)n2 * a.kp + k) : (uint16_t)0;
-        }
-        cnt_next = __ldg(a.nbr_cnt + n2);
-      }
-      const int* tb_idx = reinterpret_cast<const int*>(tbl0 + buf * tbl_pitch);
-      const uint16_t* tb_tap = reinterpret_cast<const uint16_t*>(tbl0 + buf * tbl_pitch + (size_t)a.kp * 4);
+      const size_t at = (size_t)it.d1 * a.kp + k;
+      if (lane == 0) sel = __ldg(a.nbr_idx + at);
+      if (lane == 1) sel = __ldg(a.nbr_tap + at);
+    };
+    if (item < a.total_items) settle();
+    while (item < a.total_items) {
+      const uint32_t full_leader = map_to_cta(smem_u32(&hdr->full[s]), 0);
+      const uint32_t sa = stages0 + s * a.stage_bytes;
+      bool mine = true;
       if (lane == 0) {
-        const int m0 = (mt2 * 2 + (int)rank) * BM;            // this CTA's 128 batch rows
-        const int o0 = ctile * a.ct + (int)rank * half;       // this CTA's half of the c_out tile
-        const int steps = cnt * chunks;
-        int k = 0, cc = 0;
-        for (int st = 0; st < steps; ++st) {
-          if (!mbar_wait(smem_u32(&hdr->empty[s]), ph ^ 1u, abort_flag, a.status, 11, a.wait_limit)) { ok = false; break; }
-          const uint32_t full_leader = map_to_cta(smem_u32(&hdr->full[s]), 0);
-          if (rank == 0) mbar_expect_tx(smem_u32(&hdr->full[s]), 2u * a.stage_bytes);   // both CTAs' bytes
-          const uint32_t sa = stages0 + s * a.stage_bytes;
-          tma_load_3d_pair(sa, &tmA, full_leader, cc * 64, tb_idx[k], m0);
-          tma_load_3d_pair(sa + A_STAGE_BYTES, &tmB, full_leader, cc * 64, o0, tb_tap[k]);
-          if (++cc == chunks) { cc = 0; ++k; }
-          if (++s == (uint32_t)a.nstage) { s = 0; ph ^= 1u; }
-        }
+        mine = mbar_wait(smem_u32(&hdr->empty[s]), ph ^ 1u, abort_flag, a.status, 11, a.wait_limit);
+        if (mine && rank == 0) mbar_expect_tx(smem_u32(&hdr->full[s]), 2u * a.stage_bytes);   // both CTAs' bytes
       }
-      __syncwarp();
-      if (next < a.total_items) {
-        int* ti = reinterpret_cast<int*>(tbl0 + (buf ^ 1) * tbl_pitch);
-        uint16_t* tt = reinterpret_cast<uint16_t*>(tbl0 + (buf ^ 1) * tbl_pitch + (size_t)a.kp * 4);
-#pragma unroll
-        for (int q = 0; q < TBQ; ++q) {
-          const int k = lane + 32 * q;
-          if (k < a.kp) { ti[k] = r_idx[q]; tt[k] = r_tap[q]; }
-        }
-      }
-      __syncwarp();
-      s = __shfl_sync(0xffffffffu, s, 0); ph = __shfl_sync(0xffffffffu, ph, 0);
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      buf ^= 1; cnt = cnt_next; item = next;
+      if (!__all_sync(0xffffffffu, mine)) break;
+      if (lane == 0) tma_load_3d_pair(sa, &tmA, full_leader, cc * 64, sel, (it.d2 * 2 + (int)rank) * BM);            // this CTA's 128 batch rows
+      if (lane == 1) tma_load_3d_pair(sa + A_STAGE_BYTES, &tmB, full_leader, cc * 64, it.d0 * a.ct + (int)rank * half, sel);   // half of the c_out tile
+      cc += W;
+      settle();
+      for (s += W; s >= (uint32_t)a.nstage; s -= (uint32_t)a.nstage) ph ^= 1u;
     }
     if (lane == 0 && *abort_flag) {
       // Give copies that are still in flight time to land before this CTA's shared memory goes away.
       for (int i = 0; i < 64; ++i) __nanosleep(1000);
     }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+  } else if (warp == 4) {
+    // ------------------------------------------------------------ MMA issuer (leader CTA only; see elect_one)
+    if (rank == 0) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.ct >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+      const uint64_t desc0 = smem_desc(0, 16u, 1024u, 2u);
+      const uint32_t u_stages0 = warp_uniform(stages0), u_tmem = warp_uniform(tmem);
       uint32_t s = 0, ph = 0, acc = 0, aph = 0;
       bool ok = true;
       int cnt = pair < a.total_items ? __ldg(a.nbr_cnt + (pair / a.n_ct) % a.n_out) : 0;
       for (int item = pair; item < a.total_items && ok; item += n_pairs) {
         const int next = item + n_pairs;
         const int cnt_next = next < a.total_items ? __ldg(a.nbr_cnt + (next / a.n_ct) % a.n_out) : 0;
-        const int steps = cnt * chunks;
-        if (!mbar_wait(smem_u32(&hdr->acc_empty[acc]), aph ^ 1u, abort_flag, a.status, 12, a.wait_limit)) { ok = false; break; }
+        const int steps = warp_uniform(cnt) * chunks;
+        ok = mbar_wait_warp(smem_u32(&hdr->acc_empty[acc]), aph ^ 1u, abort_flag, a.status, 12, a.wait_limit);
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem + acc * 256u;
+        const uint32_t d_tmem = u_tmem + acc * 256u;
         for (int st = 0; st < steps; ++st) {
-          if (!mbar_wait(smem_u32(&hdr->full[s]), ph, abort_flag, a.status, 13, a.wait_limit)) { ok = false; break; }
+          ok = mbar_wait_warp(smem_u32(&hdr->full[s]), ph, abort_flag, a.status, 13, a.wait_limit);
+          if (!ok) break;
           tc_fence_after();
-          const uint32_t sa = stages0 + s * a.stage_bytes, sb = sa + A_STAGE_BYTES;
+          const uint32_t sa = u_stages0 + s * a.stage_bytes;
+          const uint64_t da = desc0 + (sa >> 4), db = desc0 + ((sa + A_STAGE_BYTES) >> 4);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            tc_mma_bf16_pair(d_tmem, smem_desc(sa + kk * 32u, 16u, 1024u, 2u), smem_desc(sb + kk * 32u, 16u, 1024u, 2u), idesc,
-                             (st | kk) ? 1u : 0u);
-          tc_commit_pair(smem_u32(&hdr->empty[s]));      // frees the stage in both CTAs
+            for (int kk = 0; kk < 4; ++kk) tc_mma_bf16_pair(d_tmem, da + kk * 2u, db + kk * 2u, idesc, (st | kk) ? 1u : 0u);
+            tc_commit_pair(smem_u32(&hdr->empty[s]));      // frees the stage in both CTAs
+            if (st == steps - 1) tc_commit_pair(smem_u32(&hdr->acc_full[acc]));   // accumulator halves complete in both CTAs
+          }
+          __syncwarp();
           if (++s == (uint32_t)a.nstage) { s = 0; ph ^= 1u; }
         }
         if (!ok) break;
-        tc_commit_pair(smem_u32(&hdr->acc_full[acc]));   // accumulator halves complete in both CTAs
+        if (steps == 0) {                                  // a point without neighbours: nothing to wait for
+          if (elect_one()) tc_commit_pair(smem_u32(&hdr->acc_full[acc]));
+          __syncwarp();
+        }
         if (++acc == 2) { acc = 0; aph ^= 1u; }
         cnt = cnt_next;
       }
-      if (*abort_flag) {
+      if (*abort_flag && elect_one()) {
         asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&hdr->drain)) : "memory");
         for (uint32_t it = 0; it < (1u << 20); ++it)
           if (mbar_try_wait(smem_u32(&hdr->drain), 0)) break;
@@ -305,7 +293,7 @@ fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
 
   tc_fence_before();
   cluster_sync_all();   // nobody frees tensor memory or leaves while the other CTA may still signal or read
-  if (warp == 1) {
+  if (warp == 4) {
     __syncwarp();
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
@@ -332,11 +320,11 @@ int fovi::launch_knnconv_tc_pair(const fovi_knnconv_plan* p, const void* X, cons
   if (items >= (1ll << 31) || a.kp > 32 * TBQ) return FOVI_ERR_UNSUPPORTED;
   a.total_items = (int)items;
   a.stage_bytes = A_STAGE_BYTES + (uint32_t)(ct / 2) * 128u;
-  a.table_bytes = (2u * (((uint32_t)a.kp * 6u + 15u) & ~15u) + (uint32_t)p->c_out * 4u + 1023u) & ~1023u;
-  const uint32_t budget = 220u * 1024u - 2048u - a.table_bytes;
+  a.bias_bytes = ((uint32_t)p->c_out * 4u + 1023u) & ~1023u;
+  const uint32_t budget = 220u * 1024u - 2048u - a.bias_bytes;
   a.nstage = (int)std::min<uint32_t>(MAX_STAGES, budget / a.stage_bytes);
   if (a.nstage < 2) return FOVI_ERR_UNSUPPORTED;
-  const size_t smem = 1024 + 1024 + a.table_bytes + (size_t)a.nstage * a.stage_bytes;
+  const size_t smem = 1024 + 1024 + a.bias_bytes + (size_t)a.nstage * a.stage_bytes;
 
   CUtensorMap tmA, tmB;
   int rc = fovi::encode_3d(&tmA, X, (uint64_t)cp, (uint64_t)p->n_in, (uint64_t)B, (uint64_t)cp * 2, (uint64_t)p->n_in * cp * 2, 64, 1, BM, true);
@@ -346,6 +334,6 @@ int fovi::launch_knnconv_tc_pair(const fovi_knnconv_plan* p, const void* X, cons
 
   FOVI_CUDA(cudaFuncSetAttribute(fovi_knnconv_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int pairs = (int)std::min<long long>(items, sms / 2);
-  FOVI_CUDA(fovi::launch_pdl(fovi_knnconv_tc_pair_kernel, 2 * pairs, 192, smem, st, tmA, tmB, a));   // cluster size 2 comes from __cluster_dims__
+  FOVI_CUDA(fovi::launch_pdl(fovi_knnconv_tc_pair_kernel, 2 * pairs, TC_THREADS, smem, st, tmA, tmB, a));   // cluster size 2 comes from __cluster_dims__
   return fovi::after_launch("fovi_knnconv_tc_pair_kernel");
 }

@@ -2,6 +2,7 @@
 // tcgen05 PTX wrappers (every wait bounded), shared-memory descriptors.  Everything has internal linkage.
 #pragma once
 #include <cuda.h>
+#include <algorithm>
 #include <stdlib.h>
 #include <string.h>
 #include <utility>
@@ -20,6 +21,11 @@ namespace {
 
 constexpr int BM = 128;            // batch rows per tile (UMMA M)
 constexpr int MAX_STAGES = 8;
+#ifndef FOVI_TC_PRODUCER_WARPS
+#define FOVI_TC_PRODUCER_WARPS 4
+#endif
+constexpr int PRODUCER_WARPS = FOVI_TC_PRODUCER_WARPS;            // CTA-pair kernels: see knnconv_tc2.cu
+constexpr int TC_THREADS = (5 + PRODUCER_WARPS) * 32;            // 4 epilogue warps, the MMA warp, the producers
 constexpr uint32_t A_STAGE_BYTES = 16384;
 constexpr uint32_t WAIT_LIMIT = 1u << 22;  // try_wait attempts before giving up
 
@@ -144,6 +150,22 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes
   return d;
 }
 
+// One lane of a converged warp.  The MMA warps run their loops with all 32 lanes and issue from the elected one: loop counters,
+// descriptors and addresses are then warp-uniform and live in uniform registers, which is where the MMA instruction takes them
+// from.  Issued from a loop of a single thread, every MMA costs 76 (cta_group::1) or 102 (cta_group::2) clocks to issue, whatever its
+// width -- 409 clocks per K = 64 stage where N = 192 needs 384 and N = 128 256, and ~650 with the stage's barriers; from a uniform
+// loop the tensor core's own rate is reached (512 / 384 / 256 clocks at N = 256 / 192 / 128).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+// Bounded wait of a converged warp.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code, uint32_t limit) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code, limit)) != 0;
+}
+
 // Shared-memory header at the 1024-aligned base of the dynamic allocation.
 struct SmemHeader {
   uint64_t full[MAX_STAGES];
@@ -156,6 +178,20 @@ struct SmemHeader {
 };
 
 constexpr int TBQ = 8;  // table entries prefetched per producer lane: list pitch <= 32 * TBQ
+
+// Items first, first + stride, ... written in mixed radix (d0 fastest, radix r0; d1, radix r1; d2) without a division per item.
+struct ItemWalk {
+  int r0, r1, d0, d1, d2, i0, i1, i2;
+  __device__ __forceinline__ ItemWalk(int first, int stride, int r0_, int r1_) : r0(r0_), r1(r1_) {
+    d0 = first % r0; d1 = first / r0 % r1; d2 = first / r0 / r1;
+    i0 = stride % r0; i1 = stride / r0 % r1; i2 = stride / r0 / r1;
+  }
+  __device__ __forceinline__ void next() {
+    d0 += i0; d1 += i1; d2 += i2;
+    if (d0 >= r0) { d0 -= r0; ++d1; }
+    if (d1 >= r1) { d1 -= r1; ++d2; }
+  }
+};
 
 // Work item -> (output point, batch tile, c_out tile).  Consecutive items run at the same time on neighbouring SMs:
 // with the point varying fastest they share activations (neighbouring points read the same inputs), with the batch
@@ -197,7 +233,12 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, siz
 // Tiled 3-D bf16 tensor map (box b0 x b1 x b2 of a tensor d0 x d1 x d2 with byte strides for d1, d2).
 int encode_3d(CUtensorMap* m, const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1_bytes,
               uint64_t stride2_bytes, uint32_t b0, uint32_t b1, uint32_t b2, bool swizzle128);
+// Tiled 4-D bf16 tensor map without swizzle (strides: bytes of dimensions 1 to 3).
+int encode_4d(CUtensorMap* m, const void* ptr, const uint64_t (&dims)[4], const uint64_t (&strides)[3], const uint32_t (&box)[4]);
 // CTA-pair variant of the 64-channel mode (knnconv_tc2.cu).  Returns FOVI_ERR_UNSUPPORTED when it does not apply.
 int launch_knnconv_tc_pair(const fovi_knnconv_plan* p, const void* X, const void* Wt, const float* bias, void* Y, int y_dtype,
                            int B, int relu, cudaStream_t st, int skip_loads, uint32_t wait_limit, const OutMode& om);
+// CTA-pair kernel of the pair layout (knnconv_tcp.cu).  Returns FOVI_ERR_UNSUPPORTED when it does not apply.
+int launch_knnconv_tc_pairs2(const fovi_knnconv_plan* p, const void* X, const void* Wt, const float* bias, void* Y, int y_dtype, int B,
+                           int relu, cudaStream_t st, int skip_loads, uint32_t wait_limit);
 }  // namespace fovi
