@@ -366,7 +366,7 @@ extern "C" int fovi_knnconv_plan_create(const int32_t* knn_idx_pad, const uint16
   // (2p, 2p+1).  A neighbour takes the free half of a slot of its pair, or opens a new slot (so a
   // table that lists the same input point twice still adds both taps).
   std::vector<int> pidx, pcnt;
-  std::vector<uint16_t> ptap, prun;
+  std::vector<uint16_t> ptap, prun, pbox;
   if (c_in <= 4) {
     p->x_layout = FOVI_X_PAIRS;
     p->n_pairs = (n_in + 1) / 2;
@@ -405,6 +405,7 @@ extern "C" int fovi_knnconv_plan_create(const int32_t* knn_idx_pad, const uint16
     // Copy plan: inside every 8-slot stage, consecutive pair indices are consecutive 2 KB blocks of the
     // activations, so each run moves with one copy; the unused tail of the last stage is one run of zeros.
     prun.assign((size_t)n_out * p->sp, 0);
+    pbox.assign((size_t)n_out * p->sp, 0);
     for (int n = 0; n < n_out; ++n) {
       const int* row = &pidx[(size_t)n * p->sp];
       for (int s0 = 0; s0 < p->sp; s0 += 8) {
@@ -414,6 +415,12 @@ extern "C" int fovi_knnconv_plan_create(const int32_t* knn_idx_pad, const uint16
           if (row[s0 + j] >= p->n_pairs) len = 8 - j;
           else while (j + len < 8 && row[s0 + j + len] == row[s0 + j] + len && row[s0 + j + len] < p->n_pairs) ++len;
           prun[(size_t)n * p->sp + s0 + j] = (uint16_t)len;
+          for (int at = j, left = len; left > 0;) {
+            int lg = 3;
+            while ((1 << lg) > left) --lg;
+            pbox[(size_t)n * p->sp + s0 + at] = (uint16_t)(lg + 1);
+            at += 1 << lg; left -= 1 << lg;
+          }
           j += len;
         }
       }
@@ -426,6 +433,8 @@ extern "C" int fovi_knnconv_plan_create(const int32_t* knn_idx_pad, const uint16
     if (e == cudaSuccess) e = cudaMalloc(&p->pair_tap, sizeof(uint16_t) * ptap.size());
     if (e == cudaSuccess) e = cudaMalloc(&p->pair_run, sizeof(uint16_t) * prun.size());
     if (e == cudaSuccess) e = cudaMemcpy(p->pair_run, prun.data(), sizeof(uint16_t) * prun.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&p->pair_box, sizeof(uint16_t) * pbox.size());
+    if (e == cudaSuccess) e = cudaMemcpy(p->pair_box, pbox.data(), sizeof(uint16_t) * pbox.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMalloc(&p->zero_block, 16384);
     if (e == cudaSuccess) e = cudaMemset(p->zero_block, 0, 16384);
     if (e == cudaSuccess) e = cudaMemcpy(p->pair_idx, pidx.data(), sizeof(int) * pidx.size(), cudaMemcpyHostToDevice);
@@ -459,6 +468,7 @@ extern "C" void fovi_knnconv_plan_destroy(fovi_knnconv_plan* p) {
   if (p->pair_tap) cudaFree(p->pair_tap);
   if (p->zero_block) cudaFree(p->zero_block);
   if (p->pair_run) cudaFree(p->pair_run);
+  if (p->pair_box) cudaFree(p->pair_box);
   delete p;
 }
 

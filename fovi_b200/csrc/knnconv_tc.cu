@@ -511,6 +511,12 @@ static int knnconv_forward_impl(fovi_knnconv_plan* p, const void* X, const void*
   }
 
   const bool pairs = p->x_layout == FOVI_X_PAIRS;
+  // The pair layout with more than one batch tile: CTA pairs (knnconv_tcp.cu).
+  if (pairs && !FOVI_TC_SINGLE_CTA_ONLY && B > BM && !om.out_map) {
+    const int rc2 = fovi::launch_knnconv_tc_pairs2(p, X, Wt, bias, Y, y_dtype, B, relu, reinterpret_cast<cudaStream_t>(stream), skip_loads, wait_limit);
+    if (rc2 != FOVI_ERR_UNSUPPORTED) return rc2;
+  }
+
   TcArgs a;
   a.nbr_idx = pairs ? p->pair_idx : p->nbr_idx; a.nbr_tap = pairs ? p->pair_run : p->nbr_tap; a.nbr_cnt = pairs ? p->pair_cnt : p->nbr_cnt;
   a.bias = bias; a.Y = Y; a.status = p->status;
