@@ -49,6 +49,12 @@ SIGNATURES = {
     "fovi_sensor_ring_layout": (C.c_longlong, [C.c_double, C.c_double, C.c_int, _P, _P]),
     "fovi_sensor_points": (C.c_int, [C.c_double, C.c_double, C.c_int, C.c_double, C.c_longlong, _P, _P, _P]),
     "fovi_sensor_pad_points": (C.c_longlong, [C.c_double, C.c_double, C.c_int, C.c_double, C.c_double, C.c_longlong, _P, _P]),
+    "fovi_relu_mask_colsum": (C.c_int, [_P, _P, _P, _P, C.c_longlong, C.c_int, _P]),
+    "fovi_knndw_plan_create": (C.c_int, [_P, _P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(_P)]),
+    "fovi_knndw_plan_destroy": (None, [_P]),
+    "fovi_knndw_run": (C.c_int, [_P, _P, C.c_int, _P, C.c_int, C.c_int, _P, _P]),
+    "fovi_knndw_check": (C.c_int, [_P, _P]),
+    "fovi_knnconv_weight_grad_pairs": (C.c_int, [_P, _P, _P, C.c_int, _P, _P]),
     "fovi_column_sum": (C.c_int, [_P, C.c_int, C.c_longlong, C.c_int, _P, _P]),
     "fovi_relu_backward_to_inner": (C.c_int, [_P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_longlong, C.c_longlong, C.c_longlong, _P, _P, C.c_int, C.c_int, _P, _P]),
     "fovi_tap_segment_sum": (C.c_int, [_P, C.c_int, C.c_longlong, _P, _P, C.c_int, _P, C.c_int, _P]),

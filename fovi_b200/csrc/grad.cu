@@ -124,6 +124,40 @@ __global__ void __launch_bounds__(256) batch_to_inner_x2_kernel(const T* __restr
   }
 }
 
+// Start of the backward pass of a layer with a fused ReLU, on channels-last bf16: the gradient is masked where the layer's output is not
+// positive and summed over everything but the channel, in one pass (reads gradient and output, writes the masked gradient: bound by
+// memory).  One thread per 8 channels (16-byte accesses) of every step-th row; sums in registers, one shared-memory round per block.
+__global__ void relu_mask_colsum_kernel(const uint4* __restrict__ grad, const uint4* __restrict__ act, uint4* __restrict__ masked,
+                                        float* __restrict__ colsum, long long R, int c8) {
+  extern __shared__ float rm_part[];               // [rows per block][8 * c8]
+  const int cg = threadIdx.x % c8, r0 = threadIdx.x / c8, rows = blockDim.x / c8;
+  const long long step = (long long)gridDim.x * rows;
+  float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (long long r = (long long)blockIdx.x * rows + r0; r < R; r += step) {
+    const uint4 g = __ldg(grad + r * c8 + cg), y = __ldg(act + r * c8 + cg);
+    const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, yw[4] = {y.x, y.y, y.z, y.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float y0 = __uint_as_float(yw[i] << 16), y1 = __uint_as_float(yw[i] & 0xFFFF0000u);     // bf16 -> float32, exact
+      const uint32_t lo = y0 > 0.f ? gw[i] & 0xFFFFu : 0u, hi = y1 > 0.f ? gw[i] & 0xFFFF0000u : 0u;
+      o[i] = lo | hi;
+      sum[2 * i] += __uint_as_float(lo << 16); sum[2 * i + 1] += __uint_as_float(hi);
+    }
+    masked[r * c8 + cg] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  if (!colsum) return;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) rm_part[(size_t)r0 * 8 * c8 + cg * 8 + i] = sum[i];
+  __syncthreads();
+  for (int c = threadIdx.x; c < 8 * c8; c += blockDim.x) {
+    float t = 0.f;
+    for (int r = 0; r < rows; ++r) t += rm_part[(size_t)r * 8 * c8 + c];
+    atomicAdd(colsum + c, t);
+  }
+}
+
 // Column sums of a row-major [R, C] matrix (C even) into float32 dst[C] (zeroed by the caller's launch order: see the entry
 // point).  A warp reads 64 consecutive columns of a row (128 bytes of bf16); rows are strided over the 8 warps of a block
 // and over grid.y; partial sums meet in shared memory and leave with one atomic per column and block.
@@ -196,6 +230,20 @@ extern "C" int fovi_tap_segment_sum(const float* prod, int R, long long S, const
   tap_segment_sum_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(reinterpret_cast<const float4*>(prod), S, seg_start, seg_slot, R, dst,
                                                                                     dst_pitch);
   return fovi::after_launch("tap_segment_sum_kernel");
+}
+
+extern "C" int fovi_relu_mask_colsum(const void* grad, const void* act, void* masked, float* colsum, long long R, int C, void* stream) {
+  if (R < 0 || C <= 0) return FOVI_ERR_INVALID_ARGUMENT;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (C % 8 || C > 2048) return FOVI_ERR_UNSUPPORTED;
+  if (R > 0 && (!grad || !act || !masked)) return FOVI_ERR_INVALID_ARGUMENT;
+  if ((reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(act) | reinterpret_cast<uintptr_t>(masked)) & 15) return FOVI_ERR_UNSUPPORTED;
+  if (colsum) FOVI_CUDA(cudaMemsetAsync(colsum, 0, sizeof(float) * (size_t)C, st));
+  if (R == 0) return FOVI_OK;
+  const int c8 = C / 8, rows = std::max(1, 256 / c8);
+  const int grid = (int)std::min<long long>((R + rows - 1) / rows, (long long)fovi::sm_count() * 8);
+  relu_mask_colsum_kernel<<<grid, rows * c8, colsum ? sizeof(float) * rows * C : 0, st>>>((const uint4*)grad, (const uint4*)act, (uint4*)masked, colsum, R, c8);
+  return fovi::after_launch("relu_mask_colsum_kernel");
 }
 
 extern "C" int fovi_column_sum(const void* src, int dtype, long long R, int C, float* dst, void* stream) {

@@ -206,10 +206,14 @@ class KNNConvLayer(nn.Module):
         if self.precision == "fp32" or not self._plan.tc_supported:
             y = self._plan.forward_f32(X_l, self.packed_weight(torch.float32), self.bias)
             return y.to(X_l.dtype)
+        return self._forward_packed(X_l)[0]
+
+    def _forward_packed(self, X_l):
+        """(tensor-core forward of X_l, X_l in the kernel's layout)."""
         out_dtype = torch.float32 if X_l.dtype == torch.float32 else torch.bfloat16
         xp = ops.pack_points(X_l, self._plan)
         y = self._plan.forward(xp, self.packed_weight(), self.bias, out_dtype=out_dtype, batch=X_l.shape[0])
-        return y.permute(0, 2, 1).to(X_l.dtype)
+        return y.permute(0, 2, 1).to(X_l.dtype), xp
 
     def load_conv2d_weights(self, conv2d, strict=False):
         """Load a Conv2d kernel: transpose/flip from (row, col) to (x, y), resample to the reference

@@ -306,6 +306,18 @@ class KnnConvPlan:
                                                        _stream()), "fovi_knnconv_forward_scatter_add")
         return out
 
+    def weight_grad_pairs(self, gy_points, x_pairs):
+        """Weight gradient of a pair-layout layer: gy_points [B,n_out,c_out] bf16 contiguous, x_pairs from `pack_points` (its pad rows are
+        zero) -> float32 [V, c_out, 4] (channel sums of every tap).  See fovi_knnconv_weight_grad_pairs."""
+        _need_cuda(gy_points, x_pairs)
+        B = gy_points.shape[0]
+        assert self.x_layout == X_PAIRS and gy_points.dtype == torch.bfloat16 and gy_points.is_contiguous() and gy_points.shape[1:] == (self.n_out, self.c_out)
+        assert x_pairs.dtype == torch.bfloat16 and x_pairs.is_contiguous() and x_pairs.shape == ((B + 127) // 128, self.n_pairs, 128, 8)
+        out = torch.zeros((self.V, self.c_out, 4), dtype=torch.float32, device=gy_points.device)
+        with _on(gy_points.device):
+            check(lib.fovi_knnconv_weight_grad_pairs(self._h, _ptr(gy_points), _ptr(x_pairs), B, _ptr(out), _stream()), "fovi_knnconv_weight_grad_pairs")
+        return out
+
     def forward_f32(self, x, wt_f32, bias=None, relu=False, x_layout=ACT_BCN, y_layout=ACT_BCN):
         """Exact float32 path.  x [B,c_in,n_in] (BCN) or [B,n_in,c_in] (BNC)."""
         _need_cuda(x, wt_f32, bias)
@@ -393,6 +405,42 @@ def sample_knnconv_fused(splan, cplan, img, fix_rc, fix_hw, wt, bias=None, relu=
                                             {"fb": 0, "bf": 1}[row_order], _stream()),
               "fovi_sample_knnconv_fused")
     return out, intermediate
+
+
+class KnnDwPlan:
+    """Pair lists of a weight gradient on the device (fovi_knndw_plan)."""
+
+    def __init__(self, p_pt, q_pt, cnt, tap, V, n_p, n_q, device):
+        arrs = [np.ascontiguousarray(np.asarray(t, np.int32)) for t in (p_pt, q_pt, cnt, tap)]
+        self.n_out, self.kp = arrs[0].shape             # groups, longest list
+        self.V, self.n_p, self.n_q, self.device = int(V), int(n_p), int(n_q), torch.device(device)
+        assert arrs[1].shape == arrs[0].shape and arrs[2].shape == arrs[3].shape == (self.n_out,)
+        h = C.c_void_p()
+        with _on(self.device):
+            check(lib.fovi_knndw_plan_create(*[t.ctypes.data_as(C.c_void_p) for t in arrs], self.n_out, self.kp, self.V, self.n_p, self.n_q, C.byref(h)),
+                  "fovi_knndw_plan_create")
+        self._h = h
+
+    def __del__(self):
+        h, self._h = getattr(self, "_h", None), None
+        if h and lib is not None:
+            lib.fovi_knndw_plan_destroy(h)
+
+    def run(self, p, q):
+        """p [B,n_p,cp], q [B,n_q,cq] bf16 contiguous -> float32 [V, cp, cq].  See fovi_knndw_run."""
+        _need_cuda(p, q)
+        B, cp, cq = p.shape[0], p.shape[2], q.shape[2]
+        assert p.dtype == q.dtype == torch.bfloat16 and p.is_contiguous() and q.is_contiguous()
+        assert p.shape[1] == self.n_p and q.shape[:2] == (B, self.n_q), (p.shape, q.shape)
+        out = torch.zeros((self.V, cp, cq), dtype=torch.float32, device=p.device)
+        with _on(p.device):
+            check(lib.fovi_knndw_run(self._h, _ptr(p), cp, _ptr(q), cq, B, _ptr(out), _stream()), "fovi_knndw_run")
+        return out
+
+    def check(self):
+        """Synchronise the current stream and raise if a launch gave up on a wait."""
+        with _on(self.device):
+            check(lib.fovi_knndw_check(self._h, _stream()), "fovi_knndw_check")
 
 
 POOL_MODES = {"max": 0, "avg": 1, "sum": 2, "gaussian": 3}
@@ -535,6 +583,22 @@ def relu_backward_to_inner(grad, act, jp=None, bp=None, want_masked=True, want_c
         return None
     check(rc, "fovi_relu_backward_to_inner")
     return masked, out, colsum
+
+
+def relu_mask_colsum(grad, act):
+    """grad, act: contiguous bf16 [..., C] -> (gradient where act > 0 else 0, float32 [C] sums of it), or None when the shape needs the
+    separate calls."""
+    _need_cuda(grad, act)
+    assert grad.dtype == act.dtype == torch.bfloat16 and grad.is_contiguous() and act.is_contiguous() and grad.shape == act.shape
+    C_ = grad.shape[-1]
+    masked = torch.empty_like(grad)
+    colsum = torch.empty(C_, dtype=torch.float32, device=grad.device)
+    with _on(grad.device):
+        rc = lib.fovi_relu_mask_colsum(_ptr(grad), _ptr(act), _ptr(masked), _ptr(colsum), grad.numel() // C_, C_, _stream())
+    if rc == 2:   # FOVI_ERR_UNSUPPORTED
+        return None
+    check(rc, "fovi_relu_mask_colsum")
+    return masked, colsum
 
 
 def column_sum(x):

@@ -299,6 +299,27 @@ int fovi_batch_to_inner(const void* src, int dtype, int B, int I, int J, long lo
 int fovi_relu_backward_to_inner(const void* grad, const void* act, int dtype, int B, int I, int J, long long sb, long long si,
                                 long long sj, void* masked, void* dst, int Jp, int Bp, float* colsum, void* stream);
 
+/* Start of a layer's backward pass (channels-last bf16, C a multiple of 8 up to 2048, 16-byte aligned; otherwise FOVI_ERR_UNSUPPORTED: use the
+ * separate calls): masked[r][c] = act[r][c] > 0 ? grad[r][c] : 0, and colsum[c] (float32, overwritten; may be NULL) = sum over r of masked[r][c]. */
+int fovi_relu_mask_colsum(const void* grad, const void* act, void* masked, float* colsum, long long R, int C, void* stream);
+
+/* Weight gradient, read straight from channels-last activations (bf16): for every group g and every pair k < cnt[g]
+ *   out[tap[g]][i][j] += sum over b of P[b][p_pt[g][k]][i] * Q[b][q_pt[g][k]][j]        out: float32 [V][cp][cq], initialised by the caller.
+ * P [B][n_p][cp] and Q [B][n_q][cq] are the upstream gradient and the layer's input in either role; cp, cq multiples of 8.
+ * Groups whose pairs lie close together should follow each other (their operands then stay in L2).  Tables are host arrays, validated here.
+ * (The reference: autograd through fovi/arch/knn.py:538-557.) */
+typedef struct fovi_knndw_plan fovi_knndw_plan;
+int fovi_knndw_plan_create(const int32_t* p_pt, const int32_t* q_pt, const int32_t* cnt, const int32_t* tap, int n_groups, int kp, int V,
+                           int n_p, int n_q, fovi_knndw_plan** out);
+void fovi_knndw_plan_destroy(fovi_knndw_plan* plan);
+int fovi_knndw_run(fovi_knndw_plan* plan, const void* P, int cp, const void* Q, int cq, int B, float* out, void* stream);
+int fovi_knndw_check(fovi_knndw_plan* plan, void* stream);   /* as fovi_knnconv_check */
+
+/* Weight gradient of a pair-layout layer (c_in <= 4; `plan` is the layer's own, ungrouped plan): gY [B][n_out][c_out] bf16, X in the pair layout
+ * with the rows past B of the last row tile ZERO (as fovi_pack_points callers leave them).  out[v][o][0..3] += the four channel sums; float32
+ * [V][c_out][4], initialised by the caller. */
+int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* plan, const void* gY, const void* X, int B, float* out, void* stream);
+
 /* Bias gradient: dst[c] = sum over the R rows of the row-major [R, C] matrix src (bf16 or float32, C even), float32
  * accumulation; dst is overwritten.  (The reference: autograd of the bias add in F.linear, fovi/arch/knn.py:555.) */
 int fovi_column_sum(const void* src, int dtype, long long R, int C, float* dst, void* stream);
