@@ -6,17 +6,59 @@
 
 namespace {
 
-// W [c_out, c_in*V] (c-major, v-minor)  ->  slabs [V, c_out, cp]
-template <typename TW, typename TD>
-__global__ void pack_weights_kernel(const TW* __restrict__ W, TD* __restrict__ dst, int V, int c_out, int c_in, int cp) {
-  const long long total = (long long)V * c_out * cp;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % cp);
-    const int o = (int)((i / cp) % c_out);
-    const int v = (int)(i / ((long long)cp * c_out));
-    const float w = c < c_in ? ld_as_float(W + ((long long)o * c_in + c) * V + v) : 0.f;
-    dst[i] = from_float<TD>(w);
+// Changes between the reference's filter layout, W [c_out][c_in][V] (taps innermost), and tap-major slabs: transposes of [r][v] planes, one per
+// `outer` index, where r is the slabs' innermost index (an input channel, or an output channel for the transposed layer and for gradients).
+// What bounds them is memory, so a 64 x 64 tile of (r, v) goes through shared memory and both sides move in whole runs: taps on the filter's side
+// (its rows are V long), channels on the slabs' side.  384 -> 256 channels, 36 taps (14 MB in, 7 out): 29 -> PACKUS us against one thread per
+// slab element, whose reads were V apart.
+//   to slabs   dst[v * d_v + outer * d_o + r] = r < R ? W[outer * w_o + r * w_r + v] : 0   for r < Rp
+//   to filter  dst[outer * w_o + r * w_r + v] = src[v * d_v + outer * d_o + r]             for r < R
+constexpr int TAP_T = 64;
+
+template <typename TS, typename TD, bool TO_SLABS>
+__global__ void __launch_bounds__(256) tap_transpose_kernel(const TS* __restrict__ src, TD* __restrict__ dst, int R, int Rp, int V, long long w_o,
+                                                            long long w_r, long long d_v, long long d_o) {
+  __shared__ float tile[TAP_T][TAP_T + 1];
+  const int r0 = blockIdx.y * TAP_T, v0 = blockIdx.z * TAP_T;
+  const long long outer = blockIdx.x;
+  const int nv = min(TAP_T, V - v0), nr = min(TAP_T, (TO_SLABS ? Rp : R) - r0);
+  const uint32_t inv = (0xFFFFFFFFu / (uint32_t)nv) + 1u;      // i / nv == umulhi(i, inv) for the i < 4096 here (nv == 1: inv wraps to 0)
+  auto row_of = [&](int i) { return nv == 1 ? i : (int)__umulhi((uint32_t)i, inv); };
+  if (TO_SLABS) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nr * nv; i += 256) {
+      const int r = row_of(i), v = i - r * nv;
+      tile[r][v] = r0 + r < R ? ld_as_float(src + outer * w_o + (r0 + r) * w_r + v0 + v) : 0.f;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nv * TAP_T; i += 256) {
+      const int v = i / TAP_T, r = i % TAP_T;
+      if (r < nr) dst[(v0 + v) * d_v + outer * d_o + r0 + r] = from_float<TD>(tile[r][v]);
+    }
+  } else {
+    for (int i = threadIdx.x; i < nv * TAP_T; i += 256) {
+      const int v = i / TAP_T, r = i % TAP_T;
+      if (r < nr) tile[r][v] = ld_as_float(src + (v0 + v) * d_v + outer * d_o + r0 + r);
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nr * nv; i += 256) {
+      const int r = row_of(i), v = i - r * nv;
+      dst[outer * w_o + (r0 + r) * w_r + v0 + v] = from_float<TD>(tile[r][v]);
+    }
   }
+}
+
+template <bool TO_SLABS>
+int tap_transpose(const void* src, int s_dtype, void* dst, int d_dtype, int n_outer, int R, int Rp, int V, long long w_o, long long w_r, long long d_v,
+                  long long d_o, cudaStream_t st) {
+  const dim3 grid(n_outer, (Rp + TAP_T - 1) / TAP_T, (V + TAP_T - 1) / TAP_T);
+  if (grid.y > 65535 || grid.z > 65535) return FOVI_ERR_UNSUPPORTED;
+#define GO(TS, TD) tap_transpose_kernel<TS, TD, TO_SLABS><<<grid, 256, 0, st>>>((const TS*)src, (TD*)dst, R, Rp, V, w_o, w_r, d_v, d_o)
+  if (s_dtype == FOVI_F32) { if (d_dtype == FOVI_F32) GO(float, float); else GO(float, __nv_bfloat16); }
+  else { if (d_dtype == FOVI_F32) GO(__nv_bfloat16, float); else GO(__nv_bfloat16, __nv_bfloat16); }
+#undef GO
+  return fovi::after_launch("tap_transpose_kernel");
 }
 
 // Pair mode: W [c_out, c_in*V] -> per-output-point slabs [n_out, c_out/ct, sp, ct, 8] (so the eight
@@ -52,6 +94,7 @@ template <typename TW>
 __global__ void pack_weights_grouped_kernel(const TW* __restrict__ W, __nv_bfloat16* __restrict__ dst,
                                             const uint16_t* __restrict__ pair_tap, const uint16_t* __restrict__ member_tap, int n_groups,
                                             int sp, int K, int G, int V, int co, int c_in, int ct) {
+  // (any V; filters of up to GROUPED_TAPS taps take the kernel below)
   // one thread per 16-byte row of the destination (a pair slot of one output channel: 2 points x 4 channels), so the
   // index arithmetic and the two table look-ups are paid once per eight values and the store is a whole 16-byte piece
   const int c_out = G * co;
@@ -79,11 +122,61 @@ __global__ void pack_weights_grouped_kernel(const TW* __restrict__ W, __nv_bfloa
   }
 }
 
-// X [B,C,N] -> [ceil(B/128), ceil(N/2), 128, 2, 4] bf16 (pair layout), one thread per (pair, image).
+// Same result for filters whose 32-channel slice fits shared memory.  The rows are two 8-byte pieces of the filter each, and what bounds the kernel
+// above is fetching them: six 4-byte loads a thread, V * c_in apart between neighbouring lanes.  Here a CTA holds 32 channels of one member in shared
+// memory, tap-major and in bf16 (lanes read consecutive 8-byte pieces), and writes their rows for its share of the groups: a warp looks up the taps of
+// 32 slots at a time, a lane per slot, and stores 32 rows of 16 bytes per slot.  3 -> 64 channels, 484 taps, 341 groups of 3 (92 MB): 80 -> GROUPUS us.
+constexpr int GROUPED_TAPS = 800;      // 211 KB
+
+template <typename TW>
+__global__ void __launch_bounds__(512) pack_weights_grouped_smem_kernel(const TW* __restrict__ W, __nv_bfloat16* __restrict__ dst,
+                                                                        const uint16_t* __restrict__ pair_tap, const uint16_t* __restrict__ member_tap,
+                                                                        int n_groups, int sp, int K, int G, int V, int co, int c_in, int ct) {
+  extern __shared__ __align__(16) unsigned char pg_smem[];
+  __nv_bfloat16* ws = reinterpret_cast<__nv_bfloat16*>(pg_smem);          // [V][33][4]
+  const int o0 = blockIdx.x * 32, j = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int no = min(32, co - o0);
+  for (int i = threadIdx.x; i < V * 33 * 2; i += blockDim.x) reinterpret_cast<uint32_t*>(pg_smem)[i] = 0u;
+  __syncthreads();
+  for (int r = warp; r < no * c_in; r += blockDim.x >> 5) {               // a warp per filter row
+    const int o = r / c_in, c = r - o * c_in;
+    const TW* row = W + ((long long)(o0 + o) * c_in + c) * V;
+#pragma unroll 8
+    for (int t = lane; t < V; t += 32) ws[((size_t)t * 33 + o) * 4 + c] = __float2bfloat16_rn(ld_as_float(row + t));
+  }
+  __syncthreads();
+  const int op = j * co + o0 + lane, tile = op / ct, oc = op - tile * ct, n_ct = G * co / ct;
+  const int chunks = (sp + 31) / 32;
+  const long long units = (long long)n_groups * chunks;
+  const int n_warps = (blockDim.x >> 5) * gridDim.z;
+  for (long long u = (long long)blockIdx.z * (blockDim.x >> 5) + warp; u < units; u += n_warps) {
+    const long long g = u / chunks;
+    const int s0 = (int)(u - g * chunks) * 32, m = min(32, sp - s0);
+    uint32_t taps = 0xFFFFFFFFu;                                            // this lane's slot: the two halves' taps
+    if (lane < m) {
+      const uint32_t ks = *reinterpret_cast<const uint32_t*>(pair_tap + (g * sp + s0 + lane) * 2);
+      const uint32_t k0 = ks & 0xFFFFu, k1 = ks >> 16;
+      const uint32_t t0 = k0 != 0xFFFFu ? __ldg(member_tap + (g * K + k0) * G + j) : 0xFFFFu;
+      const uint32_t t1 = k1 != 0xFFFFu ? __ldg(member_tap + (g * K + k1) * G + j) : 0xFFFFu;
+      taps = t0 | (t1 << 16);
+    }
+    uint4* out = reinterpret_cast<uint4*>(dst) + ((g * n_ct + tile) * sp + s0) * ct + oc;
+#pragma unroll 4
+    for (int s = 0; s < m; ++s) {
+      const uint32_t tt = __shfl_sync(0xffffffffu, taps, s), t0 = tt & 0xFFFFu, t1 = tt >> 16;
+      uint2 a = make_uint2(0u, 0u), b = make_uint2(0u, 0u);
+      if (t0 != 0xFFFFu) a = *reinterpret_cast<const uint2*>(ws + ((size_t)t0 * 33 + lane) * 4);
+      if (t1 != 0xFFFFu) b = *reinterpret_cast<const uint2*>(ws + ((size_t)t1 * 33 + lane) * 4);
+      if (lane < no) out[(size_t)s * ct] = make_uint4(a.x, a.y, b.x, b.y);
+    }
+  }
+}
+
+// X [B,C,N] -> [ceil(B/128), ceil(N/2), 128, 2, 4] bf16 (pair layout), one thread per (pair, row); the last tile's rows past the batch are zeros.
 template <typename TX>
 __global__ void pack_points_pairs_kernel(const TX* __restrict__ x, __nv_bfloat16* __restrict__ dst, int B, int C, int N) {
   const int n_pairs = (N + 1) / 2;
-  const long long total = (long long)n_pairs * B;
+  const long long total = (long long)n_pairs * ((B + 127) / 128 * 128);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int pr = (int)(i % n_pairs), b = (int)(i / n_pairs);
     __align__(16) __nv_bfloat16 v[8];
@@ -92,7 +185,7 @@ __global__ void pack_points_pairs_kernel(const TX* __restrict__ x, __nv_bfloat16
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int n = 2 * pr + h;
-        v[h * 4 + c] = __float2bfloat16_rn((c < C && n < N) ? ld_as_float(x + ((long long)b * C + c) * N + n) : 0.f);
+        v[h * 4 + c] = __float2bfloat16_rn((c < C && n < N && b < B) ? ld_as_float(x + ((long long)b * C + c) * N + n) : 0.f);
       }
     *reinterpret_cast<uint4*>(dst + (((long long)(b >> 7) * n_pairs + pr) * 128 + (b & 127)) * 8) = *reinterpret_cast<const uint4*>(v);
   }
@@ -507,16 +600,25 @@ extern "C" int fovi_knnconv_pack_weights(const fovi_knnconv_plan* p, const void*
       pack_weights_pairs_kernel<__nv_bfloat16><<<g, 256, 0, st>>>((const __nv_bfloat16*)W, (__nv_bfloat16*)dst, p->pair_tap, p->n_out, p->sp, p->V, p->c_out, p->c_in, p->ct);
     return fovi::after_launch("pack_weights_pairs_kernel");
   }
-  const long long total = (long long)p->V * p->c_out * p->cin_packed;
-  const int grid = (int)std::min<long long>((total + 255) / 256, 148 * 16);
-#define PACK(TW, TD) \
-  pack_weights_kernel<TW, TD><<<grid, 256, 0, st>>>((const TW*)W, (TD*)dst, p->V, p->c_out, p->c_in, p->cin_packed)
-  if (w_dtype == FOVI_F32 && dst_dtype == FOVI_F32) PACK(float, float);
-  else if (w_dtype == FOVI_F32 && dst_dtype == FOVI_BF16) PACK(float, __nv_bfloat16);
-  else if (w_dtype == FOVI_BF16 && dst_dtype == FOVI_F32) PACK(__nv_bfloat16, float);
-  else PACK(__nv_bfloat16, __nv_bfloat16);
-#undef PACK
-  return fovi::after_launch("pack_weights_kernel");
+  // slabs [V][c_out][cin_packed]
+  return tap_transpose<true>(W, w_dtype, dst, dst_dtype, p->c_out, p->c_in, p->cin_packed, p->V, (long long)p->c_in * p->V, p->V,
+                             (long long)p->c_out * p->cin_packed, p->cin_packed, st);
+}
+
+extern "C" int fovi_knnconv_pack_weights_transposed(const fovi_knnconv_plan* p, const void* W, int w_dtype, void* dst, int dst_dtype, void* stream) {
+  if (!p || !W || !dst || !fovi::valid_dtype(w_dtype) || !fovi::valid_dtype(dst_dtype)) return FOVI_ERR_INVALID_ARGUMENT;
+  if (p->x_layout == FOVI_X_PAIRS) return FOVI_ERR_UNSUPPORTED;
+  return tap_transpose<true>(W, w_dtype, dst, dst_dtype, p->c_out, p->c_in, p->cin_packed, p->V, p->V, (long long)p->c_out * p->V,
+                             (long long)p->c_out * p->cin_packed, p->cin_packed, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int fovi_weight_grad_unpack(const float* src, int V, int n_i, int n_j, int swapped, int c_out, int c_in, void* dst, int dst_dtype, void* stream) {
+  if (!src || !dst || V <= 0 || c_out <= 0 || c_in <= 0 || !fovi::valid_dtype(dst_dtype)) return FOVI_ERR_INVALID_ARGUMENT;
+  if ((swapped ? n_j : n_i) < c_out || (swapped ? n_i : n_j) < c_in) return FOVI_ERR_INVALID_ARGUMENT;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const long long plane = (long long)n_i * n_j;
+  return swapped ? tap_transpose<false>(src, FOVI_F32, dst, dst_dtype, c_in, c_out, c_out, V, V, (long long)c_in * V, plane, n_j, st)
+                 : tap_transpose<false>(src, FOVI_F32, dst, dst_dtype, c_out, c_in, c_in, V, (long long)c_in * V, V, plane, n_j, st);
 }
 
 extern "C" int fovi_knnconv_pack_weights_grouped(const fovi_knnconv_plan* p, const void* W, int w_dtype, const uint16_t* member_tap, int G,
@@ -524,6 +626,22 @@ extern "C" int fovi_knnconv_pack_weights_grouped(const fovi_knnconv_plan* p, con
   if (!p || !W || !member_tap || !dst || !fovi::valid_dtype(w_dtype) || G <= 0 || V <= 0) return FOVI_ERR_INVALID_ARGUMENT;
   if (p->x_layout != FOVI_X_PAIRS || !p->ct || p->c_out % G) return FOVI_ERR_UNSUPPORTED;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (V <= GROUPED_TAPS && p->c_in <= 4) {
+    const size_t smem = (size_t)V * 33 * 8;
+    const int co = p->c_out / G;
+    const int nx = (co + 31) / 32, split = std::max(1, fovi::sm_count() / (nx * G));
+    const dim3 grid3(nx, G, split);
+#define GO(TW)                                                                                                                                   \
+  do {                                                                                                                                           \
+    if (smem > 48 * 1024)                                                                                                                        \
+      FOVI_CUDA(cudaFuncSetAttribute(pack_weights_grouped_smem_kernel<TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));             \
+    pack_weights_grouped_smem_kernel<TW><<<grid3, 512, smem, st>>>((const TW*)W, (__nv_bfloat16*)dst, p->pair_tap, member_tap, p->n_out, p->sp, p->K, \
+                                                                   G, V, co, p->c_in, p->ct);                                                    \
+  } while (0)
+    if (w_dtype == FOVI_F32) GO(float); else GO(__nv_bfloat16);
+#undef GO
+    return fovi::after_launch("pack_weights_grouped_smem_kernel");
+  }
   const long long tot = (long long)p->n_out * p->sp * p->c_out;   // 16-byte rows
   const int grid = (int)std::min<long long>((tot + 255) / 256, 148 * 32);
   if (w_dtype == FOVI_F32)
@@ -545,7 +663,7 @@ extern "C" int fovi_pack_points(const void* x, int x_dtype, int B, int C, int N,
   if (B > 65535) return FOVI_ERR_UNSUPPORTED;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (x_layout == FOVI_X_PAIRS) {
-    const long long tot = (long long)((N + 1) / 2) * B;
+    const long long tot = (long long)((N + 1) / 2) * ((B + 127) / 128 * 128);
     const int g = (int)std::min<long long>((tot + 255) / 256, 148 * 32);
     if (x_dtype == FOVI_F32) pack_points_pairs_kernel<float><<<g, 256, 0, st>>>((const float*)x, (__nv_bfloat16*)dst, B, C, N);
     else pack_points_pairs_kernel<__nv_bfloat16><<<g, 256, 0, st>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)dst, B, C, N);
@@ -642,13 +760,6 @@ extern "C" int fovi_knnconv_forward_bcn_static(fovi_knnconv_plan* p, const void*
   int rc = static_scratch_address(&scratch);
   if (rc) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (pairs && (B & 127)) {
-    // The pad rows of the last 128-row tile are never written by the repack: clear them, so that no
-    // bit pattern left by an earlier call is fed to the tensor cores.
-    const int r0 = B & 127;
-    unsigned char* tile = scratch + (size_t)(B / 128) * p->n_pairs * 2048;
-    FOVI_CUDA(cudaMemset2DAsync(tile + (size_t)r0 * 16, 2048, 0, (size_t)(128 - r0) * 16, p->n_pairs, st));
-  }
   rc = fovi_pack_points(X, x_dtype, B, p->c_in, p->n_in, scratch, p->cin_packed, p->x_layout, stream);
   if (rc) return rc;
   return fovi_knnconv_forward(p, scratch, Wt, bias, Y, y_dtype, B, relu, stream);

@@ -81,8 +81,7 @@ class KnnConvGrad:
     def input_grad(self, gy_points, weight):
         """gy_points [B, n_out, c_out] bf16 contiguous, weight [c_out, c_in*V] -> dX [B, n_in, c_in] bf16 (channels last)."""
         plan = self.dx_plan()
-        w_t = weight.detach().reshape(self.c_out, self.c_in, self.V).permute(1, 0, 2).reshape(self.c_in, self.c_out * self.V)
-        return plan.forward(gy_points, plan.pack_weights(w_t.contiguous()), out_dtype=torch.bfloat16)
+        return plan.forward(gy_points, plan.pack_weights_transposed(weight), out_dtype=torch.bfloat16)
 
     # ---- dW
     @property
@@ -116,18 +115,14 @@ class KnnConvGrad:
             self._dw_plans["dw"] = (ops.KnnDwPlan(p_pt, q_pt, cnt, owner, self.V, n_p, n_q, self.device), owner)
         return self._dw_plans["dw"]
 
-    def weight_grad(self, gy_points, x_points, plan):
+    def weight_grad(self, gy_points, x_points, plan, dtype=torch.float32):
         """gy_points [B, n_out, c_out] bf16 contiguous, x_points the layer's packed input ([B, n_in, cin_packed] bf16, or the pair layout with zero
-        pad rows), plan the layer's own -> dW [c_out, c_in*V] float32."""
+        pad rows), plan the layer's own -> dW [c_out, c_in*V] (summed in float32)."""
         if plan.x_layout == ops.X_PAIRS:
             self._few = plan
-            dw = plan.weight_grad_pairs(gy_points, x_points)                                # [V, c_out, 4]
-            return dw[:, :, :self.c_in].permute(1, 2, 0).reshape(self.c_out, self.c_in * self.V)
-        if self.dw_swapped:
-            dw = self.dw_plan()[0].run(x_points, gy_points)                                 # [V, cin_packed, c_out]
-            return dw[:, :self.c_in].permute(2, 1, 0).reshape(self.c_out, self.c_in * self.V)
-        dw = self.dw_plan()[0].run(gy_points, x_points)                                     # [V, c_out, cin_packed]
-        return dw[:, :, :self.c_in].permute(1, 2, 0).reshape(self.c_out, self.c_in * self.V)
+            return ops.weight_grad_unpack(plan.weight_grad_pairs(gy_points, x_points), self.c_out, self.c_in, dtype=dtype)
+        p, q = (x_points, gy_points) if self.dw_swapped else (gy_points, x_points)
+        return ops.weight_grad_unpack(self.dw_plan()[0].run(p, q), self.c_out, self.c_in, swapped=self.dw_swapped, dtype=dtype)
 
     # ---- exact float32 route (precision='fp32' layers and shapes outside the tensor-core kernel): the same two derived
     # layers, run on the exact float32 kernel (fovi_knnconv_forward_f32) instead of the tensor cores
@@ -210,7 +205,7 @@ class _KnnConvFunction(torch.autograd.Function):
             if ctx.needs_input_grad[0]:
                 gx = g.input_grad(gyp, weight).permute(0, 2, 1).to(ctx.x_dtype)
             if ctx.needs_input_grad[1]:
-                gw = g.weight_grad(gyp, x, ctx.layer.plan).to(weight.dtype)
+                gw = g.weight_grad(gyp, x, ctx.layer.plan, weight.dtype)
         if ctx.has_bias and ctx.needs_input_grad[2]:
             gb = gy.sum((0, 2), dtype=torch.float32)
         return gx, gw, gb, None
@@ -252,7 +247,7 @@ class _KnnConvPointsFunction(torch.autograd.Function):
                 raise NotImplementedError("input gradient of a pair-layout first layer is not built")
             gx = g.input_grad(gy, weight)                                      # [B, n_in, c_in] bf16
         if want_w:
-            gw = g.weight_grad(gy, xp, ctx.layer.plan).to(weight.dtype)
+            gw = g.weight_grad(gy, xp, ctx.layer.plan, weight.dtype)
         if not want_b:
             gb = None
         elif gb is None:

@@ -270,6 +270,18 @@ class KnnConvPlan:
             check(lib.fovi_knnconv_pack_weights(self._h, _ptr(weight), _dt(weight.dtype), _ptr(dst), _dt(dtype), _stream()), "fovi_knnconv_pack_weights")
         return dst
 
+    def pack_weights_transposed(self, weight):
+        """This plan is the transposed layer of one whose weight is [c_in, c_out*V] (this plan's channel counts): its bf16 operand, as
+        `pack_weights` gives it for the channel-transposed weight."""
+        _need_cuda(weight)
+        weight = weight.detach().contiguous()
+        assert weight.shape == (self.c_in, self.c_out * self.V) and self.x_layout != X_PAIRS
+        dst = torch.empty((self.V, self.c_out, self.cin_packed), dtype=torch.bfloat16, device=weight.device)
+        with _on(weight.device):
+            check(lib.fovi_knnconv_pack_weights_transposed(self._h, _ptr(weight), _dt(weight.dtype), _ptr(dst), BF16, _stream()),
+                  "fovi_knnconv_pack_weights_transposed")
+        return dst
+
     def forward(self, x_bnc, wt, bias=None, relu=False, out_dtype=torch.bfloat16, out=None, batch=None):
         """Tensor-core path.  x_bnc: bf16 contiguous, [B,n_in,cin_packed] or (pair layout)
         [ceil(B/128),n_pairs,128,8] with `batch` = B  ->  [B,n_out,c_out]."""
@@ -407,6 +419,17 @@ def sample_knnconv_fused(splan, cplan, img, fix_rc, fix_hw, wt, bias=None, relu=
     return out, intermediate
 
 
+def weight_grad_unpack(src, c_out, c_in, swapped=False, dtype=torch.float32):
+    """Tap-major gradient [V, n_i, n_j] float32 -> [c_out, c_in*V] in `dtype`; i is the output channel (the input channel when `swapped`)."""
+    _need_cuda(src)
+    assert src.dtype == torch.float32 and src.is_contiguous() and src.dim() == 3
+    V, n_i, n_j = src.shape
+    dst = torch.empty((c_out, c_in * V), dtype=dtype, device=src.device)
+    with _on(src.device):
+        check(lib.fovi_weight_grad_unpack(_ptr(src), V, n_i, n_j, int(swapped), c_out, c_in, _ptr(dst), _dt(dtype), _stream()), "fovi_weight_grad_unpack")
+    return dst
+
+
 class KnnDwPlan:
     """Pair lists of a weight gradient on the device (fovi_knndw_plan)."""
 
@@ -536,8 +559,7 @@ def pack_points(x, cp=8, x_layout=X_BNC):
     x = x.contiguous()
     B, Cc, N = x.shape
     shape = ((B + 127) // 128, (N + 1) // 2, 128, 8) if x_layout == X_PAIRS else (B, N, cp)
-    # the pad rows of the last 128-row tile are zeroed so that the buffer holds no stray bit patterns
-    dst = (torch.zeros if x_layout == X_PAIRS else torch.empty)(shape, dtype=torch.bfloat16, device=x.device)
+    dst = torch.empty(shape, dtype=torch.bfloat16, device=x.device)       # the kernel zeroes the last row tile's rows past the batch
     with _on(x.device):
         check(lib.fovi_pack_points(_ptr(x), _dt(x.dtype), B, Cc, N, _ptr(dst), cp, x_layout, _stream()), "fovi_pack_points")
     return dst

@@ -171,6 +171,14 @@ int64_t fovi_knnconv_nnz(const fovi_knnconv_plan* plan);
 int fovi_knnconv_pack_weights(const fovi_knnconv_plan* plan, const void* W, int w_dtype, void* dst, int dst_dtype,
                               void* stream);
 /* Bytes of the packed weight buffer for `dst_dtype`. */
+/* Packed operand of the TRANSPOSED layer (the input gradient): `plan` is the transposed layer's (c_out = the layer's c_in and the other way round), W
+ * the layer's own weight [c_out][c_in * V]; same destination as fovi_knnconv_pack_weights(plan, ...) on the channel-transposed weight. */
+int fovi_knnconv_pack_weights_transposed(const fovi_knnconv_plan* plan, const void* W, int w_dtype, void* dst, int dst_dtype, void* stream);
+
+/* Tap-major weight gradient src [V][n_i][n_j] float32 -> the weight's own layout dst [c_out][c_in][V] (float32 or bf16).  swapped = 0: i is the output
+ * channel and j the input channel; 1: the other way round.  Rows and columns past c_out / c_in are dropped. */
+int fovi_weight_grad_unpack(const float* src, int V, int n_i, int n_j, int swapped, int c_out, int c_in, void* dst, int dst_dtype, void* stream);
+
 int64_t fovi_knnconv_packed_weight_bytes(const fovi_knnconv_plan* plan, int dst_dtype);
 
 /* Grouped first layer.  With c_in <= 4 the MMA's N axis holds only c_out (64-96) columns; G consecutive output points can

@@ -63,3 +63,43 @@ def test_relu_mask_and_channel_sums(rows, C):
     err = (sums.double() - want.double().sum(0)).abs()
     assert (err <= rows * 2.0 ** -24 * want.double().abs().sum(0) + 1e-30).all()
     assert ops.relu_mask_colsum(g[:, :4].contiguous(), y[:, :4].contiguous()) is None
+
+
+# channel counts around the 64 x 64 tiles, padded channels, taps past one tile
+@pytest.mark.parametrize("cin,cout,V,dtype", [(16, 48, 9, torch.float32), (72, 64, 36, torch.bfloat16), (100, 32, 130, torch.float32), (192, 384, 64, torch.float32),
+                                              (65, 16, 65, torch.float32)])
+def test_filter_layout_changes(cin, cout, V, dtype):
+    from fovi_b200 import ops
+    torch.manual_seed(cin)
+    w = torch.randn(cout, cin * V, device="cuda").to(dtype)
+    w3 = w.view(cout, cin, V)
+    one = lambda a, b: ops.KnnConvPlan(np.zeros((1, 2), np.int32), np.zeros((2, 1), np.uint16), 3, V, a, b)   # noqa: E731
+    plan = one(cin, cout)
+    for t in (torch.bfloat16, torch.float32):
+        got = plan.pack_weights(w, t)
+        assert torch.equal(got[:, :, :cin], w3.permute(2, 0, 1).to(t)) and not got[:, :, cin:].any()
+    got = one(cout, cin).pack_weights_transposed(w)
+    assert torch.equal(got[:, :, :cout], w3.permute(2, 1, 0).to(torch.bfloat16)) and not got[:, :, cout:].any()
+    g = torch.randn(V, cout + 8, cin + 8, device="cuda")
+    assert torch.equal(ops.weight_grad_unpack(g, cout, cin, dtype=dtype), g[:, :cout, :cin].permute(1, 2, 0).reshape(cout, cin * V).to(dtype))
+    gs = torch.randn(V, cin + 8, cout, device="cuda")
+    assert torch.equal(ops.weight_grad_unpack(gs, cout, cin, swapped=True, dtype=dtype), gs[:, :cin].permute(2, 1, 0).reshape(cout, cin * V).to(dtype))
+
+
+@pytest.mark.parametrize("cin,cout,V,n_out,group", [(3, 64, 484, 12, 3), (4, 48, 25, 8, 4), (1, 96, 9, 6, 2), (3, 16, 801, 4, 4)])
+def test_grouped_weights_equal_the_ungrouped_ones(cin, cout, V, n_out, group):
+    """Every member's rows of a group's packed weights are the filter rows its own taps name (801 taps: past the shared-memory kernel)."""
+    from fovi_b200 import ops
+    rs = np.random.RandomState(V)
+    n_in, K = 60, 9
+    idx = np.stack([rs.permutation(n_in)[:K] for _ in range(n_out)], 1).astype(np.int32)
+    tap = rs.randint(0, V, (n_out, K)).astype(np.uint16)
+    plan = ops.KnnConvPlan(idx, tap, n_in, V, cin, cout, group=group)
+    assert plan.group == group
+    w = torch.randn(cout, cin * V, device="cuda")
+    x = torch.randn(3, cin, n_in, device="cuda").to(torch.bfloat16)
+    xp = ops.pack_points(x, plan)
+    got = plan.forward(xp, plan.pack_weights(w), batch=3, out_dtype=torch.float32)
+    flat = ops.KnnConvPlan(idx, tap, n_in, V, cin, cout, group=1)
+    want = flat.forward(xp, flat.pack_weights(w), batch=3, out_dtype=torch.float32)
+    assert (got - want).abs().max().item() < 1e-5 * want.abs().max().item()
