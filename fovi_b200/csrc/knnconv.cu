@@ -9,7 +9,7 @@ namespace {
 // Changes between the reference's filter layout, W [c_out][c_in][V] (taps innermost), and tap-major slabs: transposes of [r][v] planes, one per
 // `outer` index, where r is the slabs' innermost index (an input channel, or an output channel for the transposed layer and for gradients).
 // What bounds them is memory, so a 64 x 64 tile of (r, v) goes through shared memory and both sides move in whole runs: taps on the filter's side
-// (its rows are V long), channels on the slabs' side.  384 -> 256 channels, 36 taps (14 MB in, 7 out): 29 -> PACKUS us against one thread per
+// (its rows are V long), channels on the slabs' side.  384 -> 256 channels, 36 taps (14 MB in, 7 out): 22 -> 11 us against one thread per
 // slab element, whose reads were V apart.
 //   to slabs   dst[v * d_v + outer * d_o + r] = r < R ? W[outer * w_o + r * w_r + v] : 0   for r < Rp
 //   to filter  dst[outer * w_o + r * w_r + v] = src[v * d_v + outer * d_o + r]             for r < R
@@ -125,7 +125,7 @@ __global__ void pack_weights_grouped_kernel(const TW* __restrict__ W, __nv_bfloa
 // Same result for filters whose 32-channel slice fits shared memory.  The rows are two 8-byte pieces of the filter each, and what bounds the kernel
 // above is fetching them: six 4-byte loads a thread, V * c_in apart between neighbouring lanes.  Here a CTA holds 32 channels of one member in shared
 // memory, tap-major and in bf16 (lanes read consecutive 8-byte pieces), and writes their rows for its share of the groups: a warp looks up the taps of
-// 32 slots at a time, a lane per slot, and stores 32 rows of 16 bytes per slot.  3 -> 64 channels, 484 taps, 341 groups of 3 (92 MB): 80 -> GROUPUS us.
+// 32 slots at a time, a lane per slot, and stores 32 rows of 16 bytes per slot.  3 -> 64 channels, 484 taps, 341 groups of 3 (92 MB): 80 -> 39 us.
 constexpr int GROUPED_TAPS = 800;      // 211 KB
 
 template <typename TW>
