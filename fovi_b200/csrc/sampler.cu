@@ -6,10 +6,10 @@
 // fovi_sample_strip_kernel (the fast path: x-contiguous images whose rows are 16-byte aligned, C <= 4).
 //   The image, not the output row, is what a CTA holds still.  One CTA owns a horizontal strip of R rows of one
 //   image.  It hands the strip (R rows + the next row, all channel planes; for wide images only the columns the
-//   fixations of this image can touch) to the TMA unit as one bulk copy per row (cp.async.bulk onto an mbarrier) --
+//   fixations of this image can touch) to the TMA unit, as one tensor copy or one bulk copy per row --
 //   whole lines, in address order, every byte of the image fetched from DRAM once -- and then serves ALL
-//   fixations of that image from shared memory.  The plan keeps the sensor's points sorted by their grid y with a
-//   rank table over y buckets.  The fixation transform is an affine map with positive scale, so the points of one
+//   fixations of that image from shared memory.  The plan keeps the sensor's points sorted by buckets of their grid y
+//   with a rank table over the buckets (see N_ORDERS).  The fixation transform is an affine map with positive scale, so the points of one
 //   fixation whose 2x2 footprint starts in the strip's rows lie in ONE contiguous range of that order; the range is
 //   read off the rank table from the analytically inverted transform (widened by two buckets, far more than float32
 //   rounding can move a point) and every point in it is then tested with the exact float32 row it maps to.  Every
@@ -21,8 +21,7 @@
 //   The one wait (for the copies) is bounded: a strip that gives up sets the plan's status word, read back by
 //   fovi_sampler_check, and leaves.
 //
-// fovi_sample_kernel (any strides, any channel count).  One CTA per (image, fixation) walks the points in Morton
-//   order with plain loads and stages the output row in shared memory for one coalesced store.
+// fovi_sample_kernel (any strides, any channel count).  One thread per point, plain loads, points in their own order.
 //
 // Arithmetic: float32, one rounding per operation in the order of the reference
 // (fovi/sensing/coords.py:624-640 followed by torch's CPU grid_sample with align_corners=False):
@@ -35,34 +34,21 @@
 #include <algorithm>
 #include <limits.h>
 #include <type_traits>
-#include <stdlib.h>
 #include <string.h>
 #include <vector>
 
-#include "common.cuh"
+#include <cuda.h>
 
-#ifndef FOVI_STRIP_ROWS_MAX
-#define FOVI_STRIP_ROWS_MAX 8       // rows a strip owns at most (it loads one more)
-#endif
-#ifndef FOVI_STRIP_SMEM_BUDGET
-#define FOVI_STRIP_SMEM_BUDGET (27 * 1024)   // shared memory per CTA: eight CTAs per SM
-#endif
-#ifndef FOVI_STRIP_THREADS
-#define FOVI_STRIP_THREADS 128
-#endif
-#ifndef FOVI_STRIP_MIN_CTAS
-#define FOVI_STRIP_MIN_CTAS 8
-#endif
+#include "common.cuh"
 
 struct fovi_sampler_plan {
   int n_points = 0;
   int device = -1;
-  float2* sorted_xy = nullptr;  // [N] grid (x, y) in Morton order (general kernel)
-  int* sorted_idx = nullptr;    // [N] original index of each visited point
   float2* grid_xy = nullptr;    // [N] grid (x, y) in the caller's order (gradient kernel)
-  void* ys = nullptr;           // [N] {x, y, original index, 0} sorted by grid y (strip kernel); null: no such order
+  void* cells = nullptr;        // [N] {x, y, original index, 0} by cell of an 8 x 8 partition, then index (general kernel)
+  void* ys = nullptr;           // [3][N] {x, y, original index, 0} in the strip kernel's visiting orders (see N_ORDERS); null: none
   float gx_min = 0, gx_max = 0, gy_min = 0, gy_max = 0;
-  int* rank_lut = nullptr;      // [4097] rank table over gy buckets (see the strip kernel)
+  int* rank_lut = nullptr;      // [3][4097] rank tables of the orders over gy buckets (see the strip kernel)
   float lut_scale = 0;
   int* status = nullptr;        // device word: set by a strip kernel whose wait for its copies gave up
 };
@@ -74,8 +60,8 @@ struct __align__(16) YPoint { float x, y; int n; int pad_; };   // one sensor po
 struct SampleArgs {
   const void* img;
   void* out;
-  const float2* sorted_xy;   // visiting order of the kernel that runs (Morton order, or y order for the strip kernel)
-  const int* sorted_idx;
+  const float2* grid_xy;     // the grid in the caller's order (gradient kernel)
+  const YPoint* cells;       // the grid cell by cell (general kernel)
   const YPoint* ys;          // y order (null: the plan has none)
   const float* fix_rc;
   const float* fix_hw;
@@ -88,6 +74,8 @@ struct SampleArgs {
   // strip kernel only
   int R, n_strips, pitch;   // rows owned per strip, strips per image, shared-memory row pitch in elements
   int layout;               // LAY_PLANAR / LAY_NC / LAY_PAIRS
+  int q_shift;              // the order's bucket height: 2^q_shift buckets of the rank table
+  int use_map;              // 1: the strip's rows arrive as one tensor copy
   int full_rows;            // 1: rows are short enough to be copied whole, without waiting for the fixations
   const int* rank_lut;      // [RANK_LUT_Q + 1] number of points whose gy falls in a bucket below q
   float lut_scale;          // buckets per unit of gy
@@ -118,9 +106,23 @@ template <> __device__ __forceinline__ float smem_as_float<unsigned char>(const 
 // ------------------------------------------------------------------------------------------------------------
 // Strip kernel.
 // ------------------------------------------------------------------------------------------------------------
-constexpr int STRIP_THREADS = FOVI_STRIP_THREADS;
+// Two shapes of the strip kernel.  NARROW: eight CTAs of 128 threads per SM, strips of at most 8 rows; a strip's life is mostly latency, and small
+// independent CTAs overlap best (and fill the chip from the fewest images).  WIDE: three CTAs of 384 threads with strips of up to 72 KB, for the
+// planar layouts of large batches, whose bound is the scattered stores: a tall strip can be visited ring by ring (see N_ORDERS) with few foreign
+// candidates.  512 images x 4 fixations, 256 x 256 float32: NARROW 131 us (nearest 128), WIDE 113 (101), where the copy rate gives 77; pair layout,
+// 256 images: 60 / 64, and 8 bf16 fixations of 1024 images 342 / 333.
+template <bool WIDE> struct StripShape {
+  static constexpr int THREADS = WIDE ? 384 : 128, MIN_CTAS = WIDE ? 3 : 8, ROWS_MAX = WIDE ? 64 : 8, SMEM = (WIDE ? 72 : 27) * 1024;
+};
 constexpr int FCHUNK = 16;        // fixations served per pass over the strip
 constexpr int RANK_LUT_Q = 4096;  // buckets of the plan's rank table over [gy_min, gy_max]
+// Visiting orders of the sensor's points: by coarse buckets of grid y and, inside a bucket, by original index.  The finest (one rank-table bucket)
+// makes a strip's candidates almost exactly its points; in a coarser one neighbouring lanes hold neighbouring points of a ring, whose results share
+// 32-byte sectors -- the planar layout's scattered stores are what bounds the kernel (one sector per clock and SM) -- at the price of candidates
+// that turn out to be another strip's.  Per point, 4010-point sensor on a 256-row image, strips of 15 rows: 0.80 sectors and 1.0 candidates in the finest
+// order, 0.59 and 1.27 with 64 buckets, 0.44 and 1.53 with 32.
+constexpr int N_ORDERS = 3;
+constexpr int ORDER_SHIFT[N_ORDERS] = {0, 6, 7};   // 4096, 64 and 32 buckets
 constexpr uint32_t STRIP_WAIT_LIMIT = 1u << 22;   // mbarrier polls before the kernel gives up on its copies
 enum { LAY_PLANAR = 0, LAY_NC = 1, LAY_PAIRS = 2 };
 
@@ -279,13 +281,10 @@ __device__ __forceinline__ void strip_store(const SampleArgs& a, const int n, co
 }
 
 // The candidate points of all fixations are flattened into one index range so that every thread has work.
-#ifndef FOVI_STRIP_UNROLL
-#define FOVI_STRIP_UNROLL 1
-#endif
-template <typename TIn, typename TOut, int MODE, int PAD, int NCH, bool YCHECK>
+template <typename TIn, typename TOut, int MODE, int PAD, int NCH, bool YCHECK, int STRIP_THREADS>
 __device__ __forceinline__ void strip_points(const SampleArgs& a, const FixInfo* fi, const int* s_pre, const int nf, const TIn* tile,
                                              const int r0, const int nrows, const bool first, const bool last) {
-  constexpr int PU = FOVI_STRIP_UNROLL;
+  constexpr int PU = 1;
   const int total = s_pre[nf];
   const int klo = first ? INT_MIN : r0, khi = last ? INT_MAX : r0 + a.R;
   int f = 0;
@@ -314,11 +313,13 @@ __device__ __forceinline__ void strip_points(const SampleArgs& a, const FixInfo*
   }
 }
 
-template <typename TIn, typename TOut, int MODE, int PAD>
-__global__ void __launch_bounds__(STRIP_THREADS, FOVI_STRIP_MIN_CTAS) fovi_sample_strip_kernel(const SampleArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+template <typename TIn, typename TOut, int MODE, int PAD, bool WIDE>
+__global__ void __launch_bounds__(StripShape<WIDE>::THREADS, StripShape<WIDE>::MIN_CTAS)
+fovi_sample_strip_kernel(const __grid_constant__ CUtensorMap map, const SampleArgs a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  constexpr int STRIP_THREADS = StripShape<WIDE>::THREADS;
   constexpr int EPV = 16 / (int)sizeof(TIn);      // elements per 16 bytes
-  TIn* tile = reinterpret_cast<TIn*>(smem_raw) + EPV;   // [C][R+1][pitch], 16 bytes of zeros in front
+  TIn* tile = reinterpret_cast<TIn*>(smem_raw + 128);   // [C][R+1][pitch], 16 bytes of zeros in front
   __shared__ FixInfo fi[FCHUNK];
   __shared__ int s_pre[FCHUNK + 1];
   __shared__ int s_need, s_col_lo, s_col_hi;
@@ -342,7 +343,17 @@ __global__ void __launch_bounds__(STRIP_THREADS, FOVI_STRIP_MIN_CTAS) fovi_sampl
   bool loaded = false, gave_up = false;
 
   // One warp hands the strip's rows to the TMA unit, one bulk copy per (channel, row), columns [col_lo, col_hi).
+  // Images up to 2032 bytes wide: the whole tile is one tensor copy, whose columns W .. pitch - 1 and rows past the image are outside the tensor and
+  // arrive as zeros.  (Row by row the issue alone takes a warp 2000 clocks, of 13400 that a strip's CTA lives.)
   auto issue_rows = [&](int col_lo, int col_hi) {
+    if (a.use_map) {
+      if (lane == 0) {
+        s_mbar_expect_tx(bar, (uint32_t)(a.C * plane) * (uint32_t)sizeof(TIn));
+        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                     ::"r"(s_addr(tile)), "l"(&map), "r"(bar), "r"(0), "r"(r0), "r"(0), "r"(b) : "memory");
+      }
+      return;
+    }
     const uint32_t row_bytes = (uint32_t)(col_hi - col_lo) * (uint32_t)sizeof(TIn);
     const int rows = a.C * nrows;
     if (lane == 0) s_mbar_expect_tx(bar, row_bytes * (uint32_t)rows);
@@ -365,9 +376,8 @@ __global__ void __launch_bounds__(STRIP_THREADS, FOVI_STRIP_MIN_CTAS) fovi_sampl
   }
   loaded = a.full_rows != 0;
   // the zero tails (see strip_point); the copies never touch them
-  if (tid <= a.C * (a.R + 1)) {
-    int4* z = tid == 0 ? reinterpret_cast<int4*>(smem_raw)
-                       : reinterpret_cast<int4*>(tile + (tid - 1) * a.pitch + a.W);
+  for (int i = tid; i <= (a.use_map ? 0 : a.C * (a.R + 1)); i += STRIP_THREADS) {
+    int4* z = i == 0 ? reinterpret_cast<int4*>(smem_raw + 112) : reinterpret_cast<int4*>(tile + (i - 1) * a.pitch + a.W);
     *z = make_int4(0, 0, 0, 0);
   }
 
@@ -386,7 +396,7 @@ __global__ void __launch_bounds__(STRIP_THREADS, FOVI_STRIP_MIN_CTAS) fovi_sampl
     // that interval, widened by two buckets on either side (far more than the rounding of the float32 transform can
     // move a point), into a range of the y-sorted order.  Every point of the range is tested exactly later on, so the
     // range only has to be a superset.
-    const int ft = tid - (STRIP_THREADS > 32 ? 32 : 0);   // warp 1 when there is one: warp 0 is busy issuing the copies
+    const int ft = tid - 32;   // warp 1: warp 0 is busy issuing the copies
     if (ft >= 0 && ft < nf) {
       const int f = f0 + ft, bf = b * a.F + f;
       const float fr = __ldg(a.fix_rc + 2 * bf), fc = __ldg(a.fix_rc + 2 * bf + 1);
@@ -410,8 +420,8 @@ __global__ void __launch_bounds__(STRIP_THREADS, FOVI_STRIP_MIN_CTAS) fovi_sampl
         const float qlo = floorf((g_lo - a.gy_min) * a.lut_scale), qhi = floorf((g_hi - a.gy_min) * a.lut_scale);
         const int b_lo = (int)fminf(fmaxf(qlo - 2.f, 0.f), (float)RANK_LUT_Q);
         const int b_hi = (int)fminf(fmaxf(qhi + 3.f, 0.f), (float)RANK_LUT_Q);
-        if (!first) q.lo = __ldg(a.rank_lut + b_lo);
-        if (!last) q.hi = __ldg(a.rank_lut + b_hi);
+        if (!first) q.lo = __ldg(a.rank_lut + ((b_lo >> a.q_shift) << a.q_shift));       // whole buckets of the order
+        if (!last) q.hi = __ldg(a.rank_lut + min(((b_hi + (1 << a.q_shift) - 1) >> a.q_shift) << a.q_shift, RANK_LUT_Q));
       }
       if (!a.full_rows) {
         // wide images: which rows / columns of the image can this fixation touch at all?
@@ -445,10 +455,16 @@ __global__ void __launch_bounds__(STRIP_THREADS, FOVI_STRIP_MIN_CTAS) fovi_sampl
         issue_rows(col_lo, col_hi);
       }
     }
-    if (tid == 0) {
-      int acc = 0;
-      for (int f = 0; f < nf; ++f) { s_pre[f] = acc; acc += max(fi[f].hi - fi[f].lo, 0); }
-      s_pre[nf] = acc;
+    if (warp == STRIP_THREADS / 32 - 1) {   // prefix sums of the range lengths (nf <= 16); warp 0 watches the copies meanwhile
+      const int len = lane < nf ? max(fi[lane].hi - fi[lane].lo, 0) : 0;
+      int sum = len;
+#pragma unroll
+      for (int d = 1; d < 16; d <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane >= d) sum += up;
+      }
+      if (lane < nf) s_pre[lane] = sum - len;
+      if (lane == nf - 1) s_pre[nf] = sum;
     }
     if (loaded && (f0 == 0 || !a.full_rows)) {
       // one thread watches the barrier (bounded); the CTA barrier below passes what it saw on to the others
@@ -473,24 +489,24 @@ __global__ void __launch_bounds__(STRIP_THREADS, FOVI_STRIP_MIN_CTAS) fovi_sampl
 
     const bool ycheck = first || last;
     if (a.C == 3) {
-      if (ycheck) strip_points<TIn, TOut, MODE, PAD, 3, true>(a, fi, s_pre, nf, tile, r0, nrows, first, last);
-      else strip_points<TIn, TOut, MODE, PAD, 3, false>(a, fi, s_pre, nf, tile, r0, nrows, first, last);
+      if (ycheck) strip_points<TIn, TOut, MODE, PAD, 3, true, STRIP_THREADS>(a, fi, s_pre, nf, tile, r0, nrows, first, last);
+      else strip_points<TIn, TOut, MODE, PAD, 3, false, STRIP_THREADS>(a, fi, s_pre, nf, tile, r0, nrows, first, last);
     } else {
-      if (ycheck) strip_points<TIn, TOut, MODE, PAD, 0, true>(a, fi, s_pre, nf, tile, r0, nrows, first, last);
-      else strip_points<TIn, TOut, MODE, PAD, 0, false>(a, fi, s_pre, nf, tile, r0, nrows, first, last);
+      if (ycheck) strip_points<TIn, TOut, MODE, PAD, 0, true, STRIP_THREADS>(a, fi, s_pre, nf, tile, r0, nrows, first, last);
+      else strip_points<TIn, TOut, MODE, PAD, 0, false, STRIP_THREADS>(a, fi, s_pre, nf, tile, r0, nrows, first, last);
     }
   }
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// General kernel.
-// NC == false: out row is [C][N];  NC == true: out row is [N][cp] with channels >= C zeroed.
-// STAGE: stage the whole output row in shared memory before one coalesced store.
+// General kernel: any strides, any channel count, any alignment.  One thread per (image, fixation, point).  The points are visited cell by cell (8 x 8
+// cells of the grid) and ring by ring inside a cell, so that a warp's gathers share lines and its stores come in runs.  What bounds it is the latency
+// of the gathers, so the points of a row are split over as many CTAs as fill the chip (61 byte images of 375 x 500, 3 fixations, 3976 points: one CTA
+// per row, which staged the row in shared memory for whole stores, took 28 us; this takes 19).
+// NC == false: out row is [C][N];  NC == true: out row is [N][cp] with channels >= C zeroed (pair layout: see SampleArgs).
 // ------------------------------------------------------------------------------------------------------------
-template <typename TIn, typename TOut, int MODE, int PAD, bool NC, bool STAGE>
-__global__ void __launch_bounds__(256, 3) fovi_sample_kernel(const SampleArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  TOut* stage = reinterpret_cast<TOut*>(smem_raw);
+template <typename TIn, typename TOut, int MODE, int PAD, bool NC>
+__global__ void __launch_bounds__(256) fovi_sample_kernel(const SampleArgs a, const int per_cta) {
   // Programmatic dependent launch: once every CTA of this grid has started, a following kernel launched with the
   // programmatic-serialization attribute (the first KNNConv) may be scheduled onto SMs as they free up and run its
   // prologue; it still waits for this grid's completion before it reads the output.  A no-op otherwise.
@@ -499,11 +515,9 @@ __global__ void __launch_bounds__(256, 3) fovi_sample_kernel(const SampleArgs a)
   const int bf = blockIdx.x;  // b*F + f
   const int b = bf / a.F, f = bf - b * a.F;
   const long long row = a.f_major ? ((long long)f * a.B + b) : (long long)bf;
-  const int row_elems = NC ? (a.pairs ? ((a.N + 1) / 2) * 8 : a.N * a.cp) : a.C * a.N;
   // pair layout: rows are tiled by 128; this row's 16-byte slot of pair p sits at ((tile*n_pairs + p)*128 + r)*8
   TOut* out_row = reinterpret_cast<TOut*>(a.out) +
-                  (a.pairs ? ((row >> 7) * (long long)((a.N + 1) / 2) * 128 + (row & 127)) * 8 : row * row_elems);
-  TOut* dst = STAGE ? stage : out_row;
+                  (a.pairs ? ((row >> 7) * (long long)((a.N + 1) / 2) * 128 + (row & 127)) * 8 : row * (long long)(NC ? a.N * a.cp : a.C * a.N));
 
   const float fr = __ldg(a.fix_rc + 2 * bf), fc = __ldg(a.fix_rc + 2 * bf + 1);
   const float fh = __ldg(a.fix_hw + 2 * bf), fw = __ldg(a.fix_hw + 2 * bf + 1);
@@ -513,73 +527,61 @@ __global__ void __launch_bounds__(256, 3) fovi_sample_kernel(const SampleArgs a)
   const float sxw = Wf * 0.5f, syh = Hf * 0.5f;  // exact
   const float inv_w = 1.f / Wf, inv_h = 1.f / Hf; // exact when a.pow2 (the only case they are used in)
   const TIn* img_b = reinterpret_cast<const TIn*>(a.img) + (long long)b * a.sb;
-  const int pitch = a.pairs ? 4 : a.cp;  // per-point element pitch of the points-major layouts
 
-  if (NC && STAGE) {  // zero the pad channels once
-    for (int i = threadIdx.x; i < row_elems; i += blockDim.x) stage[i] = from_float<TOut>(0.f);
-    __syncthreads();
-  }
-
+  const int n_end = min(a.N, (int)(blockIdx.y + 1) * per_cta);
 #pragma unroll 2
-  for (int i = threadIdx.x; i < a.N; i += blockDim.x) {
-    const float2 g = __ldg(a.sorted_xy + i);
-    const int n = __ldg(a.sorted_idx + i);
+  for (int i = blockIdx.y * per_cta + threadIdx.x; i < n_end; i += blockDim.x) {
+    const float4 pt = __ldg(reinterpret_cast<const float4*>(a.cells + i));
+    const float2 g = make_float2(pt.x, pt.y);
+    const int n = __float_as_int(pt.z);
+    // the point's first channel and the distance to its next one
+    TOut* dst = out_row + (a.pairs ? (long long)(n >> 1) * 1024 + (n & 1) * 4 : NC ? (long long)n * a.cp : (long long)n);
+    const long long dc = NC ? 1 : a.N;
     float ix = grid_to_pixel(g.x, half_w, cx, Wf, inv_w, sxw, a.pow2);
     float iy = grid_to_pixel(g.y, half_h, cy, Hf, inv_h, syh, a.pow2);
     if (PAD == FOVI_PAD_BORDER) {
       ix = fminf(fmaxf(ix, 0.f), Wf - 1.f);
       iy = fminf(fmaxf(iy, 0.f), Hf - 1.f);
     }
+    float w_nw = 0.f, w_ne = 0.f, w_sw = 0.f, w_se = 0.f;
+    int x0, y0;
     if (MODE == FOVI_NEAREST) {
-      const int x = (int)rintf(ix), y = (int)rintf(iy);
-      for (int c = 0; c < a.C; ++c) {
-        const float v = tap<TIn, PAD>(img_b + c * a.sc, a.sy, a.sx, x, y, a.W, a.H);
-        dst[NC ? (n * pitch + c) : (c * a.N + n)] = from_float<TOut>(v);
-      }
+      x0 = (int)rintf(ix); y0 = (int)rintf(iy);
     } else {
       const float x0f = floorf(ix), y0f = floorf(iy);
       const float tx = __fsub_rn(ix, x0f), ty = __fsub_rn(iy, y0f);
       const float ux = __fsub_rn(1.f, tx), uy = __fsub_rn(1.f, ty);
-      const float w_nw = __fmul_rn(uy, ux), w_ne = __fmul_rn(uy, tx);
-      const float w_sw = __fmul_rn(ty, ux), w_se = __fmul_rn(ty, tx);
-      const int x0 = (int)x0f, y0 = (int)y0f;
-#pragma unroll 3
-      for (int c = 0; c < a.C; ++c) {
-        const TIn* plane = img_b + c * a.sc;
-        const float v_nw = tap<TIn, PAD>(plane, a.sy, a.sx, x0, y0, a.W, a.H);
-        const float v_ne = tap<TIn, PAD>(plane, a.sy, a.sx, x0 + 1, y0, a.W, a.H);
-        const float v_sw = tap<TIn, PAD>(plane, a.sy, a.sx, x0, y0 + 1, a.W, a.H);
-        const float v_se = tap<TIn, PAD>(plane, a.sy, a.sx, x0 + 1, y0 + 1, a.W, a.H);
-        float acc = __fmul_rn(v_nw, w_nw);
-        acc = __fmaf_rn(v_ne, w_ne, acc);
-        acc = __fmaf_rn(v_sw, w_sw, acc);
-        acc = __fmaf_rn(v_se, w_se, acc);
-        dst[NC ? (n * pitch + c) : (c * a.N + n)] = from_float<TOut>(acc);
-      }
+      w_nw = __fmul_rn(uy, ux); w_ne = __fmul_rn(uy, tx);
+      w_sw = __fmul_rn(ty, ux); w_se = __fmul_rn(ty, tx);
+      x0 = (int)x0f; y0 = (int)y0f;
     }
-    if (NC && !STAGE) {
-      for (int c = a.C; c < pitch; ++c) dst[n * pitch + c] = from_float<TOut>(0.f);
-    }
-  }
-
-  if (STAGE && NC && a.pairs) {
-    // pair layout: this row owns one 16-byte slot in each pair's 128-row block of its row tile
-    __syncthreads();
-    const long long rows = 128;
-    const int4* s4 = reinterpret_cast<const int4*>(stage);
-    int4* d4 = reinterpret_cast<int4*>(out_row);
-    const int n_pairs = (a.N + 1) / 2;
-    for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) d4[(long long)i * rows] = s4[i];
-  } else if (STAGE) {
-    __syncthreads();
-    const size_t bytes = (size_t)row_elems * sizeof(TOut);
-    const bool vec = ((reinterpret_cast<uintptr_t>(out_row) & 15) == 0) && (bytes % 16 == 0);
-    if (vec) {
-      const int4* s4 = reinterpret_cast<const int4*>(stage);
-      int4* d4 = reinterpret_cast<int4*>(out_row);
-      for (int i = threadIdx.x; i < (int)(bytes / 16); i += blockDim.x) d4[i] = s4[i];
+    auto value = [&](int c) {
+      const TIn* plane = img_b + c * a.sc;
+      if (MODE == FOVI_NEAREST) return tap<TIn, PAD>(plane, a.sy, a.sx, x0, y0, a.W, a.H);
+      const float v_nw = tap<TIn, PAD>(plane, a.sy, a.sx, x0, y0, a.W, a.H);
+      const float v_ne = tap<TIn, PAD>(plane, a.sy, a.sx, x0 + 1, y0, a.W, a.H);
+      const float v_sw = tap<TIn, PAD>(plane, a.sy, a.sx, x0, y0 + 1, a.W, a.H);
+      const float v_se = tap<TIn, PAD>(plane, a.sy, a.sx, x0 + 1, y0 + 1, a.W, a.H);
+      float acc = __fmul_rn(v_nw, w_nw);
+      acc = __fmaf_rn(v_ne, w_ne, acc);
+      acc = __fmaf_rn(v_sw, w_sw, acc);
+      return __fmaf_rn(v_se, w_se, acc);
+    };
+    if (NC && a.pairs) {              // at most four channels: one 8-byte store per point
+      float v[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) v[c] = c < a.C ? value(c) : 0.f;
+      __nv_bfloat162 h01 = __floats2bfloat162_rn(v[0], v[1]), h23 = __floats2bfloat162_rn(v[2], v[3]);
+      uint2 w;
+      w.x = *reinterpret_cast<uint32_t*>(&h01); w.y = *reinterpret_cast<uint32_t*>(&h23);
+      uint2* d = reinterpret_cast<uint2*>(dst);
+      *d = w;
+      if ((a.N & 1) && n == a.N - 1) d[1] = make_uint2(0u, 0u);   // the odd last point's empty partner
     } else {
-      for (int i = threadIdx.x; i < row_elems; i += blockDim.x) out_row[i] = stage[i];
+#pragma unroll 3
+      for (int c = 0; c < a.C; ++c) dst[c * dc] = from_float<TOut>(value(c));
+      if (NC)
+        for (int c = a.C; c < a.cp; ++c) dst[c] = from_float<TOut>(0.f);   // pad channels
     }
   }
 }
@@ -600,7 +602,7 @@ __global__ void __launch_bounds__(256) fovi_sample_backward_kernel(const SampleA
     const int b = bf / a.F, f = bf - b * a.F;
     const float fr = __ldg(a.fix_rc + 2 * bf), fc = __ldg(a.fix_rc + 2 * bf + 1);
     const float fh = __ldg(a.fix_hw + 2 * bf), fw = __ldg(a.fix_hw + 2 * bf + 1);
-    const float2 g = __ldg(a.sorted_xy + n);      // here: the grid in its ORIGINAL order
+    const float2 g = __ldg(a.grid_xy + n);
     float ix = grid_to_pixel(g.x, __fdiv_rn(fw, 2.f), __fmul_rn(fc, Wf), Wf, inv_w, sxw, a.pow2);
     float iy = grid_to_pixel(g.y, __fdiv_rn(fh, 2.f), __fmul_rn(fr, Hf), Hf, inv_h, syh, a.pow2);
     if (PAD == FOVI_PAD_BORDER) {
@@ -633,8 +635,8 @@ __global__ void __launch_bounds__(256) fovi_sample_backward_kernel(const SampleA
   }
 }
 
-// Does the strip kernel apply?  Fills R, n_strips, pitch.
-template <typename TIn>
+// Does the strip kernel apply in this shape?  Fills R, n_strips, pitch and the visiting order.
+template <typename TIn, bool WIDE>
 bool plan_strips(SampleArgs& a, bool nc) {
   constexpr int EPV = 16 / (int)sizeof(TIn);
   if (a.C > 4 || a.sx != 1 || !a.ys) return false;
@@ -642,42 +644,85 @@ bool plan_strips(SampleArgs& a, bool nc) {
   if ((a.W % EPV) || (a.sy % EPV) || (a.sc % EPV) || (a.sb % EPV) || (reinterpret_cast<uintptr_t>(a.img) & 15)) return false;
   a.pitch = a.W + EPV;   // one 16-byte piece of padding: vertically adjacent pixels fall in different banks
   const long long row_bytes = (long long)a.C * a.pitch * sizeof(TIn);
-  const int rows_fit = (int)std::min<long long>((FOVI_STRIP_SMEM_BUDGET - 16) / row_bytes, 1 << 20);
-  a.R = std::min(std::min(rows_fit - 1, FOVI_STRIP_ROWS_MAX), a.H);
+  const int rows_fit = (int)std::min<long long>((StripShape<WIDE>::SMEM - 128) / row_bytes, 1 << 20);
+  a.R = std::min(std::min(rows_fit - 1, StripShape<WIDE>::ROWS_MAX), a.H);
   if (a.R < 4) return false;   // very wide rows: the extra row per strip would dominate
   a.n_strips = (a.H + a.R - 1) / a.R;
   a.full_rows = (size_t)a.W * sizeof(TIn) <= 4096 ? 1 : 0;
+  // coarsest order whose buckets, on an image sampled at its own height, are at most 0.6 strips high
+  int order = 0;
+  for (int i = 1; WIDE && i < N_ORDERS; ++i) {
+    const float rows = (a.gy_max - a.gy_min) * 0.5f * (float)a.H * (float)(1 << ORDER_SHIFT[i]) / (float)RANK_LUT_Q;
+    if (rows <= 0.6f * (float)a.R) order = i;
+  }
+  a.ys += (size_t)order * a.N;
+  if (a.rank_lut) a.rank_lut += (size_t)order * (RANK_LUT_Q + 1);
+  a.q_shift = ORDER_SHIFT[order];
   return (long long)a.B * a.n_strips < (1ll << 31);
 }
 
+// The image batch as a tensor of 8-byte elements (x, y, channel, image); false where a tensor copy cannot take it (then rows are copied one by one).
+bool encode_image_map(CUtensorMap* m, const SampleArgs& a, size_t esz) {
+  typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                               const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const EncodeFn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
+               ? reinterpret_cast<EncodeFn>(p) : nullptr;
+  }();
+  const size_t row = (size_t)a.W * esz;
+  const long long limit = 1ll << 40;
+  if (!fn || row > 2032 || a.R + 1 > 256 || a.sy <= 0 || a.sc <= 0 || a.sb <= 0 || a.sy * (long long)esz >= limit || a.sc * (long long)esz >= limit ||
+      a.sb * (long long)esz >= limit)
+    return false;
+  const cuuint64_t dims[4] = {row / 8, (cuuint64_t)a.H, (cuuint64_t)a.C, (cuuint64_t)a.B};
+  const cuuint64_t strides[3] = {(cuuint64_t)a.sy * esz, (cuuint64_t)a.sc * esz, (cuuint64_t)a.sb * esz};
+  const cuuint32_t box[4] = {(cuuint32_t)((row + 16) / 8), (cuuint32_t)(a.R + 1), (cuuint32_t)a.C, 1}, estr[4] = {1, 1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, const_cast<void*>(a.img), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <typename TIn, typename TOut, int MODE, int PAD, bool WIDE>
+int launch_strips(SampleArgs& a, int layout, cudaStream_t st) {
+  const size_t smem = 128 + (size_t)a.C * (a.R + 1) * a.pitch * sizeof(TIn);
+  const dim3 grid(a.n_strips, std::min(a.B, 65535), (a.B + 65534) / 65535);   // strips of one image are neighbours
+  a.layout = layout;
+  CUtensorMap map;
+  memset(&map, 0, sizeof(map));
+  // (a call of a few strips is bound by the host, where making the map costs 2 us)
+  a.use_map = (long long)a.B * a.n_strips >= 8ll * fovi::sm_count() && encode_image_map(&map, a, sizeof(TIn)) ? 1 : 0;
+  auto k = fovi_sample_strip_kernel<TIn, TOut, MODE, PAD, WIDE>;
+  if (smem > 48 * 1024) FOVI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k<<<grid, StripShape<WIDE>::THREADS, smem, st>>>(map, a);
+  return fovi::after_launch("fovi_sample_strip_kernel");
+}
+
 template <typename TIn, typename TOut, int MODE, int PAD, bool NC>
-int launch_sample(SampleArgs a, size_t stage_bytes, cudaStream_t st) {
-  if (plan_strips<TIn>(a, NC) && (!a.pairs || std::is_same<TOut, __nv_bfloat16>::value)) {
-    const size_t smem = 16 + (size_t)a.C * (a.R + 1) * a.pitch * sizeof(TIn);
-    const dim3 grid(a.n_strips, std::min(a.B, 65535), (a.B + 65534) / 65535);   // strips of one image are neighbours
-    a.layout = a.pairs ? LAY_PAIRS : (NC ? LAY_NC : LAY_PLANAR);
-    auto k = fovi_sample_strip_kernel<TIn, TOut, MODE, PAD>;
-    FOVI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<grid, STRIP_THREADS, smem, st>>>(a);
-    return fovi::after_launch("fovi_sample_strip_kernel");
+int launch_sample(SampleArgs a, cudaStream_t st) {
+  if (!a.pairs || std::is_same<TOut, __nv_bfloat16>::value) {
+    if (!NC) {   // WIDE only where its strips still fill every SM's three places three times over
+      SampleArgs w = a;
+      if (plan_strips<TIn, true>(w, NC) && w.q_shift > 0 && (long long)w.B * w.n_strips >= 9ll * fovi::sm_count())
+        return launch_strips<TIn, TOut, MODE, PAD, true>(w, LAY_PLANAR, st);
+    }
+    SampleArgs n = a;
+    if (plan_strips<TIn, false>(n, NC)) return launch_strips<TIn, TOut, MODE, PAD, false>(n, n.pairs ? LAY_PAIRS : (NC ? LAY_NC : LAY_PLANAR), st);
   }
-  const int grid = a.B * a.F;
-  if (stage_bytes <= 200 * 1024) {
-    auto k = fovi_sample_kernel<TIn, TOut, MODE, PAD, NC, true>;
-    if (stage_bytes > 48 * 1024) FOVI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_bytes));
-    k<<<grid, 256, stage_bytes, st>>>(a);
-  } else {
-    if (a.pairs) return FOVI_ERR_UNSUPPORTED;  // the pair layout is only written from the staged row
-    fovi_sample_kernel<TIn, TOut, MODE, PAD, NC, false><<<grid, 256, 0, st>>>(a);
-  }
+  // points per CTA: few enough that small calls give every SM eight CTAs, at most eight per thread
+  const long long rows = (long long)a.B * a.F;
+  if (rows >= (1ll << 31)) return FOVI_ERR_UNSUPPORTED;
+  const long long share = rows * a.N / (256ll * 8 * fovi::sm_count());
+  const int per_cta = 256 * (int)std::max(1ll, std::min(8ll, share));
+  const dim3 grid((unsigned)rows, (a.N + per_cta - 1) / per_cta);
+  if (grid.y > 65535) return FOVI_ERR_UNSUPPORTED;
+  fovi_sample_kernel<TIn, TOut, MODE, PAD, NC><<<grid, 256, 0, st>>>(a, per_cta);
   return fovi::after_launch("fovi_sample_kernel");
 }
 
 template <typename TIn, typename TOut, int MODE, int PAD>
 int dispatch_layout(const SampleArgs& a, bool nc, cudaStream_t st) {
-  const size_t stage_bytes = (size_t)(nc ? (a.pairs ? ((a.N + 1) / 2) * 8 : a.N * a.cp) : a.C * a.N) * sizeof(TOut);
-  return nc ? launch_sample<TIn, TOut, MODE, PAD, true>(a, stage_bytes, st)
-            : launch_sample<TIn, TOut, MODE, PAD, false>(a, stage_bytes, st);
+  return nc ? launch_sample<TIn, TOut, MODE, PAD, true>(a, st) : launch_sample<TIn, TOut, MODE, PAD, false>(a, st);
 }
 
 template <typename TIn, typename TOut>
@@ -689,48 +734,10 @@ int dispatch_mode(const SampleArgs& a, int mode, int pad, bool nc, cudaStream_t 
                                : dispatch_layout<TIn, TOut, FOVI_BILINEAR, FOVI_PAD_BORDER>(a, nc, st);
 }
 
-// Interleave the low 16 bits of x and y (Morton / Z-order key).
-uint32_t morton16(uint32_t x, uint32_t y) {
-  auto spread = [](uint32_t v) {
-    v &= 0xFFFF;
-    v = (v | (v << 8)) & 0x00FF00FF;
-    v = (v | (v << 4)) & 0x0F0F0F0F;
-    v = (v | (v << 2)) & 0x33333333;
-    v = (v | (v << 1)) & 0x55555555;
-    return v;
-  };
-  return spread(x) | (spread(y) << 1);
-}
-
 }  // namespace
 
 extern "C" int fovi_sampler_plan_create(const float* grid_xy, int n_points, fovi_sampler_plan** out) {
   if (!grid_xy || !out || n_points <= 0) return FOVI_ERR_INVALID_ARGUMENT;
-  std::vector<std::pair<uint32_t, int>> keys(n_points);
-  for (int i = 0; i < n_points; ++i) {
-    // Quantise [-1.5, 1.5] to 12 bits per axis; the fixation transform is a positive-scale
-    // affine map, so spatial order on the sensor grid is spatial order in the image.
-    auto q = [](float v) {
-      float t = (std::min(std::max(v, -1.5f), 1.5f) + 1.5f) * (4095.f / 3.f);
-      return (uint32_t)t;
-    };
-    keys[i] = {morton16(q(grid_xy[2 * i]), q(grid_xy[2 * i + 1])), i};
-  }
-  std::stable_sort(keys.begin(), keys.end());
-  std::vector<float2> xy(n_points);
-  std::vector<YPoint> ypts(n_points);
-  std::vector<int> idx(n_points), yidx(n_points);
-  for (int i = 0; i < n_points; ++i) {
-    idx[i] = keys[i].second;
-    xy[i] = make_float2(grid_xy[2 * idx[i]], grid_xy[2 * idx[i] + 1]);
-  }
-  // second order: by grid y (ties by x, then index), for the strip kernel's range search
-  for (int i = 0; i < n_points; ++i) yidx[i] = i;
-  std::stable_sort(yidx.begin(), yidx.end(), [&](int p, int q) {
-    const float yp = grid_xy[2 * p + 1], yq = grid_xy[2 * q + 1];
-    if (yp != yq) return yp < yq;
-    return grid_xy[2 * p] < grid_xy[2 * q];
-  });
   auto* p = new fovi_sampler_plan();
   p->n_points = n_points;
   p->gx_min = p->gx_max = grid_xy[0];
@@ -738,37 +745,55 @@ extern "C" int fovi_sampler_plan_create(const float* grid_xy, int n_points, fovi
   bool finite = true;
   for (int i = 0; i < n_points; ++i) {
     const float x = grid_xy[2 * i], y = grid_xy[2 * i + 1];
-    ypts[i] = YPoint{grid_xy[2 * yidx[i]], grid_xy[2 * yidx[i] + 1], yidx[i], 0};
     finite = finite && (x - x == 0.f) && (y - y == 0.f);
     p->gx_min = std::min(p->gx_min, x); p->gx_max = std::max(p->gx_max, x);
     p->gy_min = std::min(p->gy_min, y); p->gy_max = std::max(p->gy_max, y);
   }
   cudaError_t e = cudaGetDevice(&p->device);
-  if (e == cudaSuccess) e = cudaMalloc(&p->sorted_xy, sizeof(float2) * n_points);
-  if (e == cudaSuccess) e = cudaMalloc(&p->sorted_idx, sizeof(int) * n_points);
-  if (e == cudaSuccess) e = cudaMemcpy(p->sorted_xy, xy.data(), sizeof(float2) * n_points, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(p->sorted_idx, idx.data(), sizeof(int) * n_points, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(&p->grid_xy, sizeof(float2) * n_points);
   if (e == cudaSuccess) e = cudaMemcpy(p->grid_xy, grid_xy, sizeof(float2) * n_points, cudaMemcpyHostToDevice);
+  {
+    // cells of the grid's bounding box; coordinates that are not numbers go to cell 0 (the order is a permutation all the same)
+    auto cell_of = [](float v, float lo, float hi) {
+      const float t = (v - lo) / (hi - lo) * 8.f;
+      return t == t ? (int)std::min(std::max(t, 0.f), 7.f) : 0;
+    };
+    std::vector<int> cell(n_points), order(n_points);
+    std::vector<YPoint> pts(n_points);
+    for (int i = 0; i < n_points; ++i) {
+      cell[i] = cell_of(grid_xy[2 * i + 1], p->gy_min, p->gy_max) * 8 + cell_of(grid_xy[2 * i], p->gx_min, p->gx_max);
+      order[i] = i;
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int u, int v) { return cell[u] < cell[v]; });
+    for (int i = 0; i < n_points; ++i) pts[i] = YPoint{grid_xy[2 * order[i]], grid_xy[2 * order[i] + 1], order[i], 0};
+    if (e == cudaSuccess) e = cudaMalloc(&p->cells, sizeof(YPoint) * n_points);
+    if (e == cudaSuccess) e = cudaMemcpy(p->cells, pts.data(), sizeof(YPoint) * n_points, cudaMemcpyHostToDevice);
+  }
   if (e == cudaSuccess) e = cudaMalloc(&p->status, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(p->status, 0, sizeof(int));
-  if (e == cudaSuccess && finite) {
-    // rank table: lut[q] = number of points whose bucket floor((gy - gy_min) * scale) is below q
+  if (e == cudaSuccess && finite) {   // a grid with NaN / Inf entries has no y order: the general kernel serves it
     const float span = p->gy_max - p->gy_min;
     p->lut_scale = span > 0.f ? (float)RANK_LUT_Q / span : 0.f;
-    std::vector<int> lut(RANK_LUT_Q + 1, 0);
+    std::vector<int> bucket(n_points), yidx(n_points);
     for (int i = 0; i < n_points; ++i) {
       const float t = floorf((grid_xy[2 * i + 1] - p->gy_min) * p->lut_scale);
-      const int q = (int)std::min(std::max(t, 0.f), (float)(RANK_LUT_Q - 1));
-      lut[q + 1] += 1;
+      bucket[i] = (int)std::min(std::max(t, 0.f), (float)(RANK_LUT_Q - 1));
     }
+    // rank table: lut[q] = number of points whose bucket floor((gy - gy_min) * scale) is below q; the same for every order at its bucket edges
+    std::vector<int> lut(RANK_LUT_Q + 1, 0), luts;
+    for (int i = 0; i < n_points; ++i) lut[bucket[i] + 1] += 1;
     for (int q = 0; q < RANK_LUT_Q; ++q) lut[q + 1] += lut[q];
-    e = cudaMalloc(&p->rank_lut, sizeof(int) * lut.size());
-    if (e == cudaSuccess) e = cudaMemcpy(p->rank_lut, lut.data(), sizeof(int) * lut.size(), cudaMemcpyHostToDevice);
-  }
-  if (e == cudaSuccess && finite) {   // a grid with NaN / Inf entries has no y order: the general kernel serves it
-    e = cudaMalloc(&p->ys, sizeof(YPoint) * n_points);
-    if (e == cudaSuccess) e = cudaMemcpy(p->ys, ypts.data(), sizeof(YPoint) * n_points, cudaMemcpyHostToDevice);
+    std::vector<YPoint> ypts;
+    for (int o = 0; o < N_ORDERS; ++o) {
+      for (int i = 0; i < n_points; ++i) yidx[i] = i;
+      std::stable_sort(yidx.begin(), yidx.end(), [&](int u, int v) { return (bucket[u] >> ORDER_SHIFT[o]) < (bucket[v] >> ORDER_SHIFT[o]); });
+      for (int i = 0; i < n_points; ++i) ypts.push_back(YPoint{grid_xy[2 * yidx[i]], grid_xy[2 * yidx[i] + 1], yidx[i], 0});
+      luts.insert(luts.end(), lut.begin(), lut.end());
+    }
+    e = cudaMalloc(&p->rank_lut, sizeof(int) * luts.size());
+    if (e == cudaSuccess) e = cudaMemcpy(p->rank_lut, luts.data(), sizeof(int) * luts.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&p->ys, sizeof(YPoint) * ypts.size());
+    if (e == cudaSuccess) e = cudaMemcpy(p->ys, ypts.data(), sizeof(YPoint) * ypts.size(), cudaMemcpyHostToDevice);
   }
   if (e != cudaSuccess) {
     fovi_sampler_plan_destroy(p);
@@ -780,10 +805,9 @@ extern "C" int fovi_sampler_plan_create(const float* grid_xy, int n_points, fovi
 
 extern "C" void fovi_sampler_plan_destroy(fovi_sampler_plan* plan) {
   if (!plan) return;
-  if (plan->sorted_xy) cudaFree(plan->sorted_xy);
-  if (plan->sorted_idx) cudaFree(plan->sorted_idx);
   if (plan->ys) cudaFree(plan->ys);
   if (plan->grid_xy) cudaFree(plan->grid_xy);
+  if (plan->cells) cudaFree(plan->cells);
   if (plan->rank_lut) cudaFree(plan->rank_lut);
   if (plan->status) cudaFree(plan->status);
   delete plan;
@@ -811,7 +835,8 @@ extern "C" int fovi_sample_forward(const fovi_sampler_plan* plan, const void* im
     return FOVI_ERR_UNSUPPORTED;
   if (B == 0) return FOVI_OK;
   SampleArgs a;
-  a.img = img; a.out = out; a.sorted_xy = plan->sorted_xy; a.sorted_idx = plan->sorted_idx;
+  memset(&a, 0, sizeof(a));
+  a.img = img; a.out = out; a.cells = static_cast<const YPoint*>(plan->cells);
   a.fix_rc = fix_rc; a.fix_hw = fix_hw;
   a.sb = img_strides[0]; a.sc = img_strides[1]; a.sy = img_strides[2]; a.sx = img_strides[3];
   a.B = B; a.C = C; a.H = H; a.W = W; a.F = F; a.N = plan->n_points;
@@ -821,7 +846,7 @@ extern "C" int fovi_sample_forward(const fovi_sampler_plan* plan, const void* im
   a.pow2 = ((W & (W - 1)) == 0 && (H & (H - 1)) == 0) ? 1 : 0;
   a.ys = static_cast<const YPoint*>(plan->ys);
   a.gx_min = plan->gx_min; a.gx_max = plan->gx_max; a.gy_min = plan->gy_min; a.gy_max = plan->gy_max;
-  a.R = a.n_strips = a.pitch = a.layout = a.full_rows = 0;
+  a.R = a.n_strips = a.pitch = a.layout = a.full_rows = a.q_shift = a.use_map = 0;
   a.rank_lut = plan->rank_lut; a.lut_scale = plan->lut_scale; a.status = plan->status;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (dtype == FOVI_U8 && out_dtype == FOVI_F32) return dispatch_mode<unsigned char, float>(a, mode, pad, nc, st);
@@ -858,7 +883,7 @@ extern "C" int fovi_sample_backward(const fovi_sampler_plan* plan, const void* g
   if (!grad_out || !fix_rc || !fix_hw || !grad_img || !plan->grid_xy) return FOVI_ERR_INVALID_ARGUMENT;
   SampleArgs a;
   memset(&a, 0, sizeof(a));
-  a.sorted_xy = plan->grid_xy; a.fix_rc = fix_rc; a.fix_hw = fix_hw;
+  a.grid_xy = plan->grid_xy; a.fix_rc = fix_rc; a.fix_hw = fix_hw;
   a.B = B; a.C = C; a.H = H; a.W = W; a.F = F; a.N = plan->n_points;
   a.f_major = layout == FOVI_OUT_FBCN ? 1 : 0;
   a.pow2 = ((W & (W - 1)) == 0 && (H & (H - 1)) == 0) ? 1 : 0;
