@@ -36,8 +36,6 @@ SIGNATURES = {
     "fovi_knnconv_packed_weight_bytes": (C.c_int64, [_P, C.c_int]),
     "fovi_pack_points": (C.c_int, [_P, C.c_int, C.c_int, C.c_int, C.c_int, _P, C.c_int, C.c_int, _P]),
     "fovi_knnconv_forward": (C.c_int, [_P, _P, _P, _P, _P, C.c_int, C.c_int, C.c_int, _P]),
-    "fovi_knnconv_workspace_bytes": (C.c_int64, [_P, C.c_int]),
-    "fovi_knnconv_forward_ws": (C.c_int, [_P, _P, _P, _P, _P, C.c_int, C.c_int, C.c_int, _P, C.c_int64, _P]),
     "fovi_knnconv_forward_f32": (C.c_int, [_P, _P, C.c_int, C.c_int, _P, _P, _P, C.c_int, C.c_int, C.c_int, _P]),
     "fovi_knnconv_forward_scatter_add": (C.c_int, [_P, _P, _P, _P, C.c_int, _P, C.c_int, _P]),
     "fovi_knnconv_selftest_wait_timeout": (C.c_int, [_P, _P, _P, _P, C.c_int, C.c_int, _P]),

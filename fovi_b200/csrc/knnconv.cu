@@ -546,11 +546,6 @@ extern "C" int fovi_knnconv_plan_create(const int32_t* knn_idx_pad, const uint16
     fovi_knnconv_plan_destroy(p);
     return fovi::cuda_fail(e, "fovi_knnconv_plan_create");
   }
-  const int rc = fovi::build_small_tables(p, idx, tp, cnt);
-  if (rc) {
-    fovi_knnconv_plan_destroy(p);
-    return rc;
-  }
   *out = p;
   return FOVI_OK;
 }
@@ -567,11 +562,6 @@ extern "C" void fovi_knnconv_plan_destroy(fovi_knnconv_plan* p) {
   if (p->zero_block) cudaFree(p->zero_block);
   if (p->pair_run) cudaFree(p->pair_run);
   if (p->pair_box) cudaFree(p->pair_box);
-  for (auto& t : p->small) {
-    if (t.tap) cudaFree(t.tap);
-    if (t.idx) cudaFree(t.idx);
-    if (t.cnt) cudaFree(t.cnt);
-  }
   delete p;
 }
 

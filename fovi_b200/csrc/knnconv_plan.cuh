@@ -1,7 +1,5 @@
 // Plan object shared by the KNNConv translation units.
 #pragma once
-#include <vector>
-
 #include "common.cuh"
 
 namespace fovi {
@@ -38,13 +36,6 @@ struct fovi_knnconv_plan {
   uint16_t* pair_run = nullptr; // [n_out, sp] at the first slot of a run of consecutive pairs inside an 8-slot stage: the run's length; else 0
   uint16_t* pair_box = nullptr; // [n_out, sp] the same runs cut into 8, 4, 2 and 1 pairs: 1 + log2(size) at the first slot of a piece; else 0
   void* zero_block = nullptr;   // 16 KB of zeros: the operand blocks read for unused pair slots
-  // Small-batch kernel (knnconv_small.cu): entries of groups of 32 and 16 consecutive output points.
-  struct SmallTables { int n_groups = 0, u_max = 0; uint16_t* tap = nullptr; int* idx = nullptr; int* cnt = nullptr; } small[2];
-  int small_ok = 0;
   int bias_period = 0;          // channel o reads bias[o % bias_period] (c_out, or a member's channels in a grouped plan)
   int ct = 0;                   // c_out tile of the tensor-core path (UMMA N), 0 = unsupported c_out
 };
-
-namespace fovi {
-int build_small_tables(fovi_knnconv_plan* p, const std::vector<int>& idx, const std::vector<uint16_t>& tap, const std::vector<int>& cnt);
-}  // namespace fovi

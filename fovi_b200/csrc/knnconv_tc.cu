@@ -490,7 +490,7 @@ int fovi::encode_4d(CUtensorMap* m, const void* ptr, const uint64_t (&dims)[4], 
 }
 
 static int knnconv_forward_impl(fovi_knnconv_plan* p, const void* X, const void* Wt, const float* bias, void* Y, int y_dtype, int B,
-                                int relu, void* stream, int skip_loads, uint32_t wait_limit, const OutMode& om = OutMode(), void* ws = nullptr, int64_t ws_bytes = 0) {
+                                int relu, void* stream, int skip_loads, uint32_t wait_limit, const OutMode& om = OutMode()) {
   if (!p || B < 0 || !fovi::valid_dtype(y_dtype)) return FOVI_ERR_INVALID_ARGUMENT;
   if (B == 0) return FOVI_OK;  // an empty batch has no buffers to look at
   if (!X || !Wt || !Y) return FOVI_ERR_INVALID_ARGUMENT;
@@ -510,11 +510,6 @@ static int knnconv_forward_impl(fovi_knnconv_plan* p, const void* X, const void*
     if (rc2 != FOVI_ERR_UNSUPPORTED) return rc2;
   }
 
-  // 64-channel layers of a few rows: several output points per tile.
-  if (c64 && !FOVI_TC_SINGLE_CTA_ONLY && !om.out_map) {
-    const int rc2 = fovi::launch_knnconv_small(p, X, Wt, bias, Y, y_dtype, B, relu, ws, ws_bytes, reinterpret_cast<cudaStream_t>(stream), skip_loads, wait_limit);
-    if (rc2 != FOVI_ERR_UNSUPPORTED) return rc2;
-  }
   const bool pairs = p->x_layout == FOVI_X_PAIRS;
   // The pair layout with more than one batch tile: CTA pairs (knnconv_tcp.cu).
   if (pairs && !FOVI_TC_SINGLE_CTA_ONLY && B > BM && !om.out_map) {
@@ -586,11 +581,6 @@ static int knnconv_forward_impl(fovi_knnconv_plan* p, const void* X, const void*
 extern "C" int fovi_knnconv_forward(fovi_knnconv_plan* p, const void* X, const void* Wt, const float* bias, void* Y,
                                     int y_dtype, int B, int relu, void* stream) {
   return knnconv_forward_impl(p, X, Wt, bias, Y, y_dtype, B, relu, stream, 0, WAIT_LIMIT);
-}
-
-extern "C" int fovi_knnconv_forward_ws(fovi_knnconv_plan* p, const void* X, const void* Wt, const float* bias, void* Y, int y_dtype, int B, int relu,
-                                       void* workspace, int64_t workspace_bytes, void* stream) {
-  return knnconv_forward_impl(p, X, Wt, bias, Y, y_dtype, B, relu, stream, 0, WAIT_LIMIT, OutMode(), workspace, workspace_bytes);
 }
 
 extern "C" int fovi_knnconv_forward_scatter_add(fovi_knnconv_plan* p, const void* X, const void* Wt, float* Y, int B, const int* out_map,

@@ -300,12 +300,6 @@ class KnnConvPlan:
         if out is None:
             out = torch.empty((B, self.n_out, self.c_out), dtype=out_dtype, device=x_bnc.device)
         with _on(x_bnc.device):   # a grouped plan writes [B, n_out/G, G*c_out]: the same memory
-            if B <= 16 and self.x_layout != X_PAIRS:        # a few rows: the small-batch kernel wants a workspace (0 bytes: it does not apply)
-                need = lib.fovi_knnconv_workspace_bytes(self._h, B)
-                ws = torch.empty(need, dtype=torch.uint8, device=x_bnc.device) if need > 0 else None     # the allocator reuses it in stream order
-                check(lib.fovi_knnconv_forward_ws(self._h, _ptr(x_bnc), _ptr(wt), _ptr(bias) if bias is not None else None, _ptr(out), _dt(out.dtype), B,
-                                                  int(relu), _ptr(ws) if ws is not None else None, max(need, 0), _stream()), "fovi_knnconv_forward_ws")
-                return out
             check(lib.fovi_knnconv_forward(self._h_tc, _ptr(x_bnc), _ptr(wt), _ptr(bias) if bias is not None else None, _ptr(out),
                                            _dt(out.dtype), B, int(relu), _stream()), "fovi_knnconv_forward")
         return out

@@ -226,14 +226,6 @@ int64_t fovi_static_scratch_bytes(void);
 int fovi_knnconv_forward_bcn_static(fovi_knnconv_plan* plan, const void* X, int x_dtype, const void* Wt,
                                     const float* bias, void* Y, int y_dtype, int B, int relu, void* stream);
 
-/* fovi_knnconv_forward with a workspace: batches of at most 16 rows of layers with 16 or more channels then put several output points into a tile and split the
- * contraction (every split's partial sums go to the workspace and are added in order: results are deterministic).  workspace: device memory, 32-byte
- * aligned, of at least fovi_knnconv_workspace_bytes(plan, B) bytes (0: not needed), free again when the call's work on the stream is done.  Without
- * one the call runs as fovi_knnconv_forward. */
-int64_t fovi_knnconv_workspace_bytes(const fovi_knnconv_plan* plan, int B);
-int fovi_knnconv_forward_ws(fovi_knnconv_plan* plan, const void* X, const void* Wt, const float* bias, void* Y, int y_dtype, int B, int relu,
-                            void* workspace, int64_t workspace_bytes, void* stream);
-
 /* Exact float32 path (CUDA cores, float32 multiply-adds): the fp32 parity case.
  * X : [B,c_in,n_in] (FOVI_ACT_BCN) or [B,n_in,c_in] (FOVI_ACT_BNC) of x_dtype; Wt: packed
  * f32 slabs [V,c_out,cin_packed]; Y: float32 in y_layout. */
