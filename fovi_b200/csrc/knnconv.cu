@@ -220,11 +220,19 @@ __global__ void pack_points_kernel(const TX* __restrict__ x, __nv_bfloat16* __re
 // A CTA's eight points leave through shared memory as runs of eight points (one 32-byte sector) per channel.
 // Persistent CTAs, so that the filter is staged once.  One accumulator per output, neighbours in list order, channels inside: the
 // sums are those of the general kernel below, bit for bit.
+#ifndef F32_MIN_CTAS
+#define F32_MIN_CTAS 4
+#endif
 constexpr int F32_POINTS = 8;     // output points (warps) per CTA
-constexpr int F32_NB = 32;        // neighbours staged per pass: one per lane
+constexpr int F32_NB = 16;        // neighbours staged per pass: two lanes each
+
+__host__ __device__ constexpr int f32_union_floats(int C, int BT, int OT) {
+  const int in = F32_POINTS * F32_NB * C * BT, out = BT * OT * (F32_POINTS + 1);
+  return ((in > out ? in : out) + 3) / 4 * 4;
+}
 
 template <typename TX, int BT, int NO, int CT, bool WS>
-__global__ void __launch_bounds__(F32_POINTS * 32) knnconv_f32_few_kernel(const TX* __restrict__ X, const float* __restrict__ Wt,
+__global__ void __launch_bounds__(F32_POINTS * 32, NO == 3 ? 2 : F32_MIN_CTAS) knnconv_f32_few_kernel(const TX* __restrict__ X, const float* __restrict__ Wt,
                                                                           const float* __restrict__ bias, float* __restrict__ Y,
                                                                           const int* __restrict__ nbr_idx, const uint16_t* __restrict__ nbr_tap,
                                                                           const int* __restrict__ nbr_cnt, int kp, int B, int n_in, int n_out,
@@ -234,9 +242,9 @@ __global__ void __launch_bounds__(F32_POINTS * 32) knnconv_f32_few_kernel(const 
   constexpr int OT = NO * 32;
   const int C = CT ? CT : c_in;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* xs = f32_smem + warp * (F32_NB * 4 * BT);                        // [neighbour][channel][BT images]
-  float* ys = f32_smem + F32_POINTS * F32_NB * 4 * BT;                    // [BT][OT][F32_POINTS], rows of F32_POINTS + 1
-  float* ws = ys + BT * OT * (F32_POINTS + 1);                            // [V][C][OT] (WS)
+  float* xs = f32_smem + warp * (F32_NB * C * BT);                        // [neighbour][channel][BT images]
+  float* ys = f32_smem;                                                   // [BT][OT][F32_POINTS], rows of F32_POINTS + 1: over the inputs, once used
+  float* ws = f32_smem + f32_union_floats(C, BT, OT);                     // [V][C][OT] (WS)
   int staged = -1;
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
     const int ot = item % n_ot, t = item / n_ot;                          // grid is a multiple of n_ot: a CTA keeps its channel tile
@@ -244,9 +252,14 @@ __global__ void __launch_bounds__(F32_POINTS * 32) knnconv_f32_few_kernel(const 
     const int o0 = ot * OT, b0 = bt * BT, nb = min(BT, B - b0), n = n0 + warp;
     if (WS && staged != ot) {
       __syncthreads();
-      for (int i = threadIdx.x; i < V * C * OT; i += blockDim.x) {
-        const int o = i % OT, c = (i / OT) % C, v = i / (OT * C);
-        ws[i] = o0 + o < c_out ? __ldg(Wt + ((long long)v * c_out + o0 + o) * cp + c) : 0.f;
+      // a warp per (tap, 32 channels): consecutive lanes read consecutive rows of the tap's slab
+#pragma unroll 4
+      for (int r = warp; r < V * NO; r += F32_POINTS) {
+        const int v = r / NO, o = (r - v * NO) * 32 + lane;
+        const float* src = Wt + ((long long)v * c_out + o0 + o) * cp;
+#pragma unroll
+        for (int c = 0; c < (CT ? CT : 4); ++c)
+          if (CT || c < C) ws[(v * C + c) * OT + o] = o0 + o < c_out ? __ldg(src + c) : 0.f;
       }
       staged = ot;
       __syncthreads();
@@ -261,23 +274,23 @@ __global__ void __launch_bounds__(F32_POINTS * 32) knnconv_f32_few_kernel(const 
       const int m = min(F32_NB, cnt - k0);
       int tap = 0;
       __syncwarp();      // the previous pass has been read
-      if (lane < m) {
-        const int j = __ldg(nbr_idx + (long long)n * kp + k0 + lane);
-        tap = __ldg(nbr_tap + (long long)n * kp + k0 + lane);
-        for (int c = 0; c < C; ++c) {
-          float v[BT];
+      const int nk = lane & (F32_NB - 1), bh = (lane / F32_NB) * (BT / 2);      // this lane's neighbour and its half of the images
+      if (nk < m) {
+        const int j = __ldg(nbr_idx + (long long)n * kp + k0 + nk);
+        tap = __ldg(nbr_tap + (long long)n * kp + k0 + nk);
 #pragma unroll
-          for (int b = 0; b < BT; ++b) {
-            const long long bb = b0 + b;
-            v[b] = b < nb ? ld_as_float(x_bnc ? X + (bb * n_in + j) * c_in + c : X + (bb * c_in + c) * n_in + j) : 0.f;
-          }
-          float* d = xs + (lane * C + c) * BT;
-          if constexpr (BT % 4 == 0) {
+        for (int c = 0; c < (CT ? CT : 4); ++c) {
+          if (CT == 0 && c >= C) break;
+          float v[BT / 2];
 #pragma unroll
-            for (int b = 0; b < BT; b += 4) *reinterpret_cast<float4*>(d + b) = make_float4(v[b], v[b + 1], v[b + 2], v[b + 3]);
-          } else {
-            *reinterpret_cast<float2*>(d) = make_float2(v[0], v[1]);
+          for (int b = 0; b < BT / 2; ++b) {
+            const long long bb = b0 + bh + b;
+            v[b] = bh + b < nb ? ld_as_float(x_bnc ? X + (bb * n_in + j) * c_in + c : X + (bb * c_in + c) * n_in + j) : 0.f;
           }
+          float* d = xs + (nk * C + c) * BT + bh;
+          if constexpr (BT == 8) *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1], v[2], v[3]);
+          else if constexpr (BT == 4) *reinterpret_cast<float2*>(d) = make_float2(v[0], v[1]);
+          else *d = v[0];
         }
       }
       __syncwarp();
@@ -334,7 +347,7 @@ __global__ void __launch_bounds__(F32_POINTS * 32) knnconv_f32_few_kernel(const 
       }
       continue;
     }
-    __syncthreads();     // the previous item's tile has left
+    __syncthreads();     // every warp has used its inputs
 #pragma unroll
     for (int i = 0; i < NO; ++i)
 #pragma unroll
@@ -345,6 +358,7 @@ __global__ void __launch_bounds__(F32_POINTS * 32) knnconv_f32_few_kernel(const 
       if (n0 + p < n_out && o0 + o < c_out)
         Y[((long long)(b0 + b) * c_out + o0 + o) * n_out + n0 + p] = ys[(b * OT + o) * (F32_POINTS + 1) + p];
     }
+    __syncthreads();     // the tile has left: the next item's inputs go there
   }
 }
 
@@ -377,7 +391,7 @@ int launch_f32_few(const fovi_knnconv_plan* p, const void* X, int x_bnc, const f
     const int lanes = (p->c_out + 32 * i - 1) / (32 * i) * 32 * i;
     if (lanes <= best) { best = lanes; no = i; }
   }
-  const size_t base = sizeof(float) * ((size_t)F32_POINTS * F32_NB * 4 * bt + (size_t)bt * no * 32 * (F32_POINTS + 1));
+  const size_t base = sizeof(float) * (size_t)f32_union_floats(p->c_in, bt, no * 32);
   const size_t wbytes = sizeof(float) * (size_t)p->V * p->c_in * no * 32;
   const bool ws = wbytes <= 64 * 1024;
   const size_t smem = base + (ws ? wbytes : 0);
@@ -759,7 +773,6 @@ extern "C" int fovi_knnconv_forward_bcn_static(fovi_knnconv_plan* p, const void*
   unsigned char* scratch = nullptr;
   int rc = static_scratch_address(&scratch);
   if (rc) return rc;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   rc = fovi_pack_points(X, x_dtype, B, p->c_in, p->n_in, scratch, p->cin_packed, p->x_layout, stream);
   if (rc) return rc;
   return fovi_knnconv_forward(p, scratch, Wt, bias, Y, y_dtype, B, relu, stream);
