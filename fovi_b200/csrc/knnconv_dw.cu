@@ -133,11 +133,9 @@ __device__ __forceinline__ void dw_body(const DwMaps& maps, const DwArgs& a) {
   const ItemWalk start(worker, workers, a.n_nt, a.n_mt);            // d0 tile of Q, d1 tile of P, d2 group (channels) / output point (pair)
 
   if (warp >= 5) {
-    // ------------------------------------------------------------ producers: warp w fills every W-th stage
-    constexpr int W = PRODUCER_WARPS;
-    int item = worker, cc = warp - 5, k = 0;                         // this warp's stage: row chunk cc of pair k (pair mode: k stays 0)
-    uint32_t s = (uint32_t)(warp - 5), ph = 0;
-    while (s >= (uint32_t)a.nstage) { s -= (uint32_t)a.nstage; ph ^= 1u; }
+    // ------------------------------------------------------------ producers: the warps take turns on the stages (see ring.cuh)
+    RingTurn ring(warp - 5, a.nstage);
+    int item = ring.idle ? a.total : worker, cc = warp - 5, k = 0;   // this warp's stage: row chunk cc of pair k (pair mode: k stays 0)
     ItemWalk it = start, ahead = start;
     int cnt = item < a.total ? (PAIRS ? 1 : __ldg(a.cnt + it.d2)) : 0, cnt_ahead = 0;
     auto look_ahead = [&]() {
@@ -174,8 +172,8 @@ __device__ __forceinline__ void dw_body(const DwMaps& maps, const DwArgs& a) {
     };
     if (item < a.total) settle();
     while (item < a.total) {
-      const uint32_t full = CG == 2 ? dw_map(smem_u32(&hdr->full[s]), 0) : smem_u32(&hdr->full[s]);
-      const uint32_t sa = stages0 + s * a.stage_bytes, sb = sa + 2u * DW_BOX;
+      const uint32_t full = CG == 2 ? dw_map(smem_u32(&hdr->full[ring.s]), 0) : smem_u32(&hdr->full[ring.s]);
+      const uint32_t sa = stages0 + ring.s * a.stage_bytes, sb = sa + 2u * DW_BOX;
       const int m0 = it.d1 * (128 * CG) + rank * 128;                                     // first P channel of this CTA
       // boxes wholly past the channels are not loaded: their rows / columns are never stored
       const int pb = min(2, max(0, (a.cp - m0 + 63) / 64));
@@ -183,14 +181,14 @@ __device__ __forceinline__ void dw_body(const DwMaps& maps, const DwArgs& a) {
       const int qb = PAIRS ? 0 : min((half + 63) / 64, max(0, (a.cq - q0 + 63) / 64));
       bool mine = true;
       if (lane == 0) {
-        mine = mbar_wait(smem_u32(&hdr->empty[s]), ph ^ 1u, abort_flag, a.status, 31, a.wait_limit);
+        mine = mbar_wait(smem_u32(&hdr->empty[ring.s]), ring.ph ^ 1u, abort_flag, a.status, 31, a.wait_limit);
         if (mine) {
           uint32_t bytes = (uint32_t)pb * DW_BOX + (PAIRS ? (uint32_t)max(slots, 0) * 1024u : (uint32_t)qb * DW_BOX);
           if (CG == 2) {                     // the leader arms for both CTAs
             const int m1 = it.d1 * 256 + 128, q1 = it.d0 * a.ct + half;
             bytes += (uint32_t)min(2, max(0, (a.cp - m1 + 63) / 64)) * DW_BOX + (uint32_t)min((half + 63) / 64, max(0, (a.cq - q1 + 63) / 64)) * DW_BOX;
           }
-          if (rank == 0) mbar_expect_tx(smem_u32(&hdr->full[s]), bytes);
+          if (rank == 0) mbar_expect_tx(smem_u32(&hdr->full[ring.s]), bytes);
         }
       }
       if (!__all_sync(0xffffffffu, mine)) break;
@@ -201,9 +199,9 @@ __device__ __forceinline__ void dw_body(const DwMaps& maps, const DwArgs& a) {
         if (lane < pb) dw_load3<CG>(sa + lane * DW_BOX, &maps.p, full, m0 + lane * 64, sel, cc * DW_ROWS);
         else if (lane >= 2 && lane - 2 < qb) dw_load3<CG>(sb + (lane - 2) * DW_BOX, &maps.q[0], full, q0 + (lane - 2) * 64, sel, cc * DW_ROWS);
       }
-      cc += W;
+      cc += (int)ring.step;
       settle();
-      for (s += W; s >= (uint32_t)a.nstage; s -= (uint32_t)a.nstage) ph ^= 1u;
+      ring.next();
     }
     if (lane == 0 && *abort_flag) {
       for (int i = 0; i < 64; ++i) __nanosleep(1000);    // copies in flight land before this CTA's shared memory goes away

@@ -101,12 +101,10 @@ fovi_knnconv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   const uint32_t tmem = hdr->tmem_base;
 
   if (warp >= 5 && C64) {
-    // ------------------------------------------------------------ producers: warp w fills every W-th stage (see knnconv_tc2.cu); lane 0
+    // ------------------------------------------------------------ producers: the warps take turns on the stages (see ring.cuh); lane 0
     // copies the activations, lane 1 the weights
-    constexpr int W = PRODUCER_WARPS;
-    int item = a.skip_loads ? a.total_items : (int)blockIdx.x, k = 0, cc = warp - 5, sel = 0;   // this warp's stage: chunk cc of neighbour k
-    uint32_t s = (uint32_t)(warp - 5), ph = 0;
-    while (s >= (uint32_t)a.nstage) { s -= (uint32_t)a.nstage; ph ^= 1u; }
+    RingTurn ring(warp - 5, a.nstage);
+    int item = a.skip_loads || ring.idle ? a.total_items : (int)blockIdx.x, k = 0, cc = warp - 5, sel = 0;   // this warp's stage: chunk cc of neighbour k
     ItemWalk it(blockIdx.x, gridDim.x, a.n_ct, a.n_out), ahead = it;        // d0 c_out tile, d1 output point, d2 batch tile
     int cnt = item < a.total_items ? __ldg(a.nbr_cnt + it.d1) : 0, cnt_ahead = 0;
     auto look_ahead = [&]() {
@@ -130,19 +128,19 @@ fovi_knnconv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     if (item < a.total_items) settle();
     uint32_t last_s = a.nstage, last_ph = 0;    // this warp's last armed stage
     while (item < a.total_items) {
-      const uint32_t full = smem_u32(&hdr->full[s]), sa = stages0 + s * a.stage_bytes;
+      const uint32_t full = smem_u32(&hdr->full[ring.s]), sa = stages0 + ring.s * a.stage_bytes;
       bool mine = true;
       if (lane == 0) {
-        mine = mbar_wait(smem_u32(&hdr->empty[s]), ph ^ 1u, abort_flag, a.status, 1, a.wait_limit);
+        mine = mbar_wait(smem_u32(&hdr->empty[ring.s]), ring.ph ^ 1u, abort_flag, a.status, 1, a.wait_limit);
         if (mine) mbar_expect_tx(full, a.stage_bytes);
       }
       if (!__all_sync(0xffffffffu, mine)) break;
       if (lane == 0) tma_load_3d(sa, &tmA, full, cc * 64, sel, it.d2 * BM);
       if (lane == 1) tma_load_3d(sa + b_stage_off, &tmB, full, cc * 64, it.d0 * a.ct, sel);
-      last_s = s; last_ph = ph;
-      cc += W;
+      last_s = ring.s; last_ph = ring.ph;
+      cc += (int)ring.step;
       settle();
-      for (s += W; s >= (uint32_t)a.nstage; s -= (uint32_t)a.nstage) ph ^= 1u;
+      ring.next();
     }
     if (lane == 0 && *abort_flag) {
       // Drain: wait (bounded, errors ignored) for this warp's last copies, then give the others time to land.

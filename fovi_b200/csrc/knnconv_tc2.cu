@@ -8,7 +8,7 @@
 //
 // Roles per CTA: warps 0-3 epilogue (both CTAs, each for its own 128 rows), warp 4 MMA issuer (leader CTA only; both
 // CTAs allocate and free tensor memory), four producer warps (both CTAs; loads land in the CTA's own shared memory
-// but complete on the LEADER's "full" barrier), each filling every fourth stage.  One producer thread takes 518 clocks to wait for a
+// but complete on the LEADER's "full" barrier), taking turns on the stages.  One producer thread takes 518 clocks to wait for a
 // free slot and issue a stage's two copies (a stage's MMAs: 384 at N = 192) and 2500 to change to the next item's list, and the copies land
 // 430 clocks later: the ring never held more than a stage.  Four warps with their entries requested a turn ahead keep it full.
 // 1024 rows, 225 points, one producer -> four: layer 64->192 (25 neighbours) 120 -> 106 us, 192->384 240 -> 211, 384->256 273 -> 266,
@@ -115,12 +115,10 @@ fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
   const uint32_t tmem = hdr->tmem_base;
 
   if (warp >= 5) {
-    // ------------------------------------------------------------ producers (both CTAs): warp w fills every W-th stage; lane 0
+    // ------------------------------------------------------------ producers (both CTAs): the warps take turns on the stages (see ring.cuh); lane 0
     // copies the activations, lane 1 the weights
-    constexpr int W = PRODUCER_WARPS;
-    int item = a.skip_loads ? a.total_items : pair, k = 0, cc = warp - 5, sel = 0;   // this warp's stage: chunk cc of neighbour k
-    uint32_t s = (uint32_t)(warp - 5), ph = 0;
-    while (s >= (uint32_t)a.nstage) { s -= (uint32_t)a.nstage; ph ^= 1u; }
+    RingTurn ring(warp - 5, a.nstage);
+    int item = a.skip_loads || ring.idle ? a.total_items : pair, k = 0, cc = warp - 5, sel = 0;   // this warp's stage: chunk cc of neighbour k
     ItemWalk it(pair, n_pairs, a.n_ct, a.n_out), ahead = it;                        // d0 c_out tile, d1 output point, d2 row tile
     int cnt = item < a.total_items ? __ldg(a.nbr_cnt + it.d1) : 0, cnt_ahead = 0;
     auto look_ahead = [&]() {
@@ -143,19 +141,19 @@ fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
     };
     if (item < a.total_items) settle();
     while (item < a.total_items) {
-      const uint32_t full_leader = map_to_cta(smem_u32(&hdr->full[s]), 0);
-      const uint32_t sa = stages0 + s * a.stage_bytes;
+      const uint32_t full_leader = map_to_cta(smem_u32(&hdr->full[ring.s]), 0);
+      const uint32_t sa = stages0 + ring.s * a.stage_bytes;
       bool mine = true;
       if (lane == 0) {
-        mine = mbar_wait(smem_u32(&hdr->empty[s]), ph ^ 1u, abort_flag, a.status, 11, a.wait_limit);
-        if (mine && rank == 0) mbar_expect_tx(smem_u32(&hdr->full[s]), 2u * a.stage_bytes);   // both CTAs' bytes
+        mine = mbar_wait(smem_u32(&hdr->empty[ring.s]), ring.ph ^ 1u, abort_flag, a.status, 11, a.wait_limit);
+        if (mine && rank == 0) mbar_expect_tx(smem_u32(&hdr->full[ring.s]), 2u * a.stage_bytes);   // both CTAs' bytes
       }
       if (!__all_sync(0xffffffffu, mine)) break;
       if (lane == 0) tma_load_3d_pair(sa, &tmA, full_leader, cc * 64, sel, (it.d2 * 2 + (int)rank) * BM);            // this CTA's 128 batch rows
       if (lane == 1) tma_load_3d_pair(sa + A_STAGE_BYTES, &tmB, full_leader, cc * 64, it.d0 * a.ct + (int)rank * half, sel);   // half of the c_out tile
-      cc += W;
+      cc += (int)ring.step;
       settle();
-      for (s += W; s >= (uint32_t)a.nstage; s -= (uint32_t)a.nstage) ph ^= 1u;
+      ring.next();
     }
     if (lane == 0 && *abort_flag) {
       // Give copies that are still in flight time to land before this CTA's shared memory goes away.

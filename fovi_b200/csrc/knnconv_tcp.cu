@@ -7,7 +7,7 @@
 // the c_out tile of B, which halves the weight bytes per SM and keeps more stages in flight.
 //
 // Roles per CTA: warps 0-7 epilogue; warp 8 MMA issuer (leader); four producer warps (both CTAs; copies land in the CTA's own shared memory
-// and complete on the leader's full[s]), each filling every fourth stage: issuing a stage's three to nine copies and waiting for its
+// and complete on the leader's full[s]), taking turns on the stages: issuing a stage's three to nine copies and waiting for its
 // slot takes one warp longer than the MMAs of the stage last.  The copies are tensor copies, because a plain bulk copy can only signal a barrier
 // of the CTA it writes to: a (pair, 128 rows) block is 2 KB and consecutive pairs follow each other, so a run of consecutive pairs
 // of the list moves as boxes of 8, 4, 2 and 1 blocks (the plan lists them, one tensor map per size), and a stage's weights are one box.
@@ -114,13 +114,12 @@ fovi_knnconv_tc_pairs2_kernel(const __grid_constant__ PsMaps maps, const PsArgs 
   const uint32_t tmem = hdr->tmem_base;
 
   if (warp > PS_EPI_WARPS) {
-    // ------------------------------------------------------------ producers (both CTAs): warp w fills every W-th stage, nine lanes
+    // ------------------------------------------------------------ producers (both CTAs): the warps take turns on the stages (see ring.cuh), nine lanes
     // Unit order: the row tile varies fastest, so that the pairs that run at the same time share a point's weights, which are the larger operand, and
     // the c_out tiles of a point follow each other while its activations are in L2.
-    constexpr int W = PRODUCER_WARPS;
-    int unit = a.skip_loads ? a.total : pair, st = warp - PS_EPI_WARPS - 1;
-    uint32_t s = (uint32_t)st, ph = 0;
-    while (s >= (uint32_t)a.nstage) { s -= (uint32_t)a.nstage; ph ^= 1u; }
+    int st = warp - PS_EPI_WARPS - 1;
+    RingTurn ring(st, a.nstage);
+    int unit = a.skip_loads || ring.idle ? a.total : pair;
     ItemWalk it(pair, n_cta_pairs, a.n_mt2, a.n_ct), ahead = it;             // d0 row tile, d1 c_out tile, d2 output point
     int steps = unit < a.total ? (__ldg(a.slot_cnt + it.d2) + 7) / 8 : 0, cnt_ahead = 0;
     auto look_ahead = [&]() {
@@ -146,12 +145,12 @@ fovi_knnconv_tc_pairs2_kernel(const __grid_constant__ PsMaps maps, const PsArgs 
     };
     if (unit < a.total) settle();
     while (unit < a.total) {
-      const uint32_t full_leader = ps_map(smem_u32(&hdr->full[s]), 0);
-      const uint32_t sa = stages0 + s * a.stage_bytes;
+      const uint32_t full_leader = ps_map(smem_u32(&hdr->full[ring.s]), 0);
+      const uint32_t sa = stages0 + ring.s * a.stage_bytes;
       bool mine = true;
       if (lane == 0) {
-        mine = mbar_wait(smem_u32(&hdr->empty[s]), ph ^ 1u, abort_flag, a.status, 21, a.wait_limit);
-        if (mine && rank == 0) mbar_expect_tx(smem_u32(&hdr->full[s]), 2u * a.stage_bytes);   // both CTAs' bytes
+        mine = mbar_wait(smem_u32(&hdr->empty[ring.s]), ring.ph ^ 1u, abort_flag, a.status, 21, a.wait_limit);
+        if (mine && rank == 0) mbar_expect_tx(smem_u32(&hdr->full[ring.s]), 2u * a.stage_bytes);   // both CTAs' bytes
       }
       if (!__all_sync(0xffffffffu, mine)) break;   // nobody copies into a stage before lane 0 saw it free
       if (lane < 8) {                          // a row tile past an odd last one reads as zeros; nothing of it is stored
@@ -159,9 +158,9 @@ fovi_knnconv_tc_pairs2_kernel(const __grid_constant__ PsMaps maps, const PsArgs 
       } else if (lane == 8) {
         ps_load(sa + A_STAGE_BYTES, &maps.w, full_leader, 0, (int)rank * (half >> 4), st * 8, it.d2 * a.n_ct + it.d1);
       }
-      st += W;
+      st += (int)ring.step;
       settle();
-      for (s += W; s >= (uint32_t)a.nstage; s -= (uint32_t)a.nstage) ph ^= 1u;
+      ring.next();
     }
     if (lane == 0 && *abort_flag) {
       for (int i = 0; i < 64; ++i) __nanosleep(1000);    // copies in flight land before this CTA's shared memory goes away

@@ -8,6 +8,7 @@
 #include <utility>
 
 #include "knnconv_plan.cuh"
+#include "ring.cuh"
 
 namespace fovi {
 // Where an output point's result goes.  Normally point n of the plan is point n of Y.  The weight-gradient contraction
@@ -21,10 +22,8 @@ namespace {
 
 constexpr int BM = 128;            // batch rows per tile (UMMA M)
 constexpr int MAX_STAGES = 8;
-#ifndef FOVI_TC_PRODUCER_WARPS
-#define FOVI_TC_PRODUCER_WARPS 4
-#endif
-constexpr int PRODUCER_WARPS = FOVI_TC_PRODUCER_WARPS;            // CTA-pair kernels: see knnconv_tc2.cu
+using fovi::PRODUCER_WARPS;        // why four: see knnconv_tc2.cu
+using fovi::RingTurn;
 constexpr int TC_THREADS = (5 + PRODUCER_WARPS) * 32;            // 4 epilogue warps, the MMA warp, the producers
 constexpr uint32_t A_STAGE_BYTES = 16384;
 constexpr uint32_t WAIT_LIMIT = 1u << 22;  // try_wait attempts before giving up
