@@ -47,7 +47,8 @@ def _as_bf2(v, B, device, what, F=1):
                 if len(_CONST_CACHE) > 64:
                     _CONST_CACHE.clear()
                 pair = np.broadcast_to(arr.reshape(-1), (2,)) if arr.size == 2 else np.full(2, arr.reshape(-1)[0], np.float32)
-                hit = torch.as_tensor(np.broadcast_to(pair, (B, F, 2)).copy(), device=device)
+                with torch.inference_mode(False):      # later calls may save the tensor for a backward pass
+                    hit = torch.as_tensor(np.broadcast_to(pair, (B, F, 2)).copy(), device=device)
                 _CONST_CACHE[key] = hit
             return hit, False
         t = torch.as_tensor(arr, device=device)
