@@ -23,6 +23,23 @@ _PADS = {"zeros": ops.PAD_ZEROS, "border": ops.PAD_BORDER}
 _CONST_CACHE = {}
 
 
+def _upload_pair(key, arr, B, F, device):
+    """A constant's first use with this batch and fixation count: [B,F,2] on the device, cached under `key` (..., B, F, device).  The copy for
+    one fixation is cached with it: a stream capture may not upload, so a count first met there is repeated from that copy, inside the graph
+    (and not cached: the memory is the graph's)."""
+    pair = np.broadcast_to(arr.reshape(-1), (2,)) if arr.size == 2 else np.full(2, arr.reshape(-1)[0], np.float32)
+    one_key = key[:-2] + (1, device)
+    one = _CONST_CACHE.get(one_key)
+    if one is not None and torch.device(device).type == "cuda" and torch.cuda.is_current_stream_capturing():
+        return one.expand(B, F, 2).contiguous()
+    if len(_CONST_CACHE) > 128:
+        _CONST_CACHE.clear()
+    with torch.inference_mode(False):      # later calls may save the tensor for a backward pass
+        made = {k: torch.as_tensor(np.broadcast_to(pair, (B, n, 2)).copy(), device=device) for k, n in {one_key: 1, key: F}.items()}
+    _CONST_CACHE.update(made)
+    return made[key]
+
+
 def _as_bf2(v, B, device, what, F=1):
     """Fixation argument -> float32 tensor [B,F,2] on `device` plus whether a fixation axis was given.
     A tensor that already is float32 [B,F,2] on the device is passed through untouched; Python numbers and
@@ -43,14 +60,7 @@ def _as_bf2(v, B, device, what, F=1):
         if arr.size <= 2:
             key = (arr.tobytes(), arr.shape, B, F, device) if key is None else key
             hit = _CONST_CACHE.get(key)
-            if hit is None:
-                if len(_CONST_CACHE) > 64:
-                    _CONST_CACHE.clear()
-                pair = np.broadcast_to(arr.reshape(-1), (2,)) if arr.size == 2 else np.full(2, arr.reshape(-1)[0], np.float32)
-                with torch.inference_mode(False):      # later calls may save the tensor for a backward pass
-                    hit = torch.as_tensor(np.broadcast_to(pair, (B, F, 2)).copy(), device=device)
-                _CONST_CACHE[key] = hit
-            return hit, False
+            return (hit if hit is not None else _upload_pair(key, arr, B, F, device)), False
         t = torch.as_tensor(arr, device=device)
     multi = False
     if t.dim() == 0:
