@@ -167,11 +167,17 @@ class KnnConvGrad:
         return out.reshape(self.c_out, self.c_in * self.V)
 
 
+def _aligned(t):
+    """The contiguous tensor t, copied if it does not start on the 16 bytes that the kernels' tensor copies need (an upstream gradient may be a piece
+    of a larger buffer, as the backward of a concatenation hands out)."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _channels_last(t):
-    """[B, C, N] of any strides -> contiguous [B, N, C] bf16."""
+    """[B, C, N] of any strides and alignment -> contiguous, 16-byte aligned [B, N, C] bf16."""
     p = t.permute(0, 2, 1)
     if p.is_contiguous():
-        return p.to(torch.bfloat16)
+        return _aligned(p.to(torch.bfloat16))
     return ops.pack_points(t, t.shape[1]) if t.shape[1] % 8 == 0 else p.to(torch.bfloat16).contiguous()
 
 
@@ -232,7 +238,7 @@ class _KnnConvPointsFunction(torch.autograd.Function):
     def backward(ctx, gy):
         xp, weight, y = ctx.saved_tensors
         g = ctx.layer.grad_plans
-        gy = gy.to(torch.bfloat16).contiguous()
+        gy = _aligned(gy.to(torch.bfloat16).contiguous())
         want_w, want_b = ctx.needs_input_grad[1], ctx.has_bias and ctx.needs_input_grad[2]
         gb = None
         if ctx.relu:
