@@ -91,6 +91,18 @@ class SamplerPlan:
             check(lib.fovi_sampler_check(self._h, _stream()), "fovi_sampler_check")
 
 
+def _fixations(fix_rc, fix_hw, B):
+    """(centres, sizes, F) as the kernels read them: float32, contiguous [B,F,2].  The caller keeps both tensors until its launch is issued: of two
+    copies made and dropped inside the call's argument list the second could take the first one's memory."""
+    if fix_rc.dtype != torch.float32 or not fix_rc.is_contiguous():
+        fix_rc = fix_rc.to(torch.float32).contiguous()
+    if fix_hw.dtype != torch.float32 or not fix_hw.is_contiguous():
+        fix_hw = fix_hw.to(torch.float32).contiguous()
+    F = fix_rc.shape[1]
+    assert fix_rc.shape == (B, F, 2) and fix_hw.shape == (B, F, 2)
+    return fix_rc, fix_hw, F
+
+
 def sample(plan, img, fix_rc, fix_hw, mode=BILINEAR, pad=PAD_ZEROS, out_dtype=None, layout=OUT_BFCN, channel_stride=None, out=None):
     """img [B,C,H,W] (any strides; float32, bfloat16, or uint8 sampled as the float32 values it holds);
     fix_rc, fix_hw [B,F,2] float32 CUDA.  Returns the sampled
@@ -99,12 +111,7 @@ def sample(plan, img, fix_rc, fix_hw, mode=BILINEAR, pad=PAD_ZEROS, out_dtype=No
     consumes; rows past the last one are left unwritten."""
     _need_cuda(img, fix_rc, fix_hw)
     B, Cc, H, W = img.shape
-    if fix_rc.dtype != torch.float32 or not fix_rc.is_contiguous():
-        fix_rc = fix_rc.to(torch.float32).contiguous()
-    if fix_hw.dtype != torch.float32 or not fix_hw.is_contiguous():
-        fix_hw = fix_hw.to(torch.float32).contiguous()
-    F = fix_rc.shape[1]
-    assert fix_rc.shape == (B, F, 2) and fix_hw.shape == (B, F, 2)
+    fix_rc, fix_hw, F = _fixations(fix_rc, fix_hw, B)
     if out_dtype is None:
         out_dtype = torch.float32 if img.dtype == torch.uint8 else img.dtype
     nc = layout in (OUT_BFNC, OUT_FBNC)
@@ -167,15 +174,15 @@ def sample_backward(plan, grad_out, img_shape, fix_rc, fix_hw, mode=BILINEAR, pa
     [B,C,H,W]; with `grad_img` given the gradient is accumulated into it."""
     _need_cuda(grad_out, fix_rc, fix_hw)
     B, Cc, H, W = img_shape
-    F = fix_rc.shape[1]
+    fix_rc, fix_hw, F = _fixations(fix_rc, fix_hw, B)
     grad_out = grad_out.contiguous()
     assert grad_out.shape == ((B, F, Cc, plan.n_points) if layout == OUT_BFCN else (F, B, Cc, plan.n_points)), grad_out.shape
     if grad_img is None:
         grad_img = torch.zeros((B, Cc, H, W), dtype=torch.float32, device=grad_out.device)
     assert grad_img.dtype == torch.float32 and grad_img.is_contiguous() and tuple(grad_img.shape) == (B, Cc, H, W)
     with _on(grad_out.device):
-        check(lib.fovi_sample_backward(plan._h, _ptr(grad_out), _dt(grad_out.dtype), layout, B, Cc, H, W, _ptr(fix_rc.to(torch.float32).contiguous()),
-                                       _ptr(fix_hw.to(torch.float32).contiguous()), F, mode, pad, _ptr(grad_img), _stream()), "fovi_sample_backward")
+        check(lib.fovi_sample_backward(plan._h, _ptr(grad_out), _dt(grad_out.dtype), layout, B, Cc, H, W, _ptr(fix_rc), _ptr(fix_hw), F,
+                                       mode, pad, _ptr(grad_img), _stream()), "fovi_sample_backward")
     return grad_img
 
 
@@ -400,7 +407,7 @@ def sample_knnconv_fused(splan, cplan, img, fix_rc, fix_hw, wt, bias=None, relu=
     row_order "bf", '(b f)'.  Returns ([rows, n_out, c_out], intermediate buffer)."""
     _need_cuda(img, fix_rc, fix_hw, wt, bias)
     B, Cc, H, W = img.shape
-    F = fix_rc.shape[1]
+    fix_rc, fix_hw, F = _fixations(fix_rc, fix_hw, B)
     need = lib.fovi_fused_intermediate_bytes(cplan._h_tc, B * F)
     if intermediate is None:
         intermediate = torch.zeros(need // 2, dtype=torch.bfloat16, device=img.device)
@@ -411,8 +418,8 @@ def sample_knnconv_fused(splan, cplan, img, fix_rc, fix_hw, wt, bias=None, relu=
         bias = _bias_f32(bias)
     strides = _I64x4(*img.stride())
     with _on(img.device):
-        check(lib.fovi_sample_knnconv_fused(splan._h, cplan._h_tc, _ptr(img), U8 if img.dtype == torch.uint8 else _dt(img.dtype), B, Cc, H, W, strides, _ptr(fix_rc.contiguous()),
-                                            _ptr(fix_hw.contiguous()), F, mode, pad, _ptr(intermediate), _ptr(wt),
+        check(lib.fovi_sample_knnconv_fused(splan._h, cplan._h_tc, _ptr(img), U8 if img.dtype == torch.uint8 else _dt(img.dtype), B, Cc, H, W, strides, _ptr(fix_rc),
+                                            _ptr(fix_hw), F, mode, pad, _ptr(intermediate), _ptr(wt),
                                             _ptr(bias) if bias is not None else None, _ptr(out), _dt(out.dtype), int(relu),
                                             {"fb": 0, "bf": 1}[row_order], _stream()),
               "fovi_sample_knnconv_fused")
