@@ -26,9 +26,10 @@ def _dt(t):
 
 # A launch costs a Python caller more than the smallest kernels run (a 5 us sensor call took 32 us through
 # torch.cuda.current_stream, torch.cuda.device and ctypes wrapper objects), so the launch path asks torch's own bindings for the
-# raw stream and device and hands plain integers to ctypes.
-_raw_stream = torch._C._cuda_getCurrentRawStream
-_current_device = torch._C._cuda_getDevice
+# raw stream and device and hands plain integers to ctypes.  A torch without these bindings (no CUDA build) still imports this module, for
+# the host routines; its launches fail in torch.cuda.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda device: torch.cuda.current_stream(device).cuda_stream)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
 _I64x4 = C.c_int64 * 4
 
 

@@ -2,6 +2,8 @@
 import ctypes
 import os
 import re
+import subprocess
+import sys
 
 from conftest import ROOT
 
@@ -44,3 +46,13 @@ def test_status_strings_and_argument_checks_without_gpu():
     tap_bad = (ctypes.c_uint16 * 4)(0, 9, 0, 0)
     idx_ok = (ctypes.c_int32 * 4)(0, 1, 3, 2)
     assert lib.fovi_knnconv_plan_create(idx_ok, tap_bad, 3, 2, 2, 4, 3, 16, ctypes.byref(h)) == 3
+
+
+def test_import_on_a_torch_without_cuda_bindings():
+    """The host routines (tables, geometry) need no CUDA build of torch; the launch path's private bindings may be absent."""
+    code = ("import torch\n"
+            "for n in ('_cuda_getCurrentRawStream', '_cuda_getDevice'):\n"
+            "    if hasattr(torch._C, n): delattr(torch._C, n)\n"
+            "from fovi_b200 import ops, tables, knn, sensing\n"
+            "assert callable(ops._raw_stream) and callable(ops._current_device)\n")
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT)
