@@ -56,7 +56,8 @@ SIGNATURES = {
     "fovi_knndw_plan_destroy": (None, [_P]),
     "fovi_knndw_run": (C.c_int, [_P, _P, C.c_int, _P, C.c_int, C.c_int, _P, _P]),
     "fovi_knndw_check": (C.c_int, [_P, _P]),
-    "fovi_knnconv_weight_grad_pairs": (C.c_int, [_P, _P, _P, C.c_int, _P, _P]),
+    "fovi_knnconv_weight_grad_workspace_bytes": (C.c_int64, [_P]),
+    "fovi_knnconv_weight_grad_pairs": (C.c_int, [_P, _P, _P, C.c_int, _P, C.c_int64, _P, _P]),
     "fovi_column_sum": (C.c_int, [_P, C.c_int, C.c_longlong, C.c_int, _P, _P]),
     "fovi_relu_backward_to_inner": (C.c_int, [_P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_longlong, C.c_longlong, C.c_longlong, _P, _P, C.c_int, C.c_int, _P, _P]),
     "fovi_tap_segment_sum": (C.c_int, [_P, C.c_int, C.c_longlong, _P, _P, C.c_int, _P, C.c_int, _P]),

@@ -576,6 +576,8 @@ extern "C" void fovi_knnconv_plan_destroy(fovi_knnconv_plan* p) {
   if (p->zero_block) cudaFree(p->zero_block);
   if (p->pair_run) cudaFree(p->pair_run);
   if (p->pair_box) cudaFree(p->pair_box);
+  if (p->seg_start) cudaFree(p->seg_start);
+  if (p->seg_place) cudaFree(p->seg_place);
   delete p;
 }
 

@@ -13,12 +13,14 @@
 //              role.  A stage is 64 batch rows of one pair.  Result tiles are ADDED into out[v][p channel][q channel] (float32 reductions in L2).
 //   pair       (c_in <= 4) X is in the pair layout of knnconv_tc.cu: a (pair, 64 rows) block is 64 x 16 bytes = MN-major core matrices of 8 columns
 //              (2 points x 4 channels).  A work item is one output point x 128 channels of gY x up to 32 slots of the point's list (256 columns);
-//              a stage is 64 batch rows; the four channel sums of a listed point are added into out[tap][o][0..3] as one 16-byte reduction per lane,
-//              512 contiguous bytes per warp.
+//              a stage is 64 batch rows; the four channel sums of a listed point leave as one 16-byte store per lane, 512 contiguous bytes per warp,
+//              into a workspace with a place for every (output point, listed point).  A second kernel adds each tap's places in the order of the output
+//              points: the result is the same bits every time (sums of the channels mode are float32 reductions in no fixed order).
 // CG = 2: cluster of two CTAs, M = 256 (P channels), each CTA stages its half of Q's tile.  CG = 1: M = 128.
 // Roles: warps 0-3 epilogue, warp 4 MMA issuer, the rest producers (see knnconv_tc2.cu).  All waits are bounded.
 #include "tc_common.cuh"
 
+#include <mutex>
 #include <vector>
 
 struct fovi_knndw_plan {
@@ -38,7 +40,8 @@ constexpr uint32_t DW_BOX = 8192;           // 64 channels x 64 rows
 struct DwArgs {
   const int* p_pt; const int* q_pt; const int* cnt; const int* tap;                     // channels mode
   const int* slot_pair; const uint16_t* slot_box; const uint16_t* slot_tap;             // pair mode (cnt: slots per point)
-  float* out; int* status;
+  float* out; int* status;                                                              // pair mode: out is the workspace
+  int n0;                                                                               // pair mode: first output point of this launch
   int kp, chunks, cp, cq, ct, n_mt, n_nt, total, nstage;   // ct: columns of a Q tile (pair mode: 8 per slot)
   uint32_t stage_bytes, wait_limit;
 };
@@ -194,7 +197,7 @@ __device__ __forceinline__ void dw_body(const DwMaps& maps, const DwArgs& a) {
       if (!__all_sync(0xffffffffu, mine)) break;
       if (PAIRS) {
         if (box) dw_load4(sb + lane * 1024u, &maps.q[box - 1], full, 0, (cc & 1) * 2, sel, cc >> 1);
-        if (lane < pb) dw_load3<CG>(sa + lane * DW_BOX, &maps.p, full, m0 + lane * 64, it.d2, cc * DW_ROWS);
+        if (lane < pb) dw_load3<CG>(sa + lane * DW_BOX, &maps.p, full, m0 + lane * 64, a.n0 + it.d2, cc * DW_ROWS);
       } else {
         if (lane < pb) dw_load3<CG>(sa + lane * DW_BOX, &maps.p, full, m0 + lane * 64, sel, cc * DW_ROWS);
         else if (lane >= 2 && lane - 2 < qb) dw_load3<CG>(sb + (lane - 2) * DW_BOX, &maps.q[0], full, q0 + (lane - 2) * 64, sel, cc * DW_ROWS);
@@ -255,7 +258,7 @@ __device__ __forceinline__ void dw_body(const DwMaps& maps, const DwArgs& a) {
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue: add the tile into the result
+    // ------------------------------------------------------------ epilogue: add the tile into the result (pair mode: store it)
     const int q = warp & 3;
     uint32_t acc = 0, aph = 0;
     ItemWalk it = start;
@@ -268,7 +271,8 @@ __device__ __forceinline__ void dw_body(const DwMaps& maps, const DwArgs& a) {
       const uint32_t t_base = tmem + ((uint32_t)(q * 32) << 16) + acc * 256u;
       if (PAIRS) {
         const int ts = a.ct / 8, slots = min(ts, cnt - it.d0 * ts);
-        const uint16_t* taps = a.slot_tap + ((size_t)it.d2 * a.kp + it.d0 * ts) * 2;
+        const size_t place = ((size_t)it.d2 * a.kp + it.d0 * ts) * 2;                      // of the tile's first slot
+        const uint16_t* taps = a.slot_tap + place;
         for (int s0 = 0; s0 < slots; s0 += 4) {                                           // four slots = 32 columns
           uint32_t r[32];
           tc_ld32(t_base + s0 * 8, r);
@@ -278,8 +282,7 @@ __device__ __forceinline__ void dw_body(const DwMaps& maps, const DwArgs& a) {
             if (s0 + (j >> 1) < slots) {
               const uint32_t t = __ldg(taps + s0 * 2 + j);
               if (t != 0xFFFFu && row < a.cp)
-                red_add_f32x4(a.out + ((size_t)t * a.cp + row) * 4, __uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
-                              __uint_as_float(r[4 * j + 3]));
+                reinterpret_cast<uint4*>(a.out)[(place + s0 * 2 + j) * a.cp + row] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
             }
           }
         }
@@ -328,6 +331,79 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 fovi_knnconv_dw1_kernel(const __grid_constant__ DwMaps maps, const DwArgs a) { dw_body<1, false>(maps, a); }
 __global__ void __launch_bounds__(TC_THREADS, 1)
 fovi_knnconv_dw_pairs_kernel(const __grid_constant__ DwMaps maps, const DwArgs a) { dw_body<1, true>(maps, a); }
+
+// out[v][o] += the places of tap v between `lo` and `hi` (of the whole layer's (output point, slot, half) places; the workspace starts at `lo`), in
+// ascending order: warp w adds every W-th place, the warps' sums are added in the order of the warps.  Bound by reading the workspace, which the kernel
+// above left in L2.
+constexpr int TS_WARPS = 16;
+
+__global__ void __launch_bounds__(TS_WARPS * 32) fovi_tap_sum_kernel(const float4* __restrict__ work, const int* __restrict__ seg_start,
+                                                                     const int* __restrict__ seg_place, int lo, int hi, int c_out, float4* __restrict__ out) {
+  __shared__ float4 part[TS_WARPS][32];
+  const int v = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, o = blockIdx.y * 32 + lane;
+  const int i0 = __ldg(seg_start + v), i1 = __ldg(seg_start + v + 1);
+  auto first_from = [&](int place) {      // first index in [i0, i1) whose place is not below `place`
+    int a = i0, b = i1;
+    while (a < b) {
+      const int m = (a + b) >> 1;
+      if (__ldg(seg_place + m) < place) a = m + 1; else b = m;
+    }
+    return a;
+  };
+  // (the whole list unless the layer is done in parts)
+  const int from = i0 < i1 && __ldg(seg_place + i0) < lo ? first_from(lo) : i0, to = i0 < i1 && __ldg(seg_place + i1 - 1) >= hi ? first_from(hi) : i1;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (o < c_out) {
+#pragma unroll 8
+    for (int i = from + warp; i < to; i += TS_WARPS) {
+      const float4 x = __ldg(work + (size_t)(__ldg(seg_place + i) - lo) * c_out + o);
+      s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
+    }
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && o < c_out) {
+    float4* d = out + (size_t)v * c_out + o;
+    float4 t = *d;
+#pragma unroll
+    for (int w = 0; w < TS_WARPS; ++w) { t.x += part[w][lane].x; t.y += part[w][lane].y; t.z += part[w][lane].z; t.w += part[w][lane].w; }
+    *d = t;
+  }
+}
+
+// The places of every tap, ascending: built from the plan's slot table by the first weight gradient (inference never needs them).
+int tap_places(fovi_knnconv_plan* p) {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  if (p->seg_start) return FOVI_OK;
+  const size_t n = (size_t)p->n_out * p->sp * 2;
+  if (n >= (1ull << 31)) return FOVI_ERR_UNSUPPORTED;
+  std::vector<uint16_t> tap(n);
+  FOVI_CUDA(cudaMemcpy(tap.data(), p->pair_tap, n * sizeof(uint16_t), cudaMemcpyDeviceToHost));
+  std::vector<int> start((size_t)p->V + 1, 0), place;
+  for (size_t i = 0; i < n; ++i)
+    if (tap[i] != 0xFFFF) ++start[(size_t)tap[i] + 1];
+  for (int v = 0; v < p->V; ++v) start[v + 1] += start[v];
+  place.resize(std::max<size_t>(1, start[p->V]));
+  std::vector<int> at(start.begin(), start.end() - 1);
+  for (size_t i = 0; i < n; ++i)
+    if (tap[i] != 0xFFFF) place[at[tap[i]]++] = (int)i;
+  int *d_start = nullptr, *d_place = nullptr;
+  cudaError_t e = cudaMalloc(&d_start, start.size() * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&d_place, place.size() * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemcpy(d_place, place.data(), place.size() * sizeof(int), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d_start, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    if (d_start) cudaFree(d_start);
+    if (d_place) cudaFree(d_place);
+    return fovi::cuda_fail(e, "fovi_knnconv_weight_grad_pairs");
+  }
+  p->seg_place = d_place;
+  p->seg_start = d_start;
+  return FOVI_OK;
+}
+
+int64_t place_bytes(const fovi_knnconv_plan* p) { return (int64_t)p->sp * 2 * p->c_out * 16; }    // workspace of one output point
 
 int dw_launch(int cg, bool pairs, DwMaps& maps, DwArgs& a, cudaStream_t st) {
   const uint32_t budget = 224u * 1024u - 2048u;
@@ -434,26 +510,37 @@ extern "C" int fovi_knndw_run(fovi_knndw_plan* d, const void* P, int cp, const v
   return dw_launch(cg, false, maps, a, reinterpret_cast<cudaStream_t>(stream));
 }
 
-extern "C" int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* p, const void* gY, const void* X, int B, float* out, void* stream) {
+extern "C" int64_t fovi_knnconv_weight_grad_workspace_bytes(const fovi_knnconv_plan* p) {
+  if (!p || p->x_layout != FOVI_X_PAIRS) return -1;
+  const int64_t one = place_bytes(p);
+  return std::min<int64_t>(one * p->n_out, std::max<int64_t>(one, 128ll << 20));
+}
+
+extern "C" int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* p, const void* gY, const void* X, int B, void* work, int64_t work_bytes, float* out,
+                                              void* stream) {
   if (!p || B < 0) return FOVI_ERR_INVALID_ARGUMENT;
   if (B == 0) return FOVI_OK;
-  if (!gY || !X || !out) return FOVI_ERR_INVALID_ARGUMENT;
+  if (!gY || !X || !work || !out) return FOVI_ERR_INVALID_ARGUMENT;
   if (p->x_layout != FOVI_X_PAIRS || p->c_out % 8) return FOVI_ERR_UNSUPPORTED;
-  if ((reinterpret_cast<uintptr_t>(gY) | reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(out)) & 15) return FOVI_ERR_ALIGNMENT;
+  if ((reinterpret_cast<uintptr_t>(gY) | reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(work) | reinterpret_cast<uintptr_t>(out)) & 15)
+    return FOVI_ERR_ALIGNMENT;
+  const int per_launch = (int)std::min<int64_t>(p->n_out, work_bytes / place_bytes(p));      // output points
+  if (per_launch < 1) return FOVI_ERR_INVALID_ARGUMENT;
+  int rc = tap_places(p);
+  if (rc) return rc;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   DwArgs a;
   memset(&a, 0, sizeof(a));
-  a.slot_pair = p->pair_idx; a.slot_box = p->pair_box; a.slot_tap = p->pair_tap; a.cnt = p->pair_cnt; a.out = out; a.status = p->status;
+  a.out = static_cast<float*>(work); a.status = p->status;
   a.kp = p->sp; a.chunks = (B + DW_ROWS - 1) / DW_ROWS; a.cp = p->c_out; a.cq = 0; a.wait_limit = WAIT_LIMIT;
   a.n_mt = (p->c_out + 127) / 128; a.n_nt = (p->sp + 31) / 32;
   a.ct = (p->sp / 8 + a.n_nt - 1) / a.n_nt * 64;           // equal tiles of at most 32 slots, in whole 8s
-  const long long total = (long long)p->n_out * a.n_nt * a.n_mt;
-  if (total >= (1ll << 30)) return FOVI_ERR_UNSUPPORTED;
-  a.total = (int)total;
+  if ((long long)per_launch * a.n_nt * a.n_mt >= (1ll << 30)) return FOVI_ERR_UNSUPPORTED;
   a.stage_bytes = 2u * DW_BOX + (uint32_t)a.ct * 128u;
   DwMaps maps;
   memset(&maps, 0, sizeof(maps));
   const uint64_t c = (uint64_t)p->c_out, n = (uint64_t)p->n_out, n_pairs = (uint64_t)p->n_pairs;
-  int rc = fovi::encode_3d(&maps.p, gY, c, n, (uint64_t)B, c * 2, n * c * 2, 64, 1, DW_ROWS, true);
+  rc = fovi::encode_3d(&maps.p, gY, c, n, (uint64_t)B, c * 2, n * c * 2, 64, 1, DW_ROWS, true);
   if (rc) return rc;
   for (int i = 0; i < 4; ++i) {
     const uint64_t dims[4] = {256, 4, n_pairs, (uint64_t)(B + BM - 1) / BM}, strides[3] = {512, 2048, n_pairs * 2048};
@@ -461,5 +548,17 @@ extern "C" int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* p, const void* 
     rc = fovi::encode_4d(&maps.q[i], X, dims, strides, box);
     if (rc) return rc;
   }
-  return dw_launch(1, true, maps, a, reinterpret_cast<cudaStream_t>(stream));
+  for (a.n0 = 0; a.n0 < p->n_out; a.n0 += per_launch) {
+    const int points = std::min(per_launch, p->n_out - a.n0);
+    const size_t first = (size_t)a.n0 * p->sp;
+    a.slot_pair = p->pair_idx + first; a.slot_box = p->pair_box + first; a.slot_tap = p->pair_tap + 2 * first; a.cnt = p->pair_cnt + a.n0;
+    a.total = points * a.n_nt * a.n_mt;
+    rc = dw_launch(1, true, maps, a, st);
+    if (rc) return rc;
+    fovi_tap_sum_kernel<<<dim3(p->V, (p->c_out + 31) / 32), TS_WARPS * 32, 0, st>>>(static_cast<const float4*>(work), p->seg_start, p->seg_place, (int)(2 * first),
+                                                                                 (int)(2 * first) + points * p->sp * 2, p->c_out, reinterpret_cast<float4*>(out));
+    rc = fovi::after_launch("fovi_tap_sum_kernel");
+    if (rc) return rc;
+  }
+  return FOVI_OK;
 }

@@ -37,5 +37,7 @@ struct fovi_knnconv_plan {
   uint16_t* pair_box = nullptr; // [n_out, sp] the same runs cut into 8, 4, 2 and 1 pairs: 1 + log2(size) at the first slot of a piece; else 0
   void* zero_block = nullptr;   // 16 KB of zeros: the operand blocks read for unused pair slots
   int bias_period = 0;          // channel o reads bias[o % bias_period] (c_out, or a member's channels in a grouped plan)
+  int* seg_start = nullptr;     // [V + 1], [nnz]: the (output point, slot, half) places of every tap, built by the first weight gradient
+  int* seg_place = nullptr;     // (knnconv_dw.cu)
   int ct = 0;                   // c_out tile of the tensor-core path (UMMA N), 0 = unsupported c_out
 };

@@ -326,16 +326,18 @@ class KnnConvPlan:
                                                        _stream()), "fovi_knnconv_forward_scatter_add")
         return out
 
-    def weight_grad_pairs(self, gy_points, x_pairs):
+    def weight_grad_pairs(self, gy_points, x_pairs, work_bytes=None):
         """Weight gradient of a pair-layout layer: gy_points [B,n_out,c_out] bf16 contiguous, x_pairs from `pack_points` (its pad rows are
-        zero) -> float32 [V, c_out, 4] (channel sums of every tap).  See fovi_knnconv_weight_grad_pairs."""
+        zero) -> float32 [V, c_out, 4] (channel sums of every tap, added in a fixed order).  See fovi_knnconv_weight_grad_pairs."""
         _need_cuda(gy_points, x_pairs)
         B = gy_points.shape[0]
         assert self.x_layout == X_PAIRS and gy_points.dtype == torch.bfloat16 and gy_points.is_contiguous() and gy_points.shape[1:] == (self.n_out, self.c_out)
         assert x_pairs.dtype == torch.bfloat16 and x_pairs.is_contiguous() and x_pairs.shape == ((B + 127) // 128, self.n_pairs, 128, 8)
         out = torch.zeros((self.V, self.c_out, 4), dtype=torch.float32, device=gy_points.device)
+        work = torch.empty(lib.fovi_knnconv_weight_grad_workspace_bytes(self._h) if work_bytes is None else work_bytes, dtype=torch.uint8, device=gy_points.device)
         with _on(gy_points.device):
-            check(lib.fovi_knnconv_weight_grad_pairs(self._h, _ptr(gy_points), _ptr(x_pairs), B, _ptr(out), _stream()), "fovi_knnconv_weight_grad_pairs")
+            check(lib.fovi_knnconv_weight_grad_pairs(self._h, _ptr(gy_points), _ptr(x_pairs), B, _ptr(work), work.numel(), _ptr(out), _stream()),
+                  "fovi_knnconv_weight_grad_pairs")
         return out
 
     def forward_f32(self, x, wt_f32, bias=None, relu=False, x_layout=ACT_BCN, y_layout=ACT_BCN):

@@ -313,6 +313,8 @@ int fovi_relu_mask_colsum(const void* grad, const void* act, void* masked, float
 
 /* Weight gradient, read straight from channels-last activations (bf16): for every group g and every pair k < cnt[g]
  *   out[tap[g]][i][j] += sum over b of P[b][p_pt[g][k]][i] * Q[b][q_pt[g][k]][j]        out: float32 [V][cp][cq], initialised by the caller.
+ * Groups of the same tap are added by float32 reductions in no fixed order: repeated calls agree to float32 rounding, not bit for bit.
+ * The parts of a tap are added by float32 reductions in no fixed order: repeated calls agree to float32 rounding, not bit for bit.
  * P [B][n_p][cp] and Q [B][n_q][cq] are the upstream gradient and the layer's input in either role; cp, cq multiples of 8.
  * Groups whose pairs lie close together should follow each other (their operands then stay in L2).  Tables are host arrays, validated here.
  * (The reference: autograd through fovi/arch/knn.py:538-557.) */
@@ -324,9 +326,14 @@ int fovi_knndw_run(fovi_knndw_plan* plan, const void* P, int cp, const void* Q, 
 int fovi_knndw_check(fovi_knndw_plan* plan, void* stream);   /* as fovi_knnconv_check */
 
 /* Weight gradient of a pair-layout layer (c_in <= 4; `plan` is the layer's own, ungrouped plan): gY [B][n_out][c_out] bf16, X in the pair layout
- * with the rows past B of the last row tile ZERO (as fovi_pack_points callers leave them).  out[v][o][0..3] += the four channel sums; float32
- * [V][c_out][4], initialised by the caller. */
-int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* plan, const void* gY, const void* X, int B, float* out, void* stream);
+ * with the rows past B of the last row tile ZERO (fovi_pack_points writes them so).  out[v][o][0..3] += the four channel sums; float32
+ * [V][c_out][4], initialised by the caller.  The sums are added in a fixed order: the same inputs give the same bits (fovi_knndw_run's are not).
+ * `work`: device workspace, 16-byte aligned; fovi_knnconv_weight_grad_workspace_bytes says how much one pass over the layer takes (at most 128 MB,
+ * or one output point's share); with less, at least one point's, the layer is done in parts.  The first call on a plan allocates and copies
+ * tables of its own: call it once before a stream capture. */
+int64_t fovi_knnconv_weight_grad_workspace_bytes(const fovi_knnconv_plan* plan);
+int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* plan, const void* gY, const void* X, int B, void* work, int64_t work_bytes, float* out,
+                                   void* stream);
 
 /* Bias gradient: dst[c] = sum over the R rows of the row-major [R, C] matrix src (bf16 or float32, C even), float32
  * accumulation; dst is overwritten.  (The reference: autograd of the bias add in F.linear, fovi/arch/knn.py:555.) */
