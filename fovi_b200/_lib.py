@@ -55,6 +55,8 @@ SIGNATURES = {
     "fovi_knndw_plan_create": (C.c_int, [_P, _P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(_P)]),
     "fovi_knndw_plan_destroy": (None, [_P]),
     "fovi_knndw_run": (C.c_int, [_P, _P, C.c_int, _P, C.c_int, C.c_int, _P, _P]),
+    "fovi_knndw_selftest_wait_timeout": (C.c_int, [_P, _P, C.c_int, _P, C.c_int, C.c_int, _P, _P]),
+    "fovi_knnconv_weight_grad_pairs_selftest_wait_timeout": (C.c_int, [_P, _P, _P, C.c_int, _P, C.c_int64, _P, _P]),
     "fovi_knndw_check": (C.c_int, [_P, _P]),
     "fovi_knnconv_weight_grad_workspace_bytes": (C.c_int64, [_P]),
     "fovi_knnconv_weight_grad_pairs": (C.c_int, [_P, _P, _P, C.c_int, _P, C.c_int64, _P, _P]),

@@ -44,6 +44,7 @@ struct DwArgs {
   int n0;                                                                               // pair mode: first output point of this launch
   int kp, chunks, cp, cq, ct, n_mt, n_nt, total, nstage;   // ct: columns of a Q tile (pair mode: 8 per slot)
   uint32_t stage_bytes, wait_limit;
+  int skip_loads;   // self-test: the producers withhold every copy, so the first consumer wait must give up
 };
 
 struct DwMaps { CUtensorMap p, q[4]; };     // q[0] in channels mode; boxes of 2^i pairs in pair mode
@@ -138,7 +139,7 @@ __device__ __forceinline__ void dw_body(const DwMaps& maps, const DwArgs& a) {
   if (warp >= 5) {
     // ------------------------------------------------------------ producers: the warps take turns on the stages (see ring.cuh)
     RingTurn ring(warp - 5, a.nstage);
-    int item = ring.idle ? a.total : worker, cc = warp - 5, k = 0;   // this warp's stage: row chunk cc of pair k (pair mode: k stays 0)
+    int item = a.skip_loads || ring.idle ? a.total : worker, cc = warp - 5, k = 0;   // this warp's stage: row chunk cc of pair k (pair mode: k stays 0)
     ItemWalk it = start, ahead = start;
     int cnt = item < a.total ? (PAIRS ? 1 : __ldg(a.cnt + it.d2)) : 0, cnt_ahead = 0;
     auto look_ahead = [&]() {
@@ -481,7 +482,8 @@ extern "C" int fovi_knndw_check(fovi_knndw_plan* d, void* stream) {
   return FOVI_OK;
 }
 
-extern "C" int fovi_knndw_run(fovi_knndw_plan* d, const void* P, int cp, const void* Q, int cq, int B, float* out, void* stream) {
+static int knndw_run_impl(fovi_knndw_plan* d, const void* P, int cp, const void* Q, int cq, int B, float* out, void* stream, int skip_loads,
+                          uint32_t wait_limit) {
   if (!d || B < 0 || cp <= 0 || cq <= 0) return FOVI_ERR_INVALID_ARGUMENT;
   if (B == 0) return FOVI_OK;
   if (!P || !Q || !out) return FOVI_ERR_INVALID_ARGUMENT;
@@ -490,7 +492,7 @@ extern "C" int fovi_knndw_run(fovi_knndw_plan* d, const void* P, int cp, const v
   DwArgs a;
   memset(&a, 0, sizeof(a));
   a.p_pt = d->p_pt; a.q_pt = d->q_pt; a.cnt = d->cnt; a.tap = d->tap; a.out = out; a.status = d->status;
-  a.kp = d->kp; a.chunks = (B + DW_ROWS - 1) / DW_ROWS; a.cp = cp; a.cq = cq; a.wait_limit = WAIT_LIMIT;
+  a.kp = d->kp; a.chunks = (B + DW_ROWS - 1) / DW_ROWS; a.cp = cp; a.cq = cq; a.wait_limit = wait_limit; a.skip_loads = skip_loads;
   // CTA pairs (half of Q's bytes per SM) unless one 128-channel tile covers P, where half of every M = 256 MMA would be idle.
   const int cg = cp > 128 ? 2 : 1;
   // Q's tile: the fewest tiles of at most 256 columns, equal, in whole 32s (a load brings 64 channels: what it brings past a tile is not used)
@@ -510,14 +512,22 @@ extern "C" int fovi_knndw_run(fovi_knndw_plan* d, const void* P, int cp, const v
   return dw_launch(cg, false, maps, a, reinterpret_cast<cudaStream_t>(stream));
 }
 
+extern "C" int fovi_knndw_run(fovi_knndw_plan* d, const void* P, int cp, const void* Q, int cq, int B, float* out, void* stream) {
+  return knndw_run_impl(d, P, cp, Q, cq, B, out, stream, 0, WAIT_LIMIT);
+}
+
+extern "C" int fovi_knndw_selftest_wait_timeout(fovi_knndw_plan* d, const void* P, int cp, const void* Q, int cq, int B, float* out, void* stream) {
+  return knndw_run_impl(d, P, cp, Q, cq, B, out, stream, 1, 4096u);     // as fovi_knnconv_selftest_wait_timeout
+}
+
 extern "C" int64_t fovi_knnconv_weight_grad_workspace_bytes(const fovi_knnconv_plan* p) {
   if (!p || p->x_layout != FOVI_X_PAIRS) return -1;
   const int64_t one = place_bytes(p);
   return std::min<int64_t>(one * p->n_out, std::max<int64_t>(one, 128ll << 20));
 }
 
-extern "C" int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* p, const void* gY, const void* X, int B, void* work, int64_t work_bytes, float* out,
-                                              void* stream) {
+static int weight_grad_pairs_impl(fovi_knnconv_plan* p, const void* gY, const void* X, int B, void* work, int64_t work_bytes, float* out, void* stream,
+                                  int skip_loads, uint32_t wait_limit) {
   if (!p || B < 0) return FOVI_ERR_INVALID_ARGUMENT;
   if (B == 0) return FOVI_OK;
   if (!gY || !X || !work || !out) return FOVI_ERR_INVALID_ARGUMENT;
@@ -532,7 +542,7 @@ extern "C" int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* p, const void* 
   DwArgs a;
   memset(&a, 0, sizeof(a));
   a.out = static_cast<float*>(work); a.status = p->status;
-  a.kp = p->sp; a.chunks = (B + DW_ROWS - 1) / DW_ROWS; a.cp = p->c_out; a.cq = 0; a.wait_limit = WAIT_LIMIT;
+  a.kp = p->sp; a.chunks = (B + DW_ROWS - 1) / DW_ROWS; a.cp = p->c_out; a.cq = 0; a.wait_limit = wait_limit; a.skip_loads = skip_loads;
   a.n_mt = (p->c_out + 127) / 128; a.n_nt = (p->sp + 31) / 32;
   a.ct = (p->sp / 8 + a.n_nt - 1) / a.n_nt * 64;           // equal tiles of at most 32 slots, in whole 8s
   if ((long long)per_launch * a.n_nt * a.n_mt >= (1ll << 30)) return FOVI_ERR_UNSUPPORTED;
@@ -561,4 +571,14 @@ extern "C" int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* p, const void* 
     if (rc) return rc;
   }
   return FOVI_OK;
+}
+
+extern "C" int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* p, const void* gY, const void* X, int B, void* work, int64_t work_bytes, float* out,
+                                              void* stream) {
+  return weight_grad_pairs_impl(p, gY, X, B, work, work_bytes, out, stream, 0, WAIT_LIMIT);
+}
+
+extern "C" int fovi_knnconv_weight_grad_pairs_selftest_wait_timeout(fovi_knnconv_plan* p, const void* gY, const void* X, int B, void* work,
+                                                                    int64_t work_bytes, float* out, void* stream) {
+  return weight_grad_pairs_impl(p, gY, X, B, work, work_bytes, out, stream, 1, 4096u);
 }

@@ -60,6 +60,13 @@ class KnnConvGrad:
         self._dw_plans = {}
         self.cin_packed = self.c_in if self.c_in % 64 == 0 else -(-self.c_in // 8) * 8
 
+    def check(self):
+        """Synchronise the current stream and raise if a launch of the backward pass gave up on a wait (its gradient is incomplete).  A pair-layout
+        layer's weight gradient reports through the layer's own plan."""
+        for plan in [self._dx_plan] + [p for key, plans in self._dw_plans.items() for p in (plans[:1] if key == "dw" else plans[:2])]:
+            if plan is not None:
+                plan.check()
+
     # ---- dX
     def dx_plan(self):
         if self._dx_plan is None:

@@ -199,7 +199,12 @@ class KNNConvLayer(nn.Module):
             from .grad import KnnConvGrad
             self._grad = KnnConvGrad(self.knn_indices_pad_token.numpy(), self.tap.numpy(), self.in_coords.shape[0], self.ref_coords.shape[0],
                                      self.in_channels, self.out_channels, torch.device(self.device))
+            self._plan.derived = self._grad
         return self._grad
+
+    def check(self):
+        """Synchronise the current stream and raise if a launch of this layer, forward or backward, gave up on a bounded wait."""
+        self._plan.check()
 
     def _forward(self, X_l):
         # shapes the tensor-core kernel does not cover (c_out not a multiple of 16, > 256 neighbours) run on the exact kernel
@@ -344,6 +349,12 @@ class KNNDepthwiseSeparableConvLayer(_DepthwiseBase):
             self._packed[name] = (key, self._pw_plan.pack_weights(w.detach(), dtype))
         return self._packed[name][1]
 
+    def check(self):
+        super().check()
+        self._pw_plan.check()
+        if self._pw_layer is not None:
+            self._pw_layer[0].check()
+
     def _pointwise_layer(self):
         """The pointwise map as a KNNConv layer (every point its own only neighbour, one tap) that shares ``p_conv``'s
         parameters: what the autograd path differentiates.  Kept out of the module tree so that state dicts are unchanged."""
@@ -438,6 +449,11 @@ class KNNConvStack(nn.Module):
             self._acts[key] = [torch.empty((rows, L.plan.n_out, L.out_channels), dtype=torch.bfloat16, device=device)
                                for L in self.layers[:-1]]
         return self._acts[key]
+
+    def check(self):
+        """Synchronise the current stream and raise if a launch of one of the layers, forward or backward, gave up on a bounded wait."""
+        for L in self.layers:
+            L.check()
 
     @torch.no_grad()
     def forward_points(self, x_points, rows, out_dtype=torch.bfloat16, out=None):

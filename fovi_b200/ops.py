@@ -204,6 +204,7 @@ class KnnConvPlan:
             check(lib.fovi_knnconv_plan_create(idx.ctypes.data_as(C.c_void_p), tp.ctypes.data_as(C.c_void_p), self.n_in, n_out, K,
                                                self.V, self.c_in, self.c_out, C.byref(h)), "fovi_knnconv_plan_create")
         self._h = h
+        self.derived = None        # the backward pass's plans (grad.KnnConvGrad), once there are any
         self.cin_packed = lib.fovi_knnconv_cin_packed(h)
         self.nnz = lib.fovi_knnconv_nnz(h)
         self.x_layout = lib.fovi_knnconv_x_layout(h)
@@ -326,18 +327,19 @@ class KnnConvPlan:
                                                        _stream()), "fovi_knnconv_forward_scatter_add")
         return out
 
-    def weight_grad_pairs(self, gy_points, x_pairs, work_bytes=None):
+    def weight_grad_pairs(self, gy_points, x_pairs, work_bytes=None, selftest=False):
         """Weight gradient of a pair-layout layer: gy_points [B,n_out,c_out] bf16 contiguous, x_pairs from `pack_points` (its pad rows are
-        zero) -> float32 [V, c_out, 4] (channel sums of every tap, added in a fixed order).  See fovi_knnconv_weight_grad_pairs."""
+        zero) -> float32 [V, c_out, 4] (channel sums of every tap, added in a fixed order).  See fovi_knnconv_weight_grad_pairs.
+        `selftest`: the diagnostic launch whose waits give up; check() then raises."""
         _need_cuda(gy_points, x_pairs)
         B = gy_points.shape[0]
         assert self.x_layout == X_PAIRS and gy_points.dtype == torch.bfloat16 and gy_points.is_contiguous() and gy_points.shape[1:] == (self.n_out, self.c_out)
         assert x_pairs.dtype == torch.bfloat16 and x_pairs.is_contiguous() and x_pairs.shape == ((B + 127) // 128, self.n_pairs, 128, 8)
         out = torch.zeros((self.V, self.c_out, 4), dtype=torch.float32, device=gy_points.device)
         work = torch.empty(lib.fovi_knnconv_weight_grad_workspace_bytes(self._h) if work_bytes is None else work_bytes, dtype=torch.uint8, device=gy_points.device)
+        call = lib.fovi_knnconv_weight_grad_pairs_selftest_wait_timeout if selftest else lib.fovi_knnconv_weight_grad_pairs
         with _on(gy_points.device):
-            check(lib.fovi_knnconv_weight_grad_pairs(self._h, _ptr(gy_points), _ptr(x_pairs), B, _ptr(work), work.numel(), _ptr(out), _stream()),
-                  "fovi_knnconv_weight_grad_pairs")
+            check(call(self._h, _ptr(gy_points), _ptr(x_pairs), B, _ptr(work), work.numel(), _ptr(out), _stream()), "fovi_knnconv_weight_grad_pairs")
         return out
 
     def forward_f32(self, x, wt_f32, bias=None, relu=False, x_layout=ACT_BCN, y_layout=ACT_BCN):
@@ -397,11 +399,14 @@ class KnnConvPlan:
         return gx, gw
 
     def check(self):
-        """Synchronise the current stream and raise if a tensor-core launch gave up on a wait."""
+        """Synchronise the current stream and raise if a tensor-core launch gave up on a wait: of this layer, or of its backward pass (`derived`),
+        whose gradient is then incomplete."""
         with _on(self.device):
             check(lib.fovi_knnconv_check(self._h, _stream()), "fovi_knnconv_check")
             if self._hg:
                 check(lib.fovi_knnconv_check(self._hg, _stream()), "fovi_knnconv_check")
+        if self.derived is not None:
+            self.derived.check()
 
 
 def sample_knnconv_fused(splan, cplan, img, fix_rc, fix_hw, wt, bias=None, relu=False, mode=BILINEAR, pad=PAD_ZEROS,
@@ -459,15 +464,17 @@ class KnnDwPlan:
         if h and lib is not None:
             lib.fovi_knndw_plan_destroy(h)
 
-    def run(self, p, q):
-        """p [B,n_p,cp], q [B,n_q,cq] bf16 contiguous -> float32 [V, cp, cq].  See fovi_knndw_run."""
+    def run(self, p, q, selftest=False):
+        """p [B,n_p,cp], q [B,n_q,cq] bf16 contiguous -> float32 [V, cp, cq].  See fovi_knndw_run.  `selftest`: the diagnostic launch whose waits
+        give up; check() then raises."""
         _need_cuda(p, q)
         B, cp, cq = p.shape[0], p.shape[2], q.shape[2]
         assert p.dtype == q.dtype == torch.bfloat16 and p.is_contiguous() and q.is_contiguous()
         assert p.shape[1] == self.n_p and q.shape[:2] == (B, self.n_q), (p.shape, q.shape)
         out = torch.zeros((self.V, cp, cq), dtype=torch.float32, device=p.device)
         with _on(p.device):
-            check(lib.fovi_knndw_run(self._h, _ptr(p), cp, _ptr(q), cq, B, _ptr(out), _stream()), "fovi_knndw_run")
+            check((lib.fovi_knndw_selftest_wait_timeout if selftest else lib.fovi_knndw_run)(self._h, _ptr(p), cp, _ptr(q), cq, B, _ptr(out), _stream()),
+                  "fovi_knndw_run")
         return out
 
     def check(self):

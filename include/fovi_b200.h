@@ -323,7 +323,12 @@ int fovi_knndw_plan_create(const int32_t* p_pt, const int32_t* q_pt, const int32
                            int n_p, int n_q, fovi_knndw_plan** out);
 void fovi_knndw_plan_destroy(fovi_knndw_plan* plan);
 int fovi_knndw_run(fovi_knndw_plan* plan, const void* P, int cp, const void* Q, int cq, int B, float* out, void* stream);
-int fovi_knndw_check(fovi_knndw_plan* plan, void* stream);   /* as fovi_knnconv_check */
+int fovi_knndw_check(fovi_knndw_plan* plan, void* stream);   /* as fovi_knnconv_check: a launch that gave up left an incomplete gradient */
+/* Self-tests of the two weight gradients' failure path, as fovi_knnconv_selftest_wait_timeout (`out` is left incomplete); the pair layout's status
+ * is read by fovi_knnconv_check. */
+int fovi_knndw_selftest_wait_timeout(fovi_knndw_plan* plan, const void* P, int cp, const void* Q, int cq, int B, float* out, void* stream);
+int fovi_knnconv_weight_grad_pairs_selftest_wait_timeout(fovi_knnconv_plan* plan, const void* gY, const void* X, int B, void* work, int64_t work_bytes,
+                                                         float* out, void* stream);
 
 /* Weight gradient of a pair-layout layer (c_in <= 4; `plan` is the layer's own, ungrouped plan): gY [B][n_out][c_out] bf16, X in the pair layout
  * with the rows past B of the last row tile ZERO (fovi_pack_points writes them so).  out[v][o][0..3] += the four channel sums; float32

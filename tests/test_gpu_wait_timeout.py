@@ -19,8 +19,8 @@ def _random_tables(rs, n_in, n_out, K, V):
     return idx, tap
 
 
-# (c_in, c_out, B): the three single-CTA operand modes and the CTA-pair kernel (c_in multiple of 64, B > 128)
-@pytest.mark.parametrize("c_in,c_out,B", [(3, 64, 5), (16, 32, 5), (64, 64, 5), (64, 64, 200)])
+# (c_in, c_out, B): the three single-CTA operand modes and the two CTA-pair kernels (c_in multiple of 64, pair layout; B > 128)
+@pytest.mark.parametrize("c_in,c_out,B", [(3, 64, 5), (16, 32, 5), (64, 64, 5), (64, 64, 200), (3, 64, 200)])
 def test_wait_timeout_is_reported_and_context_survives(c_in, c_out, B):
     from fovi_b200 import ops
     from fovi_b200._lib import FoviError
