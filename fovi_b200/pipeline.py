@@ -92,7 +92,8 @@ class FoveatedFrontEnd:
     @torch.no_grad()
     def run_from_host(self, images, fix_loc, out, chunks=8, fixation_size=None, kernels=True):
         """images [B,C,H,W] (float32 or bfloat16), fix_loc [B,F,2] float32, out [B,F,n_out,C_out]: PINNED host tensors.
-        Returns after the last byte of `out` has been written.  Per chunk of images: one host->device copy of the images
+        Returns once everything is queued: the current stream waits for the last byte of `out`, the host does not.  Synchronise that stream (or an
+        event recorded on it) before reading `out` on the host or overwriting `images` and `fix_loc`.  Per chunk of images: one host->device copy of the images
         (and one of the fixations), the kernels, one device->host copy of the chunk's result.
         `kernels=False` runs the copies alone (same chunks, same streams, same dependencies): the transfer floor of
         this pipeline on the machine at hand."""
