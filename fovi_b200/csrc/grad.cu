@@ -1,5 +1,5 @@
-// Layout change used by the weight-gradient contraction of KNNConv: the batch index becomes the innermost
-// (contiguous) one, so that it can play the role of the channels in the tensor-core kernel.
+// Passes around the backward contractions of KNNConv: ReLU mask with bias sums, column sums, and a layout change that makes the batch index the
+// innermost (contiguous) one, so that it can play the role of the channels in the tensor-core kernel (fovi_knnconv_forward_scatter_add).
 #include <algorithm>
 
 #include <cuda_bf16.h>
@@ -35,23 +35,15 @@ __global__ void batch_to_inner_kernel(const T* __restrict__ src, __nv_bfloat16* 
 
 // Same, 64x64 tiles with two elements per access: a warp reads 64 consecutive source elements per row and writes 64 consecutive
 // batch entries (128 bytes) per row.  Needs an even fast extent and even strides (so that pairs are aligned).
-// Optionally fused, for the backward pass of a layer with a fused ReLU (src = upstream gradient, `act` = the layer's
-// output, same layout): the gradient is masked where the output is not positive before it is transposed, the masked
-// gradient is also written back in the source layout (`masked`, for the input-gradient GEMM) and its sums over
-// everything but the fast index (the channels: the bias gradient) are added into `colsum` -- one read of the gradient
-// instead of three.
 constexpr int X2_SLOW = 4;   // consecutive values of the slow index one block works through
 
 template <typename T, bool FAST_I>
 __global__ void __launch_bounds__(256) batch_to_inner_x2_kernel(const T* __restrict__ src, __nv_bfloat16* __restrict__ dst, int B, int I, int J,
-                                                               int Jp, int Bp, long long sb, long long si, long long sj,
-                                                               const T* __restrict__ act, T* __restrict__ masked, float* __restrict__ colsum) {
+                                                               int Jp, int Bp, long long sb, long long si, long long sj) {
   __shared__ __nv_bfloat16 tile[64][66];
-  __shared__ float part[8][64];
   const int b0 = blockIdx.x * 64, f0 = blockIdx.y * 64;
   const int F = FAST_I ? I : J, n_slow = FAST_I ? Jp : I;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  float s0 = 0.f, s1 = 0.f;
   for (int sl = 0; sl < X2_SLOW; ++sl) {
     const int slow = blockIdx.z * X2_SLOW + sl;
     if (slow >= n_slow) break;           // uniform over the block
@@ -70,27 +62,6 @@ __global__ void __launch_bounds__(256) batch_to_inner_x2_kernel(const T* __restr
           const float2 q = *reinterpret_cast<const float2*>(p);
           v0 = q.x; v1 = q.y;
         }
-        if (act) {
-          float a0, a1;
-          if (sizeof(T) == 2) {
-            const __nv_bfloat162 q = *reinterpret_cast<const __nv_bfloat162*>(act + off);
-            a0 = __bfloat162float(q.x); a1 = __bfloat162float(q.y);
-          } else {
-            const float2 q = *reinterpret_cast<const float2*>(act + off);
-            a0 = q.x; a1 = q.y;
-          }
-          v0 = a0 > 0.f ? v0 : 0.f; v1 = a1 > 0.f ? v1 : 0.f;
-        }
-        if (masked) {
-          if (sizeof(T) == 2) {
-            __nv_bfloat162 q;
-            q.x = __float2bfloat16_rn(v0); q.y = __float2bfloat16_rn(v1);
-            *reinterpret_cast<__nv_bfloat162*>(masked + off) = q;
-          } else {
-            *reinterpret_cast<float2*>(masked + off) = make_float2(v0, v1);
-          }
-        }
-        s0 += v0; s1 += v1;
       }
       __nv_bfloat162 t2;
       t2.x = __float2bfloat16_rn(v0); t2.y = __float2bfloat16_rn(v1);
@@ -105,20 +76,6 @@ __global__ void __launch_bounds__(256) batch_to_inner_x2_kernel(const T* __restr
         __nv_bfloat162 q;
         q.x = tile[2 * tx][r]; q.y = tile[2 * tx + 1][r];
         *reinterpret_cast<__nv_bfloat162*>(dst + ((long long)i * Jp + j) * Bp + b) = q;
-      }
-    }
-  }
-  if (colsum) {
-    // in the FAST_I == false orientation the fast index (the channel) is the same for every slow index of the block, and in
-    // the FAST_I orientation too: the sums of all X2_SLOW passes belong to the same 64 channels
-    part[ty][2 * tx] = s0; part[ty][2 * tx + 1] = s1;
-    __syncthreads();
-    if (ty == 0) {
-      for (int e = 0; e < 2; ++e) {
-        float t = 0.f;
-        for (int w = 0; w < 8; ++w) t += part[w][2 * tx + e];
-        const int f = f0 + 2 * tx + e;
-        if (f < F) atomicAdd(colsum + f, t);
       }
     }
   }
@@ -192,45 +149,7 @@ __global__ void __launch_bounds__(256) column_sum_kernel(const T* __restrict__ s
   }
 }
 
-// Segment sums for the weight gradient of a layer with few input channels.  prod [R][S][4] float32 holds, per output
-// channel o (row) and per slot s = (output point, neighbour), the four channel products of that pair; every slot
-// belongs to one filter tap.  dst[o][v*4 + c] += sum over the slots of tap v (listed in seg_slot[seg_start[v] ..
-// seg_start[v+1])) of prod[o][s][c].  One block per (tap, 64 rows): 4 groups of 64 threads walk the list, each thread
-// keeps the float4 of its row, the groups meet in shared memory.  Every dst element has one owner, so no atomics.
-__global__ void __launch_bounds__(256) tap_segment_sum_kernel(const float4* __restrict__ prod, long long S, const int* __restrict__ seg_start,
-                                                             const int* __restrict__ seg_slot, int R, float* __restrict__ dst, int dst_pitch) {
-  __shared__ float4 part[4][64];
-  const int v = blockIdx.x, o = blockIdx.y * 64 + (threadIdx.x & 63), g = threadIdx.x >> 6;
-  const int p0 = __ldg(seg_start + v), p1 = __ldg(seg_start + v + 1);
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (o < R) {
-    const float4* row = prod + (long long)o * S;
-    for (int p = p0 + g; p < p1; p += 4) {
-      const float4 q = __ldg(row + __ldg(seg_slot + p));
-      acc.x += q.x; acc.y += q.y; acc.z += q.z; acc.w += q.w;
-    }
-  }
-  part[g][threadIdx.x & 63] = acc;
-  __syncthreads();
-  if (g == 0 && o < R) {
-    for (int w = 1; w < 4; ++w) { const float4 q = part[w][threadIdx.x]; acc.x += q.x; acc.y += q.y; acc.z += q.z; acc.w += q.w; }
-    float* d = dst + (long long)o * dst_pitch + 4 * v;
-    d[0] += acc.x; d[1] += acc.y; d[2] += acc.z; d[3] += acc.w;
-  }
-}
-
 }  // namespace
-
-extern "C" int fovi_tap_segment_sum(const float* prod, int R, long long S, const int* seg_start, const int* seg_slot, int V, float* dst,
-                                    int dst_pitch, void* stream) {
-  if (!prod || !seg_start || !seg_slot || !dst || R <= 0 || S <= 0 || V <= 0 || dst_pitch < 4 * V) return FOVI_ERR_INVALID_ARGUMENT;
-  if (reinterpret_cast<uintptr_t>(prod) & 15) return FOVI_ERR_ALIGNMENT;
-  if ((R + 63) / 64 > 65535) return FOVI_ERR_UNSUPPORTED;
-  dim3 grid(V, (R + 63) / 64);
-  tap_segment_sum_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(reinterpret_cast<const float4*>(prod), S, seg_start, seg_slot, R, dst,
-                                                                                    dst_pitch);
-  return fovi::after_launch("tap_segment_sum_kernel");
-}
 
 extern "C" int fovi_relu_mask_colsum(const void* grad, const void* act, void* masked, float* colsum, long long R, int C, void* stream) {
   if (R < 0 || C <= 0) return FOVI_ERR_INVALID_ARGUMENT;
@@ -259,12 +178,11 @@ extern "C" int fovi_column_sum(const void* src, int dtype, long long R, int C, f
   return fovi::after_launch("column_sum_kernel");
 }
 
-static int batch_to_inner_impl(const void* src, int dtype, int B, int I, int J, long long sb, long long si, long long sj, void* dst, int Jp, int Bp,
-                               const void* act, void* masked, float* colsum, void* stream) {
+extern "C" int fovi_batch_to_inner(const void* src, int dtype, int B, int I, int J, long long sb, long long si, long long sj, void* dst,
+                                   int Jp, int Bp, void* stream) {
   if (!fovi::valid_dtype(dtype) || B < 0 || I <= 0 || J <= 0 || Jp < J || Bp < B || Bp <= 0) return FOVI_ERR_INVALID_ARGUMENT;
   if (!src || !dst) return FOVI_ERR_INVALID_ARGUMENT;
   if (si != 1 && sj != 1) return FOVI_ERR_UNSUPPORTED;
-  const bool fused = act || masked || colsum;
   const bool fast_i = si == 1 && !(sj == 1 && J >= I);
   const int fast = fast_i ? I : Jp, slow = fast_i ? Jp : I;
   if (slow > 65535 || (fast + 31) / 32 > 65535) return FOVI_ERR_UNSUPPORTED;
@@ -273,16 +191,9 @@ static int batch_to_inner_impl(const void* src, int dtype, int B, int I, int J, 
   const size_t esz = fovi::dtype_size(dtype);
   const bool x2 = F % 2 == 0 && Bp % 2 == 0 && sb % 2 == 0 && (fast_i ? sj : si) % 2 == 0 &&
                   reinterpret_cast<uintptr_t>(src) % (2 * esz) == 0 && reinterpret_cast<uintptr_t>(dst) % 4 == 0 && (fast + 63) / 64 <= 65535;
-  if (fused) {
-    // the fused form exists for the two-element kernel only; the masked copy and the activations share the source's layout
-    if (!x2 || (act && reinterpret_cast<uintptr_t>(act) % (2 * esz)) || (masked && reinterpret_cast<uintptr_t>(masked) % (2 * esz)))
-      return FOVI_ERR_UNSUPPORTED;
-    if (colsum) FOVI_CUDA(cudaMemsetAsync(colsum, 0, sizeof(float) * (size_t)F, st));
-  }
   if (x2) {
     dim3 grid2((Bp + 63) / 64, (fast + 63) / 64, (slow + X2_SLOW - 1) / X2_SLOW), block2(32, 8);
-#define RUN2(T, FI) batch_to_inner_x2_kernel<T, FI><<<grid2, block2, 0, st>>>((const T*)src, (__nv_bfloat16*)dst, B, I, J, Jp, Bp, sb, si, sj, \
-                                                                              (const T*)act, (T*)masked, colsum)
+#define RUN2(T, FI) batch_to_inner_x2_kernel<T, FI><<<grid2, block2, 0, st>>>((const T*)src, (__nv_bfloat16*)dst, B, I, J, Jp, Bp, sb, si, sj)
     if (dtype == FOVI_F32) { if (fast_i) RUN2(float, true); else RUN2(float, false); }
     else { if (fast_i) RUN2(__nv_bfloat16, true); else RUN2(__nv_bfloat16, false); }
 #undef RUN2
@@ -294,15 +205,4 @@ static int batch_to_inner_impl(const void* src, int dtype, int B, int I, int J, 
   else { if (fast_i) RUN(__nv_bfloat16, true); else RUN(__nv_bfloat16, false); }
 #undef RUN
   return fovi::after_launch("batch_to_inner_kernel");
-}
-
-extern "C" int fovi_batch_to_inner(const void* src, int dtype, int B, int I, int J, long long sb, long long si, long long sj, void* dst,
-                                   int Jp, int Bp, void* stream) {
-  return batch_to_inner_impl(src, dtype, B, I, J, sb, si, sj, dst, Jp, Bp, nullptr, nullptr, nullptr, stream);
-}
-
-extern "C" int fovi_relu_backward_to_inner(const void* grad, const void* act, int dtype, int B, int I, int J, long long sb, long long si,
-                                           long long sj, void* masked, void* dst, int Jp, int Bp, float* colsum, void* stream) {
-  if (!act && !masked && !colsum) return FOVI_ERR_INVALID_ARGUMENT;
-  return batch_to_inner_impl(grad, dtype, B, I, J, sb, si, sj, dst, Jp, Bp, act, masked, colsum, stream);
 }

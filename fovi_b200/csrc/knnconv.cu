@@ -220,9 +220,6 @@ __global__ void pack_points_kernel(const TX* __restrict__ x, __nv_bfloat16* __re
 // A CTA's eight points leave through shared memory as runs of eight points (one 32-byte sector) per channel.
 // Persistent CTAs, so that the filter is staged once.  One accumulator per output, neighbours in list order, channels inside: the
 // sums are those of the general kernel below, bit for bit.
-#ifndef F32_MIN_CTAS
-#define F32_MIN_CTAS 4
-#endif
 constexpr int F32_POINTS = 8;     // output points (warps) per CTA
 constexpr int F32_NB = 16;        // neighbours staged per pass: two lanes each
 
@@ -232,7 +229,7 @@ __host__ __device__ constexpr int f32_union_floats(int C, int BT, int OT) {
 }
 
 template <typename TX, int BT, int NO, int CT, bool WS>
-__global__ void __launch_bounds__(F32_POINTS * 32, NO == 3 ? 2 : F32_MIN_CTAS) knnconv_f32_few_kernel(const TX* __restrict__ X, const float* __restrict__ Wt,
+__global__ void __launch_bounds__(F32_POINTS * 32, NO == 3 ? 2 : 4) knnconv_f32_few_kernel(const TX* __restrict__ X, const float* __restrict__ Wt,
                                                                           const float* __restrict__ bias, float* __restrict__ Y,
                                                                           const int* __restrict__ nbr_idx, const uint16_t* __restrict__ nbr_tap,
                                                                           const int* __restrict__ nbr_cnt, int kp, int B, int n_in, int n_out,

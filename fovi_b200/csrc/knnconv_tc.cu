@@ -64,8 +64,8 @@ fovi_knnconv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* basep = smem_raw + (base - raw);
   SmemHeader* hdr = reinterpret_cast<SmemHeader*>(basep);
-  // two table buffers (the next item's list is prefetched while the current one is issued), then the bias
-  const uint32_t tbl_pitch = ((uint32_t)a.kp * 6u + 15u) & ~15u;
+  // two table buffers (the next item's list is prefetched while the current one is issued; the C64 mode has none), then the bias
+  const uint32_t tbl_pitch = MODE == MODE_C64 ? 0u : ((uint32_t)a.kp * 6u + 15u) & ~15u;
   unsigned char* tbl0 = basep + 1024;
   float* bias_s = reinterpret_cast<float*>(basep + 1024 + 2 * tbl_pitch);
   const uint32_t stages0 = base + 1024u + a.table_bytes;  // 1024-aligned
@@ -530,7 +530,7 @@ static int knnconv_forward_impl(fovi_knnconv_plan* p, const void* X, const void*
   a.total_items = (int)items;
   a.stage_bytes = A_STAGE_BYTES + (uint32_t)ct * 128u;  // A: 128 rows x 128 B;  B: ct rows x 128 B (any mode)
   if (a.kp > 32 * TBQ) return FOVI_ERR_UNSUPPORTED;  // neighbour lists longer than 256 entries
-  a.table_bytes = (2u * (((uint32_t)a.kp * 6u + 15u) & ~15u) + (uint32_t)p->c_out * 4u + 1023u) & ~1023u;
+  a.table_bytes = ((c64 ? 0u : 2u * (((uint32_t)a.kp * 6u + 15u) & ~15u)) + (uint32_t)p->c_out * 4u + 1023u) & ~1023u;
   a.acc_cols = 32;
   while ((int)a.acc_cols < ct) a.acc_cols <<= 1;
   a.tmem_cols = 2 * a.acc_cols;

@@ -55,7 +55,6 @@ class KnnConvGrad:
         self.K, self.n_out = idx.shape
         ks, ns = np.nonzero(idx != n_in)
         self._n, self._m, self._v, self._k = ns, idx[ks, ns], tp[ns, ks], ks
-        self._few = None          # the plan that served a pair-layout layer's weight gradient
         self._dx_plan = None
         self._dw_plans = {}
         self.cin_packed = self.c_in if self.c_in % 64 == 0 else -(-self.c_in // 8) * 8
@@ -97,7 +96,7 @@ class KnnConvGrad:
         with few input and many output channels (64 -> 192) wastes less with the input's channels as rows."""
         return self.cin_packed <= 128 < self.c_out
 
-    def dw_plan(self, bp=None):
+    def dw_plan(self):
         """(plan, result row of each group).  A tap's pairs, sorted by output point, are cut into parts, a few hundred in all (several per CTA
         pair), and the parts of all taps are ordered by position: products that run at the same time then share points in L2 (tap by tap, every tap
         sweeps all of both operands: 2.5 GB from DRAM where they hold 0.3)."""
@@ -126,7 +125,6 @@ class KnnConvGrad:
         """gy_points [B, n_out, c_out] bf16 contiguous, x_points the layer's packed input ([B, n_in, cin_packed] bf16, or the pair layout with zero
         pad rows), plan the layer's own -> dW [c_out, c_in*V] (summed in float32)."""
         if plan.x_layout == ops.X_PAIRS:
-            self._few = plan
             return ops.weight_grad_unpack(plan.weight_grad_pairs(gy_points, x_points), self.c_out, self.c_in, dtype=dtype)
         p, q = (x_points, gy_points) if self.dw_swapped else (gy_points, x_points)
         return ops.weight_grad_unpack(self.dw_plan()[0].run(p, q), self.c_out, self.c_in, swapped=self.dw_swapped, dtype=dtype)

@@ -600,30 +600,6 @@ def batch_to_inner(src, jp=None, bp=None, out=None):
     return out
 
 
-def relu_backward_to_inner(grad, act, jp=None, bp=None, want_masked=True, want_colsum=True):
-    """Fused start of a layer's backward pass.  grad / act: logical [B, I, J] tensors of the same dtype and strides (one
-    of the last two contiguous).  Returns (masked gradient in grad's layout or None, [I, jp, bp] bf16 batch-innermost copy
-    of the masked gradient, float32 sums over everything but the contiguous index or None), or None when the shapes need
-    the separate calls (odd extents or strides)."""
-    _need_cuda(grad, act)
-    B, I, J = grad.shape
-    jp, bp = J if jp is None else int(jp), B if bp is None else int(bp)
-    sb, si, sj = grad.stride()
-    if (si != 1 and sj != 1) or act.stride() != grad.stride() or act.dtype != grad.dtype or act.shape != grad.shape:
-        return None
-    F = I if (si == 1 and not (sj == 1 and J >= I)) else J
-    masked = torch.empty_strided(grad.shape, grad.stride(), dtype=grad.dtype, device=grad.device) if want_masked else None
-    out = torch.empty((I, jp, bp), dtype=torch.bfloat16, device=grad.device)
-    colsum = torch.empty(F, dtype=torch.float32, device=grad.device) if want_colsum else None
-    with _on(grad.device):
-        rc = lib.fovi_relu_backward_to_inner(_ptr(grad), _ptr(act), _dt(grad.dtype), B, I, J, sb, si, sj, _ptr(masked) if masked is not None else None,
-                                             _ptr(out), jp, bp, _ptr(colsum) if colsum is not None else None, _stream())
-    if rc == 2:   # FOVI_ERR_UNSUPPORTED: shapes the fused kernel does not take
-        return None
-    check(rc, "fovi_relu_backward_to_inner")
-    return masked, out, colsum
-
-
 def relu_mask_colsum(grad, act):
     """grad, act: contiguous bf16 [..., C] -> (gradient where act > 0 else 0, float32 [C] sums of it), or None when the shape needs the
     separate calls."""
@@ -649,19 +625,6 @@ def column_sum(x):
     with _on(x.device):
         check(lib.fovi_column_sum(_ptr(x), _dt(x.dtype), x.numel() // Cc, Cc, _ptr(out), _stream()), "fovi_column_sum")
     return out
-
-
-def tap_segment_sum(prod, seg_start, seg_slot, dst):
-    """dst[o, 4*v + c] += sum over the slots of tap v of prod[o, slot, c]  (prod float32 [R, S, 4] contiguous, seg_start int32 [V+1],
-    seg_slot int32, dst float32 [R, >= 4*V] contiguous).  See fovi_tap_segment_sum."""
-    _need_cuda(prod, seg_start, seg_slot, dst)
-    assert prod.dtype == torch.float32 and prod.is_contiguous() and prod.dim() == 3 and prod.shape[2] == 4
-    assert seg_start.dtype == torch.int32 and seg_slot.dtype == torch.int32 and dst.dtype == torch.float32 and dst.is_contiguous()
-    V = seg_start.numel() - 1
-    with _on(prod.device):
-        check(lib.fovi_tap_segment_sum(_ptr(prod), prod.shape[0], prod.shape[1], _ptr(seg_start), _ptr(seg_slot), V, _ptr(dst), dst.shape[1],
-                                       _stream()), "fovi_tap_segment_sum")
-    return dst
 
 
 def launch_count():

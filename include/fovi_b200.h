@@ -298,15 +298,6 @@ int fovi_knn_depthwise_backward(const fovi_knnconv_plan* plan, const void* X, in
 int fovi_batch_to_inner(const void* src, int dtype, int B, int I, int J, long long sb, long long si, long long sj, void* dst, int Jp,
                         int Bp, void* stream);
 
-/* fovi_batch_to_inner fused with the first steps of a layer's backward pass (fovi_b200/grad.py): `grad` is the upstream
- * gradient and `act` (may be NULL: no ReLU) the layer's output in the same layout and dtype; the gradient is zeroed where the
- * output is not positive (ReLU backward), written back in the source layout to `masked` (may be NULL), transposed to `dst`
- * like fovi_batch_to_inner, and summed over everything but the contiguous source index into colsum (float32, one entry per
- * value of that index: the bias gradient when the channels are contiguous; may be NULL; zeroed here).  Needs even extents and
- * strides (FOVI_ERR_UNSUPPORTED otherwise: use the separate calls). */
-int fovi_relu_backward_to_inner(const void* grad, const void* act, int dtype, int B, int I, int J, long long sb, long long si,
-                                long long sj, void* masked, void* dst, int Jp, int Bp, float* colsum, void* stream);
-
 /* Start of a layer's backward pass (channels-last bf16, C a multiple of 8 up to 2048, 16-byte aligned; otherwise FOVI_ERR_UNSUPPORTED: use the
  * separate calls): masked[r][c] = act[r][c] > 0 ? grad[r][c] : 0, and colsum[c] (float32, overwritten; may be NULL) = sum over r of masked[r][c]. */
 int fovi_relu_mask_colsum(const void* grad, const void* act, void* masked, float* colsum, long long R, int C, void* stream);
@@ -314,7 +305,6 @@ int fovi_relu_mask_colsum(const void* grad, const void* act, void* masked, float
 /* Weight gradient, read straight from channels-last activations (bf16): for every group g and every pair k < cnt[g]
  *   out[tap[g]][i][j] += sum over b of P[b][p_pt[g][k]][i] * Q[b][q_pt[g][k]][j]        out: float32 [V][cp][cq], initialised by the caller.
  * Groups of the same tap are added by float32 reductions in no fixed order: repeated calls agree to float32 rounding, not bit for bit.
- * The parts of a tap are added by float32 reductions in no fixed order: repeated calls agree to float32 rounding, not bit for bit.
  * P [B][n_p][cp] and Q [B][n_q][cq] are the upstream gradient and the layer's input in either role; cp, cq multiples of 8.
  * Groups whose pairs lie close together should follow each other (their operands then stay in L2).  Tables are host arrays, validated here.
  * (The reference: autograd through fovi/arch/knn.py:538-557.) */
@@ -344,12 +334,6 @@ int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* plan, const void* gY, cons
  * accumulation; dst is overwritten.  (The reference: autograd of the bias add in F.linear, fovi/arch/knn.py:555.) */
 int fovi_column_sum(const void* src, int dtype, long long R, int C, float* dst, void* stream);
 
-/* Segment sums of the weight gradient of a layer with at most 4 input channels (fovi_b200/grad.py): prod is float32
- * [R][S][4] (row = output channel, slot = (output point, neighbour) pair, 4 channel products); the slots of filter tap v are
- * seg_slot[seg_start[v] .. seg_start[v+1]) (device int32 arrays, seg_start has V+1 entries).
- * dst[o*dst_pitch + 4*v + c] += sum of prod[o][slot][c] over the tap's slots.  No atomics: results are deterministic. */
-int fovi_tap_segment_sum(const float* prod, int R, long long S, const int* seg_start, const int* seg_slot, int V, float* dst,
-                         int dst_pitch, void* stream);
 
 
 /* ------------------------------------------------------------------------------------------

@@ -52,8 +52,8 @@ def test_gradients_match_reference_autograd(golden):
 
 
 def test_first_layer_weight_gradient(golden):
-    """A 3-channel first layer (pair-layout forward): its weight gradient runs as one GEMM per output point (columns =
-    neighbour x channel, contraction over the batch) followed by a scatter-add onto the taps; its input needs no gradient."""
+    """A 3-channel first layer (pair-layout forward): its weight gradient is one product per output point (columns =
+    neighbour x channel, contraction over the batch) whose columns are then summed tap by tap; its input needs no gradient."""
     g = golden("config1.npz")
     V, n_in = int(g["V"]), int(g["n_in"])
     n_out = g["knn_idx_pad"].shape[1]
@@ -68,14 +68,18 @@ def test_first_layer_weight_gradient(golden):
         layer.weight.copy_(torch.from_numpy(w))
     y = layer(torch.from_numpy(x).cuda())
     y.backward(torch.from_numpy(gy).cuda())
+    # the full batch in float64, neighbour by neighbour, in torch (it would take minutes in the oracle, which checks 8 rows of it below)
+    xd, gd, want = torch.from_numpy(x).cuda().double(), torch.from_numpy(gy).cuda().double(), torch.zeros(64, 3, V, dtype=torch.float64, device="cuda")
+    xd = torch.cat([xd, xd.new_zeros(70, 3, 1)], 2)
+    for k in range(g["knn_idx_pad"].shape[0]):
+        pair = torch.einsum("bon,bcn->ocn", gd, xd[:, :, torch.from_numpy(g["knn_idx_pad"][k].astype(np.int64)).cuda()])
+        want.index_add_(2, torch.from_numpy(g["tap"][:, k].astype(np.int64)).cuda(), pair)
+    assert rel_l2(layer.weight.grad.cpu().numpy(), want.reshape(64, 3 * V).cpu().numpy()) < TOL
     _, dW, _ = oracle.knnconv_backward(x[:8], g["knn_idx_pad"], g["tap"].astype(np.int64), V, w, gy[:8])
-    # the oracle on 8 rows is the check of a second, smaller run (the full batch would take minutes in NumPy)
     layer.weight.grad = None
     y8 = layer(torch.from_numpy(x[:8]).cuda())
     y8.backward(torch.from_numpy(gy[:8]).cuda())
     assert rel_l2(layer.weight.grad.cpu().numpy(), dW) < TOL
-    assert layer.grad_plans._few is not None                        # the per-point path ran
-    assert layer.grad_plans.dw_plan(64)[0].n_out > V                # the per-tap path would cut its 3800-entry lists
     with pytest.raises(NotImplementedError):
         xt = torch.from_numpy(x[:8]).cuda().requires_grad_(True)
         layer(xt).sum().backward()
