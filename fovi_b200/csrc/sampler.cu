@@ -21,7 +21,8 @@
 //   The one wait (for the copies) is bounded: a strip that gives up sets the plan's status word, read back by
 //   fovi_sampler_check, and leaves.
 //
-// fovi_sample_kernel (any strides, any channel count).  One thread per point, plain loads, points in their own order.
+// fovi_sample_kernel (any strides, any channel count).  One thread per point, plain loads, points cell by cell.  Two further forms of it for many rows:
+// fovi_sample_points16_kernel (points-major rows in 16-byte pieces) and fovi_sample_row_kernel (one CTA per row, staged in shared memory).
 //
 // Arithmetic: float32, one rounding per operation in the order of the reference
 // (fovi/sensing/coords.py:624-640 followed by torch's CPU grid_sample with align_corners=False):
@@ -46,6 +47,8 @@ struct fovi_sampler_plan {
   int device = -1;
   float2* grid_xy = nullptr;    // [N] grid (x, y) in the caller's order (gradient kernel)
   void* cells = nullptr;        // [N] {x, y, original index, 0} by cell of an 8 x 8 partition, then index (general kernel)
+  float2* row_xy = nullptr;     // [N] grid (x, y) along a Z curve, and the points' original indices (row kernel)
+  int* row_idx = nullptr;
   void* ys = nullptr;           // [3][N] {x, y, original index, 0} in the strip kernel's visiting orders (see N_ORDERS); null: none
   float gx_min = 0, gx_max = 0, gy_min = 0, gy_max = 0;
   int* rank_lut = nullptr;      // [3][4097] rank tables of the orders over gy buckets (see the strip kernel)
@@ -62,6 +65,8 @@ struct SampleArgs {
   void* out;
   const float2* grid_xy;     // the grid in the caller's order (gradient kernel)
   const YPoint* cells;       // the grid cell by cell (general kernel)
+  const float2* row_xy;      // the grid along a Z curve and the points' original indices (row kernel)
+  const int* row_idx;
   const YPoint* ys;          // y order (null: the plan has none)
   const float* fix_rc;
   const float* fix_hw;
@@ -586,6 +591,122 @@ __global__ void __launch_bounds__(256) fovi_sample_kernel(const SampleArgs a, co
   }
 }
 
+// Footprint of one sensor point in the image: upper-left pixel (nearest: the pixel) and bilinear weights.
+struct Footprint { int x0, y0; float w_nw, w_ne, w_sw, w_se; };
+struct Fixation { float cx, cy, half_w, half_h; };
+
+__device__ __forceinline__ Fixation load_fixation(const SampleArgs& a, int bf) {
+  return {__fmul_rn(__ldg(a.fix_rc + 2 * bf + 1), (float)a.W), __fmul_rn(__ldg(a.fix_rc + 2 * bf), (float)a.H), __fdiv_rn(__ldg(a.fix_hw + 2 * bf + 1), 2.f),
+          __fdiv_rn(__ldg(a.fix_hw + 2 * bf), 2.f)};
+}
+
+template <int MODE, int PAD>
+__device__ __forceinline__ Footprint footprint(const SampleArgs& a, const Fixation& f, float gx, float gy) {
+  const float Wf = (float)a.W, Hf = (float)a.H;
+  float ix = grid_to_pixel(gx, f.half_w, f.cx, Wf, 1.f / Wf, Wf * 0.5f, a.pow2);
+  float iy = grid_to_pixel(gy, f.half_h, f.cy, Hf, 1.f / Hf, Hf * 0.5f, a.pow2);
+  if (PAD == FOVI_PAD_BORDER) {
+    ix = fminf(fmaxf(ix, 0.f), Wf - 1.f);
+    iy = fminf(fmaxf(iy, 0.f), Hf - 1.f);
+  }
+  if (MODE == FOVI_NEAREST) return {(int)rintf(ix), (int)rintf(iy), 0.f, 0.f, 0.f, 0.f};
+  const float x0f = floorf(ix), y0f = floorf(iy);
+  const float tx = __fsub_rn(ix, x0f), ty = __fsub_rn(iy, y0f);
+  const float ux = __fsub_rn(1.f, tx), uy = __fsub_rn(1.f, ty);
+  return {(int)x0f, (int)y0f, __fmul_rn(uy, ux), __fmul_rn(uy, tx), __fmul_rn(ty, ux), __fmul_rn(ty, tx)};
+}
+
+template <typename TIn, int MODE, int PAD>
+__device__ __forceinline__ float footprint_value(const SampleArgs& a, const TIn* plane, const Footprint& q) {
+  if (MODE == FOVI_NEAREST) return tap<TIn, PAD>(plane, a.sy, a.sx, q.x0, q.y0, a.W, a.H);
+  const float v_nw = tap<TIn, PAD>(plane, a.sy, a.sx, q.x0, q.y0, a.W, a.H);
+  const float v_ne = tap<TIn, PAD>(plane, a.sy, a.sx, q.x0 + 1, q.y0, a.W, a.H);
+  const float v_sw = tap<TIn, PAD>(plane, a.sy, a.sx, q.x0, q.y0 + 1, a.W, a.H);
+  const float v_se = tap<TIn, PAD>(plane, a.sy, a.sx, q.x0 + 1, q.y0 + 1, a.W, a.H);
+  float acc = __fmul_rn(v_nw, q.w_nw);
+  acc = __fmaf_rn(v_ne, q.w_ne, acc);
+  acc = __fmaf_rn(v_sw, q.w_sw, acc);
+  return __fmaf_rn(v_se, q.w_se, acc);
+}
+
+// Points-major rows of many points whose points are whole 16-byte pieces: a thread writes its point's channels, pad channels with them, 16 bytes at a
+// time.  Channel by channel (the kernel above) the stores' 2- and 4-byte pieces bound it: 512 x 4 rows of 4010 points, bf16 in and out, one channel
+// padded to eight: 238 -> 86 us; three channels 215 -> 121; 16 channels, nearest 745 -> 254.  Four channels' taps are in flight per thread.
+template <typename TIn, typename TOut, int MODE, int PAD>
+__global__ void __launch_bounds__(256, 4) fovi_sample_points16_kernel(const SampleArgs a, const int per_cta) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // see fovi_sample_kernel
+  constexpr int PIECE = 16 / (int)sizeof(TOut);
+  const int bf = blockIdx.x, b = bf / a.F, f = bf - b * a.F;
+  const long long row = a.f_major ? ((long long)f * a.B + b) : (long long)bf;
+  TOut* out_row = reinterpret_cast<TOut*>(a.out) + row * (long long)a.N * a.cp;
+  const Fixation fix = load_fixation(a, bf);
+  const TIn* img_b = reinterpret_cast<const TIn*>(a.img) + (long long)b * a.sb;
+  const int n_end = min(a.N, (int)(blockIdx.y + 1) * per_cta);
+#pragma unroll 2
+  for (int i = blockIdx.y * per_cta + threadIdx.x; i < n_end; i += blockDim.x) {
+    const float4 pt = __ldg(reinterpret_cast<const float4*>(a.cells + i));
+    const Footprint q = footprint<MODE, PAD>(a, fix, pt.x, pt.y);
+    TOut* dst = out_row + (long long)__float_as_int(pt.z) * a.cp;
+#pragma unroll 1
+    for (int c0 = 0; c0 < a.cp; c0 += PIECE) {
+      __align__(16) TOut v[PIECE];
+#pragma unroll
+      for (int e = 0; e < PIECE; ++e) v[e] = from_float<TOut>(0.f);
+#pragma unroll
+      for (int h = 0; h < PIECE; h += 4) {
+        if (c0 + h < a.C) {
+#pragma unroll
+          for (int e = h; e < h + 4; ++e)
+            if (c0 + e < a.C) v[e] = from_float<TOut>(footprint_value<TIn, MODE, PAD>(a, img_b + (c0 + e) * a.sc, q));
+        }
+      }
+      *reinterpret_cast<uint4*>(dst + c0) = *reinterpret_cast<const uint4*>(v);
+    }
+  }
+}
+
+// Many rows: bound by the sectors that gathers and stores touch, not by latency.  One CTA per (image, fixation) visits the points along a Z curve,
+// so that a warp's footprints share the most sectors, and stages the row in shared memory, so that it leaves as whole lines whatever the order.
+// Three CTAs per SM: their registers hold two points' taps, and what shared memory leaves of L1 still caches the image (four CTAs of float32 rows: 1.3 x
+// slower).  Where it is the faster one: see row_kernel_pays.
+template <typename TIn, typename TOut, int MODE, int PAD, bool NC>
+__global__ void __launch_bounds__(256, 3) fovi_sample_row_kernel(const SampleArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TOut* stage = reinterpret_cast<TOut*>(smem_raw);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // see fovi_sample_kernel
+  const int bf = blockIdx.x, b = bf / a.F, f = bf - b * a.F;
+  const long long row = a.f_major ? ((long long)f * a.B + b) : (long long)bf;
+  const int row_elems = NC ? (a.pairs ? ((a.N + 1) / 2) * 8 : a.N * a.cp) : a.C * a.N;
+  TOut* out_row = reinterpret_cast<TOut*>(a.out) +
+                  (a.pairs ? ((row >> 7) * (long long)((a.N + 1) / 2) * 128 + (row & 127)) * 8 : row * row_elems);
+  const Fixation fix = load_fixation(a, bf);
+  const TIn* img_b = reinterpret_cast<const TIn*>(a.img) + (long long)b * a.sb;
+  const int pitch = a.pairs ? 4 : a.cp;  // per-point element pitch of the points-major layouts
+  if (NC) {                              // pad channels
+    for (int i = threadIdx.x; i < row_elems; i += blockDim.x) stage[i] = from_float<TOut>(0.f);
+    __syncthreads();
+  }
+#pragma unroll 2
+  for (int i = threadIdx.x; i < a.N; i += blockDim.x) {
+    const float2 g = __ldg(a.row_xy + i);
+    const int n = __ldg(a.row_idx + i);
+    const Footprint q = footprint<MODE, PAD>(a, fix, g.x, g.y);
+#pragma unroll 3
+    for (int c = 0; c < a.C; ++c) stage[NC ? n * pitch + c : c * a.N + n] = from_float<TOut>(footprint_value<TIn, MODE, PAD>(a, img_b + c * a.sc, q));
+  }
+  __syncthreads();
+  if (NC && a.pairs) {
+    // this row owns one 16-byte slot in each pair's 128-row block of its row tile
+    const int n_pairs = (a.N + 1) / 2;
+    for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) reinterpret_cast<uint4*>(out_row)[(long long)i * 128] = reinterpret_cast<const uint4*>(stage)[i];
+  } else if ((reinterpret_cast<uintptr_t>(out_row) & 15) == 0 && (size_t)row_elems * sizeof(TOut) % 16 == 0) {
+    for (int i = threadIdx.x; i < (int)((size_t)row_elems * sizeof(TOut) / 16); i += blockDim.x)
+      reinterpret_cast<uint4*>(out_row)[i] = reinterpret_cast<const uint4*>(stage)[i];
+  } else {
+    for (int i = threadIdx.x; i < row_elems; i += blockDim.x) out_row[i] = stage[i];
+  }
+}
+
 // ------------------------------------------------------------------------------------------------------------
 // Gradient with respect to the image (what autograd through F.grid_sample gives the reference, samplers.py:108): every
 // output gradient is scattered onto the taps of its footprint with the forward's weights.  One thread per
@@ -698,6 +819,31 @@ int launch_strips(SampleArgs& a, int layout, cudaStream_t st) {
   return fovi::after_launch("fovi_sample_strip_kernel");
 }
 
+// Where the row kernel is faster than the split one (us, split / row, 4010-point sensors on images at their own strides).  It needs several rounds of
+// three CTAs per SM, images whose footprints do not stay in L1 anyway, and stores that the split form scatters:
+//   planar, C >= 3       375 x 499 float32 1024 rows 186 / 162, 2048 344 / 279, bf16 1536 182 / 156, 255 x 251 bf16 1024 84 / 87, float32 1024 107 / 104, 512 55 / 70 (not yet);
+//                        bytes 2048 rows 186 / 164, 1024 98 / 96 and 255 x 251 74 / 80; 96 x 97 float32 2048 127 / 131 (never)
+//   two channels         375 x 499 float32 2048 rows 209 / 186; 255 x 251 135 / 150, bf16 148 / 157 (never); one channel never
+//   rows above 48 KB     eight bf16 channels 1024 rows 168 / 158, four float32 channels of 255 x 251 2048 rows 283 / 268, of 375 x 499 485 / 510 (never)
+//   channels last        pixels share lines: float32 375 x 499 1024 rows 149 / 135, bytes 88 / 94, 2048 167 / 158
+//   nearest              a quarter of the gathers: 375 x 499 float32 1536 rows and more, 2048 264 / 209; 255 x 251 1024 86 / 106
+//   pair layout          8-byte stores: float32 375 x 499 2048 rows 299 / 282, 1024 159 / 164; bf16 213 / 221 (never)
+//   other points-major   2-byte channels that are no 16-byte pieces: 9 of 12, 256 rows 92 / 78, 2048 627 / 457; 3 of 3, 1024 82 / 90
+bool row_kernel_pays(const SampleArgs& a, bool nc, int mode, size_t in_size, size_t out_size, size_t stage, long long rows) {
+  const long long sms = fovi::sm_count(), image = (long long)a.C * a.H * a.W * (long long)in_size;
+  if (nc && !a.pairs) {
+    if (out_size == 2 && a.C > 4) return 2 * rows >= 3 * sms && stage <= 200 * 1024;
+    return rows >= 10 * sms && stage <= 72 * 1024;
+  }
+  if (stage > 72 * 1024) return false;
+  if (a.pairs) return in_size == 4 && rows >= 10 * sms && image >= (mode == FOVI_NEAREST ? 2500000 : 2000000);
+  if (mode == FOVI_NEAREST) return a.C >= 3 && rows >= 10 * sms && image >= 1000000;
+  if (a.C < 3) return a.C == 2 && in_size == 4 && rows >= 5 * sms && image >= 1000000;
+  if (stage > 49 * 1024) return in_size == 2 ? 2 * rows >= 13 * sms : rows >= 13 * sms && (in_size == 1 || image < 2000000);
+  if (rows >= 10 * sms) return image >= (a.sx == 1 ? 160000 : 400000);
+  return rows >= 5 * sms && in_size > 1 && image >= (a.sx != 1 ? 700000 : in_size == 2 ? 600000 : 350000);
+}
+
 template <typename TIn, typename TOut, int MODE, int PAD, bool NC>
 int launch_sample(SampleArgs a, cudaStream_t st) {
   if (!a.pairs || std::is_same<TOut, __nv_bfloat16>::value) {
@@ -709,13 +855,25 @@ int launch_sample(SampleArgs a, cudaStream_t st) {
     SampleArgs n = a;
     if (plan_strips<TIn, false>(n, NC)) return launch_strips<TIn, TOut, MODE, PAD, false>(n, n.pairs ? LAY_PAIRS : (NC ? LAY_NC : LAY_PLANAR), st);
   }
-  // points per CTA: few enough that small calls give every SM eight CTAs, at most eight per thread
   const long long rows = (long long)a.B * a.F;
   if (rows >= (1ll << 31)) return FOVI_ERR_UNSUPPORTED;
+  const size_t stage = (size_t)(NC ? (a.pairs ? (a.N + 1) / 2 * 8 : a.N * a.cp) : a.C * a.N) * sizeof(TOut);
+  const bool points16 = NC && !a.pairs && (a.cp * sizeof(TOut)) % 16 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
+  if (!points16 && row_kernel_pays(a, NC, MODE, sizeof(TIn), sizeof(TOut), stage, rows)) {
+    auto k = fovi_sample_row_kernel<TIn, TOut, MODE, PAD, NC>;
+    if (stage > 48 * 1024) FOVI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage));
+    k<<<(unsigned)rows, 256, stage, st>>>(a);
+    return fovi::after_launch("fovi_sample_row_kernel");
+  }
+  // points per CTA: few enough that small calls give every SM eight CTAs, at most eight per thread unless the grid's y extent asks for more
   const long long share = rows * a.N / (256ll * 8 * fovi::sm_count());
-  const int per_cta = 256 * (int)std::max(1ll, std::min(8ll, share));
+  const int per_cta = 256 * (int)std::max({1ll, std::min(8ll, share), (a.N + 256ll * 65535 - 1) / (256ll * 65535)});
   const dim3 grid((unsigned)rows, (a.N + per_cta - 1) / per_cta);
-  if (grid.y > 65535) return FOVI_ERR_UNSUPPORTED;
+  // (below 128 K points the channels' taps in turn take longer than their stores: 16 rows of 4010 points, 8 channels: 12.3 us / 14.3; 64: 43 / 49)
+  if (points16 && rows * a.N >= (128 << 10)) {
+    if constexpr (NC) fovi_sample_points16_kernel<TIn, TOut, MODE, PAD><<<grid, 256, 0, st>>>(a, per_cta);
+    return fovi::after_launch("fovi_sample_points16_kernel");
+  }
   fovi_sample_kernel<TIn, TOut, MODE, PAD, NC><<<grid, 256, 0, st>>>(a, per_cta);
   return fovi::after_launch("fovi_sample_kernel");
 }
@@ -769,6 +927,30 @@ extern "C" int fovi_sampler_plan_create(const float* grid_xy, int n_points, fovi
     if (e == cudaSuccess) e = cudaMalloc(&p->cells, sizeof(YPoint) * n_points);
     if (e == cudaSuccess) e = cudaMemcpy(p->cells, pts.data(), sizeof(YPoint) * n_points, cudaMemcpyHostToDevice);
   }
+  {
+    // Z curve over [-1.5, 1.5]^2 in 4096 steps a side (the fixation transform has positive scale: near on the grid is near in the image)
+    auto spread = [](float v) {
+      const float s = (std::min(std::max(v, -1.5f), 1.5f) + 1.5f) * (4095.f / 3.f);
+      uint32_t u = s == s ? (uint32_t)s : 0u;
+      u = (u | (u << 8)) & 0x00FF00FFu;
+      u = (u | (u << 4)) & 0x0F0F0F0Fu;
+      u = (u | (u << 2)) & 0x33333333u;
+      return (u | (u << 1)) & 0x55555555u;
+    };
+    std::vector<uint32_t> key(n_points);
+    std::vector<int> order(n_points);
+    std::vector<float2> xy(n_points);
+    for (int i = 0; i < n_points; ++i) {
+      key[i] = spread(grid_xy[2 * i]) | (spread(grid_xy[2 * i + 1]) << 1);
+      order[i] = i;
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int u, int v) { return key[u] < key[v]; });
+    for (int i = 0; i < n_points; ++i) xy[i] = make_float2(grid_xy[2 * order[i]], grid_xy[2 * order[i] + 1]);
+    if (e == cudaSuccess) e = cudaMalloc(&p->row_xy, sizeof(float2) * n_points);
+    if (e == cudaSuccess) e = cudaMemcpy(p->row_xy, xy.data(), sizeof(float2) * n_points, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&p->row_idx, sizeof(int) * n_points);
+    if (e == cudaSuccess) e = cudaMemcpy(p->row_idx, order.data(), sizeof(int) * n_points, cudaMemcpyHostToDevice);
+  }
   if (e == cudaSuccess) e = cudaMalloc(&p->status, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(p->status, 0, sizeof(int));
   if (e == cudaSuccess && finite) {   // a grid with NaN / Inf entries has no y order: the general kernel serves it
@@ -808,6 +990,8 @@ extern "C" void fovi_sampler_plan_destroy(fovi_sampler_plan* plan) {
   if (plan->ys) cudaFree(plan->ys);
   if (plan->grid_xy) cudaFree(plan->grid_xy);
   if (plan->cells) cudaFree(plan->cells);
+  if (plan->row_xy) cudaFree(plan->row_xy);
+  if (plan->row_idx) cudaFree(plan->row_idx);
   if (plan->rank_lut) cudaFree(plan->rank_lut);
   if (plan->status) cudaFree(plan->status);
   delete plan;
@@ -837,6 +1021,7 @@ extern "C" int fovi_sample_forward(const fovi_sampler_plan* plan, const void* im
   SampleArgs a;
   memset(&a, 0, sizeof(a));
   a.img = img; a.out = out; a.cells = static_cast<const YPoint*>(plan->cells);
+  a.row_xy = plan->row_xy; a.row_idx = plan->row_idx;
   a.fix_rc = fix_rc; a.fix_hw = fix_hw;
   a.sb = img_strides[0]; a.sc = img_strides[1]; a.sy = img_strides[2]; a.sx = img_strides[3];
   a.B = B; a.C = C; a.H = H; a.W = W; a.F = F; a.N = plan->n_points;
