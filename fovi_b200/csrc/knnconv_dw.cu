@@ -334,10 +334,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 fovi_knnconv_dw_pairs_kernel(const __grid_constant__ DwMaps maps, const DwArgs a) { dw_body<1, true>(maps, a); }
 
 // out[v][o] += the places of tap v between `lo` and `hi` (of the whole layer's (output point, slot, half) places; the workspace starts at `lo`), in
-// ascending order: warp w adds every W-th place, the warps' sums are added in the order of the warps.  Bound by reading the workspace, which the kernel
-// above left in L2.
-constexpr int TS_WARPS = 16;
-
+// ascending order: warp w adds every W-th place, the warps' sums are added in the order of the warps.  Bound by writing and reading the workspace.  Both
+// kernels, 1024 rows, against float32 reductions in no order: 3 -> 64 onto 1023 points 165 us / 132, 3 -> 384 onto 63 tokens 54 / 44, 3 -> 1280 128 / 95.
+template <int TS_WARPS>
 __global__ void __launch_bounds__(TS_WARPS * 32) fovi_tap_sum_kernel(const float4* __restrict__ work, const int* __restrict__ seg_start,
                                                                      const int* __restrict__ seg_place, int lo, int hi, int c_out, float4* __restrict__ out) {
   __shared__ float4 part[TS_WARPS][32];
@@ -522,8 +521,8 @@ extern "C" int fovi_knndw_selftest_wait_timeout(fovi_knndw_plan* d, const void* 
 
 extern "C" int64_t fovi_knnconv_weight_grad_workspace_bytes(const fovi_knnconv_plan* p) {
   if (!p || p->x_layout != FOVI_X_PAIRS) return -1;
-  const int64_t one = place_bytes(p);
-  return std::min<int64_t>(one * p->n_out, std::max<int64_t>(one, 128ll << 20));
+  const int64_t one = place_bytes(p);      // (in two parts of 128 MB the first of those layers takes 185 us)
+  return std::min<int64_t>(one * p->n_out, std::max<int64_t>(one, 256ll << 20));
 }
 
 static int weight_grad_pairs_impl(fovi_knnconv_plan* p, const void* gY, const void* X, int B, void* work, int64_t work_bytes, float* out, void* stream,
@@ -534,8 +533,10 @@ static int weight_grad_pairs_impl(fovi_knnconv_plan* p, const void* gY, const vo
   if (p->x_layout != FOVI_X_PAIRS || p->c_out % 8) return FOVI_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(gY) | reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(work) | reinterpret_cast<uintptr_t>(out)) & 15)
     return FOVI_ERR_ALIGNMENT;
-  const int per_launch = (int)std::min<int64_t>(p->n_out, work_bytes / place_bytes(p));      // output points
-  if (per_launch < 1) return FOVI_ERR_INVALID_ARGUMENT;
+  const int64_t fit = std::min<int64_t>(p->n_out, work_bytes / place_bytes(p));              // output points
+  if (fit < 1) return FOVI_ERR_INVALID_ARGUMENT;
+  const int64_t launches = (p->n_out + fit - 1) / fit;
+  const int per_launch = (int)((p->n_out + launches - 1) / launches);                         // in equal parts
   int rc = tap_places(p);
   if (rc) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -565,8 +566,13 @@ static int weight_grad_pairs_impl(fovi_knnconv_plan* p, const void* gY, const vo
     a.total = points * a.n_nt * a.n_mt;
     rc = dw_launch(1, true, maps, a, st);
     if (rc) return rc;
-    fovi_tap_sum_kernel<<<dim3(p->V, (p->c_out + 31) / 32), TS_WARPS * 32, 0, st>>>(static_cast<const float4*>(work), p->seg_start, p->seg_place, (int)(2 * first),
-                                                                                 (int)(2 * first) + points * p->sp * 2, p->c_out, reinterpret_cast<float4*>(out));
+    const dim3 grid(p->V, (p->c_out + 31) / 32);
+    const int lo = (int)(2 * first), hi = lo + points * p->sp * 2;
+    // about eight places per warp (26 per tap, 1280 channels: sixteen warps 148 us in all, four 128; 243 per tap, 64 channels: sixteen)
+    const int64_t per_tap = p->nnz / p->V;
+    auto k = per_tap >= 128 ? fovi_tap_sum_kernel<16> : per_tap >= 32 ? fovi_tap_sum_kernel<8> : fovi_tap_sum_kernel<4>;
+    k<<<grid, (per_tap >= 128 ? 16 : per_tap >= 32 ? 8 : 4) * 32, 0, st>>>(static_cast<const float4*>(work), p->seg_start, p->seg_place, lo, hi, p->c_out,
+                                                                           reinterpret_cast<float4*>(out));
     rc = fovi::after_launch("fovi_tap_sum_kernel");
     if (rc) return rc;
   }

@@ -323,8 +323,8 @@ int fovi_knnconv_weight_grad_pairs_selftest_wait_timeout(fovi_knnconv_plan* plan
 /* Weight gradient of a pair-layout layer (c_in <= 4; `plan` is the layer's own, ungrouped plan): gY [B][n_out][c_out] bf16, X in the pair layout
  * with the rows past B of the last row tile ZERO (fovi_pack_points writes them so).  out[v][o][0..3] += the four channel sums; float32
  * [V][c_out][4], initialised by the caller.  The sums are added in a fixed order: the same inputs give the same bits (fovi_knndw_run's are not).
- * `work`: device workspace, 16-byte aligned; fovi_knnconv_weight_grad_workspace_bytes says how much one pass over the layer takes (at most 128 MB,
- * or one output point's share); with less, at least one point's, the layer is done in parts.  The first call on a plan allocates and copies
+ * `work`: device workspace, 16-byte aligned; fovi_knnconv_weight_grad_workspace_bytes says how much one pass over the layer takes (at most 256 MB,
+ * or one output point's share); with less, at least one point's, the layer is done in equal parts.  The first call on a plan allocates and copies
  * tables of its own: call it once before a stream capture. */
 int64_t fovi_knnconv_weight_grad_workspace_bytes(const fovi_knnconv_plan* plan);
 int fovi_knnconv_weight_grad_pairs(fovi_knnconv_plan* plan, const void* gY, const void* X, int B, void* work, int64_t work_bytes, float* out,
