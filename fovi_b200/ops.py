@@ -112,7 +112,11 @@ def sample(plan, img, fix_rc, fix_hw, mode=BILINEAR, pad=PAD_ZEROS, out_dtype=No
     consumes; rows past the last one are left unwritten."""
     _need_cuda(img, fix_rc, fix_hw)
     B, Cc, H, W = img.shape
-    fix_rc, fix_hw, F = _fixations(fix_rc, fix_hw, B)
+    if fix_rc.dtype == torch.float32 and fix_hw.dtype == torch.float32 and fix_rc.is_contiguous() and fix_hw.is_contiguous():
+        F = fix_rc.shape[1]
+        assert fix_rc.shape == (B, F, 2) and fix_hw.shape == (B, F, 2)
+    else:
+        fix_rc, fix_hw, F = _fixations(fix_rc, fix_hw, B)
     if out_dtype is None:
         out_dtype = torch.float32 if img.dtype == torch.uint8 else img.dtype
     nc = layout in (OUT_BFNC, OUT_FBNC)
