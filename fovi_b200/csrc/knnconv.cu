@@ -215,11 +215,15 @@ __global__ void pack_points_kernel(const TX* __restrict__ x, __nv_bfloat16* __re
 // The contraction is short (K * c_in = 27..147 products) and every output point has its own taps, so what bounds a plain
 // kernel is not arithmetic (8 us of FMAs at 8 images, 3 -> 64 channels, 49 neighbours, 3976 points) but two loads per FMA and
 // 4-byte stores a point apart.  Here one warp owns an output point: a lane holds NO output channels x BT images in registers, the
-// neighbours' inputs are gathered once per point into shared memory (a lane per neighbour, read back as broadcasts), and the
+// neighbours' inputs are gathered once per point into shared memory (two lanes per neighbour, half of the images each; read back as broadcasts), and the
 // filter is held in shared memory tap-major / channel-minor, so that a tap costs NO conflict-free loads for BT * NO FMAs.
 // A CTA's eight points leave through shared memory as runs of eight points (one 32-byte sector) per channel.
 // Persistent CTAs, so that the filter is staged once.  One accumulator per output, neighbours in list order, channels inside: the
 // sums are those of the general kernel below, bit for bit.
+// CTAs per SM (register limit): up to 64 registers hold the accumulators of 32 or 64 channels, so four CTAs hide the gathers of each other's passes;
+// 96 channels x 8 images take up to 127 registers, two CTAs.  (Spills: 12 bytes in the bf16 form of 64 channels x 8 images, none elsewhere.)  8 images,
+// 3975 points, 49 neighbours, us with 2 / 3 / 4 CTAs: 3 -> 64 channels 45 / 47 / 45, 1 -> 64 36 / 35 / 31, 4 -> 32 51 / 53 / 47; 64 images 3 -> 64 232 / 216 / 225.
+// Sixteen neighbours a pass with two lanes each, against thirty-two with one: 3 -> 64 55 -> 45, 3 -> 96 90 -> 57, one image 32 -> 25.
 constexpr int F32_POINTS = 8;     // output points (warps) per CTA
 constexpr int F32_NB = 16;        // neighbours staged per pass: two lanes each
 
@@ -361,7 +365,7 @@ __global__ void __launch_bounds__(F32_POINTS * 32, NO == 3 ? 2 : 4) knnconv_f32_
 
 // Launch of the kernel above.  Images per warp: the tiles of at most eight images are made equal and rounded up to 2, 4 or
 // 8; channels per CTA: 32, 64 or 96, whichever wastes the fewest lanes (the wider one on a tie).  The filter goes to shared memory
-// when a channel tile of it fits next to a second CTA on the SM (up to 64 KB), else it is read through L1.
+// when a channel tile of it is at most 64 KB (two CTAs per SM then, with the inputs; a 7 x 7 filter of 3 -> 64 channels is 37 KB), else it is read through L1.
 template <typename TX, int BT, int NO, int CT, bool WS>
 int launch_f32_few_t(const fovi_knnconv_plan* p, const void* X, int x_bnc, const float* Wt, const float* bias, float* Y, int y_bnc, int B,
                      int relu, size_t smem, cudaStream_t st) {

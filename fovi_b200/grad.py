@@ -1,15 +1,16 @@
-"""Backward pass of KNNConv on the forward tensor-core kernel.
+"""Backward pass of KNNConv on the tensor cores.
 
 Both gradient contractions of ``out[b,o,n] = sum_k sum_c Xpad[b,c,idx[k,n]] * W[o, c*V + tap[n,k]]``
 (fovi/arch/knn.py:538-557; the reference gets them from autograd through its gather, one-hot matmul and linear) are
-themselves table-driven gather-GEMMs, so each runs as a forward launch of ``fovi_knnconv_forward`` on a derived plan:
+themselves table-driven gather-GEMMs:
 
-* input gradient — the transposed layer: "output" points are the layer's input points m, the neighbours of m are the
+* input gradient — a forward launch of ``fovi_knnconv_forward`` on a derived plan, the transposed layer: "output" points are the layer's input points m, the neighbours of m are the
   output points n that list m, each with the tap it was given; channels swap roles
   (``dX[b,m,c] = sum_{(n,k): idx[k,n]=m} sum_o dY[b,n,o] * W[o, c*V + tap[n,k]]``).
 * weight gradient — the contraction runs over the batch, one product [c_out x c_in] per (output point, neighbour) pair, summed per filter tap
   (``dW[o,c,v] = sum_{(n,k): tap[n,k]=v} sum_b dY[b,n,o] * X[b,idx[k,n],c]``).  A kernel of its own (``csrc/knnconv_dw.cu``) reads both operands in the
-  layout the forward pass left them in: channels last, or the pair layout of a first layer with at most 4 channels.
+  layout the forward pass left them in: channels last (parts of a tap added in no fixed order, so repeated runs agree to float32 rounding), or the
+  pair layout of a first layer with at most 4 channels (added in a fixed order: the same bits every time).
 
 Operands are bf16 with float32 accumulation, as under the reference's autocast training.  Layers that run on the exact
 float32 kernel (``precision='fp32'``, or shapes outside the tensor-core kernel) take the same two derived layers through

@@ -170,7 +170,6 @@ int64_t fovi_knnconv_nnz(const fovi_knnconv_plan* plan);
  * W, dst: device pointers; size from fovi_knnconv_packed_weight_bytes. */
 int fovi_knnconv_pack_weights(const fovi_knnconv_plan* plan, const void* W, int w_dtype, void* dst, int dst_dtype,
                               void* stream);
-/* Bytes of the packed weight buffer for `dst_dtype`. */
 /* Packed operand of the TRANSPOSED layer (the input gradient): `plan` is the transposed layer's (c_out = the layer's c_in and the other way round), W
  * the layer's own weight [c_out][c_in * V]; same destination as fovi_knnconv_pack_weights(plan, ...) on the channel-transposed weight. */
 int fovi_knnconv_pack_weights_transposed(const fovi_knnconv_plan* plan, const void* W, int w_dtype, void* dst, int dst_dtype, void* stream);
@@ -179,6 +178,7 @@ int fovi_knnconv_pack_weights_transposed(const fovi_knnconv_plan* plan, const vo
  * channel and j the input channel; 1: the other way round.  Rows and columns past c_out / c_in are dropped. */
 int fovi_weight_grad_unpack(const float* src, int V, int n_i, int n_j, int swapped, int c_out, int c_in, void* dst, int dst_dtype, void* stream);
 
+/* Bytes of the packed weight buffer for `dst_dtype`. */
 int64_t fovi_knnconv_packed_weight_bytes(const fovi_knnconv_plan* plan, int dst_dtype);
 
 /* Grouped first layer.  With c_in <= 4 the MMA's N axis holds only c_out (64-96) columns; G consecutive output points can
@@ -193,7 +193,8 @@ int fovi_knnconv_pack_weights_grouped(const fovi_knnconv_plan* plan, const void*
 
 /* Convert activations [B,C,N] (x_dtype, contiguous) to a tensor-core input layout:
  * x_layout FOVI_X_BNC: [B,N,cp] bf16 with zero-filled pad channels (cp >= C, multiple of 8);
- * x_layout FOVI_X_PAIRS: [ceil(B/128),ceil(N/2),128,2,4] bf16 (C <= 4; cp ignored). */
+ * x_layout FOVI_X_PAIRS: [ceil(B/128),ceil(N/2),128,2,4] bf16 (C <= 4; cp ignored), the whole of it: the last tile's rows past B are written as
+ * zeros (the weight gradient reads them). */
 int fovi_pack_points(const void* x, int x_dtype, int B, int C, int N, void* dst, int cp, int x_layout, void* stream);
 
 /* Tensor-core path (tcgen05 MMA, bf16 operands, fp32 accumulation in tensor memory).
