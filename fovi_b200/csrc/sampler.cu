@@ -116,6 +116,9 @@ template <> __device__ __forceinline__ float smem_as_float<unsigned char>(const 
 // planar layouts of large batches, whose bound is the scattered stores: a tall strip can be visited ring by ring (see N_ORDERS) with few foreign
 // candidates.  512 images x 4 fixations, 256 x 256 float32: NARROW 131 us (nearest 128), WIDE 113 (101), where the copy rate gives 77; pair layout,
 // 256 images: 60 / 64, and 8 bf16 fixations of 1024 images 342 / 333.
+// What bounds the pair layout (NARROW) is the strips' own chain under the image stream, then the 8-byte stores, with the gathers last: 256 images x 4,
+// float32 67 us, without stores 54, without gathers 61, with neither 50 (the copy of the images alone: 31 at the copy rate); bf16 62 / 41 / 58 / 36 (15);
+// 1024 bf16 images of 224 x 224 x 8 326 / 209 / 320 / 153.  Planar, WIDE, 512 x 4: 118 / 101 / 103 / 86 (62).
 template <bool WIDE> struct StripShape {
   static constexpr int THREADS = WIDE ? 384 : 128, MIN_CTAS = WIDE ? 3 : 8, ROWS_MAX = WIDE ? 64 : 8, SMEM = (WIDE ? 72 : 27) * 1024;
 };
