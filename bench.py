@@ -33,7 +33,7 @@ CHANS = [3, 64, 192, 384, 256, 256]
 # dram__bytes_read.sum + dram__bytes_write.sum per launch from one ncu capture of this workload (256 images x 4 fixations,
 # captured directly: three metrics, one pass); sampler, then the five KNNConv launches.  `sources` is the hash of the kernel
 # sources the capture was taken on: when the sources change the figure is reported as null until the capture is redone.
-NCU_DRAM_TRAFFIC_MB = {"workload": (256, 4), "sources": "755e5d3a984b21c1", "sampler": 208.1, "conv": [220.2, 196.7, 225.7, 284.3, 207.0]}
+NCU_DRAM_TRAFFIC_MB = {"workload": (256, 4), "sources": "59fc4209eeb84ec4", "sampler": 208.7, "conv": [221.7, 194.8, 225.4, 287.7, 207.2]}
 METRIC = "images x fixations/s through sensor+KNNConv"
 UNIT = "img*fix/s"
 
@@ -689,7 +689,7 @@ def main():
                          "traffic_note": "DRAM bytes per launch, mean over this kernel's launches (ncu dram read+write; null when the kernel sources "
                                          "or the workload differ from the ones the capture was taken on)",
                          "peak_source": peaks["src"], "flops_per_launch_avg": dom_flops / n_dom, "ms_per_launch_avg": dom_ms / n_dom},
-            "roofline_all_knnconv": {"kernel": "all five KNNConv launches (first layer: fovi_knnconv_tc_kernel<PAIRS>)", "achieved": conv_tflops,
+            "roofline_all_knnconv": {"kernel": "all five KNNConv launches (first layer: fovi_knnconv_tc_pairs2_kernel)", "achieved": conv_tflops,
                                      "peak": peaks["bf16_tflops"], "unit": "TFLOP/s", "frac": conv_tflops / peaks["bf16_tflops"], "ms": float(conv_ms)},
             "layers": layer_rows,
             "sampler": {"kernel": "fovi_sample_strip_kernel", "ms": float(per[0]), "algorithmic_bytes_per_imgfix": samp_bytes_per, "mean_unique_pixels": mean_u,
