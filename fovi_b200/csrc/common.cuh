@@ -37,6 +37,13 @@ inline bool valid_dtype(int dt) { return dt == FOVI_F32 || dt == FOVI_BF16; }
 // Number of SMs of the current device (cached per device id).
 int sm_count();
 
+// Driver calls need the device's context current on the calling thread, and a thread that has made no runtime call of its own has none yet:
+// cuTensorMapEncodeTiled then answers CUDA_ERROR_INVALID_CONTEXT (201).  Selecting the current device again binds it.
+inline bool bind_context() {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+}
+
 }  // namespace fovi
 
 // ---- device-side element access shared by the kernels

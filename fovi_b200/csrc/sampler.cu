@@ -803,8 +803,13 @@ bool encode_image_map(CUtensorMap* m, const SampleArgs& a, size_t esz) {
   const cuuint64_t dims[4] = {row / 8, (cuuint64_t)a.H, (cuuint64_t)a.C, (cuuint64_t)a.B};
   const cuuint64_t strides[3] = {(cuuint64_t)a.sy * esz, (cuuint64_t)a.sc * esz, (cuuint64_t)a.sb * esz};
   const cuuint32_t box[4] = {(cuuint32_t)((row + 16) / 8), (cuuint32_t)(a.R + 1), (cuuint32_t)a.C, 1}, estr[4] = {1, 1, 1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, const_cast<void*>(a.img), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  auto encode = [&] {
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, const_cast<void*>(a.img), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT && fovi::bind_context()) r = encode();
+  return r == CUDA_SUCCESS;
 }
 
 template <typename TIn, typename TOut, int MODE, int PAD, bool WIDE>
