@@ -72,6 +72,11 @@ SIGNATURES = {
                                         C.c_int, _P]),
     "fovi_knnpool_forward": (C.c_int, [_P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P, _P]),
     "fovi_knnpool_backward": (C.c_int, [_P, _P, C.c_int, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P, _P]),
+    "fovi_points_to_channels": (C.c_int, [_P, _P, C.c_int, C.c_int, C.c_int, _P]),
+    "fovi_relu_pool_supported": (C.c_int, [C.c_int, _P]),
+    "fovi_relu_pool_forward": (C.c_int, [_P, C.c_int, C.c_int, C.c_int, C.c_int, _P, _P, _P, _P]),
+    "fovi_norm_block_workspace_bytes": (C.c_int64, [C.c_int, C.c_int, C.c_int]),
+    "fovi_norm_block_backward": (C.c_int, [_P, C.c_int, C.c_int, C.c_int, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, C.c_int64, _P]),
     "fovi_launch_count": (C.c_int64, []),
 }
 

@@ -7,15 +7,18 @@ shipped configuration, fovi/arch/norm.py:36-48, evaluated with its running stati
 packed weights and bias and ReLU runs in the convolution's epilogue; a per-sample norm (channel / coord / layer / group)
 runs as its own kernel behind the convolution with the ReLU fused into it; pooling is the gather-reduce kernel on the same
 channels-last layout, so activations stay in the kernels' layout from the sensor to the classifier.  Under autograd
-(training) the blocks run one by one: the convolution and the pooling with their own gradient kernels, the norm and the
-activation through torch as in the reference (batch norm with batch statistics in training mode).
+(training) the blocks run one by one: a block of the shipped form as one function (the norm's forward pass from torch, the rest and
+every gradient on the kernels), any other with the convolution's and the pooling's gradient kernels around torch's norm and activation.
 """
 import numpy as np
 import torch
 import torch.nn as nn
 
+from torch.nn.modules.module import _has_any_global_hook
+
 from . import ops
 from .coords import auto_match_num_coords, get_in_out_coords
+from .grad import block_autograd
 from .knn import KNNConvLayer, KNNPoolingLayer, get_knn_conv_layer
 from .norm import KNNBatchNorm, _KernelNorm, get_norm
 
@@ -106,9 +109,40 @@ class KNNAlexNetBlock(nn.Module):
     def _wants_grad(self, x):
         return torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in self.parameters()))
 
+    def _fused_training(self, x):
+        """True when the block's training step is one function on the kernels (grad.block_autograd): a bf16 KNNConv without bias, batch norm on batch
+        statistics with running ones, ReLU or nothing, max pooling or nothing, float32 in; and nobody listens between the modules (hooks, tracing)."""
+        conv, norm, act, pool = self.conv, self.norm, self.activation, self.pool
+        if type(conv) is not KNNConvLayer or type(norm) is not KNNBatchNorm or (act is not None and type(act) is not nn.ReLU):
+            return False
+        if conv.precision != "bf16" or not conv.plan.tc_supported or conv.bias is not None or not norm.training or norm.momentum is None:
+            return False
+        if not hasattr(torch, "_batch_norm_impl_index") or not ops.relu_pool_supported(conv.plan.n_out):
+            return False
+        if pool is not None and (type(pool) is not KNNPoolingLayer or pool.mode != "max" or not pool._plan.block_supported):
+            return False
+        params = (norm.weight, norm.bias, norm.running_mean, norm.running_var)
+        if any(t is None or t.dtype != torch.float32 or not t.is_contiguous() or t.data_ptr() % 16 or t.device != x.device or t.is_inference() for t in params):
+            return False
+        seen = norm.num_batches_tracked
+        if seen is None or seen.dtype != torch.int64 or seen.device != x.device or seen.is_inference():
+            return False
+        if x.dtype != torch.float32 or not x.is_cuda or x.dim() != 3 or not 0 < x.shape[0] < 65536 or conv.weight.device != x.device:
+            return False
+        rows = x.shape[0] * conv.plan.n_out
+        if rows < 2 or rows * (conv.out_channels // 4) >= 2 ** 31:
+            return False
+        if _has_any_global_hook() or torch.jit.is_tracing():
+            return False
+        return not any(m is not None and ("forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+                       for m in (conv, norm, act, pool))
+
     def _forward_train(self, x):
-        """The block under autograd: the convolution's own gradients (fovi_b200/grad.py), torch's norm and activation as in
-        the reference (batch norm with batch statistics in training mode), the pooling's own gradient."""
+        """The block under autograd.  In the shipped form everything from the convolution to the pooling is one function on the kernels; otherwise the
+        convolution's own gradients (fovi_b200/grad.py), torch's norm and activation as in the reference (batch norm with batch statistics in training
+        mode) and the pooling's own gradient.  Either way the result may be a channels-last view, as without gradients."""
+        if self._fused_training(x):
+            return block_autograd(self, x)
         if self.conv is not None:
             x = self.conv(x)
         if self.norm is not None:

@@ -4,18 +4,13 @@
 // Threads are laid out along the contiguous dimension of the activations (channels for the channels-last
 // layout, points for the reference's [B,C,N]), so every neighbour read of a warp is one or two cache lines
 // (channels-last) or a short gather (points-last).  NaN inputs are skipped like pads, as nanmean/nansum do.
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 
 #include <cuda_bf16.h>
 
-#include "common.cuh"
-
-struct fovi_knnpool_plan {
-  int n_in = 0, n_out = 0, K = 0;
-  int* idx = nullptr;   // [n_out, K] neighbour indices, pad = n_in
-  float* wgt = nullptr; // [n_out, K] neighbour weights of the 'gaussian' mode (null until set)
-};
+#include "knnpool_plan.cuh"
 
 namespace {
 
@@ -145,9 +140,24 @@ extern "C" int fovi_knnpool_plan_create(const int32_t* knn_idx_pad, int n_in, in
   p->n_in = n_in; p->n_out = n_out; p->K = K;
   cudaError_t e = cudaMalloc(&p->idx, sizeof(int) * t.size());
   if (e == cudaSuccess) e = cudaMemcpy(p->idx, t.data(), sizeof(int) * t.size(), cudaMemcpyHostToDevice);
+  if (K <= 255 && n_out < (1 << 23)) {
+    std::vector<int> start((size_t)n_in + 1, 0);
+    for (int j : t)
+      if (j < n_in) ++start[(size_t)j + 1];
+    for (int m = 0; m < n_in; ++m) start[m + 1] += start[m];
+    std::vector<int> at(start.begin(), start.end() - 1), entry(std::max(1, start[n_in]));
+    for (int n = 0; n < n_out; ++n)
+      for (int k = 0; k < K; ++k) {
+        const int j = t[(size_t)n * K + k];
+        if (j < n_in) entry[at[j]++] = n << 8 | k;
+      }
+    if (e == cudaSuccess) e = cudaMalloc(&p->t_start, sizeof(int) * start.size());
+    if (e == cudaSuccess) e = cudaMemcpy(p->t_start, start.data(), sizeof(int) * start.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&p->t_entry, sizeof(int) * entry.size());
+    if (e == cudaSuccess) e = cudaMemcpy(p->t_entry, entry.data(), sizeof(int) * entry.size(), cudaMemcpyHostToDevice);
+  }
   if (e != cudaSuccess) {
-    if (p->idx) cudaFree(p->idx);
-    delete p;
+    fovi_knnpool_plan_destroy(p);
     return fovi::cuda_fail(e, "fovi_knnpool_plan_create");
   }
   *out = p;
@@ -158,6 +168,8 @@ extern "C" void fovi_knnpool_plan_destroy(fovi_knnpool_plan* p) {
   if (!p) return;
   if (p->idx) cudaFree(p->idx);
   if (p->wgt) cudaFree(p->wgt);
+  if (p->t_start) cudaFree(p->t_start);
+  if (p->t_entry) cudaFree(p->t_entry);
   delete p;
 }
 

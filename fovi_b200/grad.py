@@ -21,7 +21,7 @@ import torch
 
 from . import ops
 
-__all__ = ["KnnConvGrad", "knnconv_autograd", "knnconv_points_autograd"]
+__all__ = ["KnnConvGrad", "knnconv_autograd", "knnconv_points_autograd", "block_autograd"]
 
 MAX_LIST = 256      # longest neighbour list the tensor-core kernel takes
 
@@ -265,6 +265,42 @@ class _KnnConvPointsFunction(torch.autograd.Function):
         elif gb is None:
             gb = ops.column_sum(gy) if gy.shape[-1] % 2 == 0 else gy.sum((0, 1), dtype=torch.float32)
         return gx, gw, gb, None, None
+
+
+class _BlockFunction(torch.autograd.Function):
+    """A block's convolution, training-mode batch norm, ReLU and max pooling (fovi/arch/knnalexnet.py:109-127).  The norm's forward pass is the module's own
+    (`torch._batch_norm_impl_index`, which torch's batch_norm calls), so the activations are those of the separate modules bit for bit; what surrounds it
+    and the whole way back run on the kernels of csrc/blocktrain.cu."""
+
+    @staticmethod
+    def forward(ctx, x, weight, gamma, beta, block):
+        conv, norm = block.conv, block.norm
+        ctx.block, ctx.pool = block, None if block.pool is None else block.pool._plan
+        relu = block.activation is not None
+        xp = ops.input_points(x, conv.plan)
+        y = conv.plan.forward(xp, conv.packed_weight(), None, out_dtype=torch.float32, batch=x.shape[0])
+        norm.num_batches_tracked.add_(1)
+        h, mean, rstd, _, _ = torch._batch_norm_impl_index(ops.points_to_channels(y), gamma, beta, norm.running_mean, norm.running_var, True, norm.momentum,
+                                                           norm.eps, torch.backends.cudnn.enabled)
+        out, arg = ops.relu_pool(h, relu, ctx.pool)
+        ctx.save_for_backward(xp if ctx.needs_input_grad[1] else None, weight, gamma, y, mean, rstd, out if relu and ctx.pool is None else None, arg)
+        return out.permute(0, 2, 1)
+
+    @staticmethod
+    def backward(ctx, gy):
+        xp, weight, gamma, y, mean, rstd, act, arg = ctx.saved_tensors
+        conv = ctx.block.conv
+        g = _aligned(gy.permute(0, 2, 1).to(torch.float32).contiguous())
+        dy, dgamma, dbeta = ops.norm_block_backward(y, mean, rstd, gamma, act, g, ctx.pool, arg)
+        need = ctx.needs_input_grad
+        gx = conv.grad_plans.input_grad(dy, weight).permute(0, 2, 1).to(torch.float32) if need[0] else None
+        gw = conv.grad_plans.weight_grad(dy, xp, conv.plan, weight.dtype) if need[1] else None
+        return gx, gw, dgamma if need[2] else None, dbeta if need[3] else None, None
+
+
+def block_autograd(block, x):
+    """The block's training step in one function; the caller has seen to it that the block is of that form."""
+    return _BlockFunction.apply(x, block.conv.weight, block.norm.weight, block.norm.bias, block)
 
 
 def knnconv_points_autograd(layer, x, relu):

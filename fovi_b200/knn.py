@@ -216,7 +216,7 @@ class KNNConvLayer(nn.Module):
     def _forward_packed(self, X_l):
         """(tensor-core forward of X_l, X_l in the kernel's layout)."""
         out_dtype = torch.float32 if X_l.dtype == torch.float32 else torch.bfloat16
-        xp = ops.pack_points(X_l, self._plan)
+        xp = ops.input_points(X_l, self._plan)
         y = self._plan.forward(xp, self.packed_weight(), self.bias, out_dtype=out_dtype, batch=X_l.shape[0])
         return y.permute(0, 2, 1).to(X_l.dtype), xp
 

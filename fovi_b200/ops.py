@@ -503,6 +503,7 @@ class KnnPoolPlan:
         with _on(self.device):
             check(lib.fovi_knnpool_plan_create(idx.ctypes.data_as(C.c_void_p), self.n_in, self.n_out, self.K, C.byref(h)), "fovi_knnpool_plan_create")
         self._h = h
+        self.block_supported = bool(lib.fovi_relu_pool_supported(self.n_in, h))      # relu_pool can use this plan
 
     def __del__(self):
         h, self._h = getattr(self, "_h", None), None
@@ -541,6 +542,54 @@ class KnnPoolPlan:
             check(lib.fovi_knnpool_backward(self._h, _ptr(x), _dt(x.dtype), _ptr(gy), _dt(gy.dtype), layout, B, Cc, POOL_MODES[mode], _ptr(dx), _stream()),
                   "fovi_knnpool_backward")
         return dx
+
+
+def points_to_channels(x):
+    """x [B,N,C] float32 contiguous -> [B,C,N] contiguous."""
+    _need_cuda(x)
+    assert x.dtype == torch.float32 and x.is_contiguous()
+    B, N, Cc = x.shape
+    out = torch.empty((B, Cc, N), dtype=torch.float32, device=x.device)
+    with _on(x.device):
+        check(lib.fovi_points_to_channels(_ptr(x), _ptr(out), B, N, Cc, _stream()), "fovi_points_to_channels")
+    return out
+
+
+def relu_pool_supported(n_points):
+    """True when `relu_pool` takes this many points without a pool (with one: KnnPoolPlan.block_supported)."""
+    return bool(lib.fovi_relu_pool_supported(n_points, None))
+
+
+def relu_pool(h, relu, pool=None):
+    """h [B,C,N] float32 contiguous -> ReLU (`relu`) and max pooling (`pool`, a KnnPoolPlan) -> (out [B,n_out,C] float32 channels last, list position of each
+    maximum [B,n_out,C] uint8 or None).  See fovi_relu_pool_forward."""
+    _need_cuda(h)
+    assert h.dtype == torch.float32 and h.is_contiguous() and (pool is None or pool.n_in == h.shape[2])
+    B, Cc, N = h.shape
+    out = torch.empty((B, N if pool is None else pool.n_out, Cc), dtype=torch.float32, device=h.device)
+    arg = None if pool is None else torch.empty(out.shape, dtype=torch.uint8, device=h.device)
+    with _on(h.device):
+        check(lib.fovi_relu_pool_forward(_ptr(h), B, N, Cc, int(relu), None if pool is None else pool._h, _ptr(out), None if arg is None else _ptr(arg), _stream()),
+              "fovi_relu_pool_forward")
+    return out, arg
+
+
+def norm_block_backward(y, mean, rstd, gamma, act, g, pool=None, arg=None):
+    """Gradient of batch norm (with the batch's statistics), ReLU and max pooling: y [B,N,C] the norm's input, act the ReLU's result or None, g [B,n_out,C], all
+    float32 contiguous -> (gradient of y as bf16 [B,N,C], dgamma [C], dbeta [C] float32).  See fovi_norm_block_backward."""
+    _need_cuda(y, mean, rstd, gamma, act, g, arg)
+    B, N, Cc = y.shape
+    assert all(t.dtype == torch.float32 and t.is_contiguous() for t in (y, mean, rstd, gamma, g)) and mean.shape == rstd.shape == gamma.shape == (Cc,)
+    assert g.shape == (B, N if pool is None else pool.n_out, Cc) and (act is None or (act.shape == y.shape and act.is_contiguous()))
+    dx = torch.empty((B, N, Cc), dtype=torch.bfloat16, device=y.device)
+    dgb = torch.empty((2, Cc), dtype=torch.float32, device=y.device)
+    nbytes = lib.fovi_norm_block_workspace_bytes(B, N, Cc)
+    work = torch.empty(nbytes, dtype=torch.uint8, device=y.device)
+    with _on(y.device):
+        check(lib.fovi_norm_block_backward(_ptr(y), B, N, Cc, _ptr(mean), _ptr(rstd), _ptr(gamma), None if act is None else _ptr(act),
+                                           None if pool is None else pool._h, None if arg is None else _ptr(arg), _ptr(g), _ptr(dgb), _ptr(dgb) + 4 * Cc,
+                                           _ptr(dx), _ptr(work), nbytes, _stream()), "fovi_norm_block_backward")
+    return dx, dgb[0], dgb[1]
 
 
 def knn_norm(x, mode, weight=None, bias=None, eps=1e-5, groups=1, layout=ACT_BCN, relu=False, out_dtype=None):
@@ -584,6 +633,16 @@ def pack_points(x, cp=8, x_layout=X_BNC):
     with _on(x.device):
         check(lib.fovi_pack_points(_ptr(x), _dt(x.dtype), B, Cc, N, _ptr(dst), cp, x_layout, _stream()), "fovi_pack_points")
     return dst
+
+
+def input_points(x, plan):
+    """x [B,C,N] in the layout `plan` consumes: pack_points, or for channels already contiguous (a channels-last view, as the layers return) the
+    conversion alone."""
+    if plan.x_layout != X_PAIRS and x.shape[1] == plan.cin_packed and x.dtype == torch.float32 and x.stride(1) == 1:
+        p = x.permute(0, 2, 1)
+        if p.is_contiguous():
+            return p.to(torch.bfloat16)
+    return pack_points(x, plan)
 
 
 def batch_to_inner(src, jp=None, bp=None, out=None):

@@ -407,6 +407,22 @@ int fovi_knnpool_forward(const fovi_knnpool_plan* plan, const void* X, int dtype
 int fovi_knnpool_backward(const fovi_knnpool_plan* plan, const void* X, int x_dtype, const void* gY, int g_dtype, int layout, int B,
                           int C, int mode, float* dX, void* stream);
 
+/* Between the batch norm of a training step and the next convolution.  float32 throughout; see csrc/blocktrain.cu.
+ * fovi_points_to_channels: [B,N,C] -> [B,C,N].
+ * fovi_relu_pool_forward: h [B,C,N] -> optional ReLU -> optional max pooling -> out [B,n_out,C] (n_out = N without a pool); arg: bytes [B,n_out,C], the list
+ *   position of each maximum, 255 where there is none or the ReLU stops it (null without a pool).  NaN as in fovi_knnpool_forward and ReLU.
+ *   fovi_relu_pool_supported: 0 where a channel's points do not fit, or the pool has more than 255 neighbours.
+ * fovi_norm_block_backward: the gradient of batch norm (batch statistics mean, rstd = 1/std), ReLU and pooling: y [B,N,C] the norm's input, act the ReLU's
+ *   result [B,N,C] (null without a ReLU, or with a pool, whose arg holds the mask), g [B,n_out,C] -> dgamma, dbeta [C] and dx, the gradient with respect to y, as
+ *   bf16 [B,N,C].  C a multiple of 4, pointers 16-byte aligned, work: fovi_norm_block_workspace_bytes.  Sums in a fixed order. */
+int fovi_points_to_channels(const float* src, float* dst, int B, int N, int C, void* stream);
+int fovi_relu_pool_supported(int N, const fovi_knnpool_plan* pool);
+int fovi_relu_pool_forward(const float* h, int B, int N, int C, int relu, const fovi_knnpool_plan* pool, float* out, unsigned char* arg, void* stream);
+int64_t fovi_norm_block_workspace_bytes(int B, int N, int C);
+int fovi_norm_block_backward(const float* y, int B, int N, int C, const float* mean, const float* rstd, const float* gamma, const float* act,
+                             const fovi_knnpool_plan* pool, const unsigned char* arg, const float* g, float* dgamma, float* dbeta, void* dx, void* work,
+                             int64_t work_bytes, void* stream);
+
 /* Number of kernels this library has launched from the calling process (all entry points). */
 int64_t fovi_launch_count(void);
 
