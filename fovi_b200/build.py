@@ -1,18 +1,22 @@
 """Build recipe of the native library: ``python -m fovi_b200.build``.
 
 Compiles ``fovi_b200/csrc/*.cu`` with nvcc for sm_100a (one object per source, in parallel, only the
-stale ones) and links them into ``fovi_b200/libfovi_b200.so`` (in-tree; objects and the shared object
-are not committed).
+stale ones) and links them into ``fovi_b200/libfovi_b200.so``; ``csrc/bind.cpp``, the launch path for torch
+tensors, becomes the extension module ``fovi_b200/_native.so`` (both in-tree; objects and shared objects are not
+committed).
 """
 import os
+import importlib.util
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libfovi_b200.so")
+NATIVE = os.path.join(HERE, "_native.so")
 SOURCES = ["capi.cu", "sampler.cu", "knnconv.cu", "knnconv_tc.cu", "knnconv_tc2.cu", "knnconv_tcp.cu", "knnpool.cu", "knnnorm.cu", "blocktrain.cu", "fused.cu", "tables.cu", "geometry.cu", "grad.cu", "knnconv_dw.cu", "depthwise.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 
@@ -22,6 +26,21 @@ def _headers_mtime():
     hs.append(os.path.join(HERE, "..", "include", "fovi_b200.h"))
     hs.append(os.path.abspath(__file__))
     return max(os.path.getmtime(h) for h in hs)
+
+
+def build_native(force=False):
+    """The extension module of the launch path, against the torch that is installed.  Returns its path."""
+    src = os.path.join(CSRC, "bind.cpp")
+    torch = importlib.util.find_spec("torch").submodule_search_locations[0]
+    newest = max(os.path.getmtime(f) for f in (src, os.path.join(HERE, "..", "include", "fovi_b200.h"), os.path.abspath(__file__), os.path.join(torch, "version.py")))
+    if force or not os.path.exists(NATIVE) or os.path.getmtime(NATIVE) < newest:
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-I{torch}/include", f"-I{torch}/include/torch/csrc/api/include",
+               "-I" + sysconfig.get_paths()["include"], src, "-o", NATIVE, f"-L{torch}/lib", "-lc10", "-ltorch_cpu", "-ltorch_python"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError("compiling bind.cpp failed")
+    return NATIVE
 
 
 def build(force=False, verbose=False, defines=(), lib=None, obj_dir=None):
@@ -54,6 +73,8 @@ def build(force=False, verbose=False, defines=(), lib=None, obj_dir=None):
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("linking libfovi_b200.so failed")
+    if lib == LIB:
+        build_native(force)
     return lib
 
 

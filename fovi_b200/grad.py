@@ -128,7 +128,7 @@ class KnnConvGrad:
         if plan.x_layout == ops.X_PAIRS:
             return ops.weight_grad_unpack(plan.weight_grad_pairs(gy_points, x_points), self.c_out, self.c_in, dtype=dtype)
         p, q = (x_points, gy_points) if self.dw_swapped else (gy_points, x_points)
-        return ops.weight_grad_unpack(self.dw_plan()[0].run(p, q), self.c_out, self.c_in, swapped=self.dw_swapped, dtype=dtype)
+        return ops.weight_grad(self.dw_plan()[0], p, q, self.c_out, self.c_in, self.dw_swapped, dtype)
 
     # ---- exact float32 route (precision='fp32' layers and shapes outside the tensor-core kernel): the same two derived
     # layers, run on the exact float32 kernel (fovi_knnconv_forward_f32) instead of the tensor cores
@@ -274,15 +274,12 @@ class _BlockFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, weight, gamma, beta, block):
-        conv, norm = block.conv, block.norm
+        conv, norm = block.conv, block.norm                 # (gamma and beta are the norm's)
         ctx.block, ctx.pool = block, None if block.pool is None else block.pool._plan
         relu = block.activation is not None
         xp = ops.input_points(x, conv.plan)
         y = conv.plan.forward(xp, conv.packed_weight(), None, out_dtype=torch.float32, batch=x.shape[0])
-        norm.num_batches_tracked.add_(1)
-        h, mean, rstd, _, _ = torch._batch_norm_impl_index(ops.points_to_channels(y), gamma, beta, norm.running_mean, norm.running_var, True, norm.momentum,
-                                                           norm.eps, torch.backends.cudnn.enabled)
-        out, arg = ops.relu_pool(h, relu, ctx.pool)
+        mean, rstd, out, arg = ops.block_forward(y, norm, relu, ctx.pool)
         ctx.save_for_backward(xp if ctx.needs_input_grad[1] else None, weight, gamma, y, mean, rstd, out if relu and ctx.pool is None else None, arg)
         return out.permute(0, 2, 1)
 

@@ -5,7 +5,13 @@ import ctypes as C
 import numpy as np
 import torch
 
-from ._lib import lib, check
+from ._lib import SIGNATURES, check, lib
+
+try:      # the launch path in native code (csrc/bind.cpp); without it every call takes the Python path below
+    from . import _native
+    _native.connect({name: C.cast(getattr(lib, name), C.c_void_p).value for name in SIGNATURES})
+except ImportError:
+    _native = None
 
 F32, BF16, U8 = 0, 1, 2
 NEAREST, BILINEAR = 0, 1
@@ -64,6 +70,13 @@ def _need_cuda(*ts):
             raise ValueError("fovi_b200 kernels need CUDA tensors; there is no CPU path")
 
 
+def _checked(got, where):
+    """A native call's result; a status of the C ABI comes back as an int."""
+    if got.__class__ is int:
+        check(got, where)
+    return got
+
+
 def _bias_f32(bias):
     """The bias as the kernels read it: float32 and contiguous."""
     return bias if bias.dtype == torch.float32 and bias.is_contiguous() else bias.detach().to(torch.float32).contiguous()
@@ -110,6 +123,12 @@ def sample(plan, img, fix_rc, fix_hw, mode=BILINEAR, pad=PAD_ZEROS, out_dtype=No
     tensor in `layout`: [B,F,C,N], [F,B,C,N], [B,F,N,Cp], [F,B,N,Cp], or the pair layout
     [ceil(rows/128), ceil(N/2), 128, 8] (rows = F*B or B*F) that a KNNConv plan with c_in <= 4
     consumes; rows past the last one are left unwritten."""
+    if _native is not None and out is None and img.is_cuda:
+        dev = _current_device()
+        got = _native.sample(plan._h.value, plan.n_points, img, fix_rc, fix_hw, mode, pad, -1 if out_dtype is None else _DT.get(out_dtype, -2), layout,
+                             channel_stride or 0, dev, _raw_stream(dev))
+        if got is not None:
+            return _checked(got, "fovi_sample_forward")
     _need_cuda(img, fix_rc, fix_hw)
     B, Cc, H, W = img.shape
     if fix_rc.dtype == torch.float32 and fix_hw.dtype == torch.float32 and fix_rc.is_contiguous() and fix_hw.is_contiguous():
@@ -217,6 +236,9 @@ class KnnConvPlan:
         self.group, self._hg, self._member_tap = 1, None, None
         if self.x_layout == X_PAIRS and self.tc_supported and group != 1:
             self._make_grouped(idx, tp, (int(group),) if group else (4, 3, 2))
+        # the shapes of `forward`'s operands behind the batch, as the native call takes them
+        self._forward_shapes = ((self.n_pairs, 0, self.n_out // self.group, self.group * self.c_out, 8, 1, n_out, self.c_out) if self.x_layout == X_PAIRS
+                                else (self.n_in, self.cin_packed, self.V, self.c_out, self.cin_packed, 0, n_out, self.c_out))
 
     def _make_grouped(self, idx, tp, candidates):
         """A second plan whose "points" are groups of G consecutive output points (G*c_out channels side by side) and whose
@@ -262,6 +284,12 @@ class KnnConvPlan:
     def pack_weights(self, weight, dtype=torch.bfloat16):
         """weight [c_out, c_in*V] (KNNConvLayer.weight) -> packed operand: slabs [V, c_out, cin_packed], or
         (bf16, pair layout) per-output-point slabs [n_out, pair_slots, c_out, 8]."""
+        if _native is not None and weight.is_cuda and (self.x_layout != X_PAIRS or dtype != torch.bfloat16):
+            dev = _current_device()
+            got = _native.pack_slabs(self._h.value, weight, self.c_out, self.c_in * self.V, self.V, self.c_out, self.cin_packed, _DT.get(dtype, -2), 0, dev,
+                                     _raw_stream(dev))
+            if got is not None:
+                return _checked(got, "fovi_knnconv_pack_weights")
         _need_cuda(weight)
         weight = weight.detach().contiguous()
         assert weight.shape == (self.c_out, self.c_in * self.V)
@@ -286,6 +314,11 @@ class KnnConvPlan:
     def pack_weights_transposed(self, weight):
         """This plan is the transposed layer of one whose weight is [c_in, c_out*V] (this plan's channel counts): its bf16 operand, as
         `pack_weights` gives it for the channel-transposed weight."""
+        if _native is not None and weight.is_cuda and self.x_layout != X_PAIRS:
+            dev = _current_device()
+            got = _native.pack_slabs(self._h.value, weight, self.c_in, self.c_out * self.V, self.V, self.c_out, self.cin_packed, BF16, 1, dev, _raw_stream(dev))
+            if got is not None:
+                return _checked(got, "fovi_knnconv_pack_weights_transposed")
         _need_cuda(weight)
         weight = weight.detach().contiguous()
         assert weight.shape == (self.c_in, self.c_out * self.V) and self.x_layout != X_PAIRS
@@ -298,6 +331,12 @@ class KnnConvPlan:
     def forward(self, x_bnc, wt, bias=None, relu=False, out_dtype=torch.bfloat16, out=None, batch=None):
         """Tensor-core path.  x_bnc: bf16 contiguous, [B,n_in,cin_packed] or (pair layout)
         [ceil(B/128),n_pairs,128,8] with `batch` = B  ->  [B,n_out,c_out]."""
+        if _native is not None and out is None and x_bnc.is_cuda:
+            dev = _current_device()
+            rows = x_bnc.shape[0] if self.x_layout != X_PAIRS else x_bnc.shape[0] * 128 if batch is None else int(batch)
+            got = _native.conv_forward(self._h_tc.value, x_bnc, wt, bias, int(relu), _DT.get(out_dtype, -2), rows, *self._forward_shapes, dev, _raw_stream(dev))
+            if got is not None:
+                return _checked(got, "fovi_knnconv_forward")
         _need_cuda(x_bnc, wt, bias)
         assert x_bnc.dtype == torch.bfloat16 and x_bnc.is_contiguous() and wt.dtype == torch.bfloat16 and wt.is_contiguous()
         if self.x_layout == X_PAIRS:
@@ -348,6 +387,11 @@ class KnnConvPlan:
 
     def forward_f32(self, x, wt_f32, bias=None, relu=False, x_layout=ACT_BCN, y_layout=ACT_BCN):
         """Exact float32 path.  x [B,c_in,n_in] (BCN) or [B,n_in,c_in] (BNC)."""
+        if _native is not None and x.is_cuda and not relu and x_layout == y_layout == ACT_BCN:
+            dev = _current_device()
+            got = _native.conv_forward_f32(self._h.value, x, wt_f32, bias, self.n_in, self.c_in, self.V, self.cin_packed, self.n_out, self.c_out, dev, _raw_stream(dev))
+            if got is not None:
+                return _checked(got, "fovi_knnconv_forward_f32")
         _need_cuda(x, wt_f32, bias)
         x = x.contiguous()
         B = x.shape[0]
@@ -447,6 +491,16 @@ def weight_grad_unpack(src, c_out, c_in, swapped=False, dtype=torch.float32):
     with _on(src.device):
         check(lib.fovi_weight_grad_unpack(_ptr(src), V, n_i, n_j, int(swapped), c_out, c_in, _ptr(dst), _dt(dtype), _stream()), "fovi_weight_grad_unpack")
     return dst
+
+
+def weight_grad(plan, p, q, c_out, c_in, swapped=False, dtype=torch.float32):
+    """`KnnDwPlan.run` and `weight_grad_unpack` in one call: p [B,n_p,cp], q [B,n_q,cq] bf16 -> [c_out, c_in*V] in `dtype`."""
+    if _native is not None and p.is_cuda:
+        dev = _current_device()
+        got = _native.weight_grad(plan._h.value, p, q, plan.n_p, plan.n_q, plan.V, c_out, c_in, int(swapped), _DT.get(dtype, -2), dev, _raw_stream(dev))
+        if got is not None:
+            return _checked(got, "fovi_knndw_run")
+    return weight_grad_unpack(plan.run(p, q), c_out, c_in, swapped=swapped, dtype=dtype)
 
 
 class KnnDwPlan:
@@ -574,9 +628,31 @@ def relu_pool(h, relu, pool=None):
     return out, arg
 
 
+def block_forward(y, norm, relu, pool=None):
+    """A training block behind its convolution: y [B,N,C] float32 channels last -> batch norm (the module `norm`, whose running statistics are updated), ReLU
+    (`relu`), max pooling (`pool`) -> (mean [C], 1/std [C], out [B,n_out,C] float32 channels last, list position of each maximum or None).  The norm is what
+    torch's batch_norm calls, on [B,C,N]."""
+    gamma, beta, cudnn = norm.weight, norm.bias, torch.backends.cudnn.enabled
+    if _native is not None and y.is_cuda:
+        dev = _current_device()
+        got = _native.block_forward(y, gamma, beta, norm.running_mean, norm.running_var, norm.num_batches_tracked, norm.momentum, norm.eps, int(cudnn), int(relu),
+                                    None if pool is None else pool._h.value, y.shape[1] if pool is None else pool.n_out, dev, _raw_stream(dev))
+        if got is not None:
+            return _checked(got, "fovi_relu_pool_forward")
+    norm.num_batches_tracked.add_(1)
+    h, mean, rstd, _, _ = torch._batch_norm_impl_index(points_to_channels(y), gamma, beta, norm.running_mean, norm.running_var, True, norm.momentum, norm.eps, cudnn)
+    out, arg = relu_pool(h, relu, pool)
+    return mean, rstd, out, arg
+
+
 def norm_block_backward(y, mean, rstd, gamma, act, g, pool=None, arg=None):
     """Gradient of batch norm (with the batch's statistics), ReLU and max pooling: y [B,N,C] the norm's input, act the ReLU's result or None, g [B,n_out,C], all
     float32 contiguous -> (gradient of y as bf16 [B,N,C], dgamma [C], dbeta [C] float32).  See fovi_norm_block_backward."""
+    if _native is not None and y.is_cuda and (pool is None or g.shape[1] == pool.n_out):
+        dev = _current_device()
+        got = _native.block_backward(y, mean, rstd, gamma, act, arg, g, None if pool is None else pool._h.value, dev, _raw_stream(dev))
+        if got is not None:
+            return _checked(got, "fovi_norm_block_backward")
     _need_cuda(y, mean, rstd, gamma, act, g, arg)
     B, N, Cc = y.shape
     assert all(t.dtype == torch.float32 and t.is_contiguous() for t in (y, mean, rstd, gamma, g)) and mean.shape == rstd.shape == gamma.shape == (Cc,)
@@ -623,9 +699,14 @@ def knn_norm(x, mode, weight=None, bias=None, eps=1e-5, groups=1, layout=ACT_BCN
 def pack_points(x, cp=8, x_layout=X_BNC):
     """x [B,C,N] float32/bf16 -> tensor-core input: [B,N,cp] bf16 (pad channels zero) or the pair
     layout [ceil(B/128),ceil(N/2),128,8].  Pass a KnnConvPlan as `cp` to get the layout that plan consumes."""
-    _need_cuda(x)
     if isinstance(cp, KnnConvPlan):
         cp, x_layout = cp.cin_packed, cp.x_layout
+    if _native is not None and x.is_cuda:
+        dev = _current_device()
+        got = _native.pack_points(x, cp, x_layout, dev, _raw_stream(dev))
+        if got is not None:
+            return _checked(got, "fovi_pack_points")
+    _need_cuda(x)
     x = x.contiguous()
     B, Cc, N = x.shape
     shape = ((B + 127) // 128, (N + 1) // 2, 128, 8) if x_layout == X_PAIRS else (B, N, cp)

@@ -202,7 +202,8 @@ class RetinalTransform(nn.Module):
         """x [B,C,H,W] -> [B,C,N] in ``self.dtype`` (retina.py:118-156); with fix_loc [B,F,2] -> [B,F,C,N].  Differentiable
         with respect to the images (the gradient kernel scatters onto the footprints with the forward's weights)."""
         fix_loc, fixation_size = self._defaults(fix_loc, fixation_size)
-        return self.sampler(x, fix_loc=fix_loc, fixation_size=fixation_size).to(self.dtype)
+        y = self.sampler(x, fix_loc=fix_loc, fixation_size=fixation_size)
+        return y if y.dtype is self.dtype else y.to(self.dtype)
 
     @torch.no_grad()
     def forward_points(self, x, fix_loc, fixation_size=None, conv_plan=None, out=None, row_order="fb"):
