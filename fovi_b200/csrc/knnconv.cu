@@ -221,9 +221,8 @@ __global__ void pack_points_kernel(const TX* __restrict__ x, __nv_bfloat16* __re
 // Persistent CTAs, so that the filter is staged once.  One accumulator per output, neighbours in list order, channels inside: the
 // sums are those of the general kernel below, bit for bit.
 // CTAs per SM (register limit): up to 64 registers hold the accumulators of 32 or 64 channels, so four CTAs hide the gathers of each other's passes;
-// 96 channels x 8 images take up to 127 registers, two CTAs.  (Spills: 12 bytes in the bf16 form of 64 channels x 8 images, none elsewhere.)  8 images,
-// 3975 points, 49 neighbours, us with 2 / 3 / 4 CTAs: 3 -> 64 channels 45 / 47 / 45, 1 -> 64 36 / 35 / 31, 4 -> 32 51 / 53 / 47; 64 images 3 -> 64 232 / 216 / 225.
-// Sixteen neighbours a pass with two lanes each, against thirty-two with one: 3 -> 64 55 -> 45, 3 -> 96 90 -> 57, one image 32 -> 25.
+// 96 channels x 8 images take up to 127 registers, two CTAs.  Serves tiles of one or two images, and filters that do not fit shared memory; the others take
+// the kernel below.
 constexpr int F32_POINTS = 8;     // output points (warps) per CTA
 constexpr int F32_NB = 16;        // neighbours staged per pass: two lanes each
 
@@ -363,6 +362,171 @@ __global__ void __launch_bounds__(F32_POINTS * 32, NO == 3 ? 2 : 4) knnconv_f32_
   }
 }
 
+// The same for more than two images and a filter that fits shared memory: four points per warp, eight lanes each.
+//
+// What bounds the kernel above is the load/store pipe (72 % while an SM is busy), not the FMAs: a warp-wide broadcast of 16 bytes costs as long as 32 lanes'
+// worth of data, so a (neighbour, channel) step of 64 channels x 8 images takes 10 clocks of shared-memory reads for 4 of FMAs; and 497 CTAs of eight points
+// leave a quarter of the SMs' time empty, each with its own copy of the filter.  Here a lane holds CPL channels x BT images of one point, so that a step reads
+// 16 clocks' worth for FOUR points; a CTA per SM holds the filter once, and its warps walk the quads of points of its share, which differ by one at most.  The
+// eight lanes of a point gather eight neighbours at a time into registers, while the eight before are multiplied; the lanes of a warp then fetch the same
+// image and channel of four neighbouring points' neighbours, which share lines.  Sums as above, in the same order, bit for bit.
+// 3975 points, 49 neighbours, float32, us before -> here: 3 -> 64 channels 3 images 25 -> 17, 8 38 -> 25, 16 64 -> 49, 64 217 -> 145; 3 -> 32, 8 images 27 -> 18;
+// 3 -> 96 50 -> 34; 9 neighbours, 3 -> 64, 8 images 13 -> 10.  (Sixteen warps and 128 registers, 64 channels x 8 images: 29, 88 bytes spilled; neighbours staged by
+// 4-byte asynchronous copies, which conflict in shared memory, in CTAs of four warps: 37.)
+constexpr int QUAD_NB = 8;                   // neighbours per pass
+template <int BT, int CPL> struct QuadShape { static constexpr int WARPS = BT * CPL >= 64 ? 12 : 16; };
+
+__host__ __device__ constexpr int quad_stride(int C, int BT) { return C * BT + (C * BT / 4 % 2 ? 0 : 4); }     // floats of a staged neighbour: an odd number of 16-byte pieces
+
+template <typename TX, int BT, int CPL, int CT>
+__global__ void __launch_bounds__(QuadShape<BT, CPL>::WARPS * 32, 1) knnconv_f32_quad_kernel(const TX* __restrict__ X, const float* __restrict__ Wt, const float* __restrict__ bias,
+                                                                                           float* __restrict__ Y, const int* __restrict__ nbr_idx,
+                                                                                           const uint16_t* __restrict__ nbr_tap, const int* __restrict__ nbr_cnt, int kp,
+                                                                                           int B, int n_in, int n_out, int c_in, int c_out, int cp, int V, int relu,
+                                                                                           int x_bnc, int y_bnc, int n_ot, int n_bt, int total) {
+  extern __shared__ __align__(16) float f32_smem[];
+  constexpr int OT = CPL * 8, WARPS = QuadShape<BT, CPL>::WARPS, CMAX = CT ? CT : 4;
+  const int C = CT ? CT : c_in;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane >> 3, i = lane & 7;
+  const int stride = quad_stride(C, BT);
+  float* ws = f32_smem;                                                   // [V][C][OT]
+  float* xs = f32_smem + V * C * OT + (warp * 4 + q) * QUAD_NB * stride;  // [neighbour][channel][BT images] of this lane's point
+  const int ot = blockIdx.x % n_ot, o0 = ot * OT, share = blockIdx.x / n_ot, shares = gridDim.x / n_ot;      // the grid is a multiple of n_ot
+  // a warp per (tap, 32 channels): consecutive lanes read consecutive rows of the tap's slab
+#pragma unroll 4
+  for (int r = warp; r < V * (OT / 32); r += WARPS) {
+    const int v = r / (OT / 32), o = (r - v * (OT / 32)) * 32 + lane;
+    const float* src = Wt + ((long long)v * c_out + o0 + o) * cp;
+#pragma unroll
+    for (int c = 0; c < CMAX; ++c)
+      if (CT || c < C) ws[(v * C + c) * OT + o] = o0 + o < c_out ? __ldg(src + c) : 0.f;
+  }
+  __syncthreads();
+  const int last = (int)((long long)total * (share + 1) / shares);
+  for (int t = (int)((long long)total * share / shares) + warp; t < last; t += WARPS) {
+    const int bt = t % n_bt, n = t / n_bt * 4 + q, b0 = bt * BT, nb = min(BT, B - b0);
+    const int cnt = n < n_out ? __ldg(nbr_cnt + n) : 0;
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    const long long row = (long long)n * kp;
+    int j_next = 0, tap_next = 0, tap = 0;
+    float g[CMAX][BT];
+    auto fetch = [&](int k0) {                                            // this lane's neighbour of the pass at k0
+      if (k0 + i < cnt) { j_next = __ldg(nbr_idx + row + k0 + i); tap_next = __ldg(nbr_tap + row + k0 + i); }
+    };
+    auto gather = [&](int k0) {
+      if (k0 + i < cnt) {
+        const TX* src = X + (x_bnc ? ((long long)b0 * n_in + j_next) * c_in : (long long)b0 * c_in * n_in + j_next);
+        const long long per_c = x_bnc ? 1 : n_in, per_b = (long long)c_in * n_in;
+#pragma unroll
+        for (int b = 0; b < BT; ++b) {
+#pragma unroll
+          for (int c = 0; c < CMAX; ++c)
+            if (CT || c < C) g[c][b] = b < nb ? ld_as_float(src + c * per_c) : 0.f;
+          src += per_b;                                                   // (not read past the batch)
+        }
+      }
+    };
+    auto put = [&]() {
+#pragma unroll
+      for (int c = 0; c < CMAX; ++c)
+        if (CT || c < C) {
+#pragma unroll
+          for (int b = 0; b < BT; b += 4)
+            *reinterpret_cast<float4*>(xs + i * stride + c * BT + b) = make_float4(g[c][b], g[c][b + 1], g[c][b + 2], g[c][b + 3]);
+        }
+    };
+    float acc[CPL][BT];
+#pragma unroll
+    for (int o = 0; o < CPL; ++o)
+#pragma unroll
+      for (int b = 0; b < BT; ++b) acc[o][b] = 0.f;
+#pragma unroll
+    for (int c = 0; c < CMAX; ++c)
+#pragma unroll
+      for (int b = 0; b < BT; ++b) g[c][b] = 0.f;
+    fetch(0);
+    gather(0);
+    tap = tap_next;
+    fetch(QUAD_NB);
+    put();
+    __syncwarp();
+    for (int k0 = 0; k0 < most; k0 += QUAD_NB) {
+      const bool more = k0 + QUAD_NB < most;
+      const int tap_here = tap;
+      if (more) {
+        gather(k0 + QUAD_NB);
+        tap = tap_next;
+        fetch(k0 + 2 * QUAD_NB);
+      }
+#pragma unroll 1
+      for (int k = 0; k < min(QUAD_NB, most - k0); ++k) {
+        const int tp = __shfl_sync(0xffffffffu, tap_here, (lane & 24) + k);
+        if (k0 + k >= cnt) continue;                                      // this point's list is shorter than a neighbour's
+        const float* wr = ws + tp * C * OT + 4 * i;
+        const float* xr = xs + k * stride;
+#pragma unroll
+        for (int c = 0; c < CMAX; ++c) {
+          if (CT == 0 && c >= C) break;
+          float w[CPL], x[BT];
+#pragma unroll
+          for (int u = 0; u < CPL / 4; ++u) {
+            const float4 v = *reinterpret_cast<const float4*>(wr + c * OT + u * 32);
+            w[4 * u] = v.x; w[4 * u + 1] = v.y; w[4 * u + 2] = v.z; w[4 * u + 3] = v.w;
+          }
+#pragma unroll
+          for (int b = 0; b < BT; b += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(xr + c * BT + b);
+            x[b] = v.x; x[b + 1] = v.y; x[b + 2] = v.z; x[b + 3] = v.w;
+          }
+#pragma unroll
+          for (int o = 0; o < CPL; ++o)
+#pragma unroll
+            for (int b = 0; b < BT; ++b) acc[o][b] = fmaf(x[b], w[o], acc[o][b]);
+        }
+      }
+      __syncwarp();                                                       // the pass has been read
+      if (more) {
+        put();
+        __syncwarp();
+      }
+    }
+    if (n < n_out) {
+#pragma unroll
+      for (int o = 0; o < CPL; ++o) {
+        const int oc = o0 + (o >> 2) * 32 + 4 * i + (o & 3);
+        if (oc < c_out) {
+          const float bo = bias ? __ldg(bias + oc) : 0.f;
+          float* d = Y + (y_bnc ? ((long long)b0 * n_out + n) * c_out + oc : ((long long)b0 * c_out + oc) * n_out + n);   // (planar: four points' results side by side)
+#pragma unroll
+          for (int b = 0; b < BT; ++b) {
+            float v = acc[o][b];
+            if (bias) v += bo;
+            if (relu) v = fmaxf(v, 0.f);
+            if (b < nb) d[(long long)b * c_out * n_out] = v;
+          }
+        }
+      }
+    }
+    __syncwarp();                                                         // (the next quad's neighbours go where this one's were)
+  }
+}
+
+template <typename TX, int BT, int CPL, int CT>
+int launch_f32_quad_t(const fovi_knnconv_plan* p, const void* X, int x_bnc, const float* Wt, const float* bias, float* Y, int y_bnc, int B, int relu,
+                      cudaStream_t st) {
+  auto k = knnconv_f32_quad_kernel<TX, BT, CPL, CT>;
+  constexpr int WARPS = QuadShape<BT, CPL>::WARPS;
+  const int n_ot = (p->c_out + CPL * 8 - 1) / (CPL * 8), n_bt = (B + BT - 1) / BT;
+  const long long total = (long long)((p->n_out + 3) / 4) * n_bt;
+  if (total >= (1ll << 31)) return FOVI_ERR_UNSUPPORTED;
+  const size_t smem = sizeof(float) * ((size_t)p->V * p->c_in * CPL * 8 + (size_t)WARPS * 4 * QUAD_NB * quad_stride(p->c_in, BT));
+  if (smem > 48 * 1024) FOVI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int grid = n_ot * (int)std::min<long long>(total, std::max(1, fovi::sm_count() / n_ot));
+  k<<<grid, WARPS * 32, smem, st>>>((const TX*)X, Wt, bias, Y, p->nbr_idx, p->nbr_tap, p->nbr_cnt, p->kp, B, p->n_in, p->n_out, p->c_in, p->c_out,
+                                    p->cin_packed, p->V, relu, x_bnc, y_bnc, n_ot, n_bt, (int)total);
+  return fovi::after_launch("knnconv_f32_quad_kernel");
+}
+
 // Launch of the kernel above.  Images per warp: the tiles of at most eight images are made equal and rounded up to 2, 4 or
 // 8; channels per CTA: 32, 64 or 96, whichever wastes the fewest lanes (the wider one on a tie).  The filter goes to shared memory
 // when a channel tile of it is at most 64 KB (two CTAs per SM then, with the inputs; a 7 x 7 filter of 3 -> 64 channels is 37 KB), else it is read through L1.
@@ -396,16 +560,23 @@ int launch_f32_few(const fovi_knnconv_plan* p, const void* X, int x_bnc, const f
   const size_t wbytes = sizeof(float) * (size_t)p->V * p->c_in * no * 32;
   const bool ws = wbytes <= 64 * 1024;
   const size_t smem = base + (ws ? wbytes : 0);
+  // four points per warp where the filter is in shared memory and a lane's tile is more than two images (see the kernel)
+#define QUAD(BT_, CPL_) do { if (p->c_in == 3) return launch_f32_quad_t<TX, BT_, CPL_, 3>(p, X, x_bnc, Wt, bias, Y, y_bnc, B, relu, st);    \
+                             return launch_f32_quad_t<TX, BT_, CPL_, 0>(p, X, x_bnc, Wt, bias, Y, y_bnc, B, relu, st); } while (0)
+#define QUAD_NO(BT_) do { if (no == 1) QUAD(BT_, 4); else if (no == 2) QUAD(BT_, 8); else QUAD(BT_, 12); } while (0)
+  if (ws && bt == 8) QUAD_NO(8);
+  if (ws && bt == 4) QUAD_NO(4);
+#undef QUAD_NO
+#undef QUAD
 #define GO(BT_, NO_, CT_, WS_) return launch_f32_few_t<TX, BT_, NO_, CT_, WS_>(p, X, x_bnc, Wt, bias, Y, y_bnc, B, relu, smem, st)
-#define GO_WS(BT_, NO_, CT_) do { if (ws) GO(BT_, NO_, CT_, true); else GO(BT_, NO_, CT_, false); } while (0)
-#define GO_CT(BT_, NO_) do { if (p->c_in == 3) GO_WS(BT_, NO_, 3); else GO_WS(BT_, NO_, 0); } while (0)
-#define GO_NO(BT_) do { if (no == 1) GO_CT(BT_, 1); else if (no == 2) GO_CT(BT_, 2); else GO_CT(BT_, 3); } while (0)
-  if (bt == 2) GO_NO(2);
-  else if (bt == 4) GO_NO(4);
-  else GO_NO(8);
+#define GO_CT(BT_, NO_, WS_) do { if (p->c_in == 3) GO(BT_, NO_, 3, WS_); else GO(BT_, NO_, 0, WS_); } while (0)
+#define GO_NO(BT_, WS_) do { if (no == 1) GO_CT(BT_, 1, WS_); else if (no == 2) GO_CT(BT_, 2, WS_); else GO_CT(BT_, 3, WS_); } while (0)
+  if (ws) GO_NO(2, true);
+  if (bt == 2) GO_NO(2, false);
+  if (bt == 4) GO_NO(4, false);
+  GO_NO(8, false);
 #undef GO_NO
 #undef GO_CT
-#undef GO_WS
 #undef GO
 }
 
