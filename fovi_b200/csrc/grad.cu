@@ -1,4 +1,4 @@
-// Passes around the backward contractions of KNNConv: ReLU mask with bias sums, column sums, and a layout change that makes the batch index the
+// Passes around the backward contractions of KNNConv: ReLU mask with bias sums (where no input gradient kernel has done it: knnconv_tc2.cu), column sums, and a layout change that makes the batch index the
 // innermost (contiguous) one, so that it can play the role of the channels in the tensor-core kernel (fovi_knnconv_forward_scatter_add).
 #include <algorithm>
 

@@ -18,6 +18,9 @@
 // epilogue threads signal them through cluster addresses); empty[s] and acc_full[a] exist in both CTAs and
 // are signalled by the leader's tcgen05.commit, multicast to both.  No TMA load here is multicast.
 // All waits are bounded; both CTAs always reach the closing cluster barrier.
+// MASK: an input gradient that leaves behind the ReLU mask of the layer below, with its sums per channel (that layer's bias gradient).  The epilogue has
+// the time (54 stages of MMAs per item), where a pass of its own reads the gradient and the activations and writes the gradient again: 280 us for four layers of the
+// benchmark's stack at 1024 rows, against 30 more in these launches; the training step under the power limit 3714 -> 3609.
 #include "tc_common.cuh"
 
 namespace {
@@ -30,6 +33,7 @@ struct Tc2Args {
   uint32_t stage_bytes, bias_bytes;
   uint32_t wait_limit; int skip_loads;   // as in TcArgs
   const int* out_map; int n_out_y; int accumulate;   // see OutMode
+  const __nv_bfloat16* act; float* colsum;
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -67,6 +71,25 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
                ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
 
+// Sums over the warp's 32 lanes (rows) of 64 columns, by halving exchanges: lane l ends with columns l and 32 + l.  62 exchanges, where a tree per column takes 320.
+__device__ __forceinline__ float2 column_sums(float (&v)[64], int lane) {
+  const bool up16 = lane & 16, up8 = lane & 8, up4 = lane & 4, up2 = lane & 2, up1 = lane & 1;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {                                             // columns 32h .. 32h + 31
+    float* c = v + 32 * h;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) c[i] = (up16 ? c[i + 16] : c[i]) + __shfl_xor_sync(0xffffffffu, up16 ? c[i] : c[i + 16], 16);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) c[i] = (up8 ? c[i + 8] : c[i]) + __shfl_xor_sync(0xffffffffu, up8 ? c[i] : c[i + 8], 8);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] = (up4 ? c[i + 4] : c[i]) + __shfl_xor_sync(0xffffffffu, up4 ? c[i] : c[i + 4], 4);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) c[i] = (up2 ? c[i + 2] : c[i]) + __shfl_xor_sync(0xffffffffu, up2 ? c[i] : c[i + 2], 2);
+    c[0] = (up1 ? c[1] : c[0]) + __shfl_xor_sync(0xffffffffu, up1 ? c[0] : c[1], 1);
+  }
+  return make_float2(v[0], v[32]);
+}
+
 __device__ __forceinline__ void decode_item2(const Tc2Args& a, int item, int& n, int& mt2, int& ctile) {
   ctile = item % a.n_ct;
   const int t = item / a.n_ct;
@@ -74,6 +97,7 @@ __device__ __forceinline__ void decode_item2(const Tc2Args& a, int item, int& n,
   mt2 = t / a.n_out;
 }
 
+template <bool MASK>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Tc2Args a) {
   extern __shared__ unsigned char smem_raw[];
@@ -109,6 +133,9 @@ fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int i = threadIdx.x; i < a.c_out; i += blockDim.x) bias_s[i] = a.bias ? __ldg(a.bias + i) : 0.f;
+  float* sums_s = bias_s + a.bias_bytes / 4 / (MASK ? 5 : 1);               // MASK: [4 epilogue warps][c_out] behind the bias
+  if (MASK)
+    for (int i = threadIdx.x; i < 4 * a.c_out; i += blockDim.x) sums_s[i] = 0.f;
   tc_fence_before();
   cluster_sync_all();   // barriers of both CTAs are initialised before anyone signals across
   tc_fence_after();
@@ -235,6 +262,36 @@ fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
 #pragma unroll
           for (int i = 0; i < 64; ++i) r[i] = 0u;
         }
+        if (MASK) {               // (bf16 results, no bias, no ReLU)
+          float v[64];
+          const __nv_bfloat16* m = a.act + y_off + c0;
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            uint32_t pk[8];
+            if (g * 16 < w && row < a.B) {
+              const uint4 m0 = __ldg(reinterpret_cast<const uint4*>(m + g * 16)), m1 = __ldg(reinterpret_cast<const uint4*>(m + g * 16) + 1);
+              const uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[g * 16 + 2 * i]), __uint_as_float(r[g * 16 + 2 * i + 1]));
+                const uint32_t b = *reinterpret_cast<const uint32_t*>(&h);
+                const float y0 = __uint_as_float(mw[i] << 16), y1 = __uint_as_float(mw[i] & 0xFFFF0000u);     // bf16 -> float32, exact
+                pk[i] = (y0 > 0.f ? b & 0xFFFFu : 0u) | (y1 > 0.f ? b & 0xFFFF0000u : 0u);
+              }
+              st_global_32(reinterpret_cast<__nv_bfloat16*>(a.Y) + y_off + c0 + g * 16, pk);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) pk[i] = 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { v[g * 16 + 2 * i] = __uint_as_float(pk[i] << 16); v[g * 16 + 2 * i + 1] = __uint_as_float(pk[i] & 0xFFFF0000u); }
+          }
+          const float2 s = column_sums(v, lane);
+          float* d = sums_s + q * a.c_out + o0 + c0 + lane;                 // this warp's own
+          d[0] += s.x;
+          if (w == 64) d[32] += s.y;
+          continue;
+        }
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           if (g * 16 < w) {
@@ -287,6 +344,13 @@ fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
       if (++acc == 2) { acc = 0; aph ^= 1u; }
       cnt = cnt_next;
     }
+    if (MASK) {
+      asm volatile("bar.sync 1, 128;" ::: "memory");                        // the four epilogue warps
+      for (int c = threadIdx.x; c < a.c_out; c += 128) {
+        const float s = sums_s[c] + sums_s[a.c_out + c] + sums_s[2 * a.c_out + c] + sums_s[3 * a.c_out + c];
+        if (s != 0.f) atomicAdd(a.colsum + c, s);
+      }
+    }
   }
 
   tc_fence_before();
@@ -314,11 +378,14 @@ int fovi::launch_knnconv_tc_pair(const fovi_knnconv_plan* p, const void* X, cons
   a.relu = relu; a.y_f32 = y_dtype == FOVI_F32;
   a.wait_limit = wait_limit; a.skip_loads = skip_loads;
   a.out_map = om.out_map; a.n_out_y = om.out_map ? om.n_out_y : p->n_out; a.accumulate = om.accumulate;
+  const bool mask = om.act != nullptr;
+  if (mask && (bias || relu || om.out_map || y_dtype != FOVI_BF16)) return FOVI_ERR_UNSUPPORTED;
+  a.act = static_cast<const __nv_bfloat16*>(om.act); a.colsum = om.colsum;
   const long long items = (long long)a.n_mt2 * p->n_out * a.n_ct;
   if (items >= (1ll << 31) || a.kp > 32 * TBQ) return FOVI_ERR_UNSUPPORTED;
   a.total_items = (int)items;
   a.stage_bytes = A_STAGE_BYTES + (uint32_t)(ct / 2) * 128u;
-  a.bias_bytes = ((uint32_t)p->c_out * 4u + 1023u) & ~1023u;
+  a.bias_bytes = (((uint32_t)p->c_out * 4u + 1023u) & ~1023u) * (mask ? 5u : 1u);
   const uint32_t budget = 220u * 1024u - 2048u - a.bias_bytes;
   a.nstage = (int)std::min<uint32_t>(MAX_STAGES, budget / a.stage_bytes);
   if (a.nstage < 2) return FOVI_ERR_UNSUPPORTED;
@@ -330,8 +397,9 @@ int fovi::launch_knnconv_tc_pair(const fovi_knnconv_plan* p, const void* X, cons
   rc = fovi::encode_3d(&tmB, Wt, (uint64_t)cp, (uint64_t)p->c_out, (uint64_t)p->V, (uint64_t)cp * 2, (uint64_t)p->c_out * cp * 2, 64, (uint32_t)(ct / 2), 1, true);
   if (rc) return rc;
 
-  FOVI_CUDA(cudaFuncSetAttribute(fovi_knnconv_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto k = mask ? fovi_knnconv_tc_pair_kernel<true> : fovi_knnconv_tc_pair_kernel<false>;
+  FOVI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int pairs = (int)std::min<long long>(items, sms / 2);
-  FOVI_CUDA(fovi::launch_pdl(fovi_knnconv_tc_pair_kernel, 2 * pairs, TC_THREADS, smem, st, tmA, tmB, a));   // cluster size 2 comes from __cluster_dims__
+  FOVI_CUDA(fovi::launch_pdl(k, 2 * pairs, TC_THREADS, smem, st, tmA, tmB, a));   // cluster size 2 comes from __cluster_dims__
   return fovi::after_launch("fovi_knnconv_tc_pair_kernel");
 }

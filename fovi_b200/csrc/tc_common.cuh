@@ -14,7 +14,8 @@ namespace fovi {
 // Where an output point's result goes.  Normally point n of the plan is point n of Y.  The weight-gradient contraction
 // (one "output point" per part of a filter tap's pair list) instead ADDS every part into its tap's row of a float32 Y:
 // out_map[n] is the row, n_out_y the number of rows of Y, and the stores become float32 reductions.
-struct OutMode { const int* out_map = nullptr; int n_out_y = 0; int accumulate = 0; };
+// An input gradient (act set: bf16, laid out like Y) leaves masked where act, the ReLU result it belongs to, is not positive, and its sums per channel are added to colsum.
+struct OutMode { const int* out_map = nullptr; int n_out_y = 0; int accumulate = 0; const void* act = nullptr; float* colsum = nullptr; };
 }  // namespace fovi
 using fovi::OutMode;
 

@@ -90,6 +90,11 @@ class KnnConvGrad:
         plan = self.dx_plan()
         return plan.forward(gy_points, plan.pack_weights_transposed(weight), out_dtype=torch.bfloat16)
 
+    def input_grad_masked(self, gy_points, weight, act):
+        """`input_grad` of a layer whose input `act` [B, n_in, c_in] is a ReLU's result: (the gradient behind the mask, its sums per channel), or None."""
+        plan = self.dx_plan()
+        return plan.input_grad_masked(gy_points, plan.pack_weights_transposed(weight), act)
+
     # ---- dW
     @property
     def dw_swapped(self):
@@ -226,18 +231,22 @@ class _KnnConvFunction(torch.autograd.Function):
 class _KnnConvPointsFunction(torch.autograd.Function):
     """A layer on the kernels' own activation layout (channels last, bf16) with the ReLU fused, so that a chain of layers
     trains without a layout change between them.  `x` is [B, n_in, c_in] bf16, or for a pair-layout first layer the
-    [B, c_in, n_in] input itself (it is packed here)."""
+    [B, c_in, n_in] input itself (it is packed here).
+
+    `below` / `above`: dicts that the layer shares with the one whose ReLU result is its input / whose input its ReLU result is, when nothing else reads
+    it.  A layer's input gradient then leaves its kernel behind the mask of the layer below, and the sums of it, the bias gradient of that layer, wait in the
+    dict: the pass over the gradient that does both otherwise is left out (the mask is the same, zero or one: the gradient's bits are too)."""
 
     @staticmethod
-    def forward(ctx, x, weight, bias, layer, relu):
+    def forward(ctx, x, weight, bias, layer, relu, below=None, above=None):
         plan = layer.plan
         first = plan.x_layout == ops.X_PAIRS
         rows = x.shape[0]
         with torch.no_grad():
             xp = ops.pack_points(x, plan) if first else x.contiguous()
             y = plan.forward(xp, layer.packed_weight(), bias, relu=relu, out_dtype=torch.bfloat16, batch=rows)
-        ctx.layer, ctx.relu, ctx.first, ctx.has_bias = layer, relu, first, bias is not None
-        ctx.save_for_backward(xp if ctx.needs_input_grad[1] else None, weight, y if relu else None)
+        ctx.layer, ctx.relu, ctx.first, ctx.has_bias, ctx.below, ctx.above = layer, relu, first, bias is not None, below, above
+        ctx.save_for_backward(xp if ctx.needs_input_grad[1] or (below is not None and ctx.needs_input_grad[0]) else None, weight, y if relu else None)
         return y
 
     @staticmethod
@@ -246,8 +255,8 @@ class _KnnConvPointsFunction(torch.autograd.Function):
         g = ctx.layer.grad_plans
         gy = _aligned(gy.to(torch.bfloat16).contiguous())
         want_w, want_b = ctx.needs_input_grad[1], ctx.has_bias and ctx.needs_input_grad[2]
-        gb = None
-        if ctx.relu:
+        gb = ctx.above.pop("sums", None) if ctx.above is not None else None      # there: gy is masked
+        if ctx.relu and gb is None:
             fused = ops.relu_mask_colsum(gy, y)            # mask and bias sums in one pass over the gradient
             if fused is not None:
                 gy, gb = fused
@@ -257,14 +266,18 @@ class _KnnConvPointsFunction(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             if ctx.first:
                 raise NotImplementedError("input gradient of a pair-layout first layer is not built")
-            gx = g.input_grad(gy, weight)                                      # [B, n_in, c_in] bf16
+            both = g.input_grad_masked(gy, weight, xp) if ctx.below is not None else None
+            if both is not None:
+                gx, ctx.below["sums"] = both
+            else:
+                gx = g.input_grad(gy, weight)                                  # [B, n_in, c_in] bf16
         if want_w:
             gw = g.weight_grad(gy, xp, ctx.layer.plan, weight.dtype)
         if not want_b:
             gb = None
         elif gb is None:
             gb = ops.column_sum(gy) if gy.shape[-1] % 2 == 0 else gy.sum((0, 1), dtype=torch.float32)
-        return gx, gw, gb, None, None
+        return gx, gw, gb, None, None, None, None
 
 
 class _BlockFunction(torch.autograd.Function):
@@ -300,8 +313,8 @@ def block_autograd(block, x):
     return _BlockFunction.apply(x, block.conv.weight, block.norm.weight, block.norm.bias, block)
 
 
-def knnconv_points_autograd(layer, x, relu):
-    return _KnnConvPointsFunction.apply(x, layer.weight, layer.bias, layer, relu)
+def knnconv_points_autograd(layer, x, relu, below=None, above=None):
+    return _KnnConvPointsFunction.apply(x, layer.weight, layer.bias, layer, relu, below, above)
 
 
 def knnconv_autograd(layer, x):

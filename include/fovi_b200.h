@@ -243,6 +243,11 @@ int fovi_knnconv_forward_f32(const fovi_knnconv_plan* plan, const void* X, int x
 int fovi_knnconv_forward_scatter_add(fovi_knnconv_plan* plan, const void* X, const void* Wt, float* Y, int B, const int* out_map,
                                      int n_out_y, void* stream);
 
+/* fovi_knnconv_forward of a transposed layer (bf16 in and out, no bias) whose result is the gradient of a ReLU's result: dX leaves as zero where act (bf16,
+ * [B,n_out,c_out] like dX) is not positive, and its sums per channel are ADDED to colsum (float32 [c_out]).  FOVI_ERR_UNSUPPORTED, nothing launched: batches of at most
+ * 128 rows, and layers outside the CTA-pair kernel. */
+int fovi_knnconv_input_grad_masked(fovi_knnconv_plan* plan, const void* gY, const void* Wt, const void* act, void* dX, float* colsum, int B, void* stream);
+
 /* Diagnostic for the failure path: launches the plan's tensor-core kernel with every operand load withheld and a short
  * wait limit, so the kernel's first consumer waits run out.  Nothing faults or hangs: the kernel records the wait site,
  * all its roles leave, tensor memory is freed.  A following fovi_knnconv_check must return FOVI_ERR_DEVICE_TIMEOUT, and
