@@ -586,12 +586,17 @@ extern "C" int fovi_knnconv_forward(fovi_knnconv_plan* p, const void* X, const v
   return knnconv_forward_impl(p, X, Wt, bias, Y, y_dtype, B, relu, stream, 0, WAIT_LIMIT);
 }
 
+extern "C" int fovi_knnconv_input_grad_masked_supported(const fovi_knnconv_plan* p, int B) {
+  return p && B > BM && !FOVI_TC_SINGLE_CTA_ONLY && fovi::knnconv_tc_pair_masks(p, B) ? 1 : 0;
+}
+
 extern "C" int fovi_knnconv_input_grad_masked(fovi_knnconv_plan* p, const void* gY, const void* Wt, const void* act, void* dX, float* colsum, int B,
                                               void* stream) {
   if (!p || B < 0) return FOVI_ERR_INVALID_ARGUMENT;
   if (B > 0 && (!gY || !Wt || !act || !dX || !colsum)) return FOVI_ERR_INVALID_ARGUMENT;
-  if (B <= BM || p->x_layout != FOVI_X_BNC || FOVI_TC_SINGLE_CTA_ONLY || (reinterpret_cast<uintptr_t>(act) & 15)) return FOVI_ERR_UNSUPPORTED;
-  if ((reinterpret_cast<uintptr_t>(gY) | reinterpret_cast<uintptr_t>(Wt) | reinterpret_cast<uintptr_t>(dX)) & 15) return FOVI_ERR_ALIGNMENT;
+  if (!fovi_knnconv_input_grad_masked_supported(p, B)) return FOVI_ERR_UNSUPPORTED;
+  if ((reinterpret_cast<uintptr_t>(gY) | reinterpret_cast<uintptr_t>(Wt) | reinterpret_cast<uintptr_t>(act) | reinterpret_cast<uintptr_t>(dX)) & 15)
+    return FOVI_ERR_ALIGNMENT;
   OutMode om;
   om.act = act; om.colsum = colsum;
   return fovi::launch_knnconv_tc_pair(p, gY, Wt, nullptr, dX, FOVI_BF16, B, 0, reinterpret_cast<cudaStream_t>(stream), 0, WAIT_LIMIT, om);

@@ -364,12 +364,27 @@ fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
 
 }  // namespace
 
+namespace {
+// Shared memory of the bias table (and, with a mask, of the warps' channel sums), and how many stages fit beside it.
+uint32_t pair_bias_bytes(const fovi_knnconv_plan* p, bool mask) { return (((uint32_t)p->c_out * 4u + 1023u) & ~1023u) * (mask ? 5u : 1u); }
+uint32_t pair_stages(const fovi_knnconv_plan* p, bool mask) {
+  const uint32_t taken = 2048u + pair_bias_bytes(p, mask), all = 220u * 1024u;
+  return taken >= all ? 0u : std::min<uint32_t>(MAX_STAGES, (all - taken) / (A_STAGE_BYTES + (uint32_t)(p->ct / 2) * 128u));
+}
+bool pair_applies(const fovi_knnconv_plan* p, int B, bool mask) {
+  return p->x_layout == FOVI_X_BNC && p->cin_packed >= 16 && p->ct >= 32 && p->ct % 32 == 0 && B > BM && p->kp <= 32 * TBQ && fovi::sm_count() >= 2 &&
+         (long long)((B + 2 * BM - 1) / (2 * BM)) * p->n_out * (p->c_out / p->ct) < (1ll << 31) && pair_stages(p, mask) >= 2;
+}
+}  // namespace
+
+bool fovi::knnconv_tc_pair_masks(const fovi_knnconv_plan* p, int B) { return pair_applies(p, B, true); }
+
 int fovi::launch_knnconv_tc_pair(const fovi_knnconv_plan* p, const void* X, const void* Wt, const float* bias, void* Y, int y_dtype,
                                  int B, int relu, cudaStream_t st, int skip_loads, uint32_t wait_limit, const OutMode& om) {
   const int ct = p->ct, cp = p->cin_packed;
-  if (p->x_layout != FOVI_X_BNC || cp < 16 || !ct || ct % 32 || ct < 32 || B <= BM) return FOVI_ERR_UNSUPPORTED;
+  const bool mask = om.act != nullptr;
+  if (!pair_applies(p, B, mask) || (mask && (bias || relu || om.out_map || y_dtype != FOVI_BF16))) return FOVI_ERR_UNSUPPORTED;
   const int sms = fovi::sm_count();
-  if (sms < 2) return FOVI_ERR_UNSUPPORTED;
   Tc2Args a;
   a.nbr_idx = p->nbr_idx; a.nbr_tap = p->nbr_tap; a.nbr_cnt = p->nbr_cnt;
   a.bias = bias; a.Y = Y; a.status = p->status;
@@ -378,17 +393,12 @@ int fovi::launch_knnconv_tc_pair(const fovi_knnconv_plan* p, const void* X, cons
   a.relu = relu; a.y_f32 = y_dtype == FOVI_F32;
   a.wait_limit = wait_limit; a.skip_loads = skip_loads;
   a.out_map = om.out_map; a.n_out_y = om.out_map ? om.n_out_y : p->n_out; a.accumulate = om.accumulate;
-  const bool mask = om.act != nullptr;
-  if (mask && (bias || relu || om.out_map || y_dtype != FOVI_BF16)) return FOVI_ERR_UNSUPPORTED;
   a.act = static_cast<const __nv_bfloat16*>(om.act); a.colsum = om.colsum;
   const long long items = (long long)a.n_mt2 * p->n_out * a.n_ct;
-  if (items >= (1ll << 31) || a.kp > 32 * TBQ) return FOVI_ERR_UNSUPPORTED;
   a.total_items = (int)items;
   a.stage_bytes = A_STAGE_BYTES + (uint32_t)(ct / 2) * 128u;
-  a.bias_bytes = (((uint32_t)p->c_out * 4u + 1023u) & ~1023u) * (mask ? 5u : 1u);
-  const uint32_t budget = 220u * 1024u - 2048u - a.bias_bytes;
-  a.nstage = (int)std::min<uint32_t>(MAX_STAGES, budget / a.stage_bytes);
-  if (a.nstage < 2) return FOVI_ERR_UNSUPPORTED;
+  a.bias_bytes = pair_bias_bytes(p, mask);
+  a.nstage = (int)pair_stages(p, mask);
   const size_t smem = 1024 + 1024 + a.bias_bytes + (size_t)a.nstage * a.stage_bytes;
 
   CUtensorMap tmA, tmB;

@@ -238,6 +238,8 @@ int encode_4d(CUtensorMap* m, const void* ptr, const uint64_t (&dims)[4], const 
 // CTA-pair variant of the 64-channel mode (knnconv_tc2.cu).  Returns FOVI_ERR_UNSUPPORTED when it does not apply.
 int launch_knnconv_tc_pair(const fovi_knnconv_plan* p, const void* X, const void* Wt, const float* bias, void* Y, int y_dtype,
                            int B, int relu, cudaStream_t st, int skip_loads, uint32_t wait_limit, const OutMode& om);
+// Its launch with a mask (OutMode::act) applies.
+bool knnconv_tc_pair_masks(const fovi_knnconv_plan* p, int B);
 // CTA-pair kernel of the pair layout (knnconv_tcp.cu).  Returns FOVI_ERR_UNSUPPORTED when it does not apply.
 int launch_knnconv_tc_pairs2(const fovi_knnconv_plan* p, const void* X, const void* Wt, const float* bias, void* Y, int y_dtype, int B,
                            int relu, cudaStream_t st, int skip_loads, uint32_t wait_limit);

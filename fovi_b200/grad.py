@@ -93,7 +93,7 @@ class KnnConvGrad:
     def input_grad_masked(self, gy_points, weight, act):
         """`input_grad` of a layer whose input `act` [B, n_in, c_in] is a ReLU's result: (the gradient behind the mask, its sums per channel), or None."""
         plan = self.dx_plan()
-        return plan.input_grad_masked(gy_points, plan.pack_weights_transposed(weight), act)
+        return plan.input_grad_masked(gy_points, plan.pack_weights_transposed(weight), act) if plan.masks_input_grad(gy_points.shape[0]) else None
 
     # ---- dW
     @property

@@ -244,8 +244,9 @@ int fovi_knnconv_forward_scatter_add(fovi_knnconv_plan* plan, const void* X, con
                                      int n_out_y, void* stream);
 
 /* fovi_knnconv_forward of a transposed layer (bf16 in and out, no bias) whose result is the gradient of a ReLU's result: dX leaves as zero where act (bf16,
- * [B,n_out,c_out] like dX) is not positive, and its sums per channel are ADDED to colsum (float32 [c_out]).  FOVI_ERR_UNSUPPORTED, nothing launched: batches of at most
- * 128 rows, and layers outside the CTA-pair kernel. */
+ * [B,n_out,c_out] like dX) is not positive, and its sums per channel are ADDED to colsum (float32 [c_out]).  FOVI_ERR_UNSUPPORTED, nothing launched, where
+ * fovi_knnconv_input_grad_masked_supported is 0: batches of at most 128 rows, and layers outside the CTA-pair kernel. */
+int fovi_knnconv_input_grad_masked_supported(const fovi_knnconv_plan* plan, int B);
 int fovi_knnconv_input_grad_masked(fovi_knnconv_plan* plan, const void* gY, const void* Wt, const void* act, void* dX, float* colsum, int B, void* stream);
 
 /* Diagnostic for the failure path: launches the plan's tensor-core kernel with every operand load withheld and a short
