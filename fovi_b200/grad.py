@@ -228,14 +228,29 @@ class _KnnConvFunction(torch.autograd.Function):
         return gx, gw, gb, None
 
 
+def _mark(grad, link, sums):
+    """Note on the gradient tensor itself that it is masked for the layer behind `link`, with its sums per channel.  (On the tensor, not in an object that the
+    two layers share: two passes over one graph run their nodes in any order.)  An inference tensor counts no writes, so it carries no mark."""
+    if not grad.is_inference():
+        grad._fovi_masked = (link, grad._version, sums)
+
+
+def _take_mark(grad, link):
+    """The sums that `_mark` left on this gradient for this link, or None, also if it was written to since.  Whoever takes them owns them."""
+    mark = grad.__dict__.pop("_fovi_masked", None)
+    return mark[2] if mark is not None and link is not None and mark[0] is link and mark[1] == grad._version else None
+
+
 class _KnnConvPointsFunction(torch.autograd.Function):
     """A layer on the kernels' own activation layout (channels last, bf16) with the ReLU fused, so that a chain of layers
     trains without a layout change between them.  `x` is [B, n_in, c_in] bf16, or for a pair-layout first layer the
     [B, c_in, n_in] input itself (it is packed here).
 
-    `below` / `above`: dicts that the layer shares with the one whose ReLU result is its input / whose input its ReLU result is, when nothing else reads
-    it.  A layer's input gradient then leaves its kernel behind the mask of the layer below, and the sums of it, the bias gradient of that layer, wait in the
-    dict: the pass over the gradient that does both otherwise is left out (the mask is the same, zero or one: the gradient's bits are too)."""
+    `below` / `above`: objects that the layer shares with the one whose ReLU result is its input / whose input its ReLU result is, when nothing else reads
+    it.  A layer's input gradient then leaves its kernel behind the mask of the layer below, and the sums of it, the bias gradient of that layer, travel ON the
+    gradient tensor (`_mark`, `_take_mark`): the pass over the gradient that does both otherwise is left out (the mask is the same, zero or one: the gradient's
+    bits are too).  A gradient that is not that tensor, or was written to since (by a hook on a node in between), takes that pass, which leaves a
+    masked gradient as it is; such a hook sees the gradient behind the mask."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, layer, relu, below=None, above=None):
@@ -253,9 +268,9 @@ class _KnnConvPointsFunction(torch.autograd.Function):
     def backward(ctx, gy):
         xp, weight, y = ctx.saved_tensors
         g = ctx.layer.grad_plans
+        gb = _take_mark(gy, ctx.above)                     # there: gy is masked, and these are its sums
         gy = _aligned(gy.to(torch.bfloat16).contiguous())
         want_w, want_b = ctx.needs_input_grad[1], ctx.has_bias and ctx.needs_input_grad[2]
-        gb = ctx.above.pop("sums", None) if ctx.above is not None else None      # there: gy is masked
         if ctx.relu and gb is None:
             fused = ops.relu_mask_colsum(gy, y)            # mask and bias sums in one pass over the gradient
             if fused is not None:
@@ -268,7 +283,8 @@ class _KnnConvPointsFunction(torch.autograd.Function):
                 raise NotImplementedError("input gradient of a pair-layout first layer is not built")
             both = g.input_grad_masked(gy, weight, xp) if ctx.below is not None else None
             if both is not None:
-                gx, ctx.below["sums"] = both
+                gx, sums = both
+                _mark(gx, ctx.below, sums)
             else:
                 gx = g.input_grad(gy, weight)                                  # [B, n_in, c_in] bf16
         if want_w:

@@ -485,7 +485,7 @@ class KNNConvStack(nn.Module):
             raise RuntimeError("the first layer's channels must be at most 4 or a multiple of 8")
         h = X if first else X.permute(0, 2, 1).to(torch.bfloat16)     # differentiable layout change
         n = len(self.layers)
-        links = [None] + [{} for _ in range(n - 1)] + [None]          # between a layer and the next, which alone reads its result
+        links = [None] + [object() for _ in range(n - 1)] + [None]    # between a layer and the next, which alone reads its result
         for i, L in enumerate(self.layers):
             h = knnconv_points_autograd(L, h, (i < n - 1) or self.final_relu, links[i], links[i + 1])
         return h.permute(0, 2, 1).to(X.dtype)
