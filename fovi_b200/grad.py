@@ -299,7 +299,7 @@ class _KnnConvPointsFunction(torch.autograd.Function):
 class _BlockFunction(torch.autograd.Function):
     """A block's convolution, training-mode batch norm, ReLU and max pooling (fovi/arch/knnalexnet.py:109-127).  The norm's forward pass is the module's own
     (`torch._batch_norm_impl_index`, which torch's batch_norm calls), so the activations are those of the separate modules bit for bit; what surrounds it
-    and the whole way back run on the kernels of csrc/blocktrain.cu."""
+    and the whole way back run on the kernels of csrc/blocktrain.cu.  The result is channels last, [B, n_out, C]."""
 
     @staticmethod
     def forward(ctx, x, weight, gamma, beta, block):
@@ -310,13 +310,13 @@ class _BlockFunction(torch.autograd.Function):
         y = conv.plan.forward(xp, conv.packed_weight(), None, out_dtype=torch.float32, batch=x.shape[0])
         mean, rstd, out, arg = ops.block_forward(y, norm, relu, ctx.pool)
         ctx.save_for_backward(xp if ctx.needs_input_grad[1] else None, weight, gamma, y, mean, rstd, out if relu and ctx.pool is None else None, arg)
-        return out.permute(0, 2, 1)
+        return out                                          # (not a view of it: of a view made in here the caller could not change a value in place)
 
     @staticmethod
     def backward(ctx, gy):
         xp, weight, gamma, y, mean, rstd, act, arg = ctx.saved_tensors
         conv = ctx.block.conv
-        g = _aligned(gy.permute(0, 2, 1).to(torch.float32).contiguous())
+        g = _aligned(gy.to(torch.float32).contiguous())
         dy, dgamma, dbeta = ops.norm_block_backward(y, mean, rstd, gamma, act, g, ctx.pool, arg)
         need = ctx.needs_input_grad
         gx = conv.grad_plans.input_grad(dy, weight).permute(0, 2, 1).to(torch.float32) if need[0] else None
@@ -326,7 +326,7 @@ class _BlockFunction(torch.autograd.Function):
 
 def block_autograd(block, x):
     """The block's training step in one function; the caller has seen to it that the block is of that form."""
-    return _BlockFunction.apply(x, block.conv.weight, block.norm.weight, block.norm.bias, block)
+    return _BlockFunction.apply(x, block.conv.weight, block.norm.weight, block.norm.bias, block).permute(0, 2, 1)
 
 
 def knnconv_points_autograd(layer, x, relu, below=None, above=None):
