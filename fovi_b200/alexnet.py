@@ -25,6 +25,11 @@ from .norm import KNNBatchNorm, _KernelNorm, get_norm
 __all__ = ["KNNBatchNorm", "get_norm", "KNNAlexNetBlock", "KNNAlexNet", "FoveatedAlexNet"]   # the norms live in fovi_b200/norm.py
 
 
+def _has_hooks(m):
+    """Somebody listens at the module or has replaced its forward."""
+    return bool("forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+
+
 class KNNAlexNetBlock(nn.Module):
     """conv -> norm -> activation -> optional pool (fovi/arch/knnalexnet.py:13-127); arguments as the reference."""
 
@@ -134,13 +139,12 @@ class KNNAlexNetBlock(nn.Module):
             return False
         if _has_any_global_hook() or torch.jit.is_tracing():
             return False
-        return not any(m is not None and ("forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
-                       for m in (conv, norm, act, pool))
+        return not any(m is not None and _has_hooks(m) for m in (conv, norm, act, pool))
 
     def _forward_train(self, x):
         """The block under autograd.  In the shipped form everything from the convolution to the pooling is one function on the kernels; otherwise the
         convolution's own gradients (fovi_b200/grad.py), torch's norm and activation as in the reference (batch norm with batch statistics in training
-        mode) and the pooling's own gradient.  Either way the result may be a channels-last view, as without gradients."""
+        mode) and the pooling's own gradient."""
         if self._fused_training(x):
             return block_autograd(self, x)
         if self.conv is not None:
@@ -225,13 +229,28 @@ class KNNAlexNet(nn.Module):
         """x [B, C_in, N_in] -> logits [B, n_classes], or features [B, C_out, N_out] without a classifier.  Under autograd
         (training) the blocks run one by one with gradients; otherwise on the kernels' channels-last path."""
         if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in self.parameters())):
-            for L in self.layers:
-                x = L(x)
+            x = self._forward_train(x)
             if self.n_classes is not None:
                 x = self.classifier(x.reshape(x.shape[0], -1))
             return x
         with torch.no_grad():
             return self._forward_eval(x)
+
+    def _forward_train(self, x):
+        """The layers under autograd.  A fused block followed by another hands its result on channels last, which is what the next convolution reads; wherever
+        anybody else could see a result, it is contiguous."""
+        def fused(i, x):      # (of x only the batch, type and device matter, which a fused block does not change)
+            L = self.layers[i] if i < len(self.layers) else None
+            return type(L) is KNNAlexNetBlock and not _has_hooks(L) and L._fused_training(x)
+        here = fused(0, x) and self.layers[0]._wants_grad(x)
+        for i, L in enumerate(self.layers):
+            if here:          # (its result needs a gradient, so the next one runs under autograd)
+                here = fused(i + 1, x)
+                x = block_autograd(L, x, points=here)
+            else:
+                x = L(x)
+                here = fused(i + 1, x) and self.layers[i + 1]._wants_grad(x)
+        return x
 
     def _forward_eval(self, x):
         if self.points_path:

@@ -299,34 +299,41 @@ class _KnnConvPointsFunction(torch.autograd.Function):
 class _BlockFunction(torch.autograd.Function):
     """A block's convolution, training-mode batch norm, ReLU and max pooling (fovi/arch/knnalexnet.py:109-127).  The norm's forward pass is the module's own
     (`torch._batch_norm_impl_index`, which torch's batch_norm calls), so the activations are those of the separate modules bit for bit; what surrounds it
-    and the whole way back run on the kernels of csrc/blocktrain.cu.  The result is channels last, [B, n_out, C]."""
+    and the whole way back run on the kernels of csrc/blocktrain.cu.  The result is contiguous [B, C, n_out], as the modules leave it, or with `points` what the
+    next block's convolution reads, channels last [B, n_out, C]."""
 
     @staticmethod
-    def forward(ctx, x, weight, gamma, beta, block):
+    def forward(ctx, x, weight, gamma, beta, block, points):
         conv, norm = block.conv, block.norm                 # (gamma and beta are the norm's)
-        ctx.block, ctx.pool = block, None if block.pool is None else block.pool._plan
+        ctx.block, ctx.pool, ctx.points = block, None if block.pool is None else block.pool._plan, points
         relu = block.activation is not None
         xp = ops.input_points(x, conv.plan)
         y = conv.plan.forward(xp, conv.packed_weight(), None, out_dtype=torch.float32, batch=x.shape[0])
         mean, rstd, out, arg = ops.block_forward(y, norm, relu, ctx.pool)
         ctx.save_for_backward(xp if ctx.needs_input_grad[1] else None, weight, gamma, y, mean, rstd, out if relu and ctx.pool is None else None, arg)
-        return out                                          # (not a view of it: of a view made in here the caller could not change a value in place)
+        return out if points else ops.points_to_channels(out)      # (no view: of one made in here the caller could not change a value in place)
 
     @staticmethod
     def backward(ctx, gy):
         xp, weight, gamma, y, mean, rstd, act, arg = ctx.saved_tensors
         conv = ctx.block.conv
-        g = _aligned(gy.to(torch.float32).contiguous())
+        g = gy.to(torch.float32)
+        if ctx.points:
+            g = _aligned(g.contiguous())
+        else:
+            g = ops.points_to_channels(g) if g.is_contiguous() else _aligned(g.permute(0, 2, 1).contiguous())
         dy, dgamma, dbeta = ops.norm_block_backward(y, mean, rstd, gamma, act, g, ctx.pool, arg)
         need = ctx.needs_input_grad
         gx = conv.grad_plans.input_grad(dy, weight).permute(0, 2, 1).to(torch.float32) if need[0] else None
         gw = conv.grad_plans.weight_grad(dy, xp, conv.plan, weight.dtype) if need[1] else None
-        return gx, gw, dgamma if need[2] else None, dbeta if need[3] else None, None
+        return gx, gw, dgamma if need[2] else None, dbeta if need[3] else None, None, None
 
 
-def block_autograd(block, x):
-    """The block's training step in one function; the caller has seen to it that the block is of that form."""
-    return _BlockFunction.apply(x, block.conv.weight, block.norm.weight, block.norm.bias, block).permute(0, 2, 1)
+def block_autograd(block, x, points=False):
+    """The block's training step in one function; the caller has seen to it that the block is of that form.  -> contiguous [B, C, n_out], or with `points` a
+    channels-last view, for a next block that takes it as it is (ops.input_points)."""
+    y = _BlockFunction.apply(x, block.conv.weight, block.norm.weight, block.norm.bias, block, points)
+    return y.permute(0, 2, 1) if points else y
 
 
 def knnconv_points_autograd(layer, x, relu, below=None, above=None):
