@@ -221,8 +221,8 @@ __global__ void pack_points_kernel(const TX* __restrict__ x, __nv_bfloat16* __re
 // Persistent CTAs, so that the filter is staged once.  One accumulator per output, neighbours in list order, channels inside: the
 // sums are those of the general kernel below, bit for bit.
 // CTAs per SM (register limit): up to 64 registers hold the accumulators of 32 or 64 channels, so four CTAs hide the gathers of each other's passes;
-// 96 channels x 8 images take up to 127 registers, two CTAs.  Serves tiles of one or two images, and filters that do not fit shared memory; the others take
-// the kernel below.
+// 96 channels x 8 images take up to 127 registers, two CTAs.  Serves tiles of one or two images, filters that do not fit shared memory, and grids too small for
+// the kernel below (see quad_pays).
 constexpr int F32_POINTS = 8;     // output points (warps) per CTA
 constexpr int F32_NB = 16;        // neighbours staged per pass: two lanes each
 
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(F32_POINTS * 32, NO == 3 ? 2 : 4) knnconv_f32_
   }
 }
 
-// The same for more than two images and a filter that fits shared memory: four points per warp, eight lanes each.
+// The same for more than two images, a filter that fits shared memory and enough points (quad_pays): four points per warp, eight lanes each.
 //
 // What bounds the kernel above is the load/store pipe (72 % while an SM is busy), not the FMAs: a warp-wide broadcast of 16 bytes costs as long as 32 lanes'
 // worth of data, so a (neighbour, channel) step of 64 channels x 8 images takes 10 clocks of shared-memory reads for 4 of FMAs; and 497 CTAs of eight points
@@ -527,9 +527,6 @@ int launch_f32_quad_t(const fovi_knnconv_plan* p, const void* X, int x_bnc, cons
   return fovi::after_launch("knnconv_f32_quad_kernel");
 }
 
-// Launch of the kernel above.  Images per warp: the tiles of at most eight images are made equal and rounded up to 2, 4 or
-// 8; channels per CTA: 32, 64 or 96, whichever wastes the fewest lanes (the wider one on a tie).  The filter goes to shared memory
-// when a channel tile of it is at most 64 KB (two CTAs per SM then, with the inputs; a 7 x 7 filter of 3 -> 64 channels is 37 KB), else it is read through L1.
 template <typename TX, int BT, int NO, int CT, bool WS>
 int launch_f32_few_t(const fovi_knnconv_plan* p, const void* X, int x_bnc, const float* Wt, const float* bias, float* Y, int y_bnc, int B,
                      int relu, size_t smem, cudaStream_t st) {
@@ -547,6 +544,30 @@ int launch_f32_few_t(const fovi_knnconv_plan* p, const void* X, int x_bnc, const
   return fovi::after_launch("knnconv_f32_few_kernel");
 }
 
+// Which of the two kernels above serves a layer whose filter is in shared memory and whose tiles hold more than two images.  A warp of the quad kernel does four
+// times the work, on one CTA per SM: a small grid leaves it with a long chain in few warps, where the eight-point kernel spreads the same points over every
+// SM.  As more of that kernel's tiles share an SM its load/store pipe saturates (sooner the more values a point gathers), while the quad kernel's time stands
+// still until its warps take a second quad.  Time of the quad kernel / the eight-point kernel by tiles per SM, over 1 to 4 -> 32 to 160 channels, 9, 25 and 49
+// neighbours, 7 to 3975 points, 3 to 64 images:
+//   up to 1    0.94 to 1.39 (8 images of 964 points, 3 -> 96, 9 neighbours: 8.4 -> 11.0 us); 4 channels, 192 values and more, 8 images in a tile of 32 channels: 0.89 to 0.95
+//   1 to 2     4 channels, or 96 values gathered and more, or 48 and more for a tile of 32 channels: 0.79 to 1.03; other 0.92 to 1.19
+//   2 to 3     also 3 channels, tiles of 96 (two CTAs of the eight-point kernel per SM, not four), 2 -> 32: 0.67 to 0.97; the rest (1 and 2 channels) 0.95 to 1.10
+//   above      0.49 to 0.96; for that rest up to 1.09 where the quad kernel's warps have just begun another round
+bool quad_pays(const fovi_knnconv_plan* p, int B, int bt, int no) {
+  const int n_ot = (p->c_out + no * 32 - 1) / (no * 32), n_bt = (B + bt - 1) / bt, gathered = p->c_in * p->kp;
+  const long long sms = fovi::sm_count(), tiles = (long long)((p->n_out + F32_POINTS - 1) / F32_POINTS) * n_bt * n_ot;        // of the eight-point kernel
+  if (p->c_in == 4 && gathered >= 192 && no == 1 && bt == 8) return true;
+  if (p->c_in >= 2 && (p->c_in == 4 || gathered >= 96 || (no == 1 && gathered >= 48))) return tiles > sms;
+  if (p->c_in == 3 || no == 3 || (p->c_in == 2 && no == 1)) return tiles > 2 * sms;
+  const long long warps = sms * (bt * no * 4 >= 64 ? QuadShape<8, 8>::WARPS : QuadShape<4, 4>::WARPS);
+  const long long rounds = ((long long)((p->n_out + 3) / 4) * n_bt * n_ot + warps - 1) / warps;
+  return rounds == 1 ? tiles > 3 * sms : 2 * tiles > 7 * rounds * sms;
+}
+
+// The exact layer of at most 4 input channels.  Images per tile: the tiles of at most eight images are made equal and rounded up to 2, 4 or 8; channels per CTA:
+// 32, 64 or 96, whichever wastes the fewest lanes (the wider one on a tie).  The filter goes to shared memory when a channel tile of it is at most 64 KB (two
+// CTAs of the eight-point kernel per SM then, with the inputs; a 7 x 7 filter of 3 -> 64 channels is 37 KB), else that kernel reads it through L1.  (The quad
+// kernel, with one CTA per SM, would hold a larger one; it has not been measured there.)
 template <typename TX>
 int launch_f32_few(const fovi_knnconv_plan* p, const void* X, int x_bnc, const float* Wt, const float* bias, float* Y, int y_bnc, int B, int relu,
                    cudaStream_t st) {
@@ -560,23 +581,25 @@ int launch_f32_few(const fovi_knnconv_plan* p, const void* X, int x_bnc, const f
   const size_t wbytes = sizeof(float) * (size_t)p->V * p->c_in * no * 32;
   const bool ws = wbytes <= 64 * 1024;
   const size_t smem = base + (ws ? wbytes : 0);
-  // four points per warp where the filter is in shared memory and a lane's tile is more than two images (see the kernel)
 #define QUAD(BT_, CPL_) do { if (p->c_in == 3) return launch_f32_quad_t<TX, BT_, CPL_, 3>(p, X, x_bnc, Wt, bias, Y, y_bnc, B, relu, st);    \
                              return launch_f32_quad_t<TX, BT_, CPL_, 0>(p, X, x_bnc, Wt, bias, Y, y_bnc, B, relu, st); } while (0)
 #define QUAD_NO(BT_) do { if (no == 1) QUAD(BT_, 4); else if (no == 2) QUAD(BT_, 8); else QUAD(BT_, 12); } while (0)
-  if (ws && bt == 8) QUAD_NO(8);
-  if (ws && bt == 4) QUAD_NO(4);
+  if (ws && bt > 2 && quad_pays(p, B, bt, no)) {
+    if (bt == 4) QUAD_NO(4);
+    QUAD_NO(8);
+  }
 #undef QUAD_NO
 #undef QUAD
 #define GO(BT_, NO_, CT_, WS_) return launch_f32_few_t<TX, BT_, NO_, CT_, WS_>(p, X, x_bnc, Wt, bias, Y, y_bnc, B, relu, smem, st)
-#define GO_CT(BT_, NO_, WS_) do { if (p->c_in == 3) GO(BT_, NO_, 3, WS_); else GO(BT_, NO_, 0, WS_); } while (0)
-#define GO_NO(BT_, WS_) do { if (no == 1) GO_CT(BT_, 1, WS_); else if (no == 2) GO_CT(BT_, 2, WS_); else GO_CT(BT_, 3, WS_); } while (0)
-  if (ws) GO_NO(2, true);
-  if (bt == 2) GO_NO(2, false);
-  if (bt == 4) GO_NO(4, false);
-  GO_NO(8, false);
+#define GO_WS(BT_, NO_, CT_) do { if (ws) GO(BT_, NO_, CT_, true); else GO(BT_, NO_, CT_, false); } while (0)
+#define GO_CT(BT_, NO_) do { if (p->c_in == 3) GO_WS(BT_, NO_, 3); else GO_WS(BT_, NO_, 0); } while (0)
+#define GO_NO(BT_) do { if (no == 1) GO_CT(BT_, 1); else if (no == 2) GO_CT(BT_, 2); else GO_CT(BT_, 3); } while (0)
+  if (bt == 2) GO_NO(2);
+  if (bt == 4) GO_NO(4);
+  GO_NO(8);
 #undef GO_NO
 #undef GO_CT
+#undef GO_WS
 #undef GO
 }
 
