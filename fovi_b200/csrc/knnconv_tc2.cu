@@ -20,7 +20,9 @@
 // All waits are bounded; both CTAs always reach the closing cluster barrier.
 // MASK: an input gradient that leaves behind the ReLU mask of the layer below, with its sums per channel (that layer's bias gradient).  The epilogue has
 // the time (54 stages of MMAs per item), where a pass of its own reads the gradient and the activations and writes the gradient again: 280 us for four layers of the
-// benchmark's stack at 1024 rows, against 30 more in these launches; the training step under the power limit 3714 -> 3609.
+// benchmark's stack at 1024 rows, against 30 more in these launches; the training step under the power limit 3714 -> 3609.  With few stages per item the epilogue is
+// what bounds the kernel: the activations of the next 64 columns are read ahead, while the accumulator fills or the columns before are worked on (each read where it
+// is used: 2.9 us per 64 columns; ahead: 2.0; 512 <- 64 channels, one neighbour, 1000 points, 256 rows 318 -> 224, where the separate pass takes 233).
 #include "tc_common.cuh"
 
 namespace {
@@ -243,14 +245,21 @@ fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
       decode_item2(a, item, n, mt2, ctile);
       const int next = item + n_pairs;
       const int cnt_next = next < a.total_items ? __ldg(a.nbr_cnt + (next / a.n_ct) % a.n_out) : 0;
-      ok = mbar_wait(smem_u32(&hdr->acc_full[acc]), aph, abort_flag, a.status, 14, a.wait_limit);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
       const int row = (mt2 * 2 + (int)rank) * BM + q * 32 + lane;
       const int o0 = ctile * a.ct;
       const int n_y = a.out_map ? __ldg(a.out_map + n) : n;
       const size_t y_off = ((size_t)row * a.n_out_y + n_y) * a.c_out + o0;
+      uint4 m[8];                           // MASK: activations of the next 64 columns, read while the accumulator fills or the columns before are worked on
+      auto fetch = [&](int c0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (row < a.B && c0 + i * 8 < a.ct) m[i] = __ldg(reinterpret_cast<const uint4*>(a.act + y_off + c0) + i);
+      };
+      if (MASK) fetch(0);
+      ok = mbar_wait(smem_u32(&hdr->acc_full[acc]), aph, abort_flag, a.status, 14, a.wait_limit);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
       const uint32_t t_base = tmem + ((uint32_t)(q * 32) << 16) + acc * 256u;
       for (int c0 = 0; c0 < a.ct; c0 += 64) {
         uint32_t r[64];
@@ -264,12 +273,15 @@ fovi_knnconv_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
         }
         if (MASK) {               // (bf16 results, no bias, no ReLU)
           float v[64];
-          const __nv_bfloat16* m = a.act + y_off + c0;
+          uint4 here[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) here[i] = m[i];
+          if (c0 + 64 < a.ct) fetch(c0 + 64);
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
             uint32_t pk[8];
             if (g * 16 < w && row < a.B) {
-              const uint4 m0 = __ldg(reinterpret_cast<const uint4*>(m + g * 16)), m1 = __ldg(reinterpret_cast<const uint4*>(m + g * 16) + 1);
+              const uint4 m0 = here[2 * g], m1 = here[2 * g + 1];
               const uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
 #pragma unroll
               for (int i = 0; i < 8; ++i) {

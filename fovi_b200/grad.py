@@ -95,6 +95,15 @@ class KnnConvGrad:
         plan = self.dx_plan()
         return plan.input_grad_masked(gy_points, plan.pack_weights_transposed(weight), act) if plan.masks_input_grad(gy_points.shape[0]) else None
 
+    def masking_pays(self, rows):
+        """Whether `input_grad_masked` is the faster form.  Per 64 columns of a tile (256 rows of an input point) the masked epilogue takes 2.0 us against 0.85, hidden behind
+        the products of the next tile where there are enough; the separate pass costs by the row.  So the masked form loses where the last tile of rows is mostly
+        empty AND a tile has few products: 129 rows, 1000 points: 512 <- 64 channels, 1 neighbour 170 -> 202 us, 9 neighbours 198 -> 218, 25 neighbours
+        gains; 300 rows 340 -> 380; 256 rows 233 -> 224; grids of a few hundred tiles gain at any fill."""
+        tiles, columns = -(-rows // 256), -(-self.c_in // 256)                    # row tiles; column tiles (of at most 256)
+        products = self._n.size / self.n_in * -(-self.c_out // 64)
+        return 3 * rows >= 2 * 256 * tiles or self.n_in * columns * tiles <= 700 or products >= 3 * (-(-self.c_in // (64 * columns)))
+
     # ---- dW
     @property
     def dw_swapped(self):
@@ -281,7 +290,7 @@ class _KnnConvPointsFunction(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             if ctx.first:
                 raise NotImplementedError("input gradient of a pair-layout first layer is not built")
-            both = g.input_grad_masked(gy, weight, xp) if ctx.below is not None else None
+            both = g.input_grad_masked(gy, weight, xp) if ctx.below is not None and g.masking_pays(gy.shape[0]) else None
             if both is not None:
                 gx, sums = both
                 _mark(gx, ctx.below, sums)

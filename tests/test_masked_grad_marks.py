@@ -24,6 +24,9 @@ class _Grads:
     def __init__(self):
         self.masked, self.after_masked = 0, lambda: None
 
+    def masking_pays(self, rows):
+        return True
+
     def input_grad(self, gy, weight):
         return (gy.float() @ weight.float()).to(torch.bfloat16)
 
