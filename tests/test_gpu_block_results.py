@@ -113,3 +113,16 @@ def test_a_frozen_first_block_in_training_mode_is_refused_as_before():
     net(x).sum().backward()
     assert net.layers[0].conv.weight.grad is None and net.layers[1].conv.weight.grad is not None
     assert net(x.clone().requires_grad_()).requires_grad
+
+
+# one sample's slab shared by several CTAs: more CTAs than points to share, a remainder, no pool; slabs of 32, 16 and 8 channels
+@pytest.mark.parametrize("N,C,n_out,K", [(5, 16, 3, 2), (230, 40, 61, 9), (1031, 16, 230, 9), (5602, 96, 1401, 5), (700, 32, 0, 0), (2001, 24, 0, 0)])
+def test_one_sample_alone_and_in_a_batch(N, C, n_out, K):
+    from fovi_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    h = torch.randn((200, C, N), generator=gen, device="cuda")
+    plan = ops.KnnPoolPlan(torch.randint(0, N + 1, (K, n_out), generator=torch.Generator().manual_seed(N)).int().numpy(), N, device="cuda") if n_out else None
+    out, arg = ops.relu_pool(h, True, plan)
+    for b in (0, 199):
+        one, who = ops.relu_pool(h[b:b + 1].contiguous(), True, plan)
+        assert torch.equal(one[0], out[b]) and (plan is None or torch.equal(who[0], arg[b]))
