@@ -326,4 +326,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nu
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&module); }
+// The module says which torch it was compiled against: its tensors are that one's C++ objects.
+PyMODINIT_FUNC PyInit__native() {
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "made_for", FOVI_TORCH_VERSION)) { Py_DECREF(m); return nullptr; }
+  return m;
+}

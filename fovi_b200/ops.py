@@ -1,6 +1,8 @@
 """Tensor-level wrappers over the C ABI: plans own device tables, functions take torch CUDA
 tensors, pass raw pointers and the current stream, and allocate outputs with torch."""
 import ctypes as C
+import os
+import warnings
 
 import numpy as np
 import torch
@@ -9,9 +11,14 @@ from ._lib import SIGNATURES, check, lib
 
 try:      # the launch path in native code (csrc/bind.cpp); without it every call takes the Python path below
     from . import _native
+    if getattr(_native, "made_for", None) != str(torch.__version__):
+        raise ImportError(f"it was built for torch {getattr(_native, 'made_for', '?')}, this is {torch.__version__}")
     _native.connect({name: C.cast(getattr(lib, name), C.c_void_p).value for name in SIGNATURES})
-except ImportError:
+except ImportError as e:
     _native = None
+    if any(f.startswith("_native.") and f.endswith(".so") for f in os.listdir(os.path.dirname(os.path.abspath(__file__)))):
+        warnings.warn(f"the native launch path of fovi_b200 is there but does not load ({e}): calls take the Python path, which is slower; "
+                      "python -m fovi_b200.build makes it anew")
 
 F32, BF16, U8 = 0, 1, 2
 NEAREST, BILINEAR = 0, 1
