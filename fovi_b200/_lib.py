@@ -74,6 +74,7 @@ SIGNATURES = {
     "fovi_knnpool_backward": (C.c_int, [_P, _P, C.c_int, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P, _P]),
     "fovi_knnconv_input_grad_masked_supported": (C.c_int, [_P, C.c_int]),
     "fovi_knnconv_input_grad_masked": (C.c_int, [_P, _P, _P, _P, _P, _P, C.c_int, _P]),
+    "fovi_knnconv_input_grad_masked_selftest_wait_timeout": (C.c_int, [_P, _P, _P, _P, _P, _P, C.c_int, _P]),
     "fovi_points_to_channels": (C.c_int, [_P, _P, C.c_int, C.c_int, C.c_int, _P]),
     "fovi_relu_pool_supported": (C.c_int, [C.c_int, _P]),
     "fovi_relu_pool_forward": (C.c_int, [_P, C.c_int, C.c_int, C.c_int, C.c_int, _P, _P, _P, _P]),

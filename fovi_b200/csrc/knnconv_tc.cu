@@ -590,8 +590,9 @@ extern "C" int fovi_knnconv_input_grad_masked_supported(const fovi_knnconv_plan*
   return p && B > BM && !FOVI_TC_SINGLE_CTA_ONLY && fovi::knnconv_tc_pair_masks(p, B) ? 1 : 0;
 }
 
-extern "C" int fovi_knnconv_input_grad_masked(fovi_knnconv_plan* p, const void* gY, const void* Wt, const void* act, void* dX, float* colsum, int B,
-                                              void* stream) {
+namespace {
+int input_grad_masked_impl(fovi_knnconv_plan* p, const void* gY, const void* Wt, const void* act, void* dX, float* colsum, int B, void* stream, int skip_loads,
+                           uint32_t wait_limit) {
   if (!p || B < 0) return FOVI_ERR_INVALID_ARGUMENT;
   if (B > 0 && (!gY || !Wt || !act || !dX || !colsum)) return FOVI_ERR_INVALID_ARGUMENT;
   if (!fovi_knnconv_input_grad_masked_supported(p, B)) return FOVI_ERR_UNSUPPORTED;
@@ -599,7 +600,18 @@ extern "C" int fovi_knnconv_input_grad_masked(fovi_knnconv_plan* p, const void* 
     return FOVI_ERR_ALIGNMENT;
   OutMode om;
   om.act = act; om.colsum = colsum;
-  return fovi::launch_knnconv_tc_pair(p, gY, Wt, nullptr, dX, FOVI_BF16, B, 0, reinterpret_cast<cudaStream_t>(stream), 0, WAIT_LIMIT, om);
+  return fovi::launch_knnconv_tc_pair(p, gY, Wt, nullptr, dX, FOVI_BF16, B, 0, reinterpret_cast<cudaStream_t>(stream), skip_loads, wait_limit, om);
+}
+}  // namespace
+
+extern "C" int fovi_knnconv_input_grad_masked(fovi_knnconv_plan* p, const void* gY, const void* Wt, const void* act, void* dX, float* colsum, int B,
+                                              void* stream) {
+  return input_grad_masked_impl(p, gY, Wt, act, dX, colsum, B, stream, 0, WAIT_LIMIT);
+}
+
+extern "C" int fovi_knnconv_input_grad_masked_selftest_wait_timeout(fovi_knnconv_plan* p, const void* gY, const void* Wt, const void* act, void* dX, float* colsum, int B,
+                                                                    void* stream) {
+  return input_grad_masked_impl(p, gY, Wt, act, dX, colsum, B, stream, 1, 4096u);       // as fovi_knnconv_selftest_wait_timeout
 }
 
 extern "C" int fovi_knnconv_forward_scatter_add(fovi_knnconv_plan* p, const void* X, const void* Wt, float* Y, int B, const int* out_map,

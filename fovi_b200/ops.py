@@ -367,17 +367,19 @@ class KnnConvPlan:
         """True when `input_grad_masked` takes this layer and batch (the CTA-pair kernel runs it)."""
         return bool(lib.fovi_knnconv_input_grad_masked_supported(self._h, B))
 
-    def input_grad_masked(self, gy, wt, act):
+    def input_grad_masked(self, gy, wt, act, selftest=False):
         """`forward` of a transposed layer onto the gradient of a ReLU's result `act` ([B,n_out,c_out] bf16 contiguous): (gradient, zero where act is not
-        positive, float32 [c_out] sums of it).  See fovi_knnconv_input_grad_masked and `masks_input_grad`."""
+        positive, float32 [c_out] sums of it).  See fovi_knnconv_input_grad_masked and `masks_input_grad`.
+        `selftest`: the diagnostic launch whose waits give up; check() then raises."""
         _need_cuda(gy, wt, act)
         B = gy.shape[0]
         assert gy.dtype == wt.dtype == act.dtype == torch.bfloat16 and gy.is_contiguous() and wt.is_contiguous() and act.is_contiguous()
         assert gy.shape[1:] == (self.n_in, self.cin_packed) and wt.shape == (self.V, self.c_out, self.cin_packed) and act.shape == (B, self.n_out, self.c_out)
         out = torch.empty_like(act)
         sums = torch.zeros(self.c_out, dtype=torch.float32, device=gy.device)
+        call = lib.fovi_knnconv_input_grad_masked_selftest_wait_timeout if selftest else lib.fovi_knnconv_input_grad_masked
         with _on(gy.device):
-            check(lib.fovi_knnconv_input_grad_masked(self._h, _ptr(gy), _ptr(wt), _ptr(act), _ptr(out), _ptr(sums), B, _stream()), "fovi_knnconv_input_grad_masked")
+            check(call(self._h, _ptr(gy), _ptr(wt), _ptr(act), _ptr(out), _ptr(sums), B, _stream()), "fovi_knnconv_input_grad_masked")
         return out, sums
 
     def forward_scatter_add(self, x_bnc, wt, out_map, out):

@@ -256,6 +256,9 @@ int fovi_knnconv_input_grad_masked(fovi_knnconv_plan* plan, const void* gY, cons
  * The reference has no counterpart (it has no device-side waits). */
 int fovi_knnconv_selftest_wait_timeout(fovi_knnconv_plan* plan, const void* X, const void* Wt, void* Y, int y_dtype, int B,
                                        void* stream);
+/* The same of fovi_knnconv_input_grad_masked (dX and colsum are left unspecified). */
+int fovi_knnconv_input_grad_masked_selftest_wait_timeout(fovi_knnconv_plan* plan, const void* gY, const void* Wt, const void* act, void* dX, float* colsum, int B,
+                                                         void* stream);
 
 /* Synchronises `stream` and returns FOVI_ERR_DEVICE_TIMEOUT if any tensor-core launch on this
  * plan since the last check gave up on a wait; clears the word. */
