@@ -122,6 +122,8 @@ class KNNAlexNetBlock(nn.Module):
             return False
         if conv.precision != "bf16" or not conv.plan.tc_supported or conv.bias is not None or not norm.training or norm.momentum is None:
             return False
+        if not norm.track_running_stats:                    # (a norm whose running statistics are held still)
+            return False
         if not hasattr(torch, "_batch_norm_impl_index") or not ops.relu_pool_supported(conv.plan.n_out):
             return False
         if pool is not None and (type(pool) is not KNNPoolingLayer or pool.mode != "max" or not pool._plan.block_supported):

@@ -126,3 +126,21 @@ def test_one_sample_alone_and_in_a_batch(N, C, n_out, K):
     for b in (0, 199):
         one, who = ops.relu_pool(h[b:b + 1].contiguous(), True, plan)
         assert torch.equal(one[0], out[b]) and (plan is None or torch.equal(who[0], arg[b]))
+
+
+@pytest.mark.parametrize("network", [False, True])
+def test_running_statistics_that_are_held_still(network):
+    """`track_running_stats = False` on a norm that has running statistics: batch statistics are used, the running ones are not written."""
+    from fovi_b200.alexnet import KNNAlexNet
+    torch.manual_seed(0)
+    m = KNNAlexNet(12, 32, [64], [1], [0], [9], cmf_a=0.5, ref_frame_mult=2, norm_type="force_batch", device="cuda").train() if network else make().train()
+    block = m.layers[0] if network else m
+    x = torch.randn((7, 32, block.in_coords.shape[0]), device="cuda")
+    want = m(x)
+    assert block.norm.num_batches_tracked == 1
+    block.norm.track_running_stats = False
+    before = [b.clone() for b in block.norm.buffers()]
+    got = m(x)
+    assert torch.equal(got, want)
+    for a, b in zip(before, block.norm.buffers(), strict=True):
+        assert torch.equal(a, b)
