@@ -33,7 +33,7 @@ CHANS = [3, 64, 192, 384, 256, 256]
 # dram__bytes_read.sum + dram__bytes_write.sum per launch from one ncu capture of this workload (256 images x 4 fixations,
 # captured directly: three metrics, one pass); sampler, then the five KNNConv launches.  `sources` is the hash of the kernel
 # sources the capture was taken on: when the sources change the figure is reported as null until the capture is redone.
-NCU_DRAM_TRAFFIC_MB = {"workload": (256, 4), "sources": "1abfc512c77552eb", "sampler": 207.4, "conv": [221.8, 195.5, 225.1, 284.0, 206.6]}
+NCU_DRAM_TRAFFIC_MB = {"workload": (256, 4), "sources": "f1b2951657cfdcf8", "sampler": 208.2, "conv": [221.7, 195.7, 224.9, 287.7, 207.4]}
 METRIC = "images x fixations/s through sensor+KNNConv"
 UNIT = "img*fix/s"
 
